@@ -59,25 +59,25 @@ def _case(name, model, kind, batch, tokens, dtype="bfloat16", ragged=True, want=
 def listed():
     return [
         # one reader of a small model's answer: the latency of a step is all there is
-        _case("compact, a token for one", "compact", "decode", 1, 300),
+        _case("compact token for 1", "compact", "decode", 1, 300),
         # a few short questions arrive together at a small model
-        _case("compact, short prompts", "compact", "prompt", 4, 250),
+        _case("compact short prompts", "compact", "prompt", 4, 250),
         # the benchmark's decode points: one, eight and 64 readers; the last draws its tokens at a temperature
-        _case("8b, a token for one", "8b", "decode", 1, 2048),
-        _case("8b, a token for eight", "8b", "decode", 8, 2048),
-        _case("8b, a token for 64", "8b", "decode", 64, 512, sampled=True),
+        _case("8b token for 1", "8b", "decode", 1, 2048),
+        _case("8b token for 8", "8b", "decode", 8, 2048),
+        _case("8b token for 64", "8b", "decode", 64, 512, sampled=True),
         # the benchmark's prompt
-        _case("8b, prompt of 2,048", "8b", "prompt", 1, 2048),
+        _case("8b prompt of 2048", "8b", "prompt", 1, 2048),
         # prompts of several users cut into pieces, so that no step takes long
-        _case("8b, prompts in pieces", "8b", "chunks", 3, 1100, chunk=400),
+        _case("8b prompts in pieces", "8b", "chunks", 3, 1100, chunk=400),
         # long documents: reading two, and answering four
-        _case("4b, long prompts", "4b", "prompt", 2, 12000),
-        _case("4b, a token for four long ones", "4b", "decode", 4, 12000),
+        _case("4b long prompts", "4b", "prompt", 2, 12000),
+        _case("4b token for 4 long ones", "4b", "decode", 4, 12000),
         # a checking run in true 32-bit: prompts and a greedy answer
-        _case("compact in float32, a reply", "compact", "reply", 3, 500, dtype="float32", steps=24),
+        _case("compact float32 reply", "compact", "reply", 3, 500, dtype="float32", steps=24),
         # the design with latent and linear attention and routed experts: a prompt scored at 64 places, a token for eight
-        _case("tefezen, prompt of 2,000", "tefezen", "prompt", 1, 2000, want=64),
-        _case("tefezen, a token for eight", "tefezen", "decode", 8, 1500),
+        _case("tefezen prompt of 2000", "tefezen", "prompt", 1, 2000, want=64),
+        _case("tefezen token for 8", "tefezen", "decode", 8, 1500),
     ]
 
 
