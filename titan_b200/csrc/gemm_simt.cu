@@ -7,158 +7,412 @@
 // fuse the residual into the epilogue (:3489-3493) and SwiGLU into gate/up (:2589).
 //
 // Epilogues:
+// One order of sums for every kernel here, whatever M: in each run of SUM_RUN neighbouring k the products at even and those at
+// odd k are added one after the other (fused multiply-adds from zero), then the two sums, and the runs' sums one after the
+// other.  A row's result is then the same bits alone and beside any other rows, in a decode step as in a prompt.  Even
+// and odd, because the two are neighbours in memory and one two-element instruction (fma.rn.f32x2) works on both.
+//
 //   TB_EPI_STORE   out[m][n] = acc                      (compute dtype), or an activation of it (activation.h)
 //   TB_EPI_F32     out[m][n] = acc                      (float32: logits)
 //   TB_EPI_ADD     out[m][n] += acc                     (float32 residual stream, in place)
 //   TB_EPI_SWIGLU  out[m][j] = gate(acc[2j], acc[2j+1]) (rows of W interleaved gate, up; N even); the gate is
 //                  silu(g) * u unless the launch names another (activation.h)
+#include <type_traits>
+
 #include "common.cuh"
 #include "gemm.h"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+// N elements of a row as one load (16 or 8 bytes) and as floats.
+template <typename T, int N> struct Vec;
+template <> struct Vec<float, 4> {
+    float4 r;
+    __device__ __forceinline__ void load(const float* p) { r = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void get(float* o) const { o[0] = r.x; o[1] = r.y; o[2] = r.z; o[3] = r.w; }
+};
+template <> struct Vec<__nv_bfloat16, 4> {
+    uint2 r;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { r = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void get(float* o) const {
+        o[0] = __uint_as_float(r.x << 16); o[1] = __uint_as_float(r.x & 0xffff0000u);
+        o[2] = __uint_as_float(r.y << 16); o[3] = __uint_as_float(r.y & 0xffff0000u);
+    }
+};
+template <> struct Vec<__nv_bfloat16, 8> {
+    uint4 r;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { r = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ void get(float* o) const {
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { o[2 * i] = __uint_as_float(w[i] << 16); o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+    }
+};
+// Activations are read through L2 by instructions that stay where they are: kernels of a step are in flight together, so a line of
+// this SM's L1 may be older than what the kernel before has written, and a load that the compiler takes for a load of
+// constants may move above the wait for that kernel (a __restrict__ pointer to const; weights, which no kernel writes, may have it).
+template <typename V> __device__ __forceinline__ V load_l2(const void* p);
+template <> __device__ __forceinline__ float load_l2<float>(const void* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+template <> __device__ __forceinline__ __nv_bfloat16 load_l2<__nv_bfloat16>(const void* p) {
+    unsigned short v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return __ushort_as_bfloat16(v);
+}
+template <> __device__ __forceinline__ float4 load_l2<float4>(const void* p) {
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+template <> __device__ __forceinline__ uint2 load_l2<uint2>(const void* p) {
+    uint2 v;
+    asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
 
-template <typename T, int EPI>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const T* __restrict__ X, const T* __restrict__ W, void* __restrict__ out_,
+// acc = a * b + acc on two neighbouring float32 at once, each rounded as fmaf rounds it (one instruction of sm_100a).
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float both(unsigned long long v) {      // the sum of the two
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+__device__ __forceinline__ void copy16(void* to, const void* from, bool real = true) {      // zeros if not real
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(real ? 16 : 0) : "memory");
+}
+
+constexpr int SUM_RUN = 32;
+
+// ---------------------------------------------------------------- many rows: tiles
+// Tiles of 64 x 64, K in steps of one run of sums, RI x 4 sums a thread: 4 x 4 (256 threads), or 8 x 4 (128 threads, fewer loads from
+// shared memory a product) where there are tiles enough for three blocks an SM all the same.  Operands lie along K in shared memory (a row 16 bytes behind a whole
+// number of banks: sixteen neighbouring rows do not collide), three steps deep; float32 rows come by cp.async and stay in flight for
+// two steps.  Bound by the FMA pipes; several blocks an SM hide what is left of the latencies.  1,125 rows
+// of K = 1,024: 5,632 columns 357 us (36 TFLOP/s), 1,024 columns 79 us; K = 2,816, 1,024 columns: 203 us (a kernel of 4 x 4 sums that
+// waited for each step's operands took 445, 230 and 640 us).
+constexpr int BM = 64, BN = 64, LDK = SUM_RUN + 4, TILE_STAGES = 3;
+constexpr size_t TILE_SMEM = (size_t)TILE_STAGES * (BM + BN) * LDK * sizeof(float);
+
+template <typename T, int EPI, int RI, bool VEC>
+__global__ void __launch_bounds__(1024 / RI, RI == 4 ? 2 : 3)
+gemm_simt_kernel(const T* X, const T* W, void* out_,
                  int M, int N, int K, int ldx, int ldo, long long sx, long long sw, long long so, int act, float limit) {
+    constexpr int THREADS = 1024 / RI;
     pdl_launch_dependents();
-    pdl_wait();
     // blockIdx.z: one of a batch of products of equal shape (the heads of a mixer, say), each at its own offset
     X += (size_t)blockIdx.z * sx;
     W += (size_t)blockIdx.z * sw;
     void* out = (EPI == TB_EPI_STORE || EPI == TB_EPI_SWIGLU) ? (void*)((T*)out_ + (size_t)blockIdx.z * so)
                                                               : (void*)((float*)out_ + (size_t)blockIdx.z * so);
-    __shared__ float xs[BK][BM + 4];
-    __shared__ float ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int tx = tid % 16, ty = tid / 16;     // thread tile: rows ty*4.., cols tx*4..
-    float acc[TM][TN];
+    extern __shared__ __align__(16) float tile_sm[];       // [TILE_STAGES][BM rows of X, BN rows of W][LDK]
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, steps = (K + SUM_RUN - 1) / SUM_RUN;
+    // Row r of the W area holds column 2 (r % 16) + r / 16 % 2 + 32 (r / 32) of the tile, so that the four a thread reads, sixteen rows
+    // apart, are two pairs of neighbouring columns.
+    auto stage = [&](bool weights, int step) {
+        float* area = tile_sm + (size_t)((step % TILE_STAGES) * (BM + BN) + (weights ? BM : 0)) * LDK;
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64 rows x 16 k of each operand: 1024 elements, 4 per thread
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int idx = tid + i * 256;
-            const int r = idx / BK, kk = idx % BK;
-            const int k = k0 + kk;
-            xs[kk][r] = (m0 + r < M && k < K) ? ldf(X + (size_t)(m0 + r) * ldx + k) : 0.f;
-            ws[kk][r] = (n0 + r < N && k < K) ? ldf(W + (size_t)(n0 + r) * K + k) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = xs[kk][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = ws[kk][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int m = m0 + ty * TM + i;
-        if (m >= M) continue;
-        if (EPI == TB_EPI_SWIGLU) {
-#pragma unroll
-            for (int j = 0; j < TN; j += 2) {
-                const int n = n0 + tx * TN + j;
-                if (n + 1 < N) {
-                    const float g = acc[i][j], u = acc[i][j + 1];
-                    stf((T*)out + (size_t)m * ldo + n / 2, tb_gated(act, limit, g, u));
-                }
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const int n = n0 + tx * TN + j;
-                if (n >= N) continue;
-                if (EPI == TB_EPI_STORE) stf((T*)out + (size_t)m * ldo + n, tb_unary(act, acc[i][j]));
-                if (EPI == TB_EPI_F32) ((float*)out)[(size_t)m * ldo + n] = acc[i][j];
-                if (EPI == TB_EPI_ADD) ((float*)out)[(size_t)m * ldo + n] += acc[i][j];
-            }
-        }
-    }
-}
-
-template <typename T>
-int launch(const void* X, const void* W, void* out, int M, int N, int K, int ldx, int ldo, int epi,
-           int batch, long long sx, long long sw, long long so, int act, float limit, cudaStream_t stream) {
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-    const T* x = (const T*)X;
-    const T* w = (const T*)W;
-    switch (epi) {
-        case TB_EPI_STORE: tb_launch(gemm_simt_kernel<T, TB_EPI_STORE>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act, limit); break;
-        case TB_EPI_F32: tb_launch(gemm_simt_kernel<T, TB_EPI_F32>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act, limit); break;
-        case TB_EPI_ADD: tb_launch(gemm_simt_kernel<T, TB_EPI_ADD>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act, limit); break;
-        case TB_EPI_SWIGLU: tb_launch(gemm_simt_kernel<T, TB_EPI_SWIGLU>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act, limit); break;
-        default: tb_set_error("gemm: unknown epilogue %d", epi); return 1;
-    }
-    return 0;
-}
-
-// A few rows (decode steps): a warp per output element of one row and one product of the batch, lanes along K with
-// 16-byte loads where the rows allow; the weights are read once per row of X through L2.  Epilogues STORE, F32 and ADD.
-template <typename T, int EPI>
-__global__ void __launch_bounds__(256)
-gemm_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, void* __restrict__ out_, int M, int N, int K, int ldx, int ldo,
-                 long long sx, long long sw, long long so, int act) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = blockIdx.x * 8 + warp, m = blockIdx.y, z = blockIdx.z;
-    if (n >= N) return;
-    const T* x = X + (size_t)z * sx + (size_t)m * ldx;
-    const T* w = W + (size_t)z * sw + (size_t)n * K;
-    constexpr int PER = 16 / sizeof(T);
-    float acc = 0.f;
-    if (K % PER == 0 && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0)) {
-        for (int k = lane * PER; k < K; k += 32 * PER) {
-            if (sizeof(T) == 4) {
-                const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
-                acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+        for (int u = 0; u < BM * SUM_RUN / 4 / THREADS; ++u) {
+            const int e = tid + THREADS * u, r = e / (SUM_RUN / 4), c = e % (SUM_RUN / 4) * 4, k = step * SUM_RUN + c;
+            const int row = weights ? n0 + 2 * (r % 16) + r / 16 % 2 + 32 * (r / 32) : m0 + r;
+            const bool real = row < (weights ? N : M) && k < K;
+            const T* from = (weights ? W + (size_t)row * K : X + (size_t)row * ldx) + k;
+            float* to = area + r * LDK + c;
+            if constexpr (VEC && sizeof(T) == 4) {          // K is a multiple of four: a unit is inside or outside
+                copy16(to, real ? from : X, real);
+            } else if constexpr (VEC) {
+                Vec<T, 4> v;
+                float f[4] = {0.f, 0.f, 0.f, 0.f};
+                if (real) { v.r = load_l2<decltype(v.r)>(from); v.get(f); }
+                *reinterpret_cast<float4*>(to) = make_float4(f[0], f[1], f[2], f[3]);
             } else {
-                const uint4 a = *reinterpret_cast<const uint4*>(x + k), b = *reinterpret_cast<const uint4*>(w + k);
-                const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    acc = fmaf(__uint_as_float(aw[i] << 16), __uint_as_float(bw[i] << 16), acc);
-                    acc = fmaf(__uint_as_float(aw[i] & 0xffff0000u), __uint_as_float(bw[i] & 0xffff0000u), acc);
+                    to[i] = 0.f;
+                    if (real && k + i < K) { const T v = load_l2<T>(from + i); to[i] = ldf(&v); }
                 }
             }
         }
-    } else {
-        for (int k = lane; k < K; k += 32) acc = fmaf(ldf(x + k), ldf(w + k), acc);
+    };
+    float total[RI][4];
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) total[i][j] = 0.f;
+    stage(true, 0);                                        // no kernel writes weights
+    if (steps > 1) stage(true, 1);
+    pdl_wait();
+    stage(false, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (steps > 1) stage(false, 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                   // this step's rows are there; the step before has been read
+        if (step + 2 < steps) { stage(true, step + 2); stage(false, step + 2); }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* xs = tile_sm + (size_t)(step % TILE_STAGES) * (BM + BN) * LDK + ty * LDK;
+        const float* ws = tile_sm + (size_t)((step % TILE_STAGES) * (BM + BN) + BM + tx) * LDK;
+        unsigned long long acc[RI][4] = {};
+#pragma unroll 2
+        for (int k = 0; k < SUM_RUN; k += 4) {
+            ulonglong2 b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(ws + 16 * j * LDK + k);
+#pragma unroll
+            for (int i = 0; i < RI; ++i) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + (64 / RI) * i * LDK + k);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { fma2(acc[i][j], a.x, b[j].x); fma2(acc[i][j], a.y, b[j].y); }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) total[i][j] += both(acc[i][j]);
     }
-    acc = warp_sum(acc);
-    if (lane != 0) return;
-    const size_t at = (size_t)z * so + (size_t)m * ldo + n;
-    if (EPI == TB_EPI_STORE) stf((T*)out_ + at, tb_unary(act, acc));
-    if (EPI == TB_EPI_F32) ((float*)out_)[at] = acc;
-    if (EPI == TB_EPI_ADD) ((float*)out_)[at] += acc;
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+        const int m = m0 + ty + (64 / RI) * i;
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            const int n = n0 + 2 * tx + 16 * j;
+            if (EPI == TB_EPI_SWIGLU) {
+                if (n + 1 < N) stf((T*)out + (size_t)m * ldo + n / 2, tb_gated(act, limit, total[i][j], total[i][j + 1]));
+                continue;
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (n + e >= N) continue;
+                const size_t at = (size_t)m * ldo + n + e;
+                const float v = total[i][j + e];
+                if (EPI == TB_EPI_STORE) stf((T*)out + at, tb_unary(act, v));
+                if (EPI == TB_EPI_F32) ((float*)out)[at] = v;
+                if (EPI == TB_EPI_ADD) ((float*)out)[at] = load_l2<float>((float*)out + at) + v;
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------- few rows: weights streamed once
+// A step of a few tokens is bound by the weights' bytes, and in 64 x 64 tiles most of the chip idles: 16 blocks for
+// 1,024 columns, each walking all of K.  Here a block takes eight columns at a time and up to MR rows, and its 256 threads the runs of
+// SUM_RUN along K, a thread one column and one run.  A unit of work is eight columns and ``pass`` runs; its weights come into shared
+// memory by cp.async, all requested at once, while the unit before is worked on, those of the first unit before the wait for the
+// kernel before (no kernel writes weights); so do the rows of X, once a block where K is one pass.  A run lies 16 bytes and a
+// column 64 bytes behind a whole number of banks, so that a warp's four runs and eight columns do not collide.  The run sums meet in shared
+// memory and are added in order by a thread an output.  Each weight is read from memory once for MR rows; rows beyond
+// are further blocks, which find the weights in L2.  Three rows: 1,024 columns
+// of K = 2,816 in 7.1 us, 5,632 of K = 1,024 in 12.9, 32,768 in 59 (64 x 64 tiles: 189, 87 and 204 us).
+constexpr int FEW_COLS = 8;
+template <typename T> constexpr int few_run() { return SUM_RUN + 16 / (int)sizeof(T); }           // elements from a run to the next in shared memory
+template <typename T> __host__ __device__ constexpr int few_col(int pass) { return (pass * few_run<T>() * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T) + 64 / (int)sizeof(T); }
+// Shared memory: per stage [FEW_COLS] columns of ``pass`` runs and, where K takes several passes, [MR] rows; else the rows once, behind
+// the stages; then two areas of run sums.
+template <typename T, int MR> size_t few_smem(int pass, int stages, bool one_pass) {
+    return (size_t)(stages * (FEW_COLS + (one_pass ? 0 : MR)) + (one_pass ? MR : 0)) * few_col<T>(pass) * sizeof(T) + (size_t)2 * pass * MR * FEW_COLS * sizeof(float);
+}
+
+template <typename T, int EPI, int MR, bool VEC>
+__global__ void __launch_bounds__(256)
+gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx, int ldo, long long sx, long long sw, long long so,
+                int pass, int stages, int act, float limit) {
+    constexpr int RS = few_run<T>(), PER = 16 / (int)sizeof(T), UNITS = SUM_RUN / PER;
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) unsigned char few_sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * MR, z = blockIdx.z;
+    const int runs = (K + SUM_RUN - 1) / SUM_RUN, passes = (runs + pass - 1) / pass, groups = (N + FEW_COLS - 1) / FEW_COLS;
+    const int cs = few_col<T>(pass), stage_elems = (FEW_COLS + (passes > 1 ? MR : 0)) * cs;
+    T* const stage0 = reinterpret_cast<T*>(few_sm);        // [stages][FEW_COLS (+ MR)][cs]
+    T* const x0 = stage0 + (passes > 1 ? FEW_COLS * cs : stages * stage_elems);        // rows of X: in every stage, or once
+    float* const sums0 = reinterpret_cast<float*>(stage0 + stages * stage_elems + (passes > 1 ? 0 : MR * cs));      // [2][pass][MR][FEW_COLS]
+    // ``here`` runs of one row from run ``first`` on into shared memory, by ``step`` threads; elements beyond K are zero
+    auto stage = [&](T* to, const T* row, int first, int here, int at, int step) {
+        for (int u = at; u < here * UNITS; u += step) {
+            T* dst = to + u / UNITS * RS + u % UNITS * PER;
+            const int k = first * SUM_RUN + u * PER;
+            if (VEC && k < K) { copy16(dst, row + k); continue; }
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                T e = T(0.f);
+                if (!VEC && k + i < K) e = load_l2<T>(row + k + i);
+                dst[i] = e;
+            }
+        }
+    };
+    // unit u of this block: group blockIdx.x + (u / passes) * gridDim.x, pass u % passes
+    const int my_groups = groups > (int)blockIdx.x ? (groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0, units = my_groups * passes;
+    auto stage_w = [&](int u) {                            // a warp loads a column; columns and rows outside: any valid ones
+        const int n = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS + warp, first = u % passes * pass;
+        stage(stage0 + (u % stages) * stage_elems + warp * cs, W + (size_t)z * sw + (size_t)min(n, N - 1) * K, first, min(pass, runs - first), lane, 32);
+    };
+    auto stage_x = [&](int u) {
+        const int first = u % passes * pass;
+        for (int m = 0; m < MR; ++m)
+            stage(x0 + (passes > 1 ? (u % stages) * stage_elems : 0) + m * cs, X + (size_t)z * sx + (size_t)min(m0 + m, M - 1) * ldx, first,
+                  min(pass, runs - first), tid, 256);
+    };
+    const int om = tid / FEW_COLS, on = tid % FEW_COLS;   // a thread's output, if it has one
+    const int col = tid % FEW_COLS;
+    float total = 0.f;
+    // unit u arrives with copy group u: the first ``stages`` - 1 units together in group 0, empty groups after it
+    for (int u = 0; u < min(units, max(1, stages - 1)); ++u) stage_w(u);
+    pdl_wait();
+    for (int u = 0; u < (passes > 1 ? min(units, max(1, stages - 1)) : 1); ++u) stage_x(u);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int u = 1; u < stages - 1; ++u) asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int u = 0; u < units; ++u) {
+        if (stages > 1 && u + stages - 1 < units) {
+            stage_w(u + stages - 1);
+            if (passes > 1) stage_x(u + stages - 1);
+        }
+        if (stages > 1) asm volatile("cp.async.commit_group;" ::: "memory");
+        if (stages == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (stages == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const int here = min(pass, runs - u % passes * pass);
+        float* sums = sums0 + (u & 1) * pass * MR * FEW_COLS;
+        const T* st = stage0 + (u % stages) * stage_elems;
+        const T* sx_ = x0 + (passes > 1 ? (u % stages) * stage_elems : 0);
+        for (int r = tid / FEW_COLS; r < here; r += 256 / FEW_COLS) {
+            unsigned long long acc[MR];
+#pragma unroll
+            for (int m = 0; m < MR; ++m) acc[m] = 0ull;
+            const T* wr = st + col * cs + r * RS;
+            const T* xr = sx_ + r * RS;
+#pragma unroll
+            for (int i = 0; i < UNITS; ++i) {
+                Vec<T, PER> v;
+                float wf[PER], xf[PER];
+                v.load(wr + i * PER);
+                v.get(wf);
+#pragma unroll
+                for (int m = 0; m < MR; ++m) {
+                    v.load(xr + m * cs + i * PER);
+                    v.get(xf);
+#pragma unroll
+                    for (int e = 0; e < PER; e += 2) fma2(acc[m], pair_of(xf[e], xf[e + 1]), pair_of(wf[e], wf[e + 1]));
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MR; ++m) sums[(r * MR + m) * FEW_COLS + col] = both(acc[m]);
+        }
+        __syncthreads();
+        if (tid >= MR * FEW_COLS) continue;
+#pragma unroll 8
+        for (int r = 0; r < here; ++r) total += sums[(r * MR + om) * FEW_COLS + on];
+        if (u % passes != passes - 1) continue;
+        const int m = m0 + om, n = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS + on;
+        // the gate of a pair: its second column is the neighbouring thread's
+        const float right = __shfl_down_sync(MR * FEW_COLS >= 32 ? 0xffffffffu : (1u << (MR * FEW_COLS % 32)) - 1u, total, 1);
+        if (m < M && n < N) {
+            const size_t at = (size_t)z * so + (size_t)m * ldo + n;
+            if (EPI == TB_EPI_SWIGLU) { if (n % 2 == 0) stf((T*)out_ + (size_t)z * so + (size_t)m * ldo + n / 2, tb_gated(act, limit, total, right)); }
+            if (EPI == TB_EPI_STORE) stf((T*)out_ + at, tb_unary(act, total));
+            if (EPI == TB_EPI_F32) ((float*)out_)[at] = total;
+            if (EPI == TB_EPI_ADD) ((float*)out_)[at] = load_l2<float>((float*)out_ + at) + total;
+        }
+        total = 0.f;
+    }
+}
+
+constexpr int SMS = 148;
+
+struct Product {
+    const void* X; const void* W; void* out;
+    int M, N, K, ldx, ldo, batch;
+    long long sx, sw, so;
+    int act; float limit;
+    cudaStream_t stream;
+};
+
+// 16-byte loads of the few-rows kernel, four-element loads of the tiles: every row of every product starts on such a boundary.
+template <typename T>
+bool aligned(const Product& p, int per) {
+    const size_t bytes = per * sizeof(T);
+    return p.K % per == 0 && p.ldx % per == 0 && (uintptr_t)p.X % bytes == 0 && (uintptr_t)p.W % bytes == 0 &&
+           (p.batch == 1 || (p.sx % per == 0 && p.sw % per == 0));
+}
+
+template <typename T, int EPI, int MR, bool VEC>
+void few_launch(const Product& p) {
+    const int runs = (p.K + SUM_RUN - 1) / SUM_RUN, groups = (p.N + FEW_COLS - 1) / FEW_COLS, others = (p.M + MR - 1) / MR * p.batch;
+    // One unit a block while the blocks fit the chip once: all of K at once.  Else passes of 32 runs (one a thread), up to four stages,
+    // and equal shares of the column groups for a block an SM.
+    const bool once = (long long)groups * others <= SMS;
+    int pass = once ? 96 : 32, x = groups;
+    if (pass > runs) pass = runs;
+    while (few_smem<T, MR>(pass, 1, pass >= runs) > 200 * 1024) --pass;
+    const int passes = (runs + pass - 1) / pass, room = SMS / others > 0 ? SMS / others : 1;
+    if (groups > room) {
+        const int each = (groups + room - 1) / room;
+        x = (groups + each - 1) / each;
+    }
+    const long long units = (long long)((groups + x - 1) / x) * passes;
+    int stages = units < 4 ? (int)units : 4;
+    while (stages > 1 && few_smem<T, MR>(pass, stages, passes == 1) > 220 * 1024) --stages;
+    if (stages == 1 && units > 1) { stages = 2; while (few_smem<T, MR>(pass, stages, false) > 220 * 1024) --pass; }
+    const size_t smem = few_smem<T, MR>(pass, stages, (runs + pass - 1) / pass == 1);
+    const dim3 grid(x, (p.M + MR - 1) / MR, p.batch);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(gemm_few_kernel<T, EPI, MR, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    tb_launch(gemm_few_kernel<T, EPI, MR, VEC>, grid, 256, smem, p.stream, (const T*)p.X, (const T*)p.W, p.out, p.M, p.N, p.K, p.ldx, p.ldo,
+              p.sx, p.sw, p.so, pass, stages, p.act, p.limit);
+}
+template <typename T, int EPI, int MR>
+void few_rows(const Product& p) {
+    if (aligned<T>(p, 16 / (int)sizeof(T))) few_launch<T, EPI, MR, true>(p);
+    else few_launch<T, EPI, MR, false>(p);
+}
+
+template <typename T, int EPI, int RI, bool VEC>
+void tiles(const Product& p) {
+    const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.batch);
+    cudaFuncSetAttribute(gemm_simt_kernel<T, EPI, RI, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM);
+    tb_launch(gemm_simt_kernel<T, EPI, RI, VEC>, grid, 1024 / RI, TILE_SMEM, p.stream, (const T*)p.X, (const T*)p.W, p.out, p.M, p.N, p.K, p.ldx, p.ldo,
+              p.sx, p.sw, p.so, p.act, p.limit);
+}
+
+template <typename T, int EPI>
+void product(const Product& p, bool few) {
+    // Few rows: up to 64 while the column groups of all groups of eight rows stay near a unit's time (measured, K = 1,024, few / tiles:
+    // 64 rows of 1,024 columns 23 / 47 us, of 2,048 37 / 42; 5,632 columns 32 rows 50 / 69, 48 rows 74 / 70; 32,768 columns
+    // 8 rows 69 / 140, 24 rows 200 / 141).
+    if (few || (p.M <= 64 && (long long)((p.M + 7) / 8) * p.N * p.batch <= 32768)) {
+        if (p.M == 1) few_rows<T, EPI, 1>(p);
+        else if (p.M == 2) few_rows<T, EPI, 2>(p);
+        else if (p.M <= 4) few_rows<T, EPI, 4>(p);
+        else few_rows<T, EPI, 8>(p);
+        return;
+    }
+    // 8 x 4 sums a thread from four tiles an SM on (5,632 columns of K = 1,024: 1,125 rows 389 -> 357 us, 3,000 rows 980 -> 888 us);
+    // below, twice the warps are worth more (1,125 rows, 1,024 columns of K = 2,816: 294 -> 203 us)
+    const long long count = (long long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
+    if (!aligned<T>(p, 4)) tiles<T, EPI, 4, false>(p);
+    else if (count >= 4 * 148) tiles<T, EPI, 8, true>(p);
+    else tiles<T, EPI, 4, true>(p);
 }
 
 template <typename T>
-static int launch_rows(const void* X, const void* W, void* out, int M, int N, int K, int ldx, int ldo, int epi, int batch,
-                       long long sx, long long sw, long long so, int act, cudaStream_t stream) {
-    dim3 grid((N + 7) / 8, M, batch);
-    const T* x = (const T*)X;
-    const T* w = (const T*)W;
-    if (epi == TB_EPI_STORE) tb_launch(gemm_rows_kernel<T, TB_EPI_STORE>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act);
-    else if (epi == TB_EPI_F32) tb_launch(gemm_rows_kernel<T, TB_EPI_F32>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act);
-    else if (epi == TB_EPI_ADD) tb_launch(gemm_rows_kernel<T, TB_EPI_ADD>, grid, 256, 0, stream, x, w, out, M, N, K, ldx, ldo, sx, sw, so, act);
-    else { tb_set_error("gemm_rows: epilogue %d is not one of store, float32, add", epi); return 1; }
+int run(const Product& p, int epi, bool few = false) {
+    switch (epi) {
+        case TB_EPI_STORE: product<T, TB_EPI_STORE>(p, few); break;
+        case TB_EPI_F32: product<T, TB_EPI_F32>(p, few); break;
+        case TB_EPI_ADD: product<T, TB_EPI_ADD>(p, few); break;
+        case TB_EPI_SWIGLU: product<T, TB_EPI_SWIGLU>(p, few); break;
+        default: tb_set_error("gemm: unknown epilogue %d", epi); return 1;
+    }
     return 0;
 }
 
@@ -175,19 +429,11 @@ extern "C" int tb_gemm_simt_gated(const void* X, const void* W, void* out, int d
     TB_REQUIRE(batch > 0 && batch <= 65535, "gemm: a batch of %d products", batch);
     TB_REQUIRE(ldx >= K, "gemm: row stride %d of X is shorter than K=%d", ldx, K);
     TB_REQUIRE(epi != TB_EPI_SWIGLU || N % 2 == 0, "gemm: the SwiGLU epilogue needs an even N, found %d", N);
-    TB_REQUIRE((M + BM - 1) / BM <= 65535, "gemm: M=%d is too large for one launch", M);
-    if (epi == TB_EPI_STORE && M <= 16 && batch > 1 && (N + 7) / 8 <= 65535) {      // a decode step's rows: a warp per output
-        int r;
-        if (dtype == TB_F32) r = launch_rows<float>(X, W, out, M, N, K, ldx, ldo, epi, batch, sx, sw, so, act, stream);
-        else if (dtype == TB_BF16) r = launch_rows<__nv_bfloat16>(X, W, out, M, N, K, ldx, ldo, epi, batch, sx, sw, so, act, stream);
-        else { tb_set_error("gemm: unknown dtype %d", dtype); return 1; }
-        if (r) return r;
-        TB_CHECK_LAUNCH("gemm_rows");
-        return 0;
-    }
+    TB_REQUIRE((M + 63) / 64 <= 65535, "gemm: M=%d is too large for one launch", M);
+    const Product p{X, W, out, M, N, K, ldx, ldo, batch, sx, sw, so, act, limit, stream};
     int rc;
-    if (dtype == TB_F32) rc = launch<float>(X, W, out, M, N, K, ldx, ldo, epi, batch, sx, sw, so, act, limit, stream);
-    else if (dtype == TB_BF16) rc = launch<__nv_bfloat16>(X, W, out, M, N, K, ldx, ldo, epi, batch, sx, sw, so, act, limit, stream);
+    if (dtype == TB_F32) rc = run<float>(p, epi);
+    else if (dtype == TB_BF16) rc = run<__nv_bfloat16>(p, epi);
     else { tb_set_error("gemm: unknown dtype %d", dtype); return 1; }
     if (rc) return rc;
     TB_CHECK_LAUNCH("gemm_simt");
@@ -205,18 +451,20 @@ extern "C" int tb_gemm_simt(const void* X, const void* W, void* out, int dtype, 
 }
 
 // ``act``: the activation of the STORE epilogue (activation.h).
-// out (epilogue store, float32 or add) = X[M,K] . W[N,K]^T for a few rows and a small matrix, a warp per output element:
-// the products of a decode step whose matrices are too small to pay for a tensor-core launch (a router, a narrow gate).
+// out (epilogue store, float32 or add) = X[M,K] . W[N,K]^T on the few-rows kernel whatever M: the products of a decode step
+// whose matrices are too small to pay for a tensor-core launch (a router, a narrow gate).
 extern "C" int tb_gemm_rows(const void* X, const void* W, void* out, int dtype, int M, int N, int K, int ldx, int ldo, int epi,
                             int act, cudaStream_t stream) {
     TB_REQUIRE(epi == TB_EPI_STORE ? act >= 0 && act < TB_UNARY_KINDS : act == 0, "gemm_rows: unknown activation %d", act);
-    TB_REQUIRE(M > 0 && N > 0 && K > 0 && M <= 65535 && (N + 7) / 8 <= 2147483647, "gemm_rows: sizes (M=%d N=%d K=%d)", M, N, K);
+    TB_REQUIRE(M > 0 && N > 0 && K > 0 && M <= 65535, "gemm_rows: sizes (M=%d N=%d K=%d)", M, N, K);
     TB_REQUIRE(ldx >= K, "gemm_rows: row stride %d of X is shorter than K=%d", ldx, K);
-    int r;
-    if (dtype == TB_F32) r = launch_rows<float>(X, W, out, M, N, K, ldx, ldo, epi, 1, 0, 0, 0, act, stream);
-    else if (dtype == TB_BF16) r = launch_rows<__nv_bfloat16>(X, W, out, M, N, K, ldx, ldo, epi, 1, 0, 0, 0, act, stream);
+    TB_REQUIRE(epi != TB_EPI_SWIGLU, "gemm_rows: epilogue %d is not one of store, float32, add", epi);
+    const Product p{X, W, out, M, N, K, ldx, ldo, 1, 0, 0, 0, act, 0.f, stream};
+    int rc;
+    if (dtype == TB_F32) rc = run<float>(p, epi, true);
+    else if (dtype == TB_BF16) rc = run<__nv_bfloat16>(p, epi, true);
     else { tb_set_error("gemm_rows: unknown dtype %d", dtype); return 1; }
-    if (r) return r;
+    if (rc) return rc;
     TB_CHECK_LAUNCH("gemm_rows");
     return 0;
 }
