@@ -19,6 +19,8 @@
 // query head h reads kv head h / (nh/nkv), partials merged with exp(m_s - m_max).
 #include <float.h>
 
+#include <atomic>
+
 #include "attention_args.h"
 #include "common.cuh"
 
@@ -40,6 +42,17 @@ template <> __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bflo
         o[2 * i] = __uint_as_float(w[i] << 16);
         o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
+}
+
+// The elements of a 16-byte unit.
+template <typename T> __device__ __forceinline__ void unpack16(const uint4& r, float* o);
+template <> __device__ __forceinline__ void unpack16<float>(const uint4& r, float* o) {
+    o[0] = __uint_as_float(r.x); o[1] = __uint_as_float(r.y); o[2] = __uint_as_float(r.z); o[3] = __uint_as_float(r.w);
+}
+template <> __device__ __forceinline__ void unpack16<__nv_bfloat16>(const uint4& r, float* o) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { o[2 * i] = __uint_as_float(w[i] << 16); o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 
 // Running softmax state of one warp: every lane holds the same m and l, and acc for dims lane + 32 j.
@@ -183,6 +196,200 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_prefill_kernel(AttnArgs a
     }
 }
 
+// ------------------------------------------------------------------ prefill in float32, tiles of queries
+// grid (query tiles of every sequence, nh), 256 threads: 64 queries of one head against tiles of 64 keys.  The kernel
+// above reads every key and value once a query and head (L1 and L2 bound: 637 us for 1,125 tokens of three sequences,
+// 16 heads of 64); here a tile of keys serves 64 queries.  Scores and outputs are sums in registers, 4 x 4 and
+// 4 x HD / 16 a thread, two at a time (fma.rn.f32x2: float32, rounded as fmaf rounds), the weights pass through shared memory.
+// Bound by the FMA pipes and shared memory: 119 us for the tokens above.  HD: the head size rounded up to 64 or 128, the rest is zero.
+__device__ __forceinline__ void att_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long att_twice(float v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float att_low(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float att_high(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+constexpr int TILE_Q = 64, TILE_K = 64, TILE_P = 68;       // rows of 64 in shared memory lie 68 apart: 16-byte aligned, spread over the banks
+template <int HD> constexpr size_t tile_smem() { return (size_t)(2 * HD * TILE_P + TILE_K * HD + TILE_K * TILE_P) * sizeof(float); }
+
+template <int HD>
+__global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm_tile[];
+    float* qt = sm_tile;                                   // [HD][TILE_P]: queries, transposed, scaled
+    float* kt = qt + HD * TILE_P;                          // [HD][TILE_P]: keys, transposed
+    float* vs = kt + HD * TILE_P;                          // [TILE_K][HD]
+    float* pt = vs + TILE_K * HD;                          // [TILE_K][TILE_P]: weights, transposed
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int h = blockIdx.y, kh = h / (a.nh / a.nkv), hd = a.hd;
+    // which sequence, which tile of it; a sequence's last tiles, which see the most keys, start first
+    int seq = 0, tile = blockIdx.x, t0 = 0, n_new = 0;
+    for (; seq < a.batch.B; ++seq) {
+        t0 = a.batch.q_start[seq];
+        n_new = a.batch.q_start[seq + 1] - t0;
+        const int tiles = (n_new + TILE_Q - 1) / TILE_Q;
+        if (tile < tiles) { tile = tiles - 1 - tile; break; }
+        tile -= tiles;
+    }
+    if (seq == a.batch.B) return;
+    const int first = a.batch.start_pos[seq], slot = a.batch.slot_of_seq[seq];
+    const int q0 = tile * TILE_Q, nq = min(TILE_Q, n_new - q0), pos0 = first + q0;
+    const int first_new = a.kv_new ? first : 0x7fffffff;
+    const float* knew = (const float*)a.kv_new;
+    const float* cache = (const float*)a.cache.storage;
+    const size_t vhalf = cache ? kv_half_elems(a.cache) : 0;
+    const int row = tid >> 2, quarter = tid & 3;           // loads: four threads a row, a row's 16-byte units in turn
+    {
+        const float* q = (const float*)a.q + (size_t)(t0 + q0 + min(row, nq - 1)) * a.q_stride + (size_t)h * hd;
+#pragma unroll
+        for (int u = 0; u < HD / 16; ++u) {
+            const int d = (u * 4 + quarter) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < nq && d < hd) v = *reinterpret_cast<const float4*>(q + d);
+            qt[d * TILE_P + row] = v.x; qt[(d + 1) * TILE_P + row] = v.y; qt[(d + 2) * TILE_P + row] = v.z; qt[(d + 3) * TILE_P + row] = v.w;
+        }
+    }
+    float m[4], l[4];
+    unsigned long long o[4][HD / 32];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -FLT_MAX; l[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < HD / 32; ++j) o[i][j] = 0ull;
+    }
+    const int hi = pos0 + nq, lo = a.window > 0 ? max(0, pos0 - a.window + 1) & ~(TILE_K - 1) : 0;      // tiles of keys begin at multiples of 64: a query's sums are the same in any step
+    for (int k0 = lo; k0 < hi; k0 += TILE_K) {
+        const int kpos = k0 + row;
+        const float* kp = nullptr;
+        const float* vp = nullptr;
+        if (kpos < hi) {
+            if (kpos >= first_new) {
+                kp = knew + (size_t)(t0 + kpos - first_new) * a.kv_stride + (size_t)kh * hd;
+                vp = kp + (size_t)a.nkv * hd;
+            } else {
+                kp = cache + kv_row_offset(a.cache, slot, kpos, kh);
+                vp = kp + vhalf;
+            }
+        }
+        __syncthreads();                                   // the tile before has been read
+        int odd = 0;                                       // a value that is not finite: it must not reach queries that do not see it
+#pragma unroll
+        for (int u = 0; u < HD / 16; ++u) {
+            const int d = (u * 4 + quarter) * 4;
+            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+            if (kp && d < hd) { kv = *reinterpret_cast<const float4*>(kp + d); vv = *reinterpret_cast<const float4*>(vp + d); }
+            kt[d * TILE_P + row] = kv.x; kt[(d + 1) * TILE_P + row] = kv.y; kt[(d + 2) * TILE_P + row] = kv.z; kt[(d + 3) * TILE_P + row] = kv.w;
+            *reinterpret_cast<float4*>(vs + row * HD + d) = vv;
+            odd |= !(fmaxf(fmaxf(fabsf(vv.x), fabsf(vv.y)), fmaxf(fabsf(vv.z), fabsf(vv.w))) <= FLT_MAX) | (vv.x != vv.x) | (vv.y != vv.y) | (vv.z != vv.z) | (vv.w != vv.w);
+        }
+        odd = __syncthreads_or(odd);
+        unsigned long long sc[4][2] = {};
+#pragma unroll 8
+        for (int d = 0; d < HD; ++d) {
+            const float4 q4 = *reinterpret_cast<const float4*>(qt + d * TILE_P + ty * 4);
+            const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(kt + d * TILE_P + tx * 4);
+            const float qv[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const unsigned long long qq = att_twice(qv[i]);
+                att_fma2(sc[i][0], qq, k2.x);
+                att_fma2(sc[i][1], qq, k2.y);
+            }
+        }
+        float p[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int pos = pos0 + ty * 4 + i;
+            float s[4] = {att_low(sc[i][0]), att_high(sc[i][0]), att_low(sc[i][1]), att_high(sc[i][1])};
+            bool ok[4];
+            float top = -FLT_MAX;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = k0 + tx * 4 + j;
+                ok[j] = key <= pos && (a.window <= 0 || key > pos - a.window);
+                s[j] *= a.scale;
+                if (ok[j]) top = fmaxf(top, s[j]);
+            }
+#pragma unroll
+            for (int x = 1; x < 16; x *= 2) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+            const float m_new = fmaxf(m[i], top), alpha = expf(m[i] - m_new);      // m = -FLT_MAX at the start: the sums it scales are zero
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { p[i][j] = ok[j] ? expf(s[j] - m_new) : 0.f; sum += p[i][j]; }
+#pragma unroll
+            for (int x = 1; x < 16; x *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+            l[i] = l[i] * alpha + sum;
+            m[i] = m_new;
+            const unsigned long long aa = att_twice(alpha);
+#pragma unroll
+            for (int j = 0; j < HD / 32; ++j) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(o[i][j]) : "l"(aa));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(pt + (tx * 4 + j) * TILE_P + ty * 4) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
+        __syncwarp();                                      // a warp reads the weights of its own eight rows only
+        const int n_keys = min(TILE_K, hi - k0);
+#pragma unroll 4
+        for (int k = 0; k < n_keys; ++k) {
+            const float4 p4 = *reinterpret_cast<const float4*>(pt + k * TILE_P + ty * 4);
+            const float pv[4] = {p4.x, p4.y, p4.z, p4.w};
+            unsigned long long v2[HD / 32];
+#pragma unroll
+            for (int j = 0; j < HD / 64; ++j) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vs + k * HD + j * 64 + tx * 4);
+                v2[2 * j] = v.x; v2[2 * j + 1] = v.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (odd && (k0 + k > pos0 + ty * 4 + i || (a.window > 0 && k0 + k <= pos0 + ty * 4 + i - a.window))) continue;
+                const unsigned long long pp = att_twice(pv[i]);
+#pragma unroll
+                for (int j = 0; j < HD / 32; ++j) att_fma2(o[i][j], pp, v2[j]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty * 4 + i;
+        if (r >= nq) continue;
+        float scale = 1.f;
+        if (a.sink) {                                      // one more term of the denominator, against the larger of the two maxima
+            const float sk = a.sink[h], m_new = fmaxf(m[i], sk);
+            scale = expf(m[i] - m_new);
+            l[i] = l[i] * scale + expf(sk - m_new);
+        }
+        const float inv = scale / l[i];
+        float* out = (float*)a.out + (size_t)(t0 + q0 + r) * a.out_stride + (size_t)h * hd;
+#pragma unroll
+        for (int j = 0; j < HD / 64; ++j) {
+            const int d = j * 64 + tx * 4;
+            if (d < hd)
+                *reinterpret_cast<float4*>(out + d) = make_float4(att_low(o[i][2 * j]) * inv, att_high(o[i][2 * j]) * inv,
+                                                                  att_low(o[i][2 * j + 1]) * inv, att_high(o[i][2 * j + 1]) * inv);
+        }
+    }
+}
+
+template <int HD>
+static int launch_tile(const AttnArgs& a, cudaStream_t stream) {
+    static std::atomic<bool> configured[64];              // a device each
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64 || !configured[dev].load()) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem<HD>());
+        TB_REQUIRE(e == cudaSuccess, "attn_prefill: cannot reserve %zu bytes of shared memory: %s", tile_smem<HD>(), cudaGetErrorString(e));
+        if (dev < 64) configured[dev].store(true);
+    }
+    const dim3 grid(a.batch.T / TILE_Q + a.batch.B, a.nh);
+    tb_launch(attn_prefill_tile_kernel<HD>, grid, 256, tile_smem<HD>(), stream, a);
+    return 0;
+}
+
 // ------------------------------------------------------------------ decode, split over the keys
 // grid (B, nkv, n_splits); the warps of a block take the query heads of one kv head in turn.
 // Partial of (sequence b, head h, split s) at scratch[((b * nh + h) * n_splits + s) * (hd + 2)]:
@@ -225,6 +432,119 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_decode_kernel(AttnArgs a)
             if (d < hdv) part[d] = st.acc[j];
         }
         if (lane == 0) { part[hdv] = st.m; part[hdv + 1] = st.l; }
+    }
+}
+
+// The same for rows of up to 32 16-byte units (float32: 128 elements, bfloat16: 256).  LPK lanes share a key, a 16-byte unit of its row
+// each, so that a load covers whole rows of 32 / LPK keys (in the kernel above every lane walks a row of its own, and a warp a
+// whole split).  Each group of LPK lanes is a stream of its own: keys st, st + streams, ... of the split, eight keys and
+// values requested at once, an own running softmax.  The streams of a head, those of up to eight warps, are merged in shared memory.
+// Bound by the latency of the loads at a few hundred keys a split: three
+// sequences of 500 tokens, 16 heads of 64 on 8, float32: 210 -> 13.7 us a layer.
+constexpr int VEC_WARPS = 8, VEC_KEYS = 8;
+
+template <typename T, int LPK>
+__global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArgs a) {
+    constexpr int PER = 16 / (int)sizeof(T), STREAMS = 32 / LPK;
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ float parts[];                   // [VEC_WARPS * STREAMS][hdv + 2]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, unit = lane % LPK;
+    const int blocks_y = a.head_blocks > 0 ? a.head_blocks : a.nkv;
+    const int b = blockIdx.x, kh = (int)blockIdx.y * a.nkv / blocks_y, split = blockIdx.z;
+    const int hd = a.hd, hdv = value_width(a), group = a.nh / blocks_y;
+    const int len = a.batch.kv_len[b];
+    const int keys = tb_split_keys(len, a.chunk, a.n_splits);
+    if ((long long)split * keys >= len) return;     // the merge reads ceil(len / keys) splits only
+    int share = 1;                                     // warps a head: two, four or eight where there are at least so many times as many warps
+    while (share * 2 * group <= VEC_WARPS) share *= 2;
+    const int pos = len - 1;
+    const int slot = a.batch.slot_of_seq[b];
+    const int wlo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    const int lo = max(wlo, split * keys), hi = min(len, (split + 1) * keys);
+    // the kept first tokens that lie in this split and before the window
+    const int klo = split * keys, khi = a.window > 0 ? min(min(a.keep_first, wlo), hi) : 0;
+    const T* cache = (const T*)a.cache.storage;
+    const size_t vhalf = a.v_alias ? 0 : kv_half_elems(a.cache);
+    const int streams = share * STREAMS, st = (warp % share) * STREAMS + lane / LPK;
+    const int at = unit * PER;
+    const bool key_part = at < hd, value_part = at < hdv;
+    for (int g0 = 0; g0 < group; g0 += VEC_WARPS / share) {
+        const int g = g0 + warp / share;
+        const int h = (int)blockIdx.y * group + min(g, group - 1);
+        float q[PER], acc[PER], m = -FLT_MAX, l = 0.f;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            q[e] = at + e < hd ? ldf((const T*)a.q + (size_t)b * a.q_stride + h * hd + at + e) : 0.f;
+            acc[e] = 0.f;
+        }
+        auto attend = [&](int first, int last) {
+            for (int base = first; base < last; base += VEC_KEYS * streams) {      // (the bounds are the warp's: its lanes stay together)
+                uint4 kr[VEC_KEYS], vr[VEC_KEYS];
+#pragma unroll
+                for (int u = 0; u < VEC_KEYS; ++u) {
+                    const T* row = cache + kv_row_offset(a.cache, slot, min(base + u * streams + st, last - 1), kh) + at;
+                    kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
+                    if (key_part) kr[u] = *reinterpret_cast<const uint4*>(row);
+                    if (value_part) vr[u] = *reinterpret_cast<const uint4*>(row + vhalf);
+                }
+                float s[VEC_KEYS], top = m;
+#pragma unroll
+                for (int u = 0; u < VEC_KEYS; ++u) {
+                    float k[PER], dot = 0.f;
+                    unpack16<T>(kr[u], k);
+#pragma unroll
+                    for (int e = 0; e < PER; ++e) dot = fmaf(q[e], k[e], dot);
+#pragma unroll
+                    for (int o = LPK / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                    s[u] = dot * a.scale;
+                    if (base + u * streams + st < last) top = fmaxf(top, s[u]);
+                }
+                const float alpha = expf(m - top);     // m = -FLT_MAX at the start: the sums it scales are zero
+                m = top;
+                l *= alpha;
+#pragma unroll
+                for (int e = 0; e < PER; ++e) acc[e] *= alpha;
+#pragma unroll
+                for (int u = 0; u < VEC_KEYS; ++u) {
+                    if (base + u * streams + st >= last) continue;
+                    const float p = expf(s[u] - m);
+                    float v[PER];
+                    unpack16<T>(vr[u], v);
+                    l += p;
+#pragma unroll
+                    for (int e = 0; e < PER; ++e) acc[e] = fmaf(p, v[e], acc[e]);
+                }
+            }
+        };
+        if (g < group) {
+            if (klo < khi) attend(klo, khi);
+            if (lo < hi) attend(lo, hi);
+        }
+        float* mine = parts + (warp * STREAMS + lane / LPK) * (hdv + 2);
+        if (share == 1) __syncwarp();                  // (the warp has read its streams of the head before)
+#pragma unroll
+        for (int e = 0; e < PER; ++e) if (at + e < hdv) mine[at + e] = acc[e];
+        if (unit == 0) { mine[hdv] = m; mine[hdv + 1] = l; }
+        if (share > 1) __syncthreads(); else __syncwarp();
+        if (warp % share != 0 || g >= group) continue;
+        const float* of = parts + warp * STREAMS * (hdv + 2);      // the head's streams lie side by side
+        float* part = a.scratch + ((size_t)(b * a.nh + h) * a.n_splits + split) * (hdv + 2);
+        float top = -FLT_MAX, sum = 0.f;
+        for (int w = 0; w < streams; ++w) if (of[w * (hdv + 2) + hdv + 1] != 0.f) top = fmaxf(top, of[w * (hdv + 2) + hdv]);
+        for (int d = lane; d < hdv; d += 32) {
+            float o = 0.f;
+            for (int w = 0; w < streams; ++w) {
+                const float* p = of + w * (hdv + 2);
+                if (p[hdv + 1] != 0.f) o = fmaf(expf(p[hdv] - top), p[d], o);      // (a stream that saw no key has l = 0)
+            }
+            part[d] = o;
+        }
+        for (int w = 0; w < streams; ++w) {
+            const float* p = of + w * (hdv + 2);
+            if (p[hdv + 1] != 0.f) sum = fmaf(expf(p[hdv] - top), p[hdv + 1], sum);
+        }
+        if (lane == 0) { part[hdv] = top; part[hdv + 1] = sum; }
     }
 }
 
@@ -378,6 +698,14 @@ extern "C" int tb_attn_prefill(const AttnArgs* args, int dtype, cudaStream_t str
     TB_REQUIRE(a.batch.T > 0, "attn_prefill: no tokens");
     TB_REQUIRE(a.kv_new || a.cache.storage, "attn_prefill: neither new keys nor a cache");
     TB_REQUIRE(!a.head_gate, "attn_prefill: a gate on the heads is applied by the merge of decode splits or by the mixed-heads kernels");
+    // The tiles take plain float32 heads: keys and values of one width of up to 128 that lie in separate planes, no kept first tokens
+    // and no pairs of heads, rows that 16-byte loads and stores can take.
+    if (dtype == TB_F32 && a.hd <= 128 && value_width(a) == a.hd && !a.v_alias && a.keep_first <= 0 && !a.pair_lambda && a.out_stride % 4 == 0 &&
+        (uintptr_t)a.q % 16 == 0 && (uintptr_t)a.kv_new % 16 == 0 && (uintptr_t)a.out % 16 == 0 && (uintptr_t)a.cache.storage % 16 == 0 && a.nh <= 65535) {
+        if (a.hd <= 64 ? launch_tile<64>(a, stream) : launch_tile<128>(a, stream)) return 1;
+        TB_CHECK_LAUNCH("attn_prefill");
+        return 0;
+    }
     dim3 grid(a.batch.T, (a.nh + ATT_WARPS - 1) / ATT_WARPS);
     const size_t smem = (size_t)ATT_WARPS * a.hd * sizeof(float);
     const bool wide = wide_rows(a);
@@ -421,9 +749,19 @@ extern "C" int tb_attn_decode(const AttnArgs* args, int dtype, cudaStream_t stre
     TB_REQUIRE(a.head_blocks == 0 || (a.head_blocks > 0 && a.nh % a.head_blocks == 0 && a.head_blocks % a.nkv == 0),
                "attn_decode: %d blocks for %d query heads on %d kv heads", a.head_blocks, a.nh, a.nkv);
     dim3 grid(a.batch.B, a.head_blocks > 0 ? a.head_blocks : a.nkv, a.n_splits);
-    const size_t smem = (size_t)ATT_WARPS * a.hd * sizeof(float);
-    const bool wide = wide_rows(a);
-    ATT_DISPATCH(attn_decode_kernel, grid, ATT_WARPS * 32, smem);
+    const int width = a.hd > value_width(a) ? a.hd : value_width(a), units = (width * (dtype == TB_F32 ? 4 : 2) + 15) / 16;
+    if (units <= 32 && a.hd % 8 == 0 && value_width(a) % (dtype == TB_F32 ? 4 : 8) == 0 && (uintptr_t)a.cache.storage % 16 == 0) {
+        // lanes a key: as few as hold its row
+#define ATT_VEC(TT, L) tb_launch(attn_decode_vec_kernel<TT, L>, grid, VEC_WARPS * 32, (size_t)VEC_WARPS * (32 / L) * (value_width(a) + 2) * sizeof(float), stream, a)
+#define ATT_VEC_ANY(TT) do { if (units <= 4) ATT_VEC(TT, 4); else if (units <= 8) ATT_VEC(TT, 8); else if (units <= 16) ATT_VEC(TT, 16); else ATT_VEC(TT, 32); } while (0)
+        if (dtype == TB_F32) ATT_VEC_ANY(float); else ATT_VEC_ANY(__nv_bfloat16);
+#undef ATT_VEC_ANY
+#undef ATT_VEC
+    } else {
+        const size_t smem = (size_t)ATT_WARPS * a.hd * sizeof(float);
+        const bool wide = wide_rows(a);
+        ATT_DISPATCH(attn_decode_kernel, grid, ATT_WARPS * 32, smem);
+    }
     TB_CHECK_LAUNCH("attn_decode");
     return tb_attn_merge(args, dtype, stream);
 }
