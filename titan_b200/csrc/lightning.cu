@@ -4,16 +4,18 @@
 //   o_t = S_t^T q_t
 // with q = silu(.), k = silu(.), v = silu(.) of the projection's columns (the projection may be in the compute
 // dtype; the activation, the state and the sums are float32).  A sequence's tokens are taken in order, so a prompt
-// run whole, in pieces or token by token leaves the same state up to the order of float32 sums (which is the same
-// here: one token after the other in every case).
+// run whole, in pieces or token by token leaves the same state up to the order of float32 sums.
 //
 // tb_lightning_scan   grid (sequences, heads, ceil(dv / 32)): a block owns 32 value columns of one head's state;
 //                     four neighbouring lanes share a column (each keeps a quarter of its rows in registers) and
 //                     add their parts of o with two shuffles.  Tokens are staged in shared memory sixteen at a time,
-//                     the next sixteen requested while these are worked through.
+//                     the next sixteen requested while these are worked through.  Runs of CHUNKED_FROM tokens and
+//                     more go chunk by chunk as small matrix products instead (lightning_prep_kernel, lightning_chunk_kernel).
 // tb_gated_rmsnorm    y = o / sqrt(mean(o^2) + eps) * w * sigmoid(g) over the concatenated heads, one block a token.
 // tb_rotary_rows      rotates heads that lie side by side in float32 rows, in place, and scales some of them: what the
 //                     retention mixer does to q and k between its projection and this recurrence (LightningArgs.plain).
+#include <atomic>
+
 #include "common.cuh"
 #include "qk_args.h"
 
@@ -26,6 +28,8 @@ struct LightningArgs {
     int B; int H; int dk; int dv;
     int max_new;                            // most tokens a sequence brings in this step (1: a step of single tokens)
     int plain;                              // 1: q, k and v enter the recurrence as they stand in the rows (no silu): the retention mixer, whose rows are float32
+    float* work; int work_chunks;           // room for the chunked form: work_chunks * H * 64 * (64 + 2 * DK) floats, work_chunks >= sum over sequences of ceil(tokens / 64); null: token by token
+    int below;                              // > 0: only runs of fewer tokens (set by the launcher)
 };
 
 namespace {
@@ -50,6 +54,7 @@ __global__ void __launch_bounds__(128) lightning_scan_kernel(LightningArgs a) {
     const int tid = threadIdx.x, s = tid & 3, col = tid >> 2, j = blockIdx.z * 32 + col;
     const int dk = a.dk, dv = a.dv;
     const int t0 = a.q_start[b], t1 = a.q_start[b + 1];
+    if (a.below > 0 && t1 - t0 >= a.below) return;
     const bool live = j < dv;
     float* S_g = a.state + (((size_t)a.slot_of_seq[b] * a.H + h) * dk) * dv + j;
     float S[R];
@@ -159,6 +164,7 @@ __global__ void __launch_bounds__(128) lightning_scan_vec_kernel(LightningArgs a
     const int tid = threadIdx.x, s = tid & 7, col = tid >> 3, j = blockIdx.z * 16 + col;
     const int dk = a.dk, dv = a.dv;
     const int t0 = a.q_start[b], t1 = a.q_start[b + 1];
+    if (a.below > 0 && t1 - t0 >= a.below) return;
     const bool live = j < dv;
     float* S_g = a.state + (((size_t)a.slot_of_seq[b] * a.H + h) * dk) * dv + j;
     float S[R];
@@ -247,6 +253,317 @@ __global__ void __launch_bounds__(128) lightning_scan_vec_kernel(LightningArgs a
     }
 }
 
+// ---------------------------------------------------------------- prompts: chunks of 64 tokens
+// Token by token the recurrence is a chain of 2,000 dependent steps of 0.75 us each (measured: 1,531 us for 2,000 tokens, 16 heads of
+// 128 x 128).  With S the state before a chunk, r a token's place in it and n its length,
+//     o_r = decay^(r+1) q_r . S + sum over j <= r of decay^(r-j) (q_r . k_j) v_j,     S' = decay^n S + sum_j decay^(n-1-j) k_j v_j^T
+// so that a chunk is four small products and only chunks wait for one another.  Everything stays float32, fused
+// multiply-adds only (two at a time, fma.rn.f32x2, each rounded as fmaf rounds); powers of the decay are formed in 64 bits.
+// lightning_prep_kernel, all chunks at once: rows A_r = [decay^(r-j) (q_r . k_j) for j < 64, zero above r | decay^(r+1) q_r]
+// and, transposed, k'_r = decay^(n-1-r) k_r.  lightning_chunk_kernel, a block for 16 value columns of a head, the state's slice in
+// registers and in shared memory behind the chunk's values: one product A . [v; S] and one k'^T v a chunk, the next chunk's rows on
+// their way meanwhile.  Every operand lies along the dimension that is summed over, so that sums over even and over odd
+// places are one two-element multiply-add and no operand has to be doubled.  16 columns: 128 blocks for one sequence of 16 heads of 128.  Bound by the FMA pipes, 2,560 cycles a chunk.
+// 2,000 tokens, 16 heads of 128 x 128: 34 us and 158 us, of which the outputs' product takes 50, the state's 30 and the
+// wait for the rows 22.
+constexpr int CHUNK = 64, VCOLS = 16;
+constexpr int CHUNKED_FROM = 32;        // tokens of the longest run from which the chunked form is the faster one
+
+__device__ __forceinline__ void lf_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float lf_low(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float lf_high(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+template <int DK> constexpr int chunk_row() { return CHUNK + DK; }                                  // floats of a row of A
+template <int DK> constexpr size_t chunk_floats() { return (size_t)CHUNK * (CHUNK + 2 * DK); }     // of a (chunk, head): A, then k'
+template <int DK> constexpr size_t prep_smem() { return (size_t)(2 * CHUNK * (DK + 4) + CHUNK + 1) * sizeof(float); }
+
+// grid (work_chunks, H), 256 threads
+template <typename T, int DK>
+__global__ void __launch_bounds__(256) lightning_prep_kernel(LightningArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int LD = DK + 4;
+    float* qs = sm;
+    float* ks = qs + CHUNK * LD;
+    float* power = ks + CHUNK * LD;                     // decay^0 .. decay^64
+    const int tid = threadIdx.x, h = blockIdx.y, dk = a.dk;
+    int b = 0, chunk = blockIdx.x, t0 = 0, n = 0;
+    for (; b < a.B; ++b) {
+        t0 = a.q_start[b];
+        const int left = a.q_start[b + 1] - t0, chunks = (left + CHUNK - 1) / CHUNK;
+        if (chunk < chunks) { t0 += chunk * CHUNK; n = left < CHUNKED_FROM ? 0 : min(CHUNK, left - chunk * CHUNK); break; }
+        chunk -= chunks;
+    }
+    if (b == a.B || n == 0) return;
+    if (tid <= CHUNK) power[tid] = (float)pow((double)a.decay[h], (double)tid);
+    const T* base = (const T*)a.proj + (size_t)t0 * a.stride + h * dk;
+    if (dk % 8 == 0 && a.stride % 8 == 0 && (uintptr_t)a.proj % 16 == 0) {
+        constexpr int UNITS = CHUNK * DK / 8 / 256;     // units of eight elements a thread, of q and of k: all requested at once
+        Pack8<T> q[UNITS], k[UNITS];
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int e = (tid + 256 * u) * 8, r = min(e / DK, n - 1), d = min(e % DK, dk - 8);
+            q[u].load(base + (size_t)r * a.stride + d);
+            k[u].load(base + (size_t)r * a.stride + a.H * dk + d);
+        }
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int e = (tid + 256 * u) * 8, r = e / DK, d = e % DK;
+            const bool real = r < n && d < dk;
+            float fq[8], fk[8];
+            q[u].get(fq); k[u].get(fk);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                fq[i] = real ? (a.plain ? fq[i] : silu_f(fq[i])) : 0.f;
+                fk[i] = real ? (a.plain ? fk[i] : silu_f(fk[i])) : 0.f;
+            }
+            float4* to = reinterpret_cast<float4*>(qs + r * LD + d);
+            to[0] = make_float4(fq[0], fq[1], fq[2], fq[3]); to[1] = make_float4(fq[4], fq[5], fq[6], fq[7]);
+            to = reinterpret_cast<float4*>(ks + r * LD + d);
+            to[0] = make_float4(fk[0], fk[1], fk[2], fk[3]); to[1] = make_float4(fk[4], fk[5], fk[6], fk[7]);
+        }
+    } else {
+        for (int e = tid; e < CHUNK * DK; e += 256) {
+            const int r = e / DK, d = e % DK;
+            float q = 0.f, k = 0.f;
+            if (r < n && d < dk) {
+                q = ldf(base + (size_t)r * a.stride + d);
+                k = ldf(base + (size_t)r * a.stride + a.H * dk + d);
+                if (!a.plain) { q = silu_f(q); k = silu_f(k); }
+            }
+            qs[r * LD + d] = q;
+            ks[r * LD + d] = k;
+        }
+    }
+    __syncthreads();
+    float* rows = a.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats<DK>();
+    float* krows = rows + CHUNK * chunk_row<DK>();
+    const int tx = tid & 15, ty = tid >> 4;             // scores of rows ty + 16 i and keys tx + 16 j
+    unsigned long long acc[4][4] = {};                  // sums over even and over odd dimensions
+#pragma unroll 4
+    for (int d = 0; d < DK; d += 4) {
+        ulonglong2 q[4], k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            q[i] = *reinterpret_cast<const ulonglong2*>(qs + (ty + 16 * i) * LD + d);
+            k[i] = *reinterpret_cast<const ulonglong2*>(ks + (tx + 16 * i) * LD + d);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j) { lf_fma2(acc[i][j], q[i].x, k[j].x); lf_fma2(acc[i][j], q[i].y, k[j].y); }      // (j > i: keys after every query)
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = ty + 16 * i, c = tx + 16 * j;
+            rows[r * chunk_row<DK>() + c] = c <= r && r < n ? (lf_low(acc[i][j]) + lf_high(acc[i][j])) * power[r - c] : 0.f;
+        }
+    for (int e = tid; e < CHUNK * DK / 4; e += 256) {
+        const int r = e / (DK / 4), d = e % (DK / 4) * 4;
+        float4 q = *reinterpret_cast<const float4*>(qs + r * LD + d);
+        const float f = power[r + 1];
+        q.x *= f; q.y *= f; q.z *= f; q.w *= f;
+        *reinterpret_cast<float4*>(rows + r * chunk_row<DK>() + CHUNK + d) = q;
+    }
+    for (int e = tid; e < DK * CHUNK / 4; e += 256) {   // a thread: one dimension, four tokens; four threads a dimension
+        const int d = e / 4 % DK, r = (e / (4 * DK) * 4 + e % 4) * 4;
+        float k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) k[i] = r + i < n ? ks[(r + i) * LD + d] * power[n - 1 - r - i] : 0.f;
+        *reinterpret_cast<float4*>(krows + d * CHUNK + r) = make_float4(k[0], k[1], k[2], k[3]);
+    }
+}
+
+__device__ __forceinline__ void copy16(float* to, const float* from) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+
+constexpr int PART_COL = CHUNK + 8;                     // floats from a column to the next of a warp's partial outputs
+template <int DK> constexpr size_t chunk_smem() {
+    // two buffers of A and of k'^T (rows padded by 4), values and the state's slice by column, eight warps' partial outputs
+    return (size_t)(2 * (CHUNK * (chunk_row<DK>() + 4) + DK * (CHUNK + 4)) + VCOLS * (chunk_row<DK>() + 4) + 8 * VCOLS * PART_COL) * sizeof(float);
+}
+
+// grid (B, H, ceil(dv / 16)), 512 threads: warps 0 .. 7 make the outputs while warps 8 .. 15 make the state after the chunk
+template <typename T, int DK>
+__global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int ROW = chunk_row<DK>(), LD = ROW + 4, LT = CHUNK + 4, RK = DK / 32, KW = ROW / 8;
+    float* rows = sm;                                   // [2][CHUNK][LD]
+    float* krows = rows + 2 * CHUNK * LD;               // [2][DK][LT]
+    float* vals = krows + 2 * DK * LT;                  // [VCOLS][LD]: by column, the chunk's values, then the state
+    float* part = vals + VCOLS * LD;                    // [8][VCOLS][PART_COL]
+    const int b = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VCOLS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int dk = a.dk, dv = a.dv, t0 = a.q_start[b], t1 = a.q_start[b + 1];
+    if (t1 - t0 < CHUNKED_FROM) return;
+    int chunk0 = 0;                                     // the sequence's first chunk
+    for (int i = 0; i < b; ++i) chunk0 += (a.q_start[i + 1] - a.q_start[i] + CHUNK - 1) / CHUNK;
+    const float decay = a.decay[h], whole = (float)pow((double)decay, (double)CHUNK);
+    // the state: a thread of the second half keeps rows sk + 32 i of columns sc and sc + 8
+    const bool keeps = tid >= 256;
+    const int sk = (tid & 255) >> 3, sc = tid & 7;
+    float* S_g = a.state + ((size_t)a.slot_of_seq[b] * a.H + h) * dk * dv + j0;
+    float S[RK][2];
+#pragma unroll
+    for (int i = 0; i < RK; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            S[i][c] = (keeps && sk + 32 * i < dk && j0 + sc + 8 * c < dv) ? S_g[(size_t)(sk + 32 * i) * dv + sc + 8 * c] : 0.f;
+            if (keeps) vals[(sc + 8 * c) * LD + CHUNK + sk + 32 * i] = S[i][c];
+        }
+    auto load_rows = [&](int c, int half) {
+        const float* from = a.work + ((size_t)(chunk0 + c) * a.H + h) * chunk_floats<DK>();
+        float* to = rows + half * CHUNK * LD;
+#pragma unroll
+        for (int u = 0; u < CHUNK * ROW / 4 / 512; ++u) { const int e = tid + 512 * u; copy16(to + e / (ROW / 4) * LD + e % (ROW / 4) * 4, from + e * 4); }
+        from += CHUNK * ROW;
+        to = krows + half * DK * LT;
+#pragma unroll
+        for (int u = 0; u < CHUNK * DK / 4 / 512; ++u) { const int e = tid + 512 * u; copy16(to + e / (CHUNK / 4) * LT + e % (CHUNK / 4) * 4, from + e * 4); }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // two values of a chunk a thread: token tid % 64, columns lc and lc + 1; and a thread of the first half's outputs: token vr, columns vc ..
+    const int vr = tid & 63, lc = tid >> 6 << 1, vc = (tid & 255) >> 6 << 2;
+    const bool two = dv % 2 == 0 && a.stride % 2 == 0 && (uintptr_t)a.proj % 8 == 0;       // one load for both
+    float next[2];
+    auto load_values = [&](int c) {
+        const int t = t0 + c * CHUNK + vr;
+        const T* v = (const T*)a.proj + (size_t)t * a.stride + 2 * a.H * dk + h * dv + j0 + lc;
+        next[0] = next[1] = 0.f;
+        if (two) {
+            if (t < t1 && j0 + lc < dv) {
+                struct alignas(2 * sizeof(T)) Two { T x, y; };
+                const Two both = *reinterpret_cast<const Two*>(v);
+                next[0] = ldf(&both.x); next[1] = ldf(&both.y);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) if (t < t1 && j0 + lc + i < dv) next[i] = ldf(v + i);
+        }
+    };
+    const bool out4 = dv % 4 == 0 && a.out_stride % 4 == 0 && (uintptr_t)a.out % 16 == 0;
+    const int chunks = (t1 - t0 + CHUNK - 1) / CHUNK;
+    load_rows(0, 0);
+    load_values(0);
+    for (int c = 0; c < chunks; ++c) {
+        const int half = c & 1, n = min(CHUNK, t1 - t0 - c * CHUNK);
+        int odd = 0;                                    // a value that is not finite: its product with a zero weight is no zero
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (!a.plain) next[i] = silu_f(next[i]);    // (silu(0) = 0: rows and columns outside stay zero)
+            odd |= !(fabsf(next[i]) <= 3.402823466e38f);
+            vals[(lc + i) * LD + vr] = next[i];
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        odd = __syncthreads_or(odd);
+        if (c + 1 < chunks) { load_rows(c + 1, half ^ 1); load_values(c + 1); }
+        const float* A = rows + half * CHUNK * LD;
+        if (!keeps) {   // this warp's KW of the columns of A: rows rg + 8 r, value columns cg + 4 j; sums over even and over odd places
+            const int cg = lane & 3, rg = lane >> 2;
+            unsigned long long acc[8][4] = {};
+#pragma unroll 2
+            for (int k = warp * KW; k < (warp + 1) * KW; k += 4) {
+                if (odd && k < CHUNK) continue;         // (done below, term by term)
+                ulonglong2 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const ulonglong2*>(vals + (cg + 4 * j) * LD + k);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(A + (rg + 8 * r) * LD + k);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { lf_fma2(acc[r][j], x.x, v[j].x); lf_fma2(acc[r][j], x.y, v[j].y); }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int r = 0; r < 8; ++r) part[(warp * VCOLS + cg + 4 * j) * PART_COL + rg + 8 * r] = lf_low(acc[r][j]) + lf_high(acc[r][j]);
+        }
+        if (keeps) {    // the state after the chunk
+            const float f = n == CHUNK ? whole : (float)pow((double)decay, (double)n);
+            const float* kr = krows + half * DK * LT + sk * LT;
+            unsigned long long acc[RK][2] = {};
+#pragma unroll 4
+            for (int t = 0; t < CHUNK; t += 4) {
+                const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(vals + sc * LD + t), v1 = *reinterpret_cast<const ulonglong2*>(vals + (sc + 8) * LD + t);
+#pragma unroll
+                for (int i = 0; i < RK; ++i) {
+                    const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(kr + 32 * i * LT + t);
+                    lf_fma2(acc[i][0], k.x, v0.x); lf_fma2(acc[i][0], k.y, v0.y);
+                    lf_fma2(acc[i][1], k.x, v1.x); lf_fma2(acc[i][1], k.y, v1.y);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < RK; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) S[i][e] = fmaf(f, S[i][e], lf_low(acc[i][e]) + lf_high(acc[i][e]));
+        }
+        __syncthreads();                                // the partial outputs are complete; the values and the old state have been read
+        if (!keeps && vr < n) {
+            float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[i] += part[(w * VCOLS + vc + i) * PART_COL + vr];
+            if (odd)
+                for (int j = 0; j <= vr; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) o[i] = fmaf(A[vr * LD + j], vals[(vc + i) * LD + j], o[i]);
+            float* to = a.out + (size_t)(t0 + c * CHUNK + vr) * a.out_stride + h * dv + j0 + vc;
+            if (out4) {
+                if (j0 + vc < dv) *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (j0 + vc + i < dv) to[i] = o[i];
+            }
+        }
+        if (odd) __syncthreads();                       // (those read the values again)
+        if (keeps)
+#pragma unroll
+            for (int i = 0; i < RK; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) vals[(sc + 8 * e) * LD + CHUNK + sk + 32 * i] = S[i][e];
+    }
+    if (!keeps) return;
+#pragma unroll
+    for (int i = 0; i < RK; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (sk + 32 * i < dk && j0 + sc + 8 * e < dv) S_g[(size_t)(sk + 32 * i) * dv + sc + 8 * e] = S[i][e];
+}
+
+template <typename T>
+int launch_scan(const LightningArgs& a, bool single, cudaStream_t stream);
+
+template <typename T, int DK>
+int launch_chunks(const LightningArgs& a, cudaStream_t stream) {
+    static std::atomic<bool> configured[64];            // a device each
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64 || !configured[dev].load()) {
+        cudaError_t e = cudaFuncSetAttribute(lightning_prep_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem<DK>());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(lightning_chunk_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem<DK>());
+        TB_REQUIRE(e == cudaSuccess, "lightning_scan: cannot reserve %zu bytes of shared memory: %s", chunk_smem<DK>(), cudaGetErrorString(e));
+        if (dev < 64) configured[dev].store(true);
+    }
+    tb_launch(lightning_prep_kernel<T, DK>, dim3(a.work_chunks, a.H), 256, prep_smem<DK>(), stream, a);
+    tb_launch(lightning_chunk_kernel<T, DK>, dim3(a.B, a.H, (a.dv + VCOLS - 1) / VCOLS), 512, chunk_smem<DK>(), stream, a);
+    if (a.B > 1) {                                      // shorter runs beside them go token by token, as they would alone
+        LightningArgs rest = a;
+        rest.work = nullptr; rest.below = CHUNKED_FROM;
+        return launch_scan<T>(rest, false, stream);
+    }
+    return 0;
+}
+
 template <typename T>
 __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ w, const T* __restrict__ gate,
                                      int ldg, T* __restrict__ y, int ldy, int N, float eps) {
@@ -324,6 +641,7 @@ int launch_vec(const LightningArgs& a, cudaStream_t stream) {
 
 template <typename T>
 int launch_scan(const LightningArgs& a, bool single, cudaStream_t stream) {
+    if (a.work) return a.dk <= 64 ? launch_chunks<T, 64>(a, stream) : launch_chunks<T, 128>(a, stream);
     // sizes in multiples of 8 and rows that 16-byte loads can take: the kernel of eight lanes a column
     if (a.dk % 8 == 0 && a.dv % 8 == 0 && a.stride % 8 == 0 && ((uintptr_t)a.proj % 16 == 0) && a.dk >= 64 && (a.dv + 15) / 16 <= 65535) {
         const int rows = a.dk / 8;
@@ -352,8 +670,17 @@ int launch_scan(const LightningArgs& a, bool single, cudaStream_t stream) {
 
 }  // namespace
 
+// Floats of ``work`` (and its chunks) with which a step of T tokens in B runs, the longest of max_new, takes the chunked form;
+// 0: none is wanted (short runs, where the two launches cost more than the chain; heads of more than 128 key dimensions).
+extern "C" long long tb_lightning_work(int T, int B, int H, int dk, int dv, int max_new, int* chunks) {
+    if (max_new < CHUNKED_FROM || dk > 128 || (dv + VCOLS - 1) / VCOLS > 65535) { *chunks = 0; return 0; }
+    *chunks = T / CHUNK + B;                            // at least the sum of every run's chunks
+    return (long long)*chunks * H * (long long)(dk <= 64 ? chunk_floats<64>() : chunk_floats<128>());
+}
+
 extern "C" int tb_lightning_scan(const LightningArgs* args, int dtype, cudaStream_t stream) {
     LightningArgs a = *args;
+    a.below = 0;
     TB_REQUIRE(a.B > 0 && a.H > 0 && a.dk > 0 && a.dv > 0, "lightning_scan: sizes must be positive");
     TB_REQUIRE(a.dk <= 256, "lightning_scan: %d key dimensions a head (at most 256)", a.dk);
     TB_REQUIRE(a.H <= 65535 && (a.dv + 31) / 32 <= 65535, "lightning_scan: too many heads or value columns");
@@ -361,6 +688,8 @@ extern "C" int tb_lightning_scan(const LightningArgs* args, int dtype, cudaStrea
     TB_REQUIRE(a.stride >= 2 * a.H * a.dk + a.H * a.dv, "lightning_scan: the projection row is too short");
     TB_REQUIRE(dtype == TB_F32 || dtype == TB_BF16, "lightning_scan: unknown dtype %d", dtype);
     const bool single = a.max_new <= 1;
+    TB_REQUIRE(!a.work || (a.dk <= 128 && a.work_chunks > 0 && (a.dv + VCOLS - 1) / VCOLS <= 65535 && (uintptr_t)a.work % 16 == 0),
+               "lightning_scan: the chunked form takes heads of up to 128 key dimensions (%d)", a.dk);
     if (dtype == TB_F32 ? launch_scan<float>(a, single, stream) : launch_scan<__nv_bfloat16>(a, single, stream)) return 1;
     TB_CHECK_LAUNCH("lightning_scan");
     return 0;

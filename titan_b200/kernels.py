@@ -120,7 +120,8 @@ class LightningArgs(Structure):
     """Arguments of the decayed linear-attention recurrence (csrc/lightning.cu)."""
     _fields_ = [("proj", c_void_p), ("stride", c_int), ("out", c_void_p), ("out_stride", c_int), ("state", c_void_p),
                 ("decay", c_void_p), ("q_start", c_void_p), ("slot_of_seq", c_void_p),
-                ("B", c_int), ("H", c_int), ("dk", c_int), ("dv", c_int), ("max_new", c_int), ("plain", c_int)]
+                ("B", c_int), ("H", c_int), ("dk", c_int), ("dv", c_int), ("max_new", c_int), ("plain", c_int),
+                ("work", c_void_p), ("work_chunks", c_int), ("below", c_int)]
 
 
 class WholeNormArgs(Structure):
@@ -264,6 +265,8 @@ def lib():
         l.tb_gelu_mul_table.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
         l.tb_latent_prep.argtypes = [POINTER(LatentArgs), c_int, c_void_p]
         l.tb_latent_append.argtypes = [c_void_p, c_int, c_int, POINTER(KvView), POINTER(Batch), c_void_p]
+        l.tb_lightning_work.argtypes = [c_int] * 6 + [POINTER(c_int)]
+        l.tb_lightning_work.restype = c_longlong
         l.tb_lightning_scan.argtypes = [POINTER(LightningArgs), c_int, c_void_p]
         l.tb_gated_rmsnorm.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p]
         l.tb_moe_route.argtypes = [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
@@ -303,7 +306,7 @@ def tlib():
         l.tb_gemm_tc_normed.argtypes = [c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
         l.tb_gemm_tc_normed_check.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
         l.tb_gemm_tc_expert_runs.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
-                                             c_int, c_float, c_void_p]
+                                             c_int, c_int, c_float, c_void_p]
         l.tb_gemm_tc_check.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]
         _tlib = l
     return _tlib
@@ -707,6 +710,15 @@ def latent_append(rows: torch.Tensor, cache: KvView, batch: Batch, stream: int) 
     _check(lib().tb_latent_append(rows.data_ptr(), rows.stride(0), dtype_code(rows.dtype), byref(cache), byref(batch), stream))
 
 
+def lightning_work(args: "LightningArgs", tokens: int, device) -> Optional[torch.Tensor]:
+    """Room for the chunked form of the recurrence, named in ``args`` (to be held until it has run); None where the step runs token by token."""
+    chunks = c_int(0)
+    n = int(lib().tb_lightning_work(tokens, args.B, args.H, args.dk, args.dv, args.max_new, byref(chunks)))
+    work = torch.empty(n, dtype=torch.float32, device=device) if n else None
+    args.work, args.work_chunks = _ptr(work), chunks.value
+    return work
+
+
 def lightning_scan(args: "LightningArgs", dtype: torch.dtype, stream: int) -> None:
     _check(lib().tb_lightning_scan(byref(args), dtype_code(dtype), stream))
 
@@ -845,21 +857,21 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, strea
                                   -1 if ordered and not splits else splits, int(gate), float(limit), stream))
 
 
-def gemm_tc_expert_runs(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, w_down: torch.Tensor, y: torch.Tensor, first, stream: int,
-                        gate: int = ACT_SILU, limit: float = 0.0) -> None:
+def gemm_tc_expert_runs(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, w_down: torch.Tensor, y: torch.Tensor, first: torch.Tensor,
+                        stream: int, gate: int = ACT_SILU, limit: float = 0.0) -> None:
     """For every run s of rows [first[s], first[s + 1]): act = swiglu(x . w_gate_up[s]^T), y = act . w_down[s]^T (float32), on the
-    tensor cores, the runs spread over a few side streams (w_gate_up [E, 2F, H] with gate and up rows interleaved, w_down [E, H, F])."""
-    global launch_count
-    _need_cuda(x, w_gate_up, act, w_down, y)
+    tensor cores, one launch a matrix for all runs (w_gate_up [E, 2F, H] with gate and up rows interleaved, w_down [E, H, F];
+    ``first`` int32 on the device, E + 1 ascending row numbers)."""
+    _need_cuda(x, w_gate_up, act, w_down, y, first)
     E, F2, H = w_gate_up.shape
+    P = x.shape[0]
     if (x.dtype != torch.bfloat16 or act.dtype != torch.bfloat16 or y.dtype != torch.float32 or w_down.shape != (E, H, F2 // 2)
-            or not (w_gate_up.is_contiguous() and w_down.is_contiguous()) or len(first) != E + 1 or first[-1] > x.shape[0]
-            or x.stride(1) != 1 or act.stride(1) != 1 or y.stride(1) != 1 or act.shape[1] != F2 // 2):
+            or w_gate_up.dtype != torch.bfloat16 or w_down.dtype != torch.bfloat16
+            or not (w_gate_up.is_contiguous() and w_down.is_contiguous()) or first.dtype != torch.int32 or first.numel() != E + 1 or not first.is_contiguous()
+            or x.stride(1) != 1 or act.stride(1) != 1 or y.stride(1) != 1 or x.shape[1] != H or act.shape != (P, F2 // 2) or y.shape != (P, H)):
         raise KernelError("gemm_tc_expert_runs: shapes or dtypes do not fit")
-    arr = (c_int * len(first))(*first)
-    launch_count += 2 * sum(1 for a, b in zip(first, first[1:]) if b > a) - 1
     _check(tlib().tb_gemm_tc_expert_runs(x.data_ptr(), x.stride(0), w_gate_up.data_ptr(), act.data_ptr(), act.stride(0), w_down.data_ptr(),
-                                        y.data_ptr(), y.stride(0), arr, E, H, F2 // 2, int(gate), float(limit), stream))
+                                        y.data_ptr(), y.stride(0), first.data_ptr(), E, P, H, F2 // 2, int(gate), float(limit), stream))
 
 
 def gemm_tc_normed_accepts(x: torch.Tensor, norm_w: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int,

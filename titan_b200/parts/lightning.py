@@ -76,7 +76,9 @@ class LightningMixer(Mixer):
         a.state, a.decay = group.layer_storage(index).data_ptr(), self.decay.data_ptr()
         a.q_start, a.slot_of_seq = lay.q_start.data_ptr(), lay.slot_of_seq.data_ptr()
         a.B, a.H, a.dk, a.dv, a.max_new = lay.B, H, dk, dv, lay.max_new
+        work = K.lightning_work(a, T, ctx.device)      # (held until the launch has been queued: freed memory is reused in stream order)
         K.lightning_scan(a, proj.dtype, ctx.stream)
+        del work
         y = ctx.empty((T, H * dv))
         K.gated_rmsnorm(o, self.norm_w, proj[:, 2 * H * dk + H * dv:], y, self.out_norm_spec.eps, ctx.stream)
         linear.matmul(y, self.w_o, out, linear.EPI_ADD, ctx)

@@ -86,7 +86,9 @@ class RetentionMixer(Mixer):
         a.state, a.decay = group.layer_storage(index).data_ptr(), self.decay.data_ptr()
         a.q_start, a.slot_of_seq = lay.q_start.data_ptr(), lay.slot_of_seq.data_ptr()
         a.B, a.H, a.dk, a.dv, a.max_new, a.plain = lay.B, H, dk, dv, lay.max_new, 1
+        work = K.lightning_work(a, T, ctx.device)      # (held until the launch has been queued: freed memory is reused in stream order)
         K.lightning_scan(a, torch.float32, ctx.stream)
+        del work
         y = ctx.empty((T, H * dv))
         K.head_norm_gate(o, self.ones, False, gate, y, H, K.GATE_SILU, 1.0, self.eps, ctx.stream)
         linear.matmul(y, self.w_o, out, linear.EPI_ADD, ctx)
