@@ -734,6 +734,149 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     }
 }
 
+// ---------------------------------------------------------------- prompts: one product per run of rows, one launch
+// Run e (an expert) is rows first[e] .. first[e + 1] - 1 of X against matrix e of W [runs][N][K].  The roles, the ring and
+// the two accumulators of gemm_tc_persistent_kernel; only the walk differs: the tiles of all runs follow one another, a run's
+// row tiles fastest, so that the CTAs at work share a panel of weights, and where a run's tiles begin is worked out by every CTA
+// from ``first`` in shared memory (nothing is read on the host).  A row tile's box may reach into the next run, a
+// column tile's into the next matrix: those rows and columns are computed and not stored.
+// Bound by the tensor cores, of whose work a run's last row tile wastes half on average.  8,000 rows of 32
+// runs, 2,048 columns: K = 2,048 with the gate 93 us, K = 1,024 57 us (64 launches on four side streams took 310 us for both, and the
+// host waited for the runs' sizes before them).
+struct RunTiles {
+    const int* first;       // [runs + 1]
+    const int* before;      // [runs + 1] row tiles of the runs before
+    int runs, tiles_n, stride, next_tile, run;
+    __device__ RunTiles(const int* first_, const int* before_, int runs_, int tiles_n_, int worker, int workers)
+        : first(first_), before(before_), runs(runs_), tiles_n(tiles_n_), stride(workers), next_tile(worker), run(0) {}
+    // the tile's run, first row, first column of its matrix; false at the end
+    template <int BN> __device__ bool next(int& e, int& row, int& col) {
+        if (next_tile >= before[runs] * tiles_n) return false;
+        while (next_tile >= before[run + 1] * tiles_n) ++run;
+        const int rows = before[run + 1] - before[run], t = next_tile - before[run] * tiles_n;
+        e = run; row = first[run] + t % rows * BM; col = t / rows * BN;
+        next_tile += stride;
+        return true;
+    }
+};
+
+template <int EPI>
+__global__ void __launch_bounds__(THREADS)
+gemm_tc_runs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcArgs a, const int* first_g, int runs) {
+    constexpr int BN = 256, STAGES = stages_for<BN>();
+    constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, TMEM_COLS = 2 * BN;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem_a = base;
+    uint8_t* smem_b = base + STAGES * A_BYTES;
+    uint64_t* full = (uint64_t*)(base + STAGES * (A_BYTES + B_BYTES));
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;          // [2]
+    uint64_t* acc_empty = acc_full + 2;           // [2]
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    int* first = (int*)(base + STAGES * (A_BYTES + B_BYTES) + 256);       // [runs + 1]
+    int* before = first + runs + 1;                                       // [runs + 1]
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_kb = (a.K + BK - 1) / BK;
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+    pdl_wait();
+    for (int e = threadIdx.x; e <= runs; e += THREADS) first[e] = __ldcg(first_g + e);        // (through L2: see load_l2 of gemm_simt.cu)
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    if (warp == 0) {                              // a warp's running sum over the runs' row tiles, 32 runs at a time
+        int sum = 0;
+        for (int e0 = 0; e0 < runs; e0 += 32) {
+            const int e = e0 + lane;
+            int t = e < runs ? (first[e + 1] - first[e] + BM - 1) / BM : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o *= 2) {
+                const int u = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o) t += u;
+            }
+            if (e < runs) before[e + 1] = sum + t;
+            sum += __shfl_sync(0xffffffffu, t, 31);
+        }
+        if (lane == 0) before[0] = 0;
+    }
+    __syncthreads();
+    RunTiles tiles(first, before, runs, (a.rows_b + BN - 1) / BN, blockIdx.x, gridDim.x);
+    int e, row0, col0;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int it = 0; tiles.next<BN>(e, row0, col0);) {
+                for (int k = 0; k < n_kb; ++k, ++it) {
+                    const int s = it % STAGES, round = it / STAGES;
+                    if (round > 0) mbar_wait(empty + s, (round - 1) & 1, 1);
+                    mbar_expect_tx(full + s, A_BYTES + B_BYTES);
+                    tma_load_2d(smem_a + s * A_BYTES, &map_a, full + s, k * BK, row0);
+                    tma_load_2d(smem_b + s * B_BYTES, &map_b, full + s, k * BK, e * a.rows_b + col0);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = instr_desc(BM, BN);
+            int it = 0;
+            for (int j = 0; tiles.next<BN>(e, row0, col0); ++j) {
+                const int buf = j & 1;
+                if (j >= 2) mbar_wait(acc_empty + buf, ((j >> 1) - 1) & 1, 4);     // the epilogue has drained this buffer
+                tc_fence_after();
+                const uint32_t acc = tmem + buf * BN;
+                for (int i = 0; i < n_kb; ++i, ++it) {
+                    const int s = it % STAGES, round = it / STAGES;
+                    mbar_wait(full + s, round & 1, 2);
+                    tc_fence_after();
+                    const uint64_t da = smem_desc(smem_u32(smem_a + s * A_BYTES));
+                    const uint64_t db = smem_desc(smem_u32(smem_b + s * B_BYTES));
+#pragma unroll
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        tc_mma(acc, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    tc_commit(empty + s);
+                }
+                tc_commit(acc_full + buf);
+            }
+        }
+    } else {
+        const int quarter = warp & 3;
+        TcArgs mine = a;
+        for (int j = 0; tiles.next<BN>(e, row0, col0); ++j) {
+            const int buf = j & 1;
+            mbar_wait(acc_full + buf, (j >> 1) & 1, 3);
+            tc_fence_after();
+            mine.rows_a = first[e + 1];               // rows of the next run are not this tile's
+            const uint32_t taddr = tmem + buf * BN + ((uint32_t)(quarter * 32) << 16);
+            if (row0 + quarter * 32 < mine.rows_a) {
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 32) {
+                    float v[32];
+                    tmem_ld32(taddr + c, v);
+                    epilogue_chunk<EPI, 32>(v, mine, row0 + quarter * 32 + lane, col0 + c, lane);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tbtma::mbar_arrive(acc_empty + buf);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
 // ---------------------------------------------------------------- prompts: pairs of CTAs (cta_group::2)
 // A cluster of two CTAs on neighbouring SMs works on one 256 x 256 tile: each CTA loads 128 rows of X and
 // 128 rows of W per k-block (32 KB instead of the 48 KB a lone CTA needs for 128 x 256, so six stages
@@ -1272,42 +1415,33 @@ extern "C" int tb_gemm_tc(const void* X, const void* W, void* out, int M, int N,
 // Names the buffer of the timeline probe (timeline.cuh); 1 if the library was built with it, 0 if not.
 TB_TIMELINE_SETTER(tb_gemm_tc_timeline)
 
-// The experts of a mixture over rows that a prompt has gathered side by side: for every run s of rows,
-//   act = gate(x . Wgu[s]^T) (activation.h)   then   y = act . Wd[s]^T   (float32),
-// two tensor-core products per run, the runs dealt round robin onto a few side streams so that several experts'
-// products, each too small to fill the machine, run beside one another.  The side streams start after what the
-// caller's stream has queued and the caller's stream goes on after all of them (events; no host wait).
+// The two products of every expert over rows that lie side by side, expert by expert: act = gate(X_e . Wgu_e^T) (rows of Wgu_e
+// interleaved gate, up) and y = act_e . Wd_e^T (float32), one launch each.  ``first`` [runs + 1] is on the device: the experts'
+// first rows, ascending, the last of them at most ``rows``, the rows of X, act and y.
 extern "C" int tb_gemm_tc_expert_runs(const void* X, int ldx, const void* Wgu, void* act, int ld_act, const void* Wd, void* y, int ldy,
-                                      const int* first, int runs, int H, int F, int gate, float limit, cudaStream_t stream) {
-    TB_REQUIRE(first && runs > 0 && H > 0 && F > 0, "gemm_tc_expert_runs: sizes must be positive");
-    constexpr int SIDE = 4;
-    static cudaStream_t side[SIDE];
-    static cudaEvent_t fork_ev, join_ev[SIDE];
-    static bool made = false;
-    if (!made) {
-        for (int i = 0; i < SIDE; ++i) {
-            TB_REQUIRE(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking) == cudaSuccess, "gemm_tc_expert_runs: cannot create a stream");
-            TB_REQUIRE(cudaEventCreateWithFlags(&join_ev[i], cudaEventDisableTiming) == cudaSuccess, "gemm_tc_expert_runs: cannot create an event");
-        }
-        TB_REQUIRE(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming) == cudaSuccess, "gemm_tc_expert_runs: cannot create an event");
-        made = true;
-    }
-    cudaEventRecord(fork_ev, stream);
-    for (int i = 0; i < SIDE; ++i) cudaStreamWaitEvent(side[i], fork_ev, 0);
-    int rc = 0, used = 0;
-    for (int s = 0; s < runs && !rc; ++s) {
-        const int a = first[s], M = first[s + 1] - a;
-        if (M < 0) { tb_set_error("gemm_tc_expert_runs: the runs' first rows must ascend"); rc = 1; break; }
-        if (M == 0) continue;
-        cudaStream_t st = side[used++ % SIDE];
-        rc = tb_gemm_tc_gated((const char*)X + (size_t)a * ldx * 2, (const char*)Wgu + (size_t)s * 2 * F * H * 2, (char*)act + (size_t)a * ld_act * 2,
-                              M, 2 * F, H, ldx, ld_act, TB_EPI_SWIGLU, 0, gate, limit, st);
-        if (!rc) rc = tb_gemm_tc((const char*)act + (size_t)a * ld_act * 2, (const char*)Wd + (size_t)s * H * F * 2, (char*)y + (size_t)a * ldy * 4,
-                                 M, H, F, ld_act, ldy, TB_EPI_F32, 0, st);
-    }
-    for (int i = 0; i < SIDE; ++i) {        // join in every case, also after a refusal: the caller's stream must not run ahead
-        cudaEventRecord(join_ev[i], side[i]);
-        cudaStreamWaitEvent(stream, join_ev[i], 0);
-    }
-    return rc;
+                                      const int* first, int runs, int rows, int H, int F, int gate, float limit, cudaStream_t stream) {
+    TB_REQUIRE(first && runs > 0 && runs <= 1024 && rows > 0 && H > 0 && F > 0, "gemm_tc_expert_runs: sizes (runs=%d rows=%d H=%d F=%d)", runs, rows, H, F);
+    TB_REQUIRE((long long)runs * (2 * F > H ? 2 * F : H) < 2147483647LL, "gemm_tc_expert_runs: too many rows of weights");
+    TB_REQUIRE(gate >= 0 && gate < TB_ACT_KINDS, "gemm_tc_expert_runs: unknown gate %d", gate);
+    if (tb_gemm_tc_check(rows, 2 * F, H, ldx, ld_act, TB_EPI_SWIGLU, X, Wgu, act) || tb_gemm_tc_check(rows, H, F, ld_act, ldy, TB_EPI_F32, act, Wd, y)) return 1;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    constexpr int BN = 256;
+    const size_t smem = 1024 + (size_t)stages_for<BN>() * (BM + BN) * BK * 2 + 256 + 2 * (size_t)(runs + 1) * sizeof(int);
+    auto go = [&](auto kernel, const void* A, int lda, const void* W, void* out, int ldo, int N, int K) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        TB_REQUIRE(e == cudaSuccess, "gemm_tc_expert_runs: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        CUtensorMap ma, mb;
+        if (tb_make_map_bf16(&ma, A, rows, K, lda, BM) || tb_make_map_bf16(&mb, W, (long long)runs * N, K, K, BN)) return 1;
+        TcArgs a = {};
+        a.out = out; a.K = K; a.ldo = ldo; a.rows_a = rows; a.rows_b = N; a.act = gate; a.limit = limit;
+        const long long most = ((long long)rows / BM + runs) * ((N + BN - 1) / BN);       // tiles, if every run ends inside one
+        tb_launch(kernel, dim3((unsigned)(most < sms ? most : sms)), THREADS, smem, stream, ma, mb, a, first, runs);
+        return 0;
+    };
+    if (go(gemm_tc_runs_kernel<TB_EPI_SWIGLU>, X, ldx, Wgu, act, ld_act, 2 * F, H)) return 1;
+    if (go(gemm_tc_runs_kernel<TB_EPI_F32>, act, ld_act, Wd, y, ldy, H, F)) return 1;
+    TB_CHECK_LAUNCH("gemm_tc_expert_runs");
+    return 0;
 }

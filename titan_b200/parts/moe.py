@@ -169,16 +169,15 @@ class MixtureOfExperts(FeedForward):
         on_tensor_cores = (not ctx.layout.all_single and h.dtype == torch.bfloat16 and ctx.options.get("gemm", "fast") != "plain"
                            and P >= int(ctx.options.get("moe_tensor_pairs", 512)))
         if on_tensor_cores:
-            # A prompt: every expert's rows side by side, one tensor-core product per expert and matrix.  How many rows
-            # each expert got is read on the host (one small copy a layer); steps of single tokens never come here,
-            # so they stay free of host reads and are captured as graphs.
-            offsets = plan.offsets.tolist()[:E + 1]                      # the rows of experts without matrices lie behind the last run
+            # A prompt: every expert's rows side by side, then one tensor-core launch a matrix for all experts, which reads how
+            # many rows each got on the device.
             xs = ctx.empty((P, H))
             K.moe_gather(h, plan, top, xs, ctx.stream)
-            if (K.gemm_tc_accepts(xs[:1], self.w_gate_up[0], act[:1], linear.EPI_SWIGLU)
-                    and K.gemm_tc_accepts(act[:1], self.w_down[0], y[:1], linear.EPI_F32)):
-                K.gemm_tc_expert_runs(xs, self.w_gate_up, act, self.w_down, y, offsets, ctx.stream, **gk)
+            if (E <= 1024 and K.gemm_tc_accepts(xs, self.w_gate_up[0], act, linear.EPI_SWIGLU)
+                    and K.gemm_tc_accepts(act, self.w_down[0], y, linear.EPI_F32)):
+                K.gemm_tc_expert_runs(xs, self.w_gate_up, act, self.w_down, y, plan.offsets[:E + 1], ctx.stream, **gk)
             else:
+                offsets = plan.offsets.tolist()[:E + 1]              # the rows of experts without matrices lie behind the last run
                 for e in range(E):
                     a, b = offsets[e], offsets[e + 1]
                     if b > a:
