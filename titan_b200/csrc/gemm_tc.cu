@@ -243,6 +243,49 @@ __device__ __forceinline__ void epilogue_rows(const float* val, float* tile, con
     }
 }
 
+// Swap mode: four neighbouring outputs n0 .. n0 + 3 of token m.
+template <int EPI>
+__device__ __forceinline__ void swap_four_out(float4 f, const TcArgs& a, int m, int n0) {
+    if (n0 >= a.rows_a) return;
+    const bool whole = n0 + 4 <= a.rows_a;
+    if (EPI == TB_EPI_SWIGLU) {
+        __nv_bfloat16* o = (__nv_bfloat16*)a.out + (size_t)m * a.ldo + n0 / 2;
+        if (whole) *reinterpret_cast<uint32_t*>(o) = pack_bf16(silu_mul(f.x, f.y), silu_mul(f.z, f.w));
+        else if (n0 + 1 < a.rows_a) o[0] = __float2bfloat16_rn(silu_mul(f.x, f.y));
+        return;
+    }
+    const float v[4] = {f.x, f.y, f.z, f.w};
+    if (EPI == TB_EPI_STORE) {
+        if (a.act != TB_UNARY_NONE) {
+            f.x = tb_unary(a.act, f.x); f.y = tb_unary(a.act, f.y); f.z = tb_unary(a.act, f.z); f.w = tb_unary(a.act, f.w);
+        }
+        __nv_bfloat16* o = (__nv_bfloat16*)a.out + (size_t)m * a.ldo + n0;
+        if (whole) {
+            *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
+        } else {
+            for (int j = 0; j < 4; ++j) if (n0 + j < a.rows_a) o[j] = __float2bfloat16_rn(tb_unary(a.act, v[j]));
+        }
+        return;
+    }
+    float* o = (float*)a.out + (size_t)m * a.ldo + n0;
+    if (whole && EPI == TB_EPI_F32) {
+        *reinterpret_cast<float4*>(o) = f;
+    } else if (whole && a.atomic) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(f.x), "f"(f.y), "f"(f.z), "f"(f.w) : "memory");
+    } else if (whole) {
+        float4 old = *reinterpret_cast<const float4*>(o);
+        old.x += f.x; old.y += f.y; old.z += f.z; old.w += f.w;
+        *reinterpret_cast<float4*>(o) = old;
+    } else {
+        for (int j = 0; j < 4; ++j) {
+            if (n0 + j >= a.rows_a) continue;
+            if (EPI == TB_EPI_F32) o[j] = v[j];
+            else if (a.atomic) atomicAdd(o + j, v[j]);
+            else o[j] += v[j];
+        }
+    }
+}
+
 // Swap mode: the tile as the epilogue warps have left it in shared memory, ``part`` [token][row of the tile = output
 // column], goes out along the output's rows: a thread takes four neighbouring columns of a token (sixteen for SwiGLU:
 // eight outputs), so a warp writes 512 contiguous bytes with one instruction where a thread that holds one column of
@@ -271,54 +314,24 @@ __device__ __forceinline__ void swap_tile_out(const float* part, const TcArgs& a
         for (int item = t; item < BN * 32; item += 128) {
             const int m = item >> 5, n0 = tile_a * BM + (item & 31) * 4;
             if (m >= a.rows_b || n0 >= a.rows_a) continue;
-            float4 f = *reinterpret_cast<const float4*>(part + m * BM + (item & 31) * 4);
-            if (EPI == TB_EPI_STORE && a.act != TB_UNARY_NONE) {
-                f.x = tb_unary(a.act, f.x); f.y = tb_unary(a.act, f.y); f.z = tb_unary(a.act, f.z); f.w = tb_unary(a.act, f.w);
-            }
-            const bool whole = n0 + 4 <= a.rows_a;
-            if (EPI == TB_EPI_STORE) {
-                __nv_bfloat16* o = (__nv_bfloat16*)a.out + (size_t)m * a.ldo + n0;
-                if (whole) {
-                    *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
-                } else {
-                    const float v[4] = {f.x, f.y, f.z, f.w};
-                    for (int j = 0; j < 4; ++j) if (n0 + j < a.rows_a) o[j] = __float2bfloat16_rn(v[j]);
-                }
-            } else {
-                float* o = (float*)a.out + (size_t)m * a.ldo + n0;
-                if (whole && EPI == TB_EPI_F32) {
-                    *reinterpret_cast<float4*>(o) = f;
-                } else if (whole && a.atomic) {
-                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(f.x), "f"(f.y), "f"(f.z), "f"(f.w) : "memory");
-                } else if (whole) {
-                    float4 old = *reinterpret_cast<const float4*>(o);
-                    old.x += f.x; old.y += f.y; old.z += f.z; old.w += f.w;
-                    *reinterpret_cast<float4*>(o) = old;
-                } else {
-                    const float v[4] = {f.x, f.y, f.z, f.w};
-                    for (int j = 0; j < 4; ++j) {
-                        if (n0 + j >= a.rows_a) continue;
-                        if (EPI == TB_EPI_F32) o[j] = v[j];
-                        else if (a.atomic) atomicAdd(o + j, v[j]);
-                        else o[j] += v[j];
-                    }
-                }
-            }
+            swap_four_out<EPI>(*reinterpret_cast<const float4*>(part + m * BM + (item & 31) * 4), a, m, n0);
         }
     }
 }
 
-// ORDERED (swap mode, ADD epilogue): the K slices of a tile are the CTAs of one thread-block cluster.  Each leaves its
+// ORDERED (swap mode): the K slices of a tile are the CTAs of one thread-block cluster.  Each leaves its
 // partial tile in its own shared memory; after a cluster barrier every CTA adds up a share of the tile's elements
 // from all slices, in slice order, through distributed shared memory, and adds the sum to the output.  An element is
 // then written once, by one CTA, from a sum whose order is fixed: the same inputs give the same bits on every run,
-// which float32 reductions that meet at L2 in the order they arrive do not.
+// which float32 reductions that meet at L2 in the order they arrive do not.  The other epilogues, which need an element's
+// whole sum at once, take their slices this way only: with a tile per CTA a product of few columns leaves most SMs
+// idle (44 tiles of 5,632 gate and up columns: a step of
+// twelve such layers for one sequence 313 -> 289 us with slices; eight rows of 2,048 columns, K = 2,048: 12.0 -> 5.2 us).
 template <int BN, int EPI, bool SWAP, bool NORMED = false, bool ORDERED = false>
 __global__ void __launch_bounds__(THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcArgs a) {
     static_assert(!NORMED || (SWAP && BN <= 32), "the folded norm is for decode tiles (swap mode, at most 32 rows of activations)");
     static_assert(SWAP, "this kernel takes the decode products (weights on the 128-row side); prompts have the persistent and the pair kernel");
-    static_assert(!ORDERED || EPI == TB_EPI_ADD, "slices in a fixed order: the ADD epilogue");
     constexpr int STAGES = stages_of<BN, EPI, SWAP>();
     constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
     constexpr uint32_t TMEM_COLS = tmem_cols_for<BN>();
@@ -478,7 +491,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 asm volatile("bar.sync 2, 128;" ::: "memory");
                 if (warp == 2 && lane < BN) {
                     const float total = norm_sh[lane] + norm_sh[BN + lane] + norm_sh[2 * BN + lane] + norm_sh[3 * BN + lane];
-                    if (a.sumsq_out) {                        // K slices: the consumer of the sums scales (a store, not an atomic: a fixed order of addition)
+                    if (ORDERED && EPI != TB_EPI_ADD) {       // this slice's part: the cluster adds them up
+                        norm_sh[5 * BN + lane] = total;
+                        norm_sh[4 * BN + lane] = 1.f;
+                    } else if (a.sumsq_out) {                 // K slices: the consumer of the sums scales (a store, not an atomic: a fixed order of addition)
                         if (tile_a == 0 && lane < a.rows_b) a.sumsq_out[blockIdx.z * 32 + lane] = total;
                         norm_sh[4 * BN + lane] = 1.f;
                     } else {
@@ -533,18 +549,40 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // every thread of every CTA of the cluster: parts written -> summed -> may leave
         __syncwarp();
         tbtma::cluster_sync();
-        const int n = (int)gridDim.z, total = a.rows_b * BM;          // tokens x rows of the tile (swap mode has one tile of tokens)
-        const int per = (total + n - 1) / n, first = (int)tbtma::cluster_rank() * per, last = min(total, first + per);
-        const float* part = reinterpret_cast<const float*>(smem_a);
-        for (int idx = first + (int)threadIdx.x; idx < last; idx += THREADS) {
-            float v[16];
-#pragma unroll
-            for (int r = 0; r < 16; ++r) v[r] = r < n ? tbtma::ld_cluster_f32(tbtma::cluster_addr(part + idx, r)) : 0.f;     // all loads first
-            float sum = 0.f;
-#pragma unroll
-            for (int r = 0; r < 16; ++r) sum += v[r];                  // in the order of the slices
-            const int m = idx / BM, row = tile_a * BM + idx % BM;
-            if (row < a.rows_a) atomicAdd((float*)a.out + (size_t)m * a.ldo + row, sum);      // the element's only writer in this launch
+        if (EPI != TB_EPI_ADD) {
+            // four neighbouring rows of the tile (outputs) of a token at a time
+            const int n = (int)gridDim.z, units = a.rows_b * (BM / 4), per = (units + n - 1) / n;
+            const int first = (int)tbtma::cluster_rank() * per, last = min(units, first + per);
+            const float* part = reinterpret_cast<const float*>(smem_a);
+            for (int u = first + (int)threadIdx.x; u < last; u += THREADS) {
+                const int m = u / (BM / 4), c = u % (BM / 4) * 4, row = tile_a * BM + c;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                float ss = 0.f;
+                for (int r = 0; r < n; ++r) {                          // in the order of the slices
+                    const float4 p = tbtma::ld_cluster_f32x4(tbtma::cluster_addr(part + m * BM + c, r));
+                    v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+                    if (NORMED) ss += tbtma::ld_cluster_f32(tbtma::cluster_addr(norm_sh + 5 * BN + m, r));
+                }
+                if (NORMED) {
+                    const float scale = 1.0f / sqrtf(ss / (float)a.K + a.norm_eps);
+                    v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
+                }
+                swap_four_out<EPI>(v, a, m, row);
+            }
+        } else {
+            const int n = (int)gridDim.z, total = a.rows_b * BM;          // tokens x rows of the tile (swap mode has one tile of tokens)
+            const int per = (total + n - 1) / n, first = (int)tbtma::cluster_rank() * per, last = min(total, first + per);
+            const float* part = reinterpret_cast<const float*>(smem_a);
+            for (int idx = first + (int)threadIdx.x; idx < last; idx += THREADS) {
+                float v[16];
+    #pragma unroll
+                for (int r = 0; r < 16; ++r) v[r] = r < n ? tbtma::ld_cluster_f32(tbtma::cluster_addr(part + idx, r)) : 0.f;     // all loads first
+                float sum = 0.f;
+    #pragma unroll
+                for (int r = 0; r < 16; ++r) sum += v[r];                  // in the order of the slices
+                const int m = idx / BM, row = tile_a * BM + idx % BM;
+                if (row < a.rows_a) atomicAdd((float*)a.out + (size_t)m * a.ldo + row, sum);      // the element's only writer in this launch
+            }
         }
         __syncwarp();
         tbtma::cluster_sync();
@@ -1036,12 +1074,12 @@ int launch_tc_normed(const CUtensorMap& ma, const TcArgs& a, dim3 grid, cudaStre
     return 0;
 }
 
-// Swap mode, ADD epilogue, the K slices of a tile as one cluster (grid.z CTAs) that adds them up in slice order.
-template <int BN, bool NORMED>
+// Swap mode, the K slices of a tile as one cluster (grid.z CTAs) that adds them up in slice order.
+template <int BN, bool NORMED, int EPI = TB_EPI_ADD>
 int launch_tc_ordered(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, dim3 grid, cudaStream_t stream) {
     static bool configured = false;
-    constexpr size_t smem = smem_for<BN, true, stages_of<BN, TB_EPI_ADD, true>()>();
-    auto kernel = gemm_tc_kernel<BN, TB_EPI_ADD, true, NORMED, true>;
+    constexpr size_t smem = smem_for<BN, true, stages_of<BN, EPI, true>()>();
+    auto kernel = gemm_tc_kernel<BN, EPI, true, NORMED, true>;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1052,6 +1090,17 @@ int launch_tc_ordered(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs
     const cudaError_t e = tb_launch_cluster_z(kernel, grid, THREADS, smem, stream, (int)grid.z, ma, mb, a);
     TB_REQUIRE(e == cudaSuccess, "gemm_tc: the launch of clusters of %d K slices failed: %s", (int)grid.z, cudaGetErrorString(e));
     return 0;
+}
+template <int BN>
+int launch_tc_sliced(int epi, const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, dim3 grid, cudaStream_t stream) {
+    switch (epi) {
+        case TB_EPI_STORE: return launch_tc_ordered<BN, false, TB_EPI_STORE>(ma, mb, a, grid, stream);
+        case TB_EPI_F32: return launch_tc_ordered<BN, false, TB_EPI_F32>(ma, mb, a, grid, stream);
+        case TB_EPI_SWIGLU: return launch_tc_ordered<BN, false, TB_EPI_SWIGLU>(ma, mb, a, grid, stream);
+        case TB_EPI_ADD: return launch_tc_ordered<BN, false>(ma, mb, a, grid, stream);
+    }
+    tb_set_error("gemm_tc: unknown epilogue %d", epi);
+    return 1;
 }
 // How many clusters of ``size`` CTAs of this kernel the device holds at once (0: it places none).  Clusters are placed
 // as wholes inside one part of the chip, so this is less than the CTAs it holds divided by the size.
@@ -1095,6 +1144,15 @@ int ordered_fit(int bn, bool normed, int tiles, int wanted) {
     return 1;
 }
 
+// K slices of an epilogue that needs whole sums (all but ADD), the tiles of at most 64 rows: 1 or a cluster's size.  As many as give every
+// SM a CTA, at least four k-blocks each, at most four (measured at most 1 / 2 / 3 / 4 / 6 / 8: a decode step of twelve layers of
+// width 1,024 314 / 290 / 288 / 289 / 292 / 291 us, of four layers with experts of width 2,048 696 / 670 / 661 / 653 / 652 / 652).
+int whole_slices(int bn, bool normed, int tiles, int kb, int sm_count) {
+    int s = sm_count / tiles;
+    if (s > kb / 4) s = kb / 4;
+    if (s > 4) s = 4;
+    return s < 2 || bn > 64 ? 1 : ordered_fit(bn, normed, tiles, s);
+}
 template <int BN, int EPI>
 int launch_persistent_epi(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, dim3 grid, cudaStream_t stream) {
     static bool configured = false;
@@ -1247,6 +1305,8 @@ static int normed_slices(int N, int K, int epi, int M = 1, bool ordered = false)
         s = s < 1 ? 1 : (s > max_s ? max_s : s);
         s = s > 16 ? 16 : s;
         if (ordered) s = ordered_fit(M <= 16 ? 16 : 32, true, tiles, s);
+    } else {
+        s = whole_slices(M <= 16 ? 16 : 32, true, tiles, kb, sm_count);
     }
     const int per = (kb + s - 1) / s;
     return (kb + per - 1) / per;
@@ -1271,13 +1331,15 @@ extern "C" int tb_gemm_tc_normed(const float* xf, int ldxf, const float* norm_w,
     TcArgs a;
     a.out = out; a.rows_a = N; a.rows_b = M; a.K = K; a.ldo = ldo; a.tiles_m = a.tiles_n = 0; a.tail_split = 1;
     a.k_blocks_per_split = (kb + s - 1) / s;
-    a.atomic = s > 1;
+    a.atomic = s > 1 && epi == TB_EPI_ADD;
     a.xf = xf; a.ldxf = ldxf; a.norm_w = norm_w; a.sumsq_out = sumsq_out; a.norm_eps = eps; a.act = 0; a.limit = 0.f;
     CUtensorMap ma;
     if (tb_make_map_bf16(&ma, W, N, K, K, BM)) return 1;
     dim3 grid(1, tiles, s);
     int rc;
-    if (ordered && epi == TB_EPI_ADD && s > 1) {
+    if (epi == TB_EPI_SWIGLU && s > 1) {
+        rc = M <= 16 ? launch_tc_ordered<16, true, TB_EPI_SWIGLU>(ma, ma, a, grid, stream) : launch_tc_ordered<32, true, TB_EPI_SWIGLU>(ma, ma, a, grid, stream);
+    } else if (ordered && epi == TB_EPI_ADD && s > 1) {
         TB_REQUIRE(ordered_clusters_for(M <= 16 ? 16 : 32, true, s) > 0, "gemm_tc_normed: this device places no cluster of %d K slices", s);
         a.atomic = 0;
         rc = M <= 16 ? launch_tc_ordered<16, true>(ma, ma, a, grid, stream) : launch_tc_ordered<32, true>(ma, ma, a, grid, stream);
@@ -1380,14 +1442,22 @@ extern "C" int tb_gemm_tc_gated(const void* X, const void* W, void* out, int M, 
             const int max_s = kb / 4 > 0 ? kb / 4 : 1;              // at least four 64-wide blocks per slice
             s = s < 1 ? 1 : (s > max_s ? max_s : s);
             if (ordered) s = ordered_fit(bn, false, tiles, s);
+        } else {
+            s = whole_slices(bn, false, tiles, kb, sm_count);
         }
         a.k_blocks_per_split = (kb + s - 1) / s;
         s = (kb + a.k_blocks_per_split - 1) / a.k_blocks_per_split;  // no empty slice
-        a.atomic = s > 1 && !ordered;
+        a.atomic = s > 1 && !ordered && epi == TB_EPI_ADD;
         if (tb_make_map_bf16(&ma, W, N, K, K, BM) || tb_make_map_bf16(&mb, X, M, K, ldx, bn)) return 1;
         dim3 grid(1, tiles, s);
         TB_REQUIRE(tiles <= 65535, "gemm_tc: N=%d is too large for one launch", N);
-        if (ordered && epi == TB_EPI_ADD && s > 1) {
+        if (epi != TB_EPI_ADD && s > 1) {
+            switch (bn) {
+                case 16: rc = launch_tc_sliced<16>(epi, ma, mb, a, grid, stream); break;
+                case 32: rc = launch_tc_sliced<32>(epi, ma, mb, a, grid, stream); break;
+                default: rc = launch_tc_sliced<64>(epi, ma, mb, a, grid, stream); break;
+            }
+        } else if (ordered && epi == TB_EPI_ADD && s > 1) {
             switch (bn) {
                 case 16: rc = launch_tc_ordered<16, false>(ma, mb, a, grid, stream); break;
                 case 32: rc = launch_tc_ordered<32, false>(ma, mb, a, grid, stream); break;

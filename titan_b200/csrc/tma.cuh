@@ -95,6 +95,11 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t cluster_addr_) {      /
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr_) : "memory");
     return v;
 }
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t cluster_addr_) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr_) : "memory");
+    return v;
+}
 // A value into another CTA's shared memory that counts its four bytes on a barrier of THAT CTA when it has landed:
 // the receiver expects the bytes of all its senders and needs no arrival after them.
 __device__ __forceinline__ void st_async_f32(uint32_t cluster_addr_, float v, uint32_t cluster_bar_addr) {
