@@ -1,0 +1,231 @@
+"""Kernels that split or regroup their sums, at the edges of their tiles, runs and chunks: products of any number of rows in one
+order of sums, float32 attention of prompts in tiles and of decode steps with lanes across a key's row, the decayed linear
+recurrence in chunks, the experts' products in one launch, and decode products cut along K."""
+import itertools
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import Paged, layout_for
+
+pytestmark = pytest.mark.gpu
+EPS32 = 2.0 ** -24
+
+
+@pytest.fixture(scope="module")
+def K():
+    from titan_b200 import kernels
+    kernels.lib()
+    return kernels
+
+
+def stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,Kd", [(1, 1), (7, 31), (8, 32), (9, 36), (64, 3104), (66, 200), (130, 4100), (1210, 72)])
+def test_a_rows_product_is_the_same_bits_beside_any_other_rows(K, dtype, N, Kd):
+    """Rows in numbers on both sides of every border (one to eight a block, the few-rows kernel's end at 64, tiles of 64, the wider tiles)."""
+    g = torch.Generator().manual_seed(N + Kd)
+    M = 1300 if N > 1000 else 200
+    x = torch.randn(M, Kd, generator=g).to(dtype).cuda()
+    w = torch.randn(N, Kd, generator=g).to(dtype).cuda()
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    bound = (16 + 1 + math.ceil(Kd / 32) + 2) * EPS32              # sixteen fused products, their sum with the other sixteen, a sum a run
+    first = torch.empty(M, N, device="cuda")
+    K.gemm_simt(x, w, first, K.EPI_F32, stream())
+    assert bool(((first.double() - want).abs() <= bound * size + 1e-30).all())
+    for m in (1, 2, 3, 4, 5, 8, 9, 33, 64, 65, 129):
+        out = torch.full((m, N), 7.0, device="cuda")
+        K.gemm_simt(x[:m], w, out, K.EPI_F32, stream())
+        assert torch.equal(out, first[:m]), m
+        K.gemm_rows(x[:m], w, out, K.EPI_F32, stream())
+        assert torch.equal(out, first[:m]), m
+        K.gemm_simt(x[:m], w, out.zero_().add_(1.0), K.EPI_ADD, stream())
+        assert torch.equal(out, first[:m] + 1.0), m
+
+
+def attend64(q, k, v, pos, scale, window):
+    """One query [nh, hd] over the keys [n, nkv, hd] of its sequence in 64 bits."""
+    lo = max(0, pos - window + 1) if window else 0
+    group = q.shape[0] // k.shape[1]
+    kk, vv = (t[lo:pos + 1].double().repeat_interleave(group, 1) for t in (k, v))
+    return torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q.double(), kk) * scale, -1), vv)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(4, 2, 64, 0), (3, 1, 8, 0), (8, 8, 72, 70), (4, 4, 128, 1), (16, 1, 24, 130)])
+def test_float32_prompts_in_tiles(K, nh, nkv, hd, window):
+    """Runs on both sides of 64 queries, fresh and going on from the cache; a value that is not finite reaches those who see it and no one else."""
+    g = torch.Generator().manual_seed(hd)
+    slots, starts, news = [3, 0, 2, 4], [0, 100, 63, 1], [1, 64, 65, 129]
+    lens = [a + n for a, n in zip(starts, news)]
+    paged = Paged(K, slots, lens, nkv, hd, torch.float32)
+    ks, vs = ([torch.randn(n, nkv, hd, generator=g) for n in lens] for _ in range(2))
+    q = torch.randn(sum(news), nh, hd, generator=g)
+    lay = layout_for(slots, starts, news)
+
+    def run():
+        for i, s in enumerate(slots):
+            for p in range(starts[i]):
+                paged.put(s, p, ks[i][p], vs[i][p])
+        rows = torch.cat([torch.cat([k[a:].reshape(-1, nkv * hd), v[a:].reshape(-1, nkv * hd)], 1) for k, v, a in zip(ks, vs, starts)]).cuda()
+        qd, out = q.reshape(-1, nh * hd).cuda(), torch.empty(sum(news), nh * hd, device="cuda")
+        a = K.AttnArgs()
+        a.q, a.q_stride, a.kv_new, a.kv_stride, a.out, a.out_stride = qd.data_ptr(), nh * hd, rows.data_ptr(), 2 * nkv * hd, out.data_ptr(), nh * hd
+        a.cache, a.batch, a.nh, a.nkv, a.hd, a.window, a.scale = paged.view, lay.c_struct(), nh, nkv, hd, window, 0.3
+        K.attn_prefill(a, torch.float32, stream())
+        return out.view(-1, nh, hd).cpu()
+
+    got, at = run(), 0
+    for i in range(4):
+        for j in range(news[i]):
+            want = attend64(q[at + j], ks[i], vs[i], starts[i] + j, 0.3, window)
+            assert float((got[at + j].double() - want).norm() / want.norm()) < 4e-6, (i, j)
+        at += news[i]
+    vs[3][40, 0, 0] = math.inf
+    again, first = run(), sum(news[:3])
+    blind = [j for j in range(news[3]) if starts[3] + j < 40 or (window and starts[3] + j >= 40 + window)]
+    assert torch.equal(again[:first], got[:first]) and torch.equal(again[first:][blind], got[first:][blind])
+    seeing = [j for j in range(news[3]) if j not in blind]
+    assert not bool(torch.isfinite(again[first:][seeing][:, 0, 0]).any())
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 4e-6), (torch.bfloat16, 6e-3)])
+@pytest.mark.parametrize("nh,nkv,hd,window,chunk", [(2, 2, 8, 0, 32), (16, 8, 64, 0, 256), (9, 1, 40, 50, 64), (6, 2, 128, 0, 128), (4, 4, 16, 3, 32)])
+def test_decode_with_lanes_across_a_row(K, dtype, tol, nh, nkv, hd, window, chunk):
+    g = torch.Generator().manual_seed(hd + nh)
+    slots, lens = [2, 0, 5, 1], [1, chunk, chunk + 1, 3 * chunk - 5]
+    paged = Paged(K, slots, lens, nkv, hd, dtype)
+    ks, vs = ([torch.randn(n, nkv, hd, generator=g).to(dtype) for n in lens] for _ in range(2))
+    for i, s in enumerate(slots):
+        for p in range(lens[i]):
+            paged.put(s, p, ks[i][p], vs[i][p])
+    q = torch.randn(4, nh, hd, generator=g).to(dtype)
+    lay = layout_for(slots, [n - 1 for n in lens], [1] * 4)
+    qd, out = q.reshape(4, -1).cuda(), torch.empty(4, nh * hd, dtype=dtype, device="cuda")
+    splits = -(-max(lens) // chunk)
+    scratch = torch.full((4 * nh * splits * (hd + 2),), math.nan, device="cuda")
+    a = K.AttnArgs()
+    a.q, a.q_stride, a.out, a.out_stride = qd.data_ptr(), nh * hd, out.data_ptr(), nh * hd
+    a.cache, a.batch, a.nh, a.nkv, a.hd, a.window, a.scale = paged.view, lay.c_struct(), nh, nkv, hd, window, 0.3
+    a.chunk, a.n_splits, a.scratch = chunk, splits, scratch.data_ptr()
+    K.attn_decode(a, dtype, stream())
+    for i in range(4):
+        want = attend64(q[i], ks[i], vs[i], lens[i] - 1, 0.3, window)
+        assert float((out[i].cpu().double().view(nh, hd) - want).norm() / want.norm()) < tol, i
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dk,dv,plain", [(8, 16, 0), (64, 17, 0), (65, 40, 1), (128, 33, 0)])
+def test_recurrence_in_chunks(K, dtype, dk, dv, plain):
+    """Runs on both sides of a chunk and of the border between the two forms, from a state that is not zero; the short runs beside long
+    ones are the bits they are alone; a value that is not finite reaches no earlier token."""
+    g = torch.Generator().manual_seed(dk)
+    lens, H, decay = [31, 32, 64, 5, 65, 130], 2, [0.9, 1.0]
+    T, stride = sum(lens), 2 * H * dk + 2 * H * dv
+    proj = torch.randn(T, stride, generator=g).to(dtype)
+    state = torch.randn(len(lens) + 1, H, dk, dv, generator=g)
+    slots = torch.tensor([3, 0, 6, 1, 5, 2], dtype=torch.int32)
+
+    def run(rows, which):
+        n = [lens[i] for i in which]
+        starts = torch.tensor([0] + list(itertools.accumulate(n)), dtype=torch.int32).cuda()
+        p, st, sl, dec = rows.cuda(), state.cuda().clone(), slots[list(which)].cuda(), torch.tensor(decay, device="cuda")
+        out = torch.empty(sum(n), H * dv, device="cuda")
+        a = K.LightningArgs()
+        a.proj, a.stride, a.out, a.out_stride = p.data_ptr(), stride, out.data_ptr(), H * dv
+        a.state, a.decay, a.q_start, a.slot_of_seq = st.data_ptr(), dec.data_ptr(), starts.data_ptr(), sl.data_ptr()
+        a.B, a.H, a.dk, a.dv, a.max_new, a.plain = len(n), H, dk, dv, max(n), plain
+        work = K.lightning_work(a, sum(n), "cuda")
+        assert (work is not None) == (max(n) >= 32)
+        K.lightning_scan(a, dtype, stream())
+        return out.cpu(), st.cpu()
+
+    out, st = run(proj, range(6))
+    f = (lambda z: z) if plain else (lambda z: z * torch.sigmoid(z))
+    at = 0
+    for i, n in enumerate(lens):
+        r = f(proj[at:at + n].double())
+        q, k = (r[:, c * H * dk:(c + 1) * H * dk].view(n, H, dk) for c in (0, 1))
+        v = r[:, 2 * H * dk:2 * H * dk + H * dv].view(n, H, dv)
+        S, want = state[slots[i]].double(), []
+        for t in range(n):
+            S = S * torch.tensor(decay).double()[:, None, None] + k[t][:, :, None] * v[t][:, None, :]
+            want.append(torch.einsum("hkv,hk->hv", S, q[t]).reshape(-1))
+        want = torch.stack(want)
+        # sums of at most dk + 64 float32 products and powers of the decay rounded once: far below 1e-5 of the result's norm
+        assert float((out[at:at + n].double() - want).norm() / want.norm()) < 1e-5, n
+        assert float((st[slots[i]].double() - S).norm() / S.norm()) < 1e-5, n
+        at += n
+    alone, st_alone = run(proj[sum(lens[:3]):sum(lens[:4])], [3])
+    assert torch.equal(alone, out[sum(lens[:3]):sum(lens[:4])]) and torch.equal(st_alone[1], st[1])
+    spoiled, place = proj.clone(), sum(lens[:5]) + 70                                     # inside the longest run's second chunk
+    spoiled[place, 2 * H * dk] = math.inf
+    bad, _ = run(spoiled, range(6))
+    assert torch.equal(bad[:sum(lens[:5]) + 64], out[:sum(lens[:5]) + 64])
+    assert float((bad[:place] - out[:place]).abs().max()) < 1e-4 * float(out.abs().max()) and not bool(torch.isfinite(bad[place:, 0]).any())
+
+
+@pytest.mark.parametrize("H,F,counts", [(64, 24, [1, 0, 127, 128, 129]), (264, 40, [0, 300, 0]), (2048, 136, [5, 260, 1, 0, 31, 33])])
+def test_experts_products_in_one_launch(K, H, F, counts):
+    """Empty runs, runs on both sides of a row tile, columns that end inside a tile; rows behind the last run are not touched."""
+    g = torch.Generator().manual_seed(H)
+    E, P = len(counts), sum(counts) + 9
+    x = torch.randn(P, H, generator=g).to(torch.bfloat16).cuda()
+    wgu = (torch.randn(E, 2 * F, H, generator=g) * 0.1).to(torch.bfloat16).cuda()
+    wd = (torch.randn(E, H, F, generator=g) * 0.1).to(torch.bfloat16).cuda()
+    first = torch.tensor([0] + list(itertools.accumulate(counts)), dtype=torch.int32).cuda()
+    act, y = torch.full((P, F), 7.0, dtype=torch.bfloat16, device="cuda"), torch.full((P, H), 7.0, device="cuda")
+    K.gemm_tc_expert_runs(x, wgu, act, wd, y, first, stream())
+    at = 0
+    for e, n in enumerate(counts):
+        if n:
+            z = x[at:at + n].double() @ wgu[e].double().t()
+            want = z[:, 0::2] * torch.sigmoid(z[:, 0::2]) * z[:, 1::2]
+            assert float((act[at:at + n].double() - want).norm() / want.norm()) < 4e-3                # one bfloat16 rounding
+            want = act[at:at + n].double() @ wd[e].double().t()
+            assert float((y[at:at + n].double() - want).norm() / want.norm()) < 2e-6
+        at += n
+    assert bool((act[at:] == 7.0).all()) and bool((y[at:] == 7.0).all())
+    with pytest.raises(K.KernelError):
+        K.gemm_tc_expert_runs(x, wgu, act, wd, y, first[:-1], stream())
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 65])
+@pytest.mark.parametrize("N,Kd", [(130, 512), (2048, 2048), (5632, 1032), (4, 1024)])
+def test_decode_products_that_need_whole_sums(K, M, N, Kd):
+    """Every epilogue but the adding one, K cut into slices of a cluster (and not: rows beyond 64); the same bits on every run."""
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, Kd, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, Kd, generator=g) * 0.05).to(torch.bfloat16).cuda()
+    z = x.double() @ w.double().t()
+    gated = z[:, 0::2] * torch.sigmoid(z[:, 0::2]) * z[:, 1::2]
+    wide = -(-N // 8) * 8
+    for epi, want, dt, tol in ((K.EPI_STORE, z, torch.bfloat16, 4e-3), (K.EPI_F32, z, torch.float32, 3e-6), (K.EPI_SWIGLU, gated, torch.bfloat16, 4e-3)):
+        out = torch.full((M, wide), 7.0, dtype=dt, device="cuda")
+        view = out[:, :want.shape[1]]
+        K.gemm_tc(x, w, view, epi, stream())
+        assert float((view.double() - want).norm() / want.norm()) < tol
+        assert bool((out[:, want.shape[1]:] == 7.0).all())
+        again = torch.empty_like(out)
+        K.gemm_tc(x, w, again[:, :want.shape[1]], epi, stream())
+        assert torch.equal(again[:, :want.shape[1]], view)
+    if M <= 32:
+        xf, norm = torch.randn(M, Kd, generator=g).cuda(), (1 + 0.1 * torch.randn(Kd, generator=g)).cuda()
+        h = (xf * norm).to(torch.bfloat16).double() / torch.sqrt((xf.double() ** 2).mean(1, keepdim=True) + 1e-6)
+        z = h @ w.double().t()
+        want = z[:, 0::2] * torch.sigmoid(z[:, 0::2]) * z[:, 1::2]
+        out = torch.empty(M, wide, dtype=torch.bfloat16, device="cuda")[:, :N // 2]
+        if K.gemm_tc_normed_accepts(xf, norm, w, out, K.EPI_SWIGLU, None):
+            K.gemm_tc_normed(xf, norm, 1e-6, w, out, K.EPI_SWIGLU, stream())
+            assert float((out.double() - want).norm() / want.norm()) < 4e-3
+
+
+def test_a_row_of_router_logits_that_are_not_numbers_chooses_experts_there_are(K):
+    z = torch.full((3, 8), math.nan, device="cuda")
+    z[1] = torch.arange(8.0)
+    ids, wts = torch.full((3, 2), -1, dtype=torch.int32, device="cuda"), torch.empty(3, 2, device="cuda")
+    K.moe_route(z, 8, 2, False, ids, wts, None, stream())
+    assert bool(((ids >= 0) & (ids < 8)).all()) and ids[1].tolist() == [7, 6]

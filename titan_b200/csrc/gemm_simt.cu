@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "gemm.h"
+#include "tma.cuh"
 
 namespace {
 
@@ -207,20 +208,23 @@ gemm_simt_kernel(const T* X, const T* W, void* out_,
 // A step of a few tokens is bound by the weights' bytes, and in 64 x 64 tiles most of the chip idles: 16 blocks for
 // 1,024 columns, each walking all of K.  Here a block takes eight columns at a time and up to MR rows, and its 256 threads the runs of
 // SUM_RUN along K, a thread one column and one run.  A unit of work is eight columns and ``pass`` runs; its weights come into shared
-// memory by cp.async, all requested at once, while the unit before is worked on, those of the first unit before the wait for the
-// kernel before (no kernel writes weights); so do the rows of X, once a block where K is one pass.  A run lies 16 bytes and a
-// column 64 bytes behind a whole number of banks, so that a warp's four runs and eight columns do not collide.  The run sums meet in shared
+// memory as one bulk copy a column, up to three units ahead, those of the first units before the wait for the kernel before (no
+// kernel writes weights); the rows of X by cp.async, once a block where K is one pass.  A column of weights lies 16 bytes behind a whole
+// number of banks and a run of X likewise, so that a warp's eight columns and four runs do not collide.  The run sums meet in shared
 // memory and are added in order by a thread an output.  Each weight is read from memory once for MR rows; rows beyond
 // are further blocks, which find the weights in L2.  Three rows: 1,024 columns
 // of K = 2,816 in 7.1 us, 5,632 of K = 1,024 in 12.9, 32,768 in 59 (64 x 64 tiles: 189, 87 and 204 us).
 constexpr int FEW_COLS = 8;
 template <typename T> constexpr int few_run() { return SUM_RUN + 16 / (int)sizeof(T); }           // elements from a run to the next in shared memory
-template <typename T> __host__ __device__ constexpr int few_col(int pass) { return (pass * few_run<T>() * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T) + 64 / (int)sizeof(T); }
-// Shared memory: per stage [FEW_COLS] columns of ``pass`` runs and, where K takes several passes, [MR] rows; else the rows once, behind
-// the stages; then two areas of run sums.
+template <typename T> __host__ __device__ constexpr int few_col(int pass) { return pass * SUM_RUN + 16 / (int)sizeof(T); }      // a column of weights
+template <typename T> __host__ __device__ constexpr int few_row(int pass) { return pass * few_run<T>(); }                         // a row of X
+// Shared memory: the barriers; per stage [FEW_COLS] columns of ``pass`` runs and, where K takes several passes, [MR] rows; else the rows
+// once, behind the stages; then two areas of run sums.
 template <typename T, int MR> size_t few_smem(int pass, int stages, bool one_pass) {
-    return (size_t)(stages * (FEW_COLS + (one_pass ? 0 : MR)) + (one_pass ? MR : 0)) * few_col<T>(pass) * sizeof(T) + (size_t)2 * pass * MR * FEW_COLS * sizeof(float);
+    return 64 + (size_t)stages * FEW_COLS * few_col<T>(pass) * sizeof(T) + (size_t)(one_pass ? 1 : stages) * MR * few_row<T>(pass) * sizeof(T) +
+           (size_t)2 * pass * MR * FEW_COLS * sizeof(float);
 }
+__device__ unsigned int g_few_error = 0;
 
 template <typename T, int EPI, int MR, bool VEC>
 __global__ void __launch_bounds__(256)
@@ -232,14 +236,15 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m0 = blockIdx.y * MR, z = blockIdx.z;
     const int runs = (K + SUM_RUN - 1) / SUM_RUN, passes = (runs + pass - 1) / pass, groups = (N + FEW_COLS - 1) / FEW_COLS;
-    const int cs = few_col<T>(pass), stage_elems = (FEW_COLS + (passes > 1 ? MR : 0)) * cs;
-    T* const stage0 = reinterpret_cast<T*>(few_sm);        // [stages][FEW_COLS (+ MR)][cs]
+    const int cs = few_col<T>(pass), rs = few_row<T>(pass), stage_elems = FEW_COLS * cs + (passes > 1 ? MR * rs : 0);
+    uint64_t* const landed = reinterpret_cast<uint64_t*>(few_sm);        // [stages]
+    T* const stage0 = reinterpret_cast<T*>(few_sm + 64);   // [stages][FEW_COLS][cs] ([MR][rs])
     T* const x0 = stage0 + (passes > 1 ? FEW_COLS * cs : stages * stage_elems);        // rows of X: in every stage, or once
-    float* const sums0 = reinterpret_cast<float*>(stage0 + stages * stage_elems + (passes > 1 ? 0 : MR * cs));      // [2][pass][MR][FEW_COLS]
+    float* const sums0 = reinterpret_cast<float*>(stage0 + stages * stage_elems + (passes > 1 ? 0 : MR * rs));      // [2][pass][MR][FEW_COLS]
     // ``here`` runs of one row from run ``first`` on into shared memory, by ``step`` threads; elements beyond K are zero
-    auto stage = [&](T* to, const T* row, int first, int here, int at, int step) {
+    auto stage = [&](T* to, int run, const T* row, int first, int here, int at, int step) {
         for (int u = at; u < here * UNITS; u += step) {
-            T* dst = to + u / UNITS * RS + u % UNITS * PER;
+            T* dst = to + u / UNITS * run + u % UNITS * PER;
             const int k = first * SUM_RUN + u * PER;
             if (VEC && k < K) { copy16(dst, row + k); continue; }
 #pragma unroll
@@ -252,20 +257,38 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     };
     // unit u of this block: group blockIdx.x + (u / passes) * gridDim.x, pass u % passes
     const int my_groups = groups > (int)blockIdx.x ? (groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0, units = my_groups * passes;
-    auto stage_w = [&](int u) {                            // a warp loads a column; columns and rows outside: any valid ones
-        const int n = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS + warp, first = u % passes * pass;
-        stage(stage0 + (u % stages) * stage_elems + warp * cs, W + (size_t)z * sw + (size_t)min(n, N - 1) * K, first, min(pass, runs - first), lane, 32);
+    auto stage_w = [&](int u) {                            // columns outside: any valid one
+        const int n0 = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS, first = u % passes * pass, here = min(pass, runs - first);
+        T* to = stage0 + (u % stages) * stage_elems;
+        const T* from = W + (size_t)z * sw;
+        if (VEC) {
+            if (lane == 0) {                               // a warp a column: one thread for all eight would be what a unit waits for
+                const uint32_t bytes = (uint32_t)(min(here * SUM_RUN, K - first * SUM_RUN) * sizeof(T));
+                tbtma::mbar_expect_tx(landed + u % stages, bytes);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tbtma::smem_u32(to + warp * cs)),
+                             "l"(from + (size_t)min(n0 + warp, N - 1) * K + first * SUM_RUN), "r"(bytes), "r"(tbtma::smem_u32(landed + u % stages)) : "memory");
+            }
+        } else {
+            stage(to + warp * cs, SUM_RUN, from + (size_t)min(n0 + warp, N - 1) * K, first, here, lane, 32);      // a warp a column
+        }
     };
-    auto stage_x = [&](int u) {
+    auto stage_x = [&](int u) {                            // rows outside: any valid one
         const int first = u % passes * pass;
         for (int m = 0; m < MR; ++m)
-            stage(x0 + (passes > 1 ? (u % stages) * stage_elems : 0) + m * cs, X + (size_t)z * sx + (size_t)min(m0 + m, M - 1) * ldx, first,
+            stage(x0 + (passes > 1 ? (u % stages) * stage_elems : 0) + m * rs, RS, X + (size_t)z * sx + (size_t)min(m0 + m, M - 1) * ldx, first,
                   min(pass, runs - first), tid, 256);
     };
+    if (VEC) {
+        if (tid == 0) {
+            for (int s = 0; s < stages; ++s) tbtma::mbar_init(landed + s, FEW_COLS);
+            tbtma::mbar_fence_init();
+        }
+        __syncthreads();
+    }
     const int om = tid / FEW_COLS, on = tid % FEW_COLS;   // a thread's output, if it has one
     const int col = tid % FEW_COLS;
     float total = 0.f;
-    // unit u arrives with copy group u: the first ``stages`` - 1 units together in group 0, empty groups after it
+    // the rows of unit u arrive with copy group u: the first ``stages`` - 1 units together in group 0, empty groups after it
     for (int u = 0; u < min(units, max(1, stages - 1)); ++u) stage_w(u);
     pdl_wait();
     for (int u = 0; u < (passes > 1 ? min(units, max(1, stages - 1)) : 1); ++u) stage_x(u);
@@ -282,6 +305,7 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
         else if (stages == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
+        if (VEC) tbtma::mbar_wait(landed + u % stages, (u / stages) & 1, &g_few_error, 1);
         const int here = min(pass, runs - u % passes * pass);
         float* sums = sums0 + (u & 1) * pass * MR * FEW_COLS;
         const T* st = stage0 + (u % stages) * stage_elems;
@@ -290,29 +314,45 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
             unsigned long long acc[MR];
 #pragma unroll
             for (int m = 0; m < MR; ++m) acc[m] = 0ull;
-            const T* wr = st + col * cs + r * RS;
+            const T* wr = st + col * cs + r * SUM_RUN;
             const T* xr = sx_ + r * RS;
-#pragma unroll
-            for (int i = 0; i < UNITS; ++i) {
+            const int k0 = (u % passes * pass + r) * SUM_RUN;
+            auto unit = [&](int i) {
                 Vec<T, PER> v;
                 float wf[PER], xf[PER];
                 v.load(wr + i * PER);
                 v.get(wf);
 #pragma unroll
                 for (int m = 0; m < MR; ++m) {
-                    v.load(xr + m * cs + i * PER);
+                    v.load(xr + m * rs + i * PER);
                     v.get(xf);
 #pragma unroll
                     for (int e = 0; e < PER; e += 2) fma2(acc[m], pair_of(xf[e], xf[e + 1]), pair_of(wf[e], wf[e + 1]));
                 }
+            };
+            if (!VEC || k0 + SUM_RUN <= K) {
+#pragma unroll
+                for (int i = 0; i < UNITS; ++i) unit(i);
+            } else {                                       // the last run, cut short: nothing was copied behind K, a multiple of PER
+                for (int i = 0; k0 + i * PER < K; ++i) unit(i);
             }
 #pragma unroll
             for (int m = 0; m < MR; ++m) sums[(r * MR + m) * FEW_COLS + col] = both(acc[m]);
         }
         __syncthreads();
         if (tid >= MR * FEW_COLS) continue;
-#pragma unroll 8
-        for (int r = 0; r < here; ++r) total += sums[(r * MR + om) * FEW_COLS + on];
+        {
+            const float* mine = sums + om * FEW_COLS + on;
+            int r = 0;
+            for (; r + 16 <= here; r += 16) {              // all loads first
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = mine[(r + i) * MR * FEW_COLS];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) total += v[i];
+            }
+            for (; r < here; ++r) total += mine[r * MR * FEW_COLS];
+        }
         if (u % passes != passes - 1) continue;
         const int m = m0 + om, n = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS + on;
         // the gate of a pair: its second column is the neighbouring thread's
@@ -349,19 +389,17 @@ bool aligned(const Product& p, int per) {
 template <typename T, int EPI, int MR, bool VEC>
 void few_launch(const Product& p) {
     const int runs = (p.K + SUM_RUN - 1) / SUM_RUN, groups = (p.N + FEW_COLS - 1) / FEW_COLS, others = (p.M + MR - 1) / MR * p.batch;
-    // One unit a block while the blocks fit the chip once: all of K at once.  Else passes of 32 runs (one a thread), up to four stages,
-    // and equal shares of the column groups for a block an SM.
+    // One unit a block while the blocks fit the chip once: all of K at once.  Else passes of 32 runs (one a thread) and equal shares of the
+    // column groups, for two blocks an SM with two stages each where their memory fits (one computes while the other waits), or
+    // one block with up to four.
     const bool once = (long long)groups * others <= SMS;
-    int pass = once ? 96 : 32, x = groups;
+    int pass = once ? 96 : 32;
     if (pass > runs) pass = runs;
     while (few_smem<T, MR>(pass, 1, pass >= runs) > 200 * 1024) --pass;
-    const int passes = (runs + pass - 1) / pass, room = SMS / others > 0 ? SMS / others : 1;
-    if (groups > room) {
-        const int each = (groups + room - 1) / room;
-        x = (groups + each - 1) / each;
-    }
+    const int passes = (runs + pass - 1) / pass, two = few_smem<T, MR>(pass, 2, passes == 1) <= 112 * 1024;
+    const int room = (two ? 2 : 1) * SMS / others > 0 ? (two ? 2 : 1) * SMS / others : 1, each = (groups + room - 1) / room, x = (groups + each - 1) / each;
     const long long units = (long long)((groups + x - 1) / x) * passes;
-    int stages = units < 4 ? (int)units : 4;
+    int stages = units < (two ? 2 : 4) ? (int)units : (two ? 2 : 4);
     while (stages > 1 && few_smem<T, MR>(pass, stages, passes == 1) > 220 * 1024) --stages;
     if (stages == 1 && units > 1) { stages = 2; while (few_smem<T, MR>(pass, stages, false) > 220 * 1024) --pass; }
     const size_t smem = few_smem<T, MR>(pass, stages, (runs + pass - 1) / pass == 1);
@@ -417,6 +455,14 @@ int run(const Product& p, int epi, bool few = false) {
 }
 
 }  // namespace
+
+// Clears and returns the code of a bounded wait that gave up (0: none): the results since the last call are then invalid.
+extern "C" int tb_gemm_few_error() {
+    unsigned int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_few_error, sizeof v) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_few_error, &zero, sizeof zero);
+    return (int)v;
+}
 
 // ldx: row stride of X in elements; ldo: row stride of out in elements.  ``batch`` products of the same shape in one
 // launch: product z reads X + z * sx and W + z * sw and writes out + z * so (offsets in elements).

@@ -1147,12 +1147,14 @@ int ordered_fit(int bn, bool normed, int tiles, int wanted) {
 // K slices of an epilogue that needs whole sums (all but ADD), the tiles of at most 64 rows: 1 or a cluster's size.  As many as give every
 // SM a CTA, at least four k-blocks each, at most four (measured at most 1 / 2 / 3 / 4 / 6 / 8: a decode step of twelve layers of
 // width 1,024 314 / 290 / 288 / 289 / 292 / 291 us, of four layers with experts of width 2,048 696 / 670 / 661 / 653 / 652 / 652).
-int whole_slices(int bn, bool normed, int tiles, int kb, int sm_count) {
+// The clusters take at most half of the places (two CTAs an SM), so all of them are held at once wherever they can be put.
+int whole_slices(int bn, int tiles, int kb, int sm_count) {
     int s = sm_count / tiles;
     if (s > kb / 4) s = kb / 4;
     if (s > 4) s = 4;
-    return s < 2 || bn > 64 ? 1 : ordered_fit(bn, normed, tiles, s);
+    return s < 2 || bn > 64 ? 1 : s;
 }
+
 template <int BN, int EPI>
 int launch_persistent_epi(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, dim3 grid, cudaStream_t stream) {
     static bool configured = false;
@@ -1306,7 +1308,7 @@ static int normed_slices(int N, int K, int epi, int M = 1, bool ordered = false)
         s = s > 16 ? 16 : s;
         if (ordered) s = ordered_fit(M <= 16 ? 16 : 32, true, tiles, s);
     } else {
-        s = whole_slices(M <= 16 ? 16 : 32, true, tiles, kb, sm_count);
+        s = whole_slices(M <= 16 ? 16 : 32, tiles, kb, sm_count);
     }
     const int per = (kb + s - 1) / s;
     return (kb + per - 1) / per;
@@ -1356,7 +1358,7 @@ extern "C" int tb_gemm_tc_normed(const float* xf, int ldxf, const float* norm_w,
 // act, limit: the gate of the SWIGLU epilogue, or the activation of the STORE epilogue (activation.h).
 extern "C" int tb_gemm_tc_gated(const void* X, const void* W, void* out, int M, int N, int K, int ldx, int ldo, int epi,
                                 int splits, int act, float limit, cudaStream_t stream) {
-    if (tb_gemm_tc_check(M, N, K, ldx, ldo, epi, X, W, out)) return 1;
+    if (tb_gemm_tc_check(M, N, K, ldx, ldo, epi, X, W, out)) return 3;       // not this kernel's: the caller may have another
     TB_REQUIRE(act >= 0 && act < (epi == TB_EPI_STORE ? TB_UNARY_KINDS : TB_ACT_KINDS), "gemm_tc: unknown gate or activation %d", act);
     const bool ordered = splits < 0;
     if (ordered) splits = 0;
@@ -1443,7 +1445,7 @@ extern "C" int tb_gemm_tc_gated(const void* X, const void* W, void* out, int M, 
             s = s < 1 ? 1 : (s > max_s ? max_s : s);
             if (ordered) s = ordered_fit(bn, false, tiles, s);
         } else {
-            s = whole_slices(bn, false, tiles, kb, sm_count);
+            s = whole_slices(bn, tiles, kb, sm_count);
         }
         a.k_blocks_per_split = (kb + s - 1) / s;
         s = (kb + a.k_blocks_per_split - 1) / a.k_blocks_per_split;  // no empty slice

@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "qk_args.h"
+#include "tma.cuh"
 
 struct LightningArgs {
     const void* proj; int stride;           // [T][stride]: q (H*dk) | k (H*dk) | v (H*dv) | g (H*dv), compute dtype
@@ -28,7 +29,7 @@ struct LightningArgs {
     int B; int H; int dk; int dv;
     int max_new;                            // most tokens a sequence brings in this step (1: a step of single tokens)
     int plain;                              // 1: q, k and v enter the recurrence as they stand in the rows (no silu): the retention mixer, whose rows are float32
-    float* work; int work_chunks;           // room for the chunked form: work_chunks * H * 64 * (64 + 2 * DK) floats, work_chunks >= sum over sequences of ceil(tokens / 64); null: token by token
+    float* work; int work_chunks;           // room for the chunked form (tb_lightning_work floats), work_chunks >= sum over sequences of ceil(tokens / 64); null: token by token
     int below;                              // > 0: only runs of fewer tokens (set by the launcher)
 };
 
@@ -276,7 +277,11 @@ __device__ __forceinline__ float lf_low(unsigned long long v) { return __uint_as
 __device__ __forceinline__ float lf_high(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
 template <int DK> constexpr int chunk_row() { return CHUNK + DK; }                                  // floats of a row of A
-template <int DK> constexpr size_t chunk_floats() { return (size_t)CHUNK * (CHUNK + 2 * DK); }     // of a (chunk, head): A, then k'
+// Of a (chunk, head): A, then k', both with the padding of their rows in shared memory, so that each is one bulk copy.
+template <int DK> constexpr int chunk_a() { return CHUNK * (chunk_row<DK>() + 4); }
+template <int DK> constexpr int chunk_k() { return DK * (CHUNK + 4); }
+template <int DK> constexpr size_t chunk_floats() { return (size_t)chunk_a<DK>() + chunk_k<DK>(); }
+__device__ unsigned int g_lightning_error = 0;
 template <int DK> constexpr size_t prep_smem() { return (size_t)(2 * CHUNK * (DK + 4) + CHUNK + 1) * sizeof(float); }
 
 // grid (work_chunks, H), 256 threads
@@ -340,7 +345,8 @@ __global__ void __launch_bounds__(256) lightning_prep_kernel(LightningArgs a) {
     }
     __syncthreads();
     float* rows = a.work + ((size_t)blockIdx.x * a.H + h) * chunk_floats<DK>();
-    float* krows = rows + CHUNK * chunk_row<DK>();
+    float* krows = rows + chunk_a<DK>();
+    constexpr int LA = chunk_row<DK>() + 4, LT = CHUNK + 4;
     const int tx = tid & 15, ty = tid >> 4;             // scores of rows ty + 16 i and keys tx + 16 j
     unsigned long long acc[4][4] = {};                  // sums over even and over odd dimensions
 #pragma unroll 4
@@ -361,32 +367,33 @@ __global__ void __launch_bounds__(256) lightning_prep_kernel(LightningArgs a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int r = ty + 16 * i, c = tx + 16 * j;
-            rows[r * chunk_row<DK>() + c] = c <= r && r < n ? (lf_low(acc[i][j]) + lf_high(acc[i][j])) * power[r - c] : 0.f;
+            rows[r * LA + c] = c <= r && r < n ? (lf_low(acc[i][j]) + lf_high(acc[i][j])) * power[r - c] : 0.f;
         }
     for (int e = tid; e < CHUNK * DK / 4; e += 256) {
         const int r = e / (DK / 4), d = e % (DK / 4) * 4;
         float4 q = *reinterpret_cast<const float4*>(qs + r * LD + d);
         const float f = power[r + 1];
         q.x *= f; q.y *= f; q.z *= f; q.w *= f;
-        *reinterpret_cast<float4*>(rows + r * chunk_row<DK>() + CHUNK + d) = q;
+        *reinterpret_cast<float4*>(rows + r * LA + CHUNK + d) = q;
     }
     for (int e = tid; e < DK * CHUNK / 4; e += 256) {   // a thread: one dimension, four tokens; four threads a dimension
         const int d = e / 4 % DK, r = (e / (4 * DK) * 4 + e % 4) * 4;
         float k[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) k[i] = r + i < n ? ks[(r + i) * LD + d] * power[n - 1 - r - i] : 0.f;
-        *reinterpret_cast<float4*>(krows + d * CHUNK + r) = make_float4(k[0], k[1], k[2], k[3]);
+        *reinterpret_cast<float4*>(krows + d * LT + r) = make_float4(k[0], k[1], k[2], k[3]);
     }
 }
 
-__device__ __forceinline__ void copy16(float* to, const float* from) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+__device__ __forceinline__ void bulk_copy(void* to, const void* from, uint32_t bytes, uint64_t* landed) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tbtma::smem_u32(to)), "l"(from), "r"(bytes),
+                 "r"(tbtma::smem_u32(landed)) : "memory");
 }
 
 constexpr int PART_COL = CHUNK + 8;                     // floats from a column to the next of a warp's partial outputs
 template <int DK> constexpr size_t chunk_smem() {
     // two buffers of A and of k'^T (rows padded by 4), values and the state's slice by column, eight warps' partial outputs
-    return (size_t)(2 * (CHUNK * (chunk_row<DK>() + 4) + DK * (CHUNK + 4)) + VCOLS * (chunk_row<DK>() + 4) + 8 * VCOLS * PART_COL) * sizeof(float);
+    return (size_t)(2 * (CHUNK * (chunk_row<DK>() + 4) + DK * (CHUNK + 4)) + VCOLS * (chunk_row<DK>() + 4) + 8 * VCOLS * PART_COL) * sizeof(float) + 16;
 }
 
 // grid (B, H, ceil(dv / 16)), 512 threads: warps 0 .. 7 make the outputs while warps 8 .. 15 make the state after the chunk
@@ -400,6 +407,7 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
     float* krows = rows + 2 * CHUNK * LD;               // [2][DK][LT]
     float* vals = krows + 2 * DK * LT;                  // [VCOLS][LD]: by column, the chunk's values, then the state
     float* part = vals + VCOLS * LD;                    // [8][VCOLS][PART_COL]
+    uint64_t* landed = reinterpret_cast<uint64_t*>(part + 8 * VCOLS * PART_COL);      // [2]
     const int b = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VCOLS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dk = a.dk, dv = a.dv, t0 = a.q_start[b], t1 = a.q_start[b + 1];
@@ -419,16 +427,18 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
             S[i][c] = (keeps && sk + 32 * i < dk && j0 + sc + 8 * c < dv) ? S_g[(size_t)(sk + 32 * i) * dv + sc + 8 * c] : 0.f;
             if (keeps) vals[(sc + 8 * c) * LD + CHUNK + sk + 32 * i] = S[i][c];
         }
-    auto load_rows = [&](int c, int half) {
+    if (tid == 0) {
+        tbtma::mbar_init(landed, 1);
+        tbtma::mbar_init(landed + 1, 1);
+        tbtma::mbar_fence_init();
+    }
+    __syncthreads();
+    auto load_rows = [&](int c, int half) {             // two bulk copies, by one thread
+        if (tid != 0) return;
         const float* from = a.work + ((size_t)(chunk0 + c) * a.H + h) * chunk_floats<DK>();
-        float* to = rows + half * CHUNK * LD;
-#pragma unroll
-        for (int u = 0; u < CHUNK * ROW / 4 / 512; ++u) { const int e = tid + 512 * u; copy16(to + e / (ROW / 4) * LD + e % (ROW / 4) * 4, from + e * 4); }
-        from += CHUNK * ROW;
-        to = krows + half * DK * LT;
-#pragma unroll
-        for (int u = 0; u < CHUNK * DK / 4 / 512; ++u) { const int e = tid + 512 * u; copy16(to + e / (CHUNK / 4) * LT + e % (CHUNK / 4) * 4, from + e * 4); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        tbtma::mbar_expect_tx(landed + half, (uint32_t)(chunk_floats<DK>() * sizeof(float)));
+        bulk_copy(rows + half * CHUNK * LD, from, chunk_a<DK>() * 4, landed + half);
+        bulk_copy(krows + half * DK * LT, from + chunk_a<DK>(), chunk_k<DK>() * 4, landed + half);
     };
     // two values of a chunk a thread: token tid % 64, columns lc and lc + 1; and a thread of the first half's outputs: token vr, columns vc ..
     const int vr = tid & 63, lc = tid >> 6 << 1, vc = (tid & 255) >> 6 << 2;
@@ -462,8 +472,8 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
             odd |= !(fabsf(next[i]) <= 3.402823466e38f);
             vals[(lc + i) * LD + vr] = next[i];
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
         odd = __syncthreads_or(odd);
+        tbtma::mbar_wait(landed + half, (c >> 1) & 1, &g_lightning_error, 1);
         if (c + 1 < chunks) { load_rows(c + 1, half ^ 1); load_values(c + 1); }
         const float* A = rows + half * CHUNK * LD;
         if (!keeps) {   // this warp's KW of the columns of A: rows rg + 8 r, value columns cg + 4 j; sums over even and over odd places
@@ -693,6 +703,14 @@ extern "C" int tb_lightning_scan(const LightningArgs* args, int dtype, cudaStrea
     if (dtype == TB_F32 ? launch_scan<float>(a, single, stream) : launch_scan<__nv_bfloat16>(a, single, stream)) return 1;
     TB_CHECK_LAUNCH("lightning_scan");
     return 0;
+}
+
+// Clears and returns the code of a bounded wait that gave up (0: none): the results since the last call are then invalid.
+extern "C" int tb_lightning_error() {
+    unsigned int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_lightning_error, sizeof v) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_lightning_error, &zero, sizeof zero);
+    return (int)v;
 }
 
 extern "C" int tb_gated_rmsnorm(const float* o, int ldo, const float* w, const void* gate, int ldg, void* y, int ldy,

@@ -838,23 +838,35 @@ def gemm_tc_accepts(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: in
 
 
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, stream: int, splits: int = 0, ordered: bool = False,
-            gate: int = ACT_SILU, limit: float = 0.0) -> None:
+            gate: int = ACT_SILU, limit: float = 0.0, optional: bool = False) -> bool:
     """out (epilogue ``epi``) = x[M,K] . w[N,K]^T on the tcgen05 tensor cores (bfloat16 operands).  ``ordered``: partial
     sums along K add up in a fixed order (the K slices of a decode product inside a thread-block cluster, no prompt tile
     cut along K), so that the same inputs give the same bits on every run; the default lets float32 reductions meet at
-    L2 in the order they arrive, which is faster and differs from run to run in the last bits."""
-    _need_cuda(x, w, out)
-    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
-        raise KernelError("gemm_tc: operands must be bfloat16")
-    want = torch.bfloat16 if epi in (EPI_STORE, EPI_SWIGLU) else torch.float32
-    if out.dtype != want:
-        raise KernelError(f"gemm_tc: this epilogue writes {want}, the output is {out.dtype}")
+    L2 in the order they arrive, which is faster and differs from run to run in the last bits.  ``optional``: a product that the kernel's
+    rules exclude (``gemm_tc_accepts``) returns False and launches nothing, instead of raising: a prompt's products ask and launch in one call."""
+    if not (x.is_cuda and w.is_cuda and out.is_cuda):
+        _need_cuda(x, w, out)
     M, K_ = x.shape
-    N = w.shape[0]
-    if w.shape[1] != K_ or not w.is_contiguous() or x.stride(1) != 1 or out.stride(1) != 1:
+    N, Kw = w.shape
+    ldx, unit_x = x.stride()
+    ldo, unit_o = out.stride()
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        if optional:
+            return False
+        raise KernelError("gemm_tc: operands must be bfloat16")
+    if Kw != K_ or unit_x != 1 or unit_o != 1 or not w.is_contiguous():
+        if optional:
+            return False
         raise KernelError(f"gemm_tc: shapes do not fit: x {tuple(x.shape)} w {tuple(w.shape)}")
-    _check(tlib().tb_gemm_tc_gated(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K_, x.stride(0), out.stride(0), epi,
-                                  -1 if ordered and not splits else splits, int(gate), float(limit), stream))
+    if out.dtype != (torch.bfloat16 if epi == EPI_STORE or epi == EPI_SWIGLU else torch.float32):
+        want = torch.bfloat16 if epi in (EPI_STORE, EPI_SWIGLU) else torch.float32
+        raise KernelError(f"gemm_tc: this epilogue writes {want}, the output is {out.dtype}")
+    rc = tlib().tb_gemm_tc_gated(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K_, ldx, ldo, epi,
+                                 -1 if ordered and not splits else splits, gate, limit, stream)
+    if rc == 3 and optional:
+        return False
+    _check(rc)
+    return True
 
 
 def gemm_tc_expert_runs(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, w_down: torch.Tensor, y: torch.Tensor, first: torch.Tensor,
@@ -1025,11 +1037,10 @@ def commit_lengths(slot_of_seq, kv_len, seq_len, stream: int) -> None:
 
 def wait_errors() -> dict:
     """The error words of the kernels whose waits are bounded (a wait that gave up leaves a code there and the
-    step's result is invalid).  Reads and clears them; synchronises the device.  Empty if all is well, and
-    if the tensor-core library was never loaded."""
-    if _tlib is None:
-        return {}
-    found = {"gemm_tc": gemm_tc_error()}
+    step's result is invalid).  Reads and clears them; synchronises the device.  Empty if all is well."""
+    found = {"gemm_few": int(lib().tb_gemm_few_error()), "lightning": int(lib().tb_lightning_error())}
+    if _tlib is not None:
+        found["gemm_tc"] = gemm_tc_error()
     if _alib is not None:
         found.update({"attn_prefill_tc": attn_tc_error(), "attn_mma": attn_mma_error(), "attn_decode_latent": int(alib().tb_attn_latent_error())})
     return {k: v for k, v in found.items() if v}

@@ -26,16 +26,13 @@ def matmul(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, ctx, g
     epilogue makes of a sum (``kernels.UNARY_*``)."""
     if unary and epi != EPI_STORE:
         raise ValueError("an activation of single sums comes with the STORE epilogue")
-    act = gate if epi == EPI_SWIGLU else unary
-    if (x.shape[0] <= ROWS_MAX_M and w.shape[0] * w.shape[1] <= ROWS_MAX_ELEMENTS and epi in (EPI_STORE, EPI_F32, EPI_ADD)
-            and ctx.options.get("small_products", True)):
+    act, options = (gate if epi == EPI_SWIGLU else unary), ctx.options
+    if x.shape[0] <= ROWS_MAX_M and epi != EPI_SWIGLU and w.numel() <= ROWS_MAX_ELEMENTS and options.get("small_products", True):
         K.gemm_rows(x, w, out, epi, ctx.stream, unary)
         return
-    if w.dtype == torch.bfloat16 and ctx.options.get("gemm", "fast") != "plain":
-        fast = getattr(K, "gemm_tc", None)
-        if fast is not None and K.gemm_tc_accepts(x, w, out, epi):
-            fast(x, w, out, epi, ctx.stream, ordered=bool(ctx.options.get("reproducible", False)), gate=act, limit=limit)
-            return
+    if (w.dtype == torch.bfloat16 and options.get("gemm", "fast") != "plain"
+            and K.gemm_tc(x, w, out, epi, ctx.stream, 0, bool(options.get("reproducible", False)), act, limit, optional=True)):
+        return
     K.gemm_simt(x, w, out, epi, ctx.stream, act, limit)
 
 
