@@ -88,7 +88,7 @@ class SequenceCache:
     def alloc_slot(self) -> int:
         slot = self.slots.take()
         self.length[slot] = 0
-        self.state.seq_len[slot] = 0
+        self.state.seq_len[slot].zero_()    # a kernel in stream order (assigning a number would copy from the host and wait for the stream)
         for g in self.groups:
             g.on_alloc(slot)
         return slot

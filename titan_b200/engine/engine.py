@@ -160,9 +160,12 @@ class Engine:
             n = len(e.tokens)
             if n == 0:
                 raise StepError(f"slot {e.slot} brings no token")
-            for t in e.tokens:
-                if not 0 <= int(t) < V:
-                    raise StepError(f"token id {t} lies outside the vocabulary of {V}")
+            # one pass in numpy over a prompt's ids; the loop names the one that is wrong (and takes what numpy does not)
+            ids = np.asarray(e.tokens)
+            if ids.ndim != 1 or ids.dtype.kind not in "iu" or int(ids.min()) < 0 or int(ids.max()) >= V:
+                for t in e.tokens:
+                    if not 0 <= int(t) < V:
+                        raise StepError(f"token id {t} lies outside the vocabulary of {V}")
             for w in e.want:
                 if not 0 <= int(w) < n:
                     raise StepError(f"logits wanted at place {w} of {n} tokens")

@@ -398,9 +398,9 @@ def scale_f32(x: torch.Tensor, factor: float, stream: int) -> None:
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, eps: float, stream: int,
             rows: Optional[torch.Tensor] = None) -> None:
-    _need_cuda(x, w, y, rows)
-    n = y.shape[0]
-    _check(lib().tb_rmsnorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), dtype_code(y.dtype), _ptr(rows), n,
+    if not (x.is_cuda and w.is_cuda and y.is_cuda and (rows is None or rows.is_cuda)):
+        _need_cuda(x, w, y, rows)
+    _check(lib().tb_rmsnorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), dtype_code(y.dtype), None if rows is None else rows.data_ptr(), y.shape[0],
                             x.shape[-1], eps, stream))
 
 
