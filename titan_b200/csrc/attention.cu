@@ -55,6 +55,15 @@ template <> __device__ __forceinline__ void unpack16<__nv_bfloat16>(const uint4&
     for (int i = 0; i < 4; ++i) { o[2 * i] = __uint_as_float(w[i] << 16); o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 
+// kv_row_offset with the page's size as a shift where it is a power of two (``shift`` >= 0): two divisions less a key.
+__device__ __forceinline__ int page_shift(const TbKvView& c) { return (c.page_size & (c.page_size - 1)) == 0 ? 31 - __clz(c.page_size) : -1; }
+__device__ __forceinline__ size_t row_offset(const TbKvView& c, int slot, int pos, int head, int shift) {
+    if (shift < 0) return kv_row_offset(c, slot, pos, head);
+    const int row = c.ring_rows ? pos % c.ring_rows : pos;
+    const int page = c.table[(size_t)slot * c.table_width + (row >> shift)];
+    return (((size_t)page * c.kv_heads + head << shift) + (row & (c.page_size - 1))) * c.head_dim;
+}
+
 // Running softmax state of one warp: every lane holds the same m and l, and acc for dims lane + 32 j.
 template <int MAXE>
 struct Running {
@@ -243,6 +252,7 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
     const float* knew = (const float*)a.kv_new;
     const float* cache = (const float*)a.cache.storage;
     const size_t vhalf = cache ? kv_half_elems(a.cache) : 0;
+    const int shift = page_shift(a.cache);
     const int row = tid >> 2, quarter = tid & 3;           // loads: four threads a row, a row's 16-byte units in turn
     {
         const float* q = (const float*)a.q + (size_t)(t0 + q0 + min(row, nq - 1)) * a.q_stride + (size_t)h * hd;
@@ -272,7 +282,7 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
                 kp = knew + (size_t)(t0 + kpos - first_new) * a.kv_stride + (size_t)kh * hd;
                 vp = kp + (size_t)a.nkv * hd;
             } else {
-                kp = cache + kv_row_offset(a.cache, slot, kpos, kh);
+                kp = cache + row_offset(a.cache, slot, kpos, kh, shift);
                 vp = kp + vhalf;
             }
         }
@@ -438,10 +448,10 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_decode_kernel(AttnArgs a)
 // The same for rows of up to 32 16-byte units (float32: 128 elements, bfloat16: 256).  LPK lanes share a key, a 16-byte unit of its row
 // each, so that a load covers whole rows of 32 / LPK keys (in the kernel above every lane walks a row of its own, and a warp a
 // whole split).  Each group of LPK lanes is a stream of its own: keys st, st + streams, ... of the split, eight keys and
-// values requested at once, an own running softmax.  The streams of a head, those of up to eight warps, are merged in shared memory.
+// values requested at once, an own running softmax.  The streams of a head, those of up to sixteen warps, are merged in shared memory.
 // Bound by the latency of the loads at a few hundred keys a split: three
 // sequences of 500 tokens, 16 heads of 64 on 8, float32: 210 -> 13.7 us a layer.
-constexpr int VEC_WARPS = 8, VEC_KEYS = 8;
+constexpr int VEC_WARPS = 16, VEC_KEYS = 8;
 
 template <typename T, int LPK>
 __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArgs a) {
@@ -456,7 +466,7 @@ __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArg
     const int len = a.batch.kv_len[b];
     const int keys = tb_split_keys(len, a.chunk, a.n_splits);
     if ((long long)split * keys >= len) return;     // the merge reads ceil(len / keys) splits only
-    int share = 1;                                     // warps a head: two, four or eight where there are at least so many times as many warps
+    int share = 1;                                     // warps a head: two, four, eight or sixteen where there are so many times as many warps
     while (share * 2 * group <= VEC_WARPS) share *= 2;
     const int pos = len - 1;
     const int slot = a.batch.slot_of_seq[b];
@@ -466,6 +476,7 @@ __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArg
     const int klo = split * keys, khi = a.window > 0 ? min(min(a.keep_first, wlo), hi) : 0;
     const T* cache = (const T*)a.cache.storage;
     const size_t vhalf = a.v_alias ? 0 : kv_half_elems(a.cache);
+    const int shift = page_shift(a.cache);
     const int streams = share * STREAMS, st = (warp % share) * STREAMS + lane / LPK;
     const int at = unit * PER;
     const bool key_part = at < hd, value_part = at < hdv;
@@ -483,7 +494,7 @@ __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArg
                 uint4 kr[VEC_KEYS], vr[VEC_KEYS];
 #pragma unroll
                 for (int u = 0; u < VEC_KEYS; ++u) {
-                    const T* row = cache + kv_row_offset(a.cache, slot, min(base + u * streams + st, last - 1), kh) + at;
+                    const T* row = cache + row_offset(a.cache, slot, min(base + u * streams + st, last - 1), kh, shift) + at;
                     kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
                     if (key_part) kr[u] = *reinterpret_cast<const uint4*>(row);
                     if (value_part) vr[u] = *reinterpret_cast<const uint4*>(row + vhalf);

@@ -206,7 +206,7 @@ gemm_simt_kernel(const T* X, const T* W, void* out_,
 
 // ---------------------------------------------------------------- few rows: weights streamed once
 // A step of a few tokens is bound by the weights' bytes, and in 64 x 64 tiles most of the chip idles: 16 blocks for
-// 1,024 columns, each walking all of K.  Here a block takes eight columns at a time and up to MR rows, and its 256 threads the runs of
+// 1,024 columns, each walking all of K.  Here a block takes eight columns (COLS) at a time and up to MR rows, and its 256 threads the runs of
 // SUM_RUN along K, a thread one column and one run.  A unit of work is eight columns and ``pass`` runs; its weights come into shared
 // memory as one bulk copy a column, up to three units ahead, those of the first units before the wait for the kernel before (no
 // kernel writes weights); the rows of X by cp.async, once a block where K is one pass.  A column of weights lies 16 bytes behind a whole
@@ -214,19 +214,18 @@ gemm_simt_kernel(const T* X, const T* W, void* out_,
 // memory and are added in order by a thread an output.  Each weight is read from memory once for MR rows; rows beyond
 // are further blocks, which find the weights in L2.  Three rows: 1,024 columns
 // of K = 2,816 in 7.1 us, 5,632 of K = 1,024 in 12.9, 32,768 in 59 (64 x 64 tiles: 189, 87 and 204 us).
-constexpr int FEW_COLS = 8;
 template <typename T> constexpr int few_run() { return SUM_RUN + 16 / (int)sizeof(T); }           // elements from a run to the next in shared memory
 template <typename T> __host__ __device__ constexpr int few_col(int pass) { return pass * SUM_RUN + 16 / (int)sizeof(T); }      // a column of weights
 template <typename T> __host__ __device__ constexpr int few_row(int pass) { return pass * few_run<T>(); }                         // a row of X
-// Shared memory: the barriers; per stage [FEW_COLS] columns of ``pass`` runs and, where K takes several passes, [MR] rows; else the rows
+// Shared memory: the barriers; per stage [COLS] columns of ``pass`` runs and, where K takes several passes, [MR] rows; else the rows
 // once, behind the stages; then two areas of run sums.
-template <typename T, int MR> size_t few_smem(int pass, int stages, bool one_pass) {
-    return 64 + (size_t)stages * FEW_COLS * few_col<T>(pass) * sizeof(T) + (size_t)(one_pass ? 1 : stages) * MR * few_row<T>(pass) * sizeof(T) +
-           (size_t)2 * pass * MR * FEW_COLS * sizeof(float);
+template <typename T, int MR, int COLS> size_t few_smem(int pass, int stages, bool one_pass) {
+    return 64 + (size_t)stages * COLS * few_col<T>(pass) * sizeof(T) + (size_t)(one_pass ? 1 : stages) * MR * few_row<T>(pass) * sizeof(T) +
+           (size_t)2 * pass * MR * COLS * sizeof(float);
 }
 __device__ unsigned int g_few_error = 0;
 
-template <typename T, int EPI, int MR, bool VEC>
+template <typename T, int EPI, int MR, int COLS, bool VEC>
 __global__ void __launch_bounds__(256)
 gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx, int ldo, long long sx, long long sw, long long so,
                 int pass, int stages, int act, float limit) {
@@ -235,12 +234,12 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     extern __shared__ __align__(16) unsigned char few_sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m0 = blockIdx.y * MR, z = blockIdx.z;
-    const int runs = (K + SUM_RUN - 1) / SUM_RUN, passes = (runs + pass - 1) / pass, groups = (N + FEW_COLS - 1) / FEW_COLS;
-    const int cs = few_col<T>(pass), rs = few_row<T>(pass), stage_elems = FEW_COLS * cs + (passes > 1 ? MR * rs : 0);
+    const int runs = (K + SUM_RUN - 1) / SUM_RUN, passes = (runs + pass - 1) / pass, groups = (N + COLS - 1) / COLS;
+    const int cs = few_col<T>(pass), rs = few_row<T>(pass), stage_elems = COLS * cs + (passes > 1 ? MR * rs : 0);
     uint64_t* const landed = reinterpret_cast<uint64_t*>(few_sm);        // [stages]
-    T* const stage0 = reinterpret_cast<T*>(few_sm + 64);   // [stages][FEW_COLS][cs] ([MR][rs])
-    T* const x0 = stage0 + (passes > 1 ? FEW_COLS * cs : stages * stage_elems);        // rows of X: in every stage, or once
-    float* const sums0 = reinterpret_cast<float*>(stage0 + stages * stage_elems + (passes > 1 ? 0 : MR * rs));      // [2][pass][MR][FEW_COLS]
+    T* const stage0 = reinterpret_cast<T*>(few_sm + 64);   // [stages][COLS][cs] ([MR][rs])
+    T* const x0 = stage0 + (passes > 1 ? COLS * cs : stages * stage_elems);        // rows of X: in every stage, or once
+    float* const sums0 = reinterpret_cast<float*>(stage0 + stages * stage_elems + (passes > 1 ? 0 : MR * rs));      // [2][pass][MR][COLS]
     // ``here`` runs of one row from run ``first`` on into shared memory, by ``step`` threads; elements beyond K are zero
     auto stage = [&](T* to, int run, const T* row, int first, int here, int at, int step) {
         for (int u = at; u < here * UNITS; u += step) {
@@ -258,18 +257,19 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     // unit u of this block: group blockIdx.x + (u / passes) * gridDim.x, pass u % passes
     const int my_groups = groups > (int)blockIdx.x ? (groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0, units = my_groups * passes;
     auto stage_w = [&](int u) {                            // columns outside: any valid one
-        const int n0 = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS, first = u % passes * pass, here = min(pass, runs - first);
+        const int n0 = (blockIdx.x + u / passes * gridDim.x) * COLS, first = u % passes * pass, here = min(pass, runs - first);
         T* to = stage0 + (u % stages) * stage_elems;
         const T* from = W + (size_t)z * sw;
         if (VEC) {
-            if (lane == 0) {                               // a warp a column: one thread for all eight would be what a unit waits for
+            if (lane < COLS / 8) {                         // every warp its columns: one thread for all would be what a unit waits for
                 const uint32_t bytes = (uint32_t)(min(here * SUM_RUN, K - first * SUM_RUN) * sizeof(T));
+                const int c = warp * (COLS / 8) + lane;
                 tbtma::mbar_expect_tx(landed + u % stages, bytes);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tbtma::smem_u32(to + warp * cs)),
-                             "l"(from + (size_t)min(n0 + warp, N - 1) * K + first * SUM_RUN), "r"(bytes), "r"(tbtma::smem_u32(landed + u % stages)) : "memory");
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tbtma::smem_u32(to + c * cs)),
+                             "l"(from + (size_t)min(n0 + c, N - 1) * K + first * SUM_RUN), "r"(bytes), "r"(tbtma::smem_u32(landed + u % stages)) : "memory");
             }
         } else {
-            stage(to + warp * cs, SUM_RUN, from + (size_t)min(n0 + warp, N - 1) * K, first, here, lane, 32);      // a warp a column
+            for (int c = warp; c < COLS; c += 8) stage(to + c * cs, SUM_RUN, from + (size_t)min(n0 + c, N - 1) * K, first, here, lane, 32);
         }
     };
     auto stage_x = [&](int u) {                            // rows outside: any valid one
@@ -280,13 +280,13 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     };
     if (VEC) {
         if (tid == 0) {
-            for (int s = 0; s < stages; ++s) tbtma::mbar_init(landed + s, FEW_COLS);
+            for (int s = 0; s < stages; ++s) tbtma::mbar_init(landed + s, COLS);
             tbtma::mbar_fence_init();
         }
         __syncthreads();
     }
-    const int om = tid / FEW_COLS, on = tid % FEW_COLS;   // a thread's output, if it has one
-    const int col = tid % FEW_COLS;
+    const int om = tid / COLS, on = tid % COLS;   // a thread's output, if it has one
+    const int col = tid % COLS;
     float total = 0.f;
     // the rows of unit u arrive with copy group u: the first ``stages`` - 1 units together in group 0, empty groups after it
     for (int u = 0; u < min(units, max(1, stages - 1)); ++u) stage_w(u);
@@ -307,10 +307,10 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
         __syncthreads();
         if (VEC) tbtma::mbar_wait(landed + u % stages, (u / stages) & 1, &g_few_error, 1);
         const int here = min(pass, runs - u % passes * pass);
-        float* sums = sums0 + (u & 1) * pass * MR * FEW_COLS;
+        float* sums = sums0 + (u & 1) * pass * MR * COLS;
         const T* st = stage0 + (u % stages) * stage_elems;
         const T* sx_ = x0 + (passes > 1 ? (u % stages) * stage_elems : 0);
-        for (int r = tid / FEW_COLS; r < here; r += 256 / FEW_COLS) {
+        for (int r = tid / COLS; r < here; r += 256 / COLS) {
             unsigned long long acc[MR];
 #pragma unroll
             for (int m = 0; m < MR; ++m) acc[m] = 0ull;
@@ -337,26 +337,26 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
                 for (int i = 0; k0 + i * PER < K; ++i) unit(i);
             }
 #pragma unroll
-            for (int m = 0; m < MR; ++m) sums[(r * MR + m) * FEW_COLS + col] = both(acc[m]);
+            for (int m = 0; m < MR; ++m) sums[(r * MR + m) * COLS + col] = both(acc[m]);
         }
         __syncthreads();
-        if (tid >= MR * FEW_COLS) continue;
+        if (tid >= MR * COLS) continue;
         {
-            const float* mine = sums + om * FEW_COLS + on;
+            const float* mine = sums + om * COLS + on;
             int r = 0;
             for (; r + 16 <= here; r += 16) {              // all loads first
                 float v[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = mine[(r + i) * MR * FEW_COLS];
+                for (int i = 0; i < 16; ++i) v[i] = mine[(r + i) * MR * COLS];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) total += v[i];
             }
-            for (; r < here; ++r) total += mine[r * MR * FEW_COLS];
+            for (; r < here; ++r) total += mine[r * MR * COLS];
         }
         if (u % passes != passes - 1) continue;
-        const int m = m0 + om, n = (blockIdx.x + u / passes * gridDim.x) * FEW_COLS + on;
+        const int m = m0 + om, n = (blockIdx.x + u / passes * gridDim.x) * COLS + on;
         // the gate of a pair: its second column is the neighbouring thread's
-        const float right = __shfl_down_sync(MR * FEW_COLS >= 32 ? 0xffffffffu : (1u << (MR * FEW_COLS % 32)) - 1u, total, 1);
+        const float right = __shfl_down_sync(MR * COLS >= 32 ? 0xffffffffu : (1u << (MR * COLS % 32)) - 1u, total, 1);
         if (m < M && n < N) {
             const size_t at = (size_t)z * so + (size_t)m * ldo + n;
             if (EPI == TB_EPI_SWIGLU) { if (n % 2 == 0) stf((T*)out_ + (size_t)z * so + (size_t)m * ldo + n / 2, tb_gated(act, limit, total, right)); }
@@ -386,32 +386,35 @@ bool aligned(const Product& p, int per) {
            (p.batch == 1 || (p.sx % per == 0 && p.sw % per == 0));
 }
 
-template <typename T, int EPI, int MR, bool VEC>
+template <typename T, int EPI, int MR, int COLS, bool VEC>
 void few_launch(const Product& p) {
-    const int runs = (p.K + SUM_RUN - 1) / SUM_RUN, groups = (p.N + FEW_COLS - 1) / FEW_COLS, others = (p.M + MR - 1) / MR * p.batch;
+    const int runs = (p.K + SUM_RUN - 1) / SUM_RUN, groups = (p.N + COLS - 1) / COLS, others = (p.M + MR - 1) / MR * p.batch;
     // One unit a block while the blocks fit the chip once: all of K at once.  Else passes of 32 runs (one a thread) and equal shares of the
     // column groups, for two blocks an SM with two stages each where their memory fits (one computes while the other waits), or
     // one block with up to four.
     const bool once = (long long)groups * others <= SMS;
     int pass = once ? 96 : 32;
     if (pass > runs) pass = runs;
-    while (few_smem<T, MR>(pass, 1, pass >= runs) > 200 * 1024) --pass;
-    const int passes = (runs + pass - 1) / pass, two = few_smem<T, MR>(pass, 2, passes == 1) <= 112 * 1024;
+    while (few_smem<T, MR, COLS>(pass, 1, pass >= runs) > 200 * 1024) --pass;
+    const int passes = (runs + pass - 1) / pass, two = few_smem<T, MR, COLS>(pass, 2, passes == 1) <= 112 * 1024;
     const int room = (two ? 2 : 1) * SMS / others > 0 ? (two ? 2 : 1) * SMS / others : 1, each = (groups + room - 1) / room, x = (groups + each - 1) / each;
     const long long units = (long long)((groups + x - 1) / x) * passes;
     int stages = units < (two ? 2 : 4) ? (int)units : (two ? 2 : 4);
-    while (stages > 1 && few_smem<T, MR>(pass, stages, passes == 1) > 220 * 1024) --stages;
-    if (stages == 1 && units > 1) { stages = 2; while (few_smem<T, MR>(pass, stages, false) > 220 * 1024) --pass; }
-    const size_t smem = few_smem<T, MR>(pass, stages, (runs + pass - 1) / pass == 1);
+    while (stages > 1 && few_smem<T, MR, COLS>(pass, stages, passes == 1) > 220 * 1024) --stages;
+    if (stages == 1 && units > 1) { stages = 2; while (few_smem<T, MR, COLS>(pass, stages, false) > 220 * 1024) --pass; }
+    const size_t smem = few_smem<T, MR, COLS>(pass, stages, (runs + pass - 1) / pass == 1);
     const dim3 grid(x, (p.M + MR - 1) / MR, p.batch);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(gemm_few_kernel<T, EPI, MR, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    tb_launch(gemm_few_kernel<T, EPI, MR, VEC>, grid, 256, smem, p.stream, (const T*)p.X, (const T*)p.W, p.out, p.M, p.N, p.K, p.ldx, p.ldo,
+    if (smem > 48 * 1024) cudaFuncSetAttribute(gemm_few_kernel<T, EPI, MR, COLS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    tb_launch(gemm_few_kernel<T, EPI, MR, COLS, VEC>, grid, 256, smem, p.stream, (const T*)p.X, (const T*)p.W, p.out, p.M, p.N, p.K, p.ldx, p.ldo,
               p.sx, p.sw, p.so, pass, stages, p.act, p.limit);
 }
 template <typename T, int EPI, int MR>
 void few_rows(const Product& p) {
-    if (aligned<T>(p, 16 / (int)sizeof(T))) few_launch<T, EPI, MR, true>(p);
-    else few_launch<T, EPI, MR, false>(p);
+    // 32 columns a unit where a column has at most eight runs (with eight columns most of the block would have no run: sixteen heads'
+    // products of 8 rows, 576 columns of K = 128, bfloat16: 9.4 -> 4.7 us)
+    if (!aligned<T>(p, 16 / (int)sizeof(T))) few_launch<T, EPI, MR, 8, false>(p);
+    else if (p.K <= 8 * SUM_RUN) few_launch<T, EPI, MR, 32, true>(p);
+    else few_launch<T, EPI, MR, 8, true>(p);
 }
 
 template <typename T, int EPI, int RI, bool VEC>
