@@ -213,7 +213,8 @@ gemm_simt_kernel(const T* X, const T* W, void* out_,
 // number of banks and a run of X likewise, so that a warp's eight columns and four runs do not collide.  The run sums meet in shared
 // memory and are added in order by a thread an output.  Each weight is read from memory once for MR rows; rows beyond
 // are further blocks, which find the weights in L2.  Three rows: 1,024 columns
-// of K = 2,816 in 7.1 us, 5,632 of K = 1,024 in 12.9, 32,768 in 59 (64 x 64 tiles: 189, 87 and 204 us).
+// of K = 2,816 in 6.4 us, 5,632 of K = 1,024 in 10.0, 32,768 in 30.5 (64 x 64 tiles: 189, 87 and 204 us; with copies of sixteen bytes a
+// thread, and one warp that issued, added and waited in turn: 7.1, 12.9 and 59).
 template <typename T> constexpr int few_run() { return SUM_RUN + 16 / (int)sizeof(T); }           // elements from a run to the next in shared memory
 template <typename T> __host__ __device__ constexpr int few_col(int pass) { return pass * SUM_RUN + 16 / (int)sizeof(T); }      // a column of weights
 template <typename T> __host__ __device__ constexpr int few_row(int pass) { return pass * few_run<T>(); }                         // a row of X
@@ -428,8 +429,8 @@ void tiles(const Product& p) {
 template <typename T, int EPI>
 void product(const Product& p, bool few) {
     // Few rows: up to 64 while the column groups of all groups of eight rows stay near a unit's time (measured, K = 1,024, few / tiles:
-    // 64 rows of 1,024 columns 23 / 47 us, of 2,048 37 / 42; 5,632 columns 32 rows 50 / 69, 48 rows 74 / 70; 32,768 columns
-    // 8 rows 69 / 140, 24 rows 200 / 141).
+    // 64 rows of 1,024 columns 20 / 47 us, of 2,048 31 / 42; 5,632 columns 32 rows 41 / 69, 64 rows 81 / 70; 32,768 columns
+    // 8 rows 56 / 140, 24 rows 168 / 141).
     if (few || (p.M <= 64 && (long long)((p.M + 7) / 8) * p.N * p.batch <= 32768)) {
         if (p.M == 1) few_rows<T, EPI, 1>(p);
         else if (p.M == 2) few_rows<T, EPI, 2>(p);

@@ -264,9 +264,10 @@ __global__ void __launch_bounds__(128) lightning_scan_vec_kernel(LightningArgs a
 // and, transposed, k'_r = decay^(n-1-r) k_r.  lightning_chunk_kernel, a block for 16 value columns of a head, the state's slice in
 // registers and in shared memory behind the chunk's values: one product A . [v; S] and one k'^T v a chunk, the next chunk's rows on
 // their way meanwhile.  Every operand lies along the dimension that is summed over, so that sums over even and over odd
-// places are one two-element multiply-add and no operand has to be doubled.  16 columns: 128 blocks for one sequence of 16 heads of 128.  Bound by the FMA pipes, 2,560 cycles a chunk.
-// 2,000 tokens, 16 heads of 128 x 128: 34 us and 158 us, of which the outputs' product takes 50, the state's 30 and the
-// wait for the rows 22.
+// places are one two-element multiply-add and no operand has to be doubled.  16 columns:
+// 128 blocks for one sequence of 16 heads of 128.  The FMA pipes would need 2,560 cycles a chunk (43 us of the second figure).
+// 2,000 tokens, 16 heads of 128 x 128: 34 us and 146 us, of which the outputs' product takes about 50 and the
+// state's 30; the rest is barriers, the merge of the warps' parts, values and stores.
 constexpr int CHUNK = 64, VCOLS = 16;
 constexpr int CHUNKED_FROM = 32;        // tokens of the longest run from which the chunked form is the faster one
 
