@@ -229,3 +229,32 @@ def test_a_row_of_router_logits_that_are_not_numbers_chooses_experts_there_are(K
     ids, wts = torch.full((3, 2), -1, dtype=torch.int32, device="cuda"), torch.empty(3, 2, device="cuda")
     K.moe_route(z, 8, 2, False, ids, wts, None, stream())
     assert bool(((ids >= 0) & (ids < 8)).all()) and ids[1].tolist() == [7, 6]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,H", [(512, 1024), (513, 2048), (8192, 2052), (8193, 2564), (8192, 4092), (512, 4096), (700, 4100), (8192, 8192)])
+def test_norms_of_long_prompts_are_the_bits_of_short_ones(K, dtype, rows, H):
+    """The kernel of 512 rows and more against the one of fewer, at both ends of every number of threads and units."""
+    g = torch.Generator().manual_seed(H)
+    x, w = (torch.randn(rows, H, generator=g) * 3).cuda(), (1 + 0.1 * torch.randn(H, generator=g)).cuda()
+    y, few = torch.empty(rows, H, dtype=dtype, device="cuda"), torch.empty(rows, H, dtype=dtype, device="cuda")
+    K.rmsnorm(x, w, y, 1e-3, stream())
+    for a in range(0, rows, 500):
+        K.rmsnorm(x[a:a + 500], w, few[a:a + 500], 1e-3, stream())
+    assert torch.equal(y, few)
+    want = x.double() / torch.sqrt((x.double() ** 2).mean(1, keepdim=True) + 1e-3) * w.double()
+    assert float((y.double() - want).norm() / want.norm()) < (1e-6 if dtype == torch.float32 else 4e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,N,Kd,batch", [(1, 576, 128, 16), (8, 40, 256, 3), (9, 33, 264, 2), (64, 100, 8, 5)])
+def test_products_of_heads_side_by_side(K, dtype, M, N, Kd, batch):
+    g = torch.Generator().manual_seed(N)
+    x = torch.randn(M, batch * Kd, generator=g).to(dtype).cuda()
+    w = torch.randn(batch, N, Kd, generator=g).to(dtype).cuda()
+    out = torch.full((M, batch * N + 8), 7.0, dtype=dtype, device="cuda")
+    K.gemm_simt_batched(x[:, :Kd], w, out[:, :N], K.EPI_STORE, stream(), batch, Kd, N)
+    for z in range(batch):
+        want = x[:, z * Kd:(z + 1) * Kd].double() @ w[z].double().t()
+        assert float((out[:, z * N:(z + 1) * N].double() - want).norm() / want.norm()) < (1e-6 if dtype == torch.float32 else 4e-3)
+    assert bool((out[:, batch * N:] == 7.0).all())
