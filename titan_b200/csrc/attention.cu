@@ -8,9 +8,10 @@
 //   tb_attn_merge    log-sum-exp merge of the chunks in chunk order (a block per sequence and head, or, with
 //                    AttnArgs.pair_lambda, per sequence and pair of heads, whose difference it finishes)
 //
-// One warp per (query, head): a lane scores one key per round with the whole query in shared
+// The general kernels have one warp per (query, head): a lane scores one key per round with the whole query in shared
 // memory, the warp folds 32 scores into the running softmax, then every lane accumulates its
 // output dims over the 32 values.  Scores, softmax and PV are float32 with precise expf.
+// Plain float32 prompts go in tiles of queries and keys, decode steps with rows of up to 32 16-byte units with lanes across a row.
 // A chunk's borders depend on the sequence's own length only, never on the batch.
 //
 // berniehans/titan: flash_attention_2_kernel (engine/engine-cuda/kernels/flash_attention_2.cu:22-106),

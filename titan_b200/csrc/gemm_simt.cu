@@ -6,12 +6,12 @@
 // (engine/engine-cuda/kernels/gemm_quant.cu:2331-2363 gemm_f32_kernel, :3365-3499 batched), which
 // fuse the residual into the epilogue (:3489-3493) and SwiGLU into gate/up (:2589).
 //
-// Epilogues:
 // One order of sums for every kernel here, whatever M: in each run of SUM_RUN neighbouring k the products at even and those at
 // odd k are added one after the other (fused multiply-adds from zero), then the two sums, and the runs' sums one after the
 // other.  A row's result is then the same bits alone and beside any other rows, in a decode step as in a prompt.  Even
 // and odd, because the two are neighbours in memory and one two-element instruction (fma.rn.f32x2) works on both.
 //
+// Epilogues:
 //   TB_EPI_STORE   out[m][n] = acc                      (compute dtype), or an activation of it (activation.h)
 //   TB_EPI_F32     out[m][n] = acc                      (float32: logits)
 //   TB_EPI_ADD     out[m][n] += acc                     (float32 residual stream, in place)
