@@ -117,6 +117,38 @@ def test_decode_with_lanes_across_a_row(K, dtype, tol, nh, nkv, hd, window, chun
         assert float((out[i].cpu().double().view(nh, hd) - want).norm() / want.norm()) < tol, i
 
 
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 4e-6), (torch.bfloat16, 6e-3)])
+@pytest.mark.parametrize("nh,nkv,hd,hd_v,alias,blocks,window,keep,chunk,page", [
+    (17, 1, 64, 64, 0, 0, 0, 0, 32, 64), (33, 1, 40, 40, 0, 0, 0, 0, 256, 64), (40, 2, 72, 72, 0, 0, 50, 0, 32, 64), (8, 2, 64, 64, 0, 4, 0, 0, 64, 64),
+    (12, 1, 96, 64, 1, 3, 0, 0, 32, 64), (8, 4, 8, 8, 0, 0, 40, 5, 32, 64), (3, 1, 24, 24, 0, 0, 33, 70, 64, 64), (6, 2, 16, 16, 0, 0, 0, 0, 64, 48)])
+def test_decode_with_lanes_across_a_row_in_every_form(K, dtype, tol, nh, nkv, hd, hd_v, alias, blocks, window, keep, chunk, page):
+    """More heads on a kv head than a block has warps, blocks that share a kv head, kept first tokens that end inside a split, values that are the
+    head of their key's row, splits that a window has left behind, pages of no power of two."""
+    g = torch.Generator().manual_seed(hd + nh)
+    slots, lens = [2, 0, 4, 1], [1, 50, 3 * chunk, 5 * chunk - 3]
+    paged = Paged(K, slots, lens, nkv, hd, dtype, page=page)
+    ks, vs = ([torch.randn(n, nkv, hd, generator=g).to(dtype) for n in lens] for _ in range(2))
+    for i, s in enumerate(slots):
+        for p in range(lens[i]):
+            paged.put(s, p, ks[i][p], vs[i][p])
+    q = torch.randn(4, nh, hd, generator=g).to(dtype)
+    lay = layout_for(slots, [n - 1 for n in lens], [1] * 4)
+    qd, out = q.reshape(4, -1).cuda(), torch.empty(4, nh * hd_v, dtype=dtype, device="cuda")
+    splits = -(-max(lens) // chunk)
+    scratch = torch.full((4 * nh * splits * (hd_v + 2),), math.nan, device="cuda")
+    a = K.AttnArgs()
+    a.q, a.q_stride, a.out, a.out_stride = qd.data_ptr(), nh * hd, out.data_ptr(), nh * hd_v
+    a.cache, a.batch, a.nh, a.nkv, a.hd, a.window, a.scale = paged.view, lay.c_struct(), nh, nkv, hd, window, 0.3
+    a.chunk, a.n_splits, a.scratch, a.hd_v, a.v_alias, a.head_blocks, a.keep_first = chunk, splits, scratch.data_ptr(), hd_v if hd_v != hd else 0, alias, blocks, keep
+    K.attn_decode(a, dtype, stream())
+    for i, n in enumerate(lens):
+        seen = [p for p in range(n) if not window or p > n - 1 - window or p < keep]
+        kk = ks[i][seen].double().repeat_interleave(nh // nkv, 1)
+        vv = (ks[i] if alias else vs[i])[seen][..., :hd_v].double().repeat_interleave(nh // nkv, 1)
+        want = torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q[i].double(), kk) * 0.3, -1), vv)
+        assert float((out[i].cpu().double().view(nh, hd_v) - want).norm() / want.norm()) < tol, i
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("dk,dv,plain", [(8, 16, 0), (64, 17, 0), (65, 40, 1), (128, 33, 0)])
 def test_recurrence_in_chunks(K, dtype, dk, dv, plain):

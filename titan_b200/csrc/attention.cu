@@ -449,17 +449,19 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_decode_kernel(AttnArgs a)
 // The same for rows of up to 32 16-byte units (float32: 128 elements, bfloat16: 256).  LPK lanes share a key, a 16-byte unit of its row
 // each, so that a load covers whole rows of 32 / LPK keys (in the kernel above every lane walks a row of its own, and a warp a
 // whole split).  Each group of LPK lanes is a stream of its own: keys st, st + streams, ... of the split, eight keys and
-// values requested at once, an own running softmax.  The streams of a head, those of up to sixteen warps, are merged in shared memory.
+// values requested at once, an own running softmax.  A warp merges its streams by shuffles; ``share`` warps, a power of two, take
+// a head together and meet in shared memory.  They are as many as leave a stream a whole round of eight keys of the launch's ``chunk``
+// (more only add parts to merge: 32 keys a split, 64 sequences of 2,000, 8 heads of 8: 2,700 us with sixteen warps a head).
 // Bound by the latency of the loads at a few hundred keys a split: three
 // sequences of 500 tokens, 16 heads of 64 on 8, float32: 210 -> 12.3 us a layer.
 constexpr int VEC_WARPS = 16, VEC_KEYS = 8;
 
 template <typename T, int LPK>
-__global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArgs a, int share) {
     constexpr int PER = 16 / (int)sizeof(T), STREAMS = 32 / LPK;
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ float parts[];                   // [VEC_WARPS * STREAMS][hdv + 2]
+    extern __shared__ float parts[];                   // [warps][hdv + 2]: what a warp made of its keys (share > 1)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, unit = lane % LPK;
     const int blocks_y = a.head_blocks > 0 ? a.head_blocks : a.nkv;
     const int b = blockIdx.x, kh = (int)blockIdx.y * a.nkv / blocks_y, split = blockIdx.z;
@@ -467,21 +469,20 @@ __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArg
     const int len = a.batch.kv_len[b];
     const int keys = tb_split_keys(len, a.chunk, a.n_splits);
     if ((long long)split * keys >= len) return;     // the merge reads ceil(len / keys) splits only
-    int share = 1;                                     // warps a head: two, four, eight or sixteen where there are so many times as many warps
-    while (share * 2 * group <= VEC_WARPS) share *= 2;
     const int pos = len - 1;
     const int slot = a.batch.slot_of_seq[b];
     const int wlo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
     const int lo = max(wlo, split * keys), hi = min(len, (split + 1) * keys);
     // the kept first tokens that lie in this split and before the window
     const int klo = split * keys, khi = a.window > 0 ? min(min(a.keep_first, wlo), hi) : 0;
+    if (lo >= hi && a.keep_first <= 0) return;         // a split before the window: the merge begins behind it
     const T* cache = (const T*)a.cache.storage;
     const size_t vhalf = a.v_alias ? 0 : kv_half_elems(a.cache);
     const int shift = page_shift(a.cache);
     const int streams = share * STREAMS, st = (warp % share) * STREAMS + lane / LPK;
-    const int at = unit * PER;
+    const int at = unit * PER, at_once = (int)(blockDim.x >> 5) / share;
     const bool key_part = at < hd, value_part = at < hdv;
-    for (int g0 = 0; g0 < group; g0 += VEC_WARPS / share) {
+    for (int g0 = 0; g0 < group; g0 += at_once) {
         const int g = g0 + warp / share;
         const int h = (int)blockIdx.y * group + min(g, group - 1);
         float q[PER], acc[PER], m = -FLT_MAX, l = 0.f;
@@ -533,30 +534,43 @@ __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArg
             if (klo < khi) attend(klo, khi);
             if (lo < hi) attend(lo, hi);
         }
-        float* mine = parts + (warp * STREAMS + lane / LPK) * (hdv + 2);
-        if (share == 1) __syncwarp();                  // (the warp has read its streams of the head before)
+        // the warp's streams as one
+        float top = m;
 #pragma unroll
-        for (int e = 0; e < PER; ++e) if (at + e < hdv) mine[at + e] = acc[e];
-        if (unit == 0) { mine[hdv] = m; mine[hdv + 1] = l; }
-        if (share > 1) __syncthreads(); else __syncwarp();
-        if (warp % share != 0 || g >= group) continue;
-        const float* of = parts + warp * STREAMS * (hdv + 2);      // the head's streams lie side by side
+        for (int o = LPK; o < 32; o *= 2) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float mine = expf(m - top);              // (a stream that saw no key: its sums are zero)
+        l *= mine;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) acc[e] *= mine;
+#pragma unroll
+        for (int o = LPK; o < 32; o *= 2) {
+            l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+            for (int e = 0; e < PER; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+        }
         float* part = a.scratch + ((size_t)(b * a.nh + h) * a.n_splits + split) * (hdv + 2);
-        float top = -FLT_MAX, sum = 0.f;
-        for (int w = 0; w < streams; ++w) if (of[w * (hdv + 2) + hdv + 1] != 0.f) top = fmaxf(top, of[w * (hdv + 2) + hdv]);
-        for (int d = lane; d < hdv; d += 32) {
-            float o = 0.f;
-            for (int w = 0; w < streams; ++w) {
+        float* to = share == 1 ? part : parts + warp * (hdv + 2);
+        if (g0 > 0 && share > 1) __syncthreads();      // the heads before have been read
+        if (lane < LPK && (share > 1 || g < group)) {
+#pragma unroll
+            for (int e = 0; e < PER; ++e) if (at + e < hdv) to[at + e] = acc[e];
+            if (unit == 0) { to[hdv] = top; to[hdv + 1] = l; }
+        }
+        if (share == 1) continue;
+        __syncthreads();
+        if (g >= group) continue;                      // (every warp takes every turn of the loop)
+        const float* of = parts + warp / share * share * (hdv + 2);      // the head's warps lie side by side
+        float all = -FLT_MAX, sum = 0.f;
+        for (int w = 0; w < share; ++w) all = fmaxf(all, of[w * (hdv + 2) + hdv]);
+        for (int d = (warp % share) * 32 + lane; d < hdv + 1; d += share * 32) {      // (place hdv: the weights' sum)
+            sum = 0.f;
+            for (int w = 0; w < share; ++w) {
                 const float* p = of + w * (hdv + 2);
-                if (p[hdv + 1] != 0.f) o = fmaf(expf(p[hdv] - top), p[d], o);      // (a stream that saw no key has l = 0)
+                sum = fmaf(expf(p[hdv] - all), p[d < hdv ? d : hdv + 1], sum);
             }
-            part[d] = o;
+            part[d < hdv ? d : hdv + 1] = sum;
         }
-        for (int w = 0; w < streams; ++w) {
-            const float* p = of + w * (hdv + 2);
-            if (p[hdv + 1] != 0.f) sum = fmaf(expf(p[hdv] - top), p[hdv + 1], sum);
-        }
-        if (lane == 0) { part[hdv] = top; part[hdv + 1] = sum; }
+        if (warp % share == 0 && lane == 0) part[hdv] = all;
     }
 }
 
@@ -763,9 +777,14 @@ extern "C" int tb_attn_decode(const AttnArgs* args, int dtype, cudaStream_t stre
     dim3 grid(a.batch.B, a.head_blocks > 0 ? a.head_blocks : a.nkv, a.n_splits);
     const int width = a.hd > value_width(a) ? a.hd : value_width(a), units = (width * (dtype == TB_F32 ? 4 : 2) + 15) / 16;
     if (units <= 32 && a.hd % 8 == 0 && value_width(a) % (dtype == TB_F32 ? 4 : 8) == 0 && (uintptr_t)a.cache.storage % 16 == 0) {
-        // lanes a key: as few as hold its row
-#define ATT_VEC(TT, L) tb_launch(attn_decode_vec_kernel<TT, L>, grid, VEC_WARPS * 32, (size_t)VEC_WARPS * (32 / L) * (value_width(a) + 2) * sizeof(float), stream, a)
-#define ATT_VEC_ANY(TT) do { if (units <= 4) ATT_VEC(TT, 4); else if (units <= 8) ATT_VEC(TT, 8); else if (units <= 16) ATT_VEC(TT, 16); else ATT_VEC(TT, 32); } while (0)
+        // lanes a key: as few as hold its row; warps a head: see the kernel (a rule of the launch's numbers, not of the lengths)
+        const int lanes = units <= 4 ? 4 : (units <= 8 ? 8 : (units <= 16 ? 16 : 32)), group = a.nh / (int)grid.y;
+        const int turns = (group + VEC_WARPS - 1) / VEC_WARPS, heads = (group + turns - 1) / turns;      // equal turns
+        int share = 1;
+        while (share * 2 * heads <= VEC_WARPS && share * 2 * (32 / lanes) * VEC_KEYS <= a.chunk) share *= 2;
+        const int warps = share * heads;
+#define ATT_VEC(TT, L) tb_launch(attn_decode_vec_kernel<TT, L>, grid, warps * 32, (size_t)warps * (value_width(a) + 2) * sizeof(float), stream, a, share)
+#define ATT_VEC_ANY(TT) do { if (lanes == 4) ATT_VEC(TT, 4); else if (lanes == 8) ATT_VEC(TT, 8); else if (lanes == 16) ATT_VEC(TT, 16); else ATT_VEC(TT, 32); } while (0)
         if (dtype == TB_F32) ATT_VEC_ANY(float); else ATT_VEC_ANY(__nv_bfloat16);
 #undef ATT_VEC_ANY
 #undef ATT_VEC
