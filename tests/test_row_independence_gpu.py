@@ -117,6 +117,52 @@ def test_decode_with_lanes_across_a_row(K, dtype, tol, nh, nkv, hd, window, chun
         assert float((out[i].cpu().double().view(nh, hd) - want).norm() / want.norm()) < tol, i
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window,ring,sink", [(4, 2, 64, 0, 0, False), (5, 5, 24, 0, 0, True), (8, 2, 128, 0, 0, False), (3, 1, 72, 70, 128, True), (2, 2, 16, 64, 64, False)])
+def test_float32_attention_is_the_same_bits_however_a_prompt_is_cut(K, nh, nkv, hd, window, ring, sink):
+    """Runs on both sides of the border between rows and tiles, alone and beside longer ones, on a cache that keeps all keys and on a ring
+    whose overwritten rows are not finite: each query against 64 bits, and the same bits as in the whole prompt."""
+    g = torch.Generator().manual_seed(hd + nh)
+    n, scale = 330, 0.3
+    ks, vs = (torch.randn(n, nkv, hd, generator=g) for _ in range(2))
+    q = torch.randn(n, nh, hd, generator=g)
+    sinks = torch.randn(nh, generator=g).cuda() if sink else None
+
+    def step(pieces):
+        """The outputs of a step with the run [a, z) of the one sequence for every (a, z), each run on a slot of its own."""
+        slots = list(range(len(pieces)))
+        paged = Paged(K, slots, [z for _, z in pieces], nkv, hd, torch.float32, ring_rows=ring)
+        if ring:
+            paged.storage.fill_(math.nan)
+        for s, (a, _) in zip(slots, pieces):
+            for p in range(max(0, a - ring) if ring else 0, a):
+                seen = not window or p > a - window                    # rows that no query of the run sees any more hold anything
+                paged.put(s, p, ks[p] if seen else torch.full((nkv, hd), math.inf), vs[p] if seen else torch.full((nkv, hd), math.nan))
+        rows = torch.cat([torch.cat([ks[a:z].reshape(z - a, -1), vs[a:z].reshape(z - a, -1)], 1) for a, z in pieces]).cuda()
+        qd = torch.cat([q[a:z] for a, z in pieces]).reshape(-1, nh * hd).cuda()
+        lay, out = layout_for(slots, [a for a, _ in pieces], [z - a for a, z in pieces]), torch.empty_like(qd)
+        a = K.AttnArgs()
+        a.q, a.q_stride, a.kv_new, a.kv_stride, a.out, a.out_stride = qd.data_ptr(), nh * hd, rows.data_ptr(), 2 * nkv * hd, out.data_ptr(), nh * hd
+        a.cache, a.batch, a.nh, a.nkv, a.hd, a.window, a.scale = paged.view, lay.c_struct(), nh, nkv, hd, window, scale
+        if sink:
+            a.sink = sinks.data_ptr()
+        K.attn_prefill(a, torch.float32, stream())
+        return torch.split(out.view(-1, nh, hd).cpu(), [z - a for a, z in pieces])
+
+    whole = step([(0, n)])[0]
+    for p in range(0, n, 7):
+        lo = max(0, p - window + 1) if window else 0
+        kk, vv = (t[lo:p + 1].double().repeat_interleave(nh // nkv, 1) for t in (ks, vs))
+        s = torch.einsum("hd,nhd->hn", q[p].double(), kk) * scale
+        if sink:
+            s = torch.cat([s, sinks.cpu().double()[:, None]], 1)
+        want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1)[:, :len(kk)], vv)
+        assert float((whole[p].double() - want).norm() / want.norm()) < 4e-6, p
+    for pieces in ([(0, 1)], [(5, 6), (9, 12), (100, 131)], [(0, 31), (31, 63), (63, 64), (64, 130), (200, 201)], [(63, 65), (300, 330)], [(0, 32), (32, 64)],
+                   [(i, i + 1) for i in range(40, 80)] + [(130, 194)]):
+        for (a, z), got in zip(pieces, step(pieces)):
+            assert torch.equal(got, whole[a:z]), (a, z, pieces)
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 4e-6), (torch.bfloat16, 6e-3)])
 @pytest.mark.parametrize("nh,nkv,hd,hd_v,alias,blocks,window,keep,chunk,page", [
     (17, 1, 64, 64, 0, 0, 0, 0, 32, 64), (33, 1, 40, 40, 0, 0, 0, 0, 256, 64), (40, 2, 72, 72, 0, 0, 50, 0, 32, 64), (8, 2, 64, 64, 0, 4, 0, 0, 64, 64),

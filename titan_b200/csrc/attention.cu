@@ -11,7 +11,8 @@
 // The general kernels have one warp per (query, head): a lane scores one key per round with the whole query in shared
 // memory, the warp folds 32 scores into the running softmax, then every lane accumulates its
 // output dims over the 32 values.  Scores, softmax and PV are float32 with precise expf.
-// Plain float32 prompts go in tiles of queries and keys, decode steps with rows of up to 32 16-byte units with lanes across a row.
+// Plain float32 prompts go in tiles of queries and keys (runs of a few tokens by the row, in the same order of sums), decode steps with rows of up to 32
+// 16-byte units with lanes across a row.
 // A chunk's borders depend on the sequence's own length only, never on the batch.
 //
 // berniehans/titan: flash_attention_2_kernel (engine/engine-cuda/kernels/flash_attention_2.cu:22-106),
@@ -207,11 +208,171 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_prefill_kernel(AttnArgs a
 }
 
 // ------------------------------------------------------------------ prefill in float32, tiles of queries
-// grid (query tiles of every sequence, nh), 256 threads: 64 queries of one head against tiles of 64 keys.  The kernel
+// Runs of TILE_FROM tokens and more: grid (query tiles, nh), 256 threads: 64 queries of one head against tiles of 64 keys.  The kernel
 // above reads every key and value once a query and head (L1 and L2 bound: 637 us for 1,125 tokens of three sequences,
 // 16 heads of 64); here a tile of keys serves 64 queries.  Scores and outputs are sums in registers, 4 x 4 and
 // 4 x HD / 16 a thread, two at a time (fma.rn.f32x2: float32, rounded as fmaf rounds), the weights pass through shared memory.
 // Bound by the FMA pipes and shared memory: 119 us for the tokens above.  HD: the head size rounded up to 64 or 128, the rest is zero.
+// Shorter runs (running sequences beside a prompt's piece, drafts): attend_row, a warp a query and head, which walks the same
+// 64 keys at a time and adds in the same order, so that a query is the same bits however its prompt is cut.  By the row / in tiles, 16 heads
+// of 64: 2 tokens at 4,000 273 / 535 us, 32 prompts of 20 19 / 25, 64 sequences of 100 with 1 or 2 tokens each 17 / 91; from 32 tokens on
+// a tile is the faster form (a prompt of 64: 20 / 11).  Where a step has both kinds, one launch holds them: beside 63 single tokens at 4,000 the
+// tiles of 64 more cost nothing.
+constexpr int TILE_FROM = 32;
+
+// The run of the step that holds the ``left``-th of the things that count(tokens of a run) counts, -1 behind the last; ``left`` becomes the
+// place within the run.  A warp's lanes look at 32 runs at a time; every lane returns the same.
+template <typename F>
+__device__ __forceinline__ int find_run(const TbBatch& batch, int& left, F count) {
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < batch.B; s0 += 32) {
+        const int s = s0 + lane, mine = s < batch.B ? count(batch.q_start[s + 1] - batch.q_start[s]) : 0;
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            const int u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+        if (left < total) {
+            const int at = __ffs(__ballot_sync(0xffffffffu, upto > left)) - 1;
+            left -= __shfl_sync(0xffffffffu, upto - mine, at);
+            return s0 + at;
+        }
+        left -= total;
+    }
+    return -1;
+}
+
+// One head of one query of a short run by one warp, VW neighbouring elements of the head a lane.  A lane scores two neighbouring keys of 64;
+// weights and value rows' addresses pass through the warp's piece of shared memory, sixteen value rows are requested at once.
+// Bound by the latency of a key's row (a lane walks it alone: a sum over a row has one order).
+constexpr int TILE_Q = 64, TILE_K = 64, TILE_P = 68;       // rows of 64 in shared memory lie 68 apart: 16-byte aligned, spread over the banks
+template <int VW> struct __align__(16) RowShared {
+    float q[32 * VW];
+    const float* v[TILE_K];
+    float p[TILE_K];
+};
+
+template <int VW>
+__device__ __forceinline__ void attend_row(const AttnArgs& a, RowShared<VW>& sh, int item) {
+    const int lane = threadIdx.x & 31, hd = a.hd, h = item % a.nh, kh = h / (a.nh / a.nkv);
+    int place = item / a.nh;
+    const int seq = find_run(a.batch, place, [](int n) { return n < TILE_FROM ? n : 0; });
+    if (seq < 0) return;
+    const int t0 = a.batch.q_start[seq], first = a.batch.start_pos[seq], slot = a.batch.slot_of_seq[seq], pos = first + place;
+    const int first_new = a.kv_new ? first : 0x7fffffff;
+    const float* knew = (const float*)a.kv_new;
+    const float* cache = (const float*)a.cache.storage;
+    const size_t vhalf = cache ? kv_half_elems(a.cache) : 0;
+    const int shift = page_shift(a.cache), at = lane * VW;
+    {
+        const float* q = (const float*)a.q + (size_t)(t0 + place) * a.q_stride + (size_t)h * hd;
+        for (int d = lane; d < hd; d += 32) sh.q[d] = q[d];
+        __syncwarp();
+    }
+    float m = -FLT_MAX, l = 0.f, o[VW];
+#pragma unroll
+    for (int e = 0; e < VW; ++e) o[e] = 0.f;
+    const int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    for (int k0 = lo & ~(TILE_K - 1); k0 <= pos; k0 += TILE_K) {
+        const float* row[2] = {nullptr, nullptr};
+        bool ok[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int key = k0 + 2 * lane + j;
+            ok[j] = key <= pos && key >= lo;
+            if (!ok[j]) continue;
+            if (key >= first_new) {
+                row[j] = knew + (size_t)(t0 + key - first_new) * a.kv_stride + (size_t)kh * hd;
+                sh.v[2 * lane + j] = row[j] + (size_t)a.nkv * hd;
+            } else {
+                row[j] = cache + row_offset(a.cache, slot, key, kh, shift);
+                sh.v[2 * lane + j] = row[j] + vhalf;
+            }
+        }
+        __syncwarp();
+        const int begin = max(0, lo - k0), end = min(TILE_K, pos + 1 - k0);
+        constexpr int AHEAD = 16;
+        float v[AHEAD][VW];
+        auto load_values = [&](int k) {
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const float* r = sh.v[min(k + u, end - 1)] + min(at, hd - VW);
+                if constexpr (VW == 4) { const float4 f = *reinterpret_cast<const float4*>(r); v[u][0] = f.x; v[u][1] = f.y; v[u][2] = f.z; v[u][3] = f.w; }
+                else if constexpr (VW == 2) { const float2 f = *reinterpret_cast<const float2*>(r); v[u][0] = f.x; v[u][1] = f.y; }
+                else v[u][0] = *r;
+            }
+        };
+        float s[2] = {0.f, 0.f};
+        if (ok[0] || ok[1]) {
+            const float* r0 = ok[0] ? row[0] : row[1];
+            const float* r1 = ok[1] ? row[1] : row[0];
+#pragma unroll 8
+            for (int d = 0; d < hd; d += 4) {
+                const float4 q4 = *reinterpret_cast<const float4*>(sh.q + d), x = *reinterpret_cast<const float4*>(r0 + d), y = *reinterpret_cast<const float4*>(r1 + d);
+                s[0] = fmaf(q4.x, x.x, s[0]); s[1] = fmaf(q4.x, y.x, s[1]);
+                s[0] = fmaf(q4.y, x.y, s[0]); s[1] = fmaf(q4.y, y.y, s[1]);
+                s[0] = fmaf(q4.z, x.z, s[0]); s[1] = fmaf(q4.z, y.z, s[1]);
+                s[0] = fmaf(q4.w, x.w, s[0]); s[1] = fmaf(q4.w, y.w, s[1]);
+            }
+        }
+        __syncwarp();
+        load_values(begin);                                // on their way while the weights are made
+        float top = -FLT_MAX, p[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            s[j] = __fmul_rn(s[j], a.scale);
+            if (ok[j]) top = fmaxf(top, s[j]);
+        }
+        const float m_new = fmaxf(m, warp_max(top)), alpha = expf(m - m_new);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) { p[j] = ok[j] ? expf(__fsub_rn(s[j], m_new)) : 0.f; sh.p[2 * lane + j] = p[j]; }
+        // the order of the tiles: four neighbouring keys one after the other, then the sixteen fours in pairs (on the odd lanes)
+        const float before = __shfl_up_sync(0xffffffffu, p[0] + p[1], 1);
+        float sum = (lane & 1 ? before : 0.f) + p[0] + p[1];
+#pragma unroll
+        for (int x = 2; x < 32; x *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+        l = __fmaf_rn(l, alpha, __shfl_sync(0xffffffffu, sum, 31));
+        m = m_new;
+#pragma unroll
+        for (int e = 0; e < VW; ++e) o[e] = __fmul_rn(o[e], alpha);
+        __syncwarp();
+        for (int k = begin; k < end; k += AHEAD) {
+            if (k > begin) load_values(k);
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+                if (k + u < end) {
+                    const float w = sh.p[k + u];
+#pragma unroll
+                    for (int e = 0; e < VW; ++e) o[e] = fmaf(w, v[u][e], o[e]);
+                }
+        }
+        __syncwarp();                                      // (weights and addresses have been read)
+    }
+    float scale = 1.f;
+    if (a.sink) {                                          // one more term of the denominator, against the larger of the two maxima
+        const float sk = a.sink[h], m_new = fmaxf(m, sk);
+        scale = expf(m - m_new);
+        l = __fmaf_rn(l, scale, expf(sk - m_new));
+    }
+    const float inv = scale / l;
+    float* out = (float*)a.out + (size_t)(t0 + place) * a.out_stride + (size_t)h * hd;
+#pragma unroll
+    for (int e = 0; e < VW; ++e) if (at < hd) out[at + e] = o[e] * inv;
+}
+
+// A step of short runs only: grid (items / 4), an item is a (token, head).
+template <int VW>
+__global__ void __launch_bounds__(ATT_WARPS * 32) attn_prefill_row_kernel(AttnArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ RowShared<VW> sh[ATT_WARPS];
+    const int warp = threadIdx.x >> 5;
+    const long long item = (long long)blockIdx.x * ATT_WARPS + warp;
+    if (item < (long long)a.batch.T * a.nh) attend_row<VW>(a, sh[warp], (int)item);
+}
+
 __device__ __forceinline__ void att_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
@@ -223,11 +384,10 @@ __device__ __forceinline__ unsigned long long att_twice(float v) {
 __device__ __forceinline__ float att_low(unsigned long long v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float att_high(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-constexpr int TILE_Q = 64, TILE_K = 64, TILE_P = 68;       // rows of 64 in shared memory lie 68 apart: 16-byte aligned, spread over the banks
 template <int HD> constexpr size_t tile_smem() { return (size_t)(2 * HD * TILE_P + TILE_K * HD + TILE_K * TILE_P) * sizeof(float); }
 
 template <int HD>
-__global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a, int tiles_x) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float sm_tile[];
@@ -237,16 +397,17 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
     float* pt = vs + TILE_K * HD;                          // [TILE_K][TILE_P]: weights, transposed
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int h = blockIdx.y, kh = h / (a.nh / a.nkv), hd = a.hd;
-    // which sequence, which tile of it; a sequence's last tiles, which see the most keys, start first
-    int seq = 0, tile = blockIdx.x, t0 = 0, n_new = 0;
-    for (; seq < a.batch.B; ++seq) {
-        t0 = a.batch.q_start[seq];
-        n_new = a.batch.q_start[seq + 1] - t0;
-        const int tiles = (n_new + TILE_Q - 1) / TILE_Q;
-        if (tile < tiles) { tile = tiles - 1 - tile; break; }
-        tile -= tiles;
+    if ((int)blockIdx.x >= tiles_x) {                      // short runs beside the long ones, eight (token, head) a block
+        const long long item = ((long long)(blockIdx.x - tiles_x) * gridDim.y + h) * 8 + (tid >> 5);
+        if (item < (long long)a.batch.T * a.nh) attend_row<HD / 32>(a, reinterpret_cast<RowShared<HD / 32>*>(sm_tile)[tid >> 5], (int)item);
+        return;
     }
-    if (seq == a.batch.B) return;
+    // which sequence, which tile of it; a sequence's last tiles, which see the most keys, start first
+    int tile = blockIdx.x;
+    const int seq = find_run(a.batch, tile, [](int n) { return n >= TILE_FROM ? (n + TILE_Q - 1) / TILE_Q : 0; });
+    if (seq < 0) return;
+    const int t0 = a.batch.q_start[seq], n_new = a.batch.q_start[seq + 1] - t0;
+    tile = (n_new + TILE_Q - 1) / TILE_Q - 1 - tile;
     const int first = a.batch.start_pos[seq], slot = a.batch.slot_of_seq[seq];
     const int q0 = tile * TILE_Q, nq = min(TILE_Q, n_new - q0), pos0 = first + q0;
     const int first_new = a.kv_new ? first : 0x7fffffff;
@@ -323,7 +484,7 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
             for (int j = 0; j < 4; ++j) {
                 const int key = k0 + tx * 4 + j;
                 ok[j] = key <= pos && (a.window <= 0 || key > pos - a.window);
-                s[j] *= a.scale;
+                s[j] = __fmul_rn(s[j], a.scale);           // (roundings spelled out: those of attend_row)
                 if (ok[j]) top = fmaxf(top, s[j]);
             }
 #pragma unroll
@@ -331,10 +492,10 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
             const float m_new = fmaxf(m[i], top), alpha = expf(m[i] - m_new);      // m = -FLT_MAX at the start: the sums it scales are zero
             float sum = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { p[i][j] = ok[j] ? expf(s[j] - m_new) : 0.f; sum += p[i][j]; }
+            for (int j = 0; j < 4; ++j) { p[i][j] = ok[j] ? expf(__fsub_rn(s[j], m_new)) : 0.f; sum += p[i][j]; }
 #pragma unroll
             for (int x = 1; x < 16; x *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-            l[i] = l[i] * alpha + sum;
+            l[i] = __fmaf_rn(l[i], alpha, sum);
             m[i] = m_new;
             const unsigned long long aa = att_twice(alpha);
 #pragma unroll
@@ -372,7 +533,7 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a) {
         if (a.sink) {                                      // one more term of the denominator, against the larger of the two maxima
             const float sk = a.sink[h], m_new = fmaxf(m[i], sk);
             scale = expf(m[i] - m_new);
-            l[i] = l[i] * scale + expf(sk - m_new);
+            l[i] = __fmaf_rn(l[i], scale, expf(sk - m_new));
         }
         const float inv = scale / l[i];
         float* out = (float*)a.out + (size_t)(t0 + q0 + r) * a.out_stride + (size_t)h * hd;
@@ -396,9 +557,19 @@ static int launch_tile(const AttnArgs& a, cudaStream_t stream) {
         TB_REQUIRE(e == cudaSuccess, "attn_prefill: cannot reserve %zu bytes of shared memory: %s", tile_smem<HD>(), cudaGetErrorString(e));
         if (dev < 64) configured[dev].store(true);
     }
-    const dim3 grid(a.batch.T / TILE_Q + a.batch.B, a.nh);
-    tb_launch(attn_prefill_tile_kernel<HD>, grid, 256, tile_smem<HD>(), stream, a);
+    // At least the tiles of all long runs, and blocks for the tokens of the short ones (none where all runs are as long as the longest).
+    const int B = a.batch.B, T = a.batch.T, most = a.batch.max_new;
+    const int tiles_x = T / TILE_Q + min(B, T / TILE_FROM), others = most > 0 ? (int)min((long long)T - most, (long long)(B - 1) * (TILE_FROM - 1)) : T;
+    const dim3 grid(tiles_x + (most > 0 && (long long)B * most == T ? 0 : (others + 7) / 8), a.nh);
+    tb_launch(attn_prefill_tile_kernel<HD>, grid, 256, tile_smem<HD>(), stream, a, tiles_x);
     return 0;
+}
+
+static void launch_rows(const AttnArgs& a, cudaStream_t stream) {
+    const unsigned blocks = (unsigned)(((long long)a.batch.T * a.nh + ATT_WARPS - 1) / ATT_WARPS);
+    if (a.hd <= 32) tb_launch(attn_prefill_row_kernel<1>, dim3(blocks), ATT_WARPS * 32, 0, stream, a);
+    else if (a.hd <= 64) tb_launch(attn_prefill_row_kernel<2>, dim3(blocks), ATT_WARPS * 32, 0, stream, a);
+    else tb_launch(attn_prefill_row_kernel<4>, dim3(blocks), ATT_WARPS * 32, 0, stream, a);
 }
 
 // ------------------------------------------------------------------ decode, split over the keys
@@ -728,7 +899,8 @@ extern "C" int tb_attn_prefill(const AttnArgs* args, int dtype, cudaStream_t str
     // and no pairs of heads, rows that 16-byte loads and stores can take.
     if (dtype == TB_F32 && a.hd <= 128 && value_width(a) == a.hd && !a.v_alias && a.keep_first <= 0 && !a.pair_lambda && a.out_stride % 4 == 0 &&
         (uintptr_t)a.q % 16 == 0 && (uintptr_t)a.kv_new % 16 == 0 && (uintptr_t)a.out % 16 == 0 && (uintptr_t)a.cache.storage % 16 == 0 && a.nh <= 65535) {
-        if (a.hd <= 64 ? launch_tile<64>(a, stream) : launch_tile<128>(a, stream)) return 1;
+        if (a.batch.max_new > 0 && a.batch.max_new < TILE_FROM) launch_rows(a, stream);
+        else if (a.hd <= 64 ? launch_tile<64>(a, stream) : launch_tile<128>(a, stream)) return 1;
         TB_CHECK_LAUNCH("attn_prefill");
         return 0;
     }
