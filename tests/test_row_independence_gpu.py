@@ -47,6 +47,32 @@ def test_a_rows_product_is_the_same_bits_beside_any_other_rows(K, dtype, N, Kd):
         assert torch.equal(out, first[:m] + 1.0), m
 
 
+def test_two_threads_launch_products_of_different_sizes(K):
+    """Two engines of different widths step in two threads: no launch is refused because another has changed its kernel's limits."""
+    import threading
+    g, wrong = torch.Generator().manual_seed(0), []
+
+    def work(M, N, Kd, times):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x, w = torch.randn(M, Kd, generator=g).cuda(), torch.randn(N, Kd, generator=g).cuda()
+                out, want = torch.empty(M, N, device="cuda"), None
+                for _ in range(times):
+                    K.gemm_simt(x, w, out, K.EPI_F32, stream())
+                torch.cuda.current_stream().synchronize()
+                want = x.double() @ w.double().t()
+                assert float((out.double() - want).norm() / want.norm()) < 1e-6
+        except Exception as e:  # noqa: BLE001 (whatever a thread met, the test reports)
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((3, 1000, 4096, 2000), (3, 2048, 1024, 2000), (4, 1600, 1024, 2000))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
+
+
 def attend64(q, k, v, pos, scale, window):
     """One query [nh, hd] over the keys [n, nkv, hd] of its sequence in 64 bits."""
     lo = max(0, pos - window + 1) if window else 0

@@ -17,6 +17,7 @@
 //   TB_EPI_ADD     out[m][n] += acc                     (float32 residual stream, in place)
 //   TB_EPI_SWIGLU  out[m][j] = gate(acc[2j], acc[2j+1]) (rows of W interleaved gate, up; N even); the gate is
 //                  silu(g) * u unless the launch names another (activation.h)
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -371,6 +372,20 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
 
 constexpr int SMS = 148;
 
+// Shared memory beyond 48 KB is asked for once a device and kernel, for the largest launch there is: a limit that each launch set for itself
+// would be lowered under the launch of another thread.
+template <auto Kernel>
+int allow_smem(size_t most) {
+    static std::atomic<bool> allowed[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && allowed[dev].load()) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    TB_REQUIRE(e == cudaSuccess, "gemm: cannot reserve %zu bytes of shared memory: %s", most, cudaGetErrorString(e));
+    if (dev < 64) allowed[dev].store(true);
+    return 0;
+}
+
 struct Product {
     const void* X; const void* W; void* out;
     int M, N, K, ldx, ldo, batch;
@@ -387,8 +402,10 @@ bool aligned(const Product& p, int per) {
            (p.batch == 1 || (p.sx % per == 0 && p.sw % per == 0));
 }
 
+constexpr size_t FEW_SMEM = 220 * 1024;
+
 template <typename T, int EPI, int MR, int COLS, bool VEC>
-void few_launch(const Product& p) {
+int few_launch(const Product& p) {
     const int runs = (p.K + SUM_RUN - 1) / SUM_RUN, groups = (p.N + COLS - 1) / COLS, others = (p.M + MR - 1) / MR * p.batch;
     // One unit a block while the blocks fit the chip once: all of K at once.  Else passes of 32 runs (one a thread) and equal shares of the
     // column groups, for two blocks an SM with two stages each where their memory fits (one computes while the other waits), or
@@ -401,61 +418,62 @@ void few_launch(const Product& p) {
     const int room = (two ? 2 : 1) * SMS / others > 0 ? (two ? 2 : 1) * SMS / others : 1, each = (groups + room - 1) / room, x = (groups + each - 1) / each;
     const long long units = (long long)((groups + x - 1) / x) * passes;
     int stages = units < (two ? 2 : 4) ? (int)units : (two ? 2 : 4);
-    while (stages > 1 && few_smem<T, MR, COLS>(pass, stages, passes == 1) > 220 * 1024) --stages;
-    if (stages == 1 && units > 1) { stages = 2; while (few_smem<T, MR, COLS>(pass, stages, false) > 220 * 1024) --pass; }
+    while (stages > 1 && few_smem<T, MR, COLS>(pass, stages, passes == 1) > FEW_SMEM) --stages;
+    if (stages == 1 && units > 1) { stages = 2; while (few_smem<T, MR, COLS>(pass, stages, false) > FEW_SMEM) --pass; }
     const size_t smem = few_smem<T, MR, COLS>(pass, stages, (runs + pass - 1) / pass == 1);
     const dim3 grid(x, (p.M + MR - 1) / MR, p.batch);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(gemm_few_kernel<T, EPI, MR, COLS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && allow_smem<gemm_few_kernel<T, EPI, MR, COLS, VEC>>(FEW_SMEM)) return 1;
     tb_launch(gemm_few_kernel<T, EPI, MR, COLS, VEC>, grid, 256, smem, p.stream, (const T*)p.X, (const T*)p.W, p.out, p.M, p.N, p.K, p.ldx, p.ldo,
               p.sx, p.sw, p.so, pass, stages, p.act, p.limit);
+    return 0;
 }
 template <typename T, int EPI, int MR>
-void few_rows(const Product& p) {
+int few_rows(const Product& p) {
     // 32 columns a unit where a column has at most eight runs (with eight columns most of the block would have no run: sixteen heads'
     // products of 8 rows, 576 columns of K = 128, bfloat16: 9.4 -> 4.7 us)
-    if (!aligned<T>(p, 16 / (int)sizeof(T))) few_launch<T, EPI, MR, 8, false>(p);
-    else if (p.K <= 8 * SUM_RUN) few_launch<T, EPI, MR, 32, true>(p);
-    else few_launch<T, EPI, MR, 8, true>(p);
+    if (!aligned<T>(p, 16 / (int)sizeof(T))) return few_launch<T, EPI, MR, 8, false>(p);
+    if (p.K <= 8 * SUM_RUN) return few_launch<T, EPI, MR, 32, true>(p);
+    return few_launch<T, EPI, MR, 8, true>(p);
 }
 
 template <typename T, int EPI, int RI, bool VEC>
-void tiles(const Product& p) {
+int tiles(const Product& p) {
     const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.batch);
-    cudaFuncSetAttribute(gemm_simt_kernel<T, EPI, RI, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM);
+    if (allow_smem<gemm_simt_kernel<T, EPI, RI, VEC>>(TILE_SMEM)) return 1;
     tb_launch(gemm_simt_kernel<T, EPI, RI, VEC>, grid, 1024 / RI, TILE_SMEM, p.stream, (const T*)p.X, (const T*)p.W, p.out, p.M, p.N, p.K, p.ldx, p.ldo,
               p.sx, p.sw, p.so, p.act, p.limit);
+    return 0;
 }
 
 template <typename T, int EPI>
-void product(const Product& p, bool few) {
+int product(const Product& p, bool few) {
     // Few rows: up to 64 while the column groups of all groups of eight rows stay near a unit's time (measured, K = 1,024, few / tiles:
     // 64 rows of 1,024 columns 20 / 47 us, of 2,048 31 / 42; 5,632 columns 32 rows 41 / 69, 64 rows 81 / 70; 32,768 columns
     // 8 rows 56 / 140, 24 rows 168 / 141).
     if (few || (p.M <= 64 && (long long)((p.M + 7) / 8) * p.N * p.batch <= 32768)) {
-        if (p.M == 1) few_rows<T, EPI, 1>(p);
-        else if (p.M == 2) few_rows<T, EPI, 2>(p);
-        else if (p.M <= 4) few_rows<T, EPI, 4>(p);
-        else few_rows<T, EPI, 8>(p);
-        return;
+        if (p.M == 1) return few_rows<T, EPI, 1>(p);
+        if (p.M == 2) return few_rows<T, EPI, 2>(p);
+        if (p.M <= 4) return few_rows<T, EPI, 4>(p);
+        return few_rows<T, EPI, 8>(p);
     }
     // 8 x 4 sums a thread from four tiles an SM on (5,632 columns of K = 1,024: 1,125 rows 389 -> 357 us, 3,000 rows 980 -> 888 us);
     // below, twice the warps are worth more (1,125 rows, 1,024 columns of K = 2,816: 294 -> 203 us)
     const long long count = (long long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
-    if (!aligned<T>(p, 4)) tiles<T, EPI, 4, false>(p);
-    else if (count >= 4 * 148) tiles<T, EPI, 8, true>(p);
-    else tiles<T, EPI, 4, true>(p);
+    if (!aligned<T>(p, 4)) return tiles<T, EPI, 4, false>(p);
+    if (count >= 4 * SMS) return tiles<T, EPI, 8, true>(p);
+    return tiles<T, EPI, 4, true>(p);
 }
 
 template <typename T>
 int run(const Product& p, int epi, bool few = false) {
     switch (epi) {
-        case TB_EPI_STORE: product<T, TB_EPI_STORE>(p, few); break;
-        case TB_EPI_F32: product<T, TB_EPI_F32>(p, few); break;
-        case TB_EPI_ADD: product<T, TB_EPI_ADD>(p, few); break;
-        case TB_EPI_SWIGLU: product<T, TB_EPI_SWIGLU>(p, few); break;
-        default: tb_set_error("gemm: unknown epilogue %d", epi); return 1;
+        case TB_EPI_STORE: return product<T, TB_EPI_STORE>(p, few);
+        case TB_EPI_F32: return product<T, TB_EPI_F32>(p, few);
+        case TB_EPI_ADD: return product<T, TB_EPI_ADD>(p, few);
+        case TB_EPI_SWIGLU: return product<T, TB_EPI_SWIGLU>(p, few);
     }
-    return 0;
+    tb_set_error("gemm: unknown epilogue %d", epi);
+    return 1;
 }
 
 }  // namespace

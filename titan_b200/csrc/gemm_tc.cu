@@ -32,6 +32,7 @@
 // berniehans/titan's counterpart is gemm_q4k_batched_kernel (engine/engine-cuda/kernels/
 // gemm_quant.cu:3365-3499), a scalar-FMA warp-per-column kernel with the residual in its
 // epilogue (:3489-3493); it has no tensor-core path.
+#include <atomic>
 #include <cuda.h>
 
 #include <mutex>
@@ -1487,33 +1488,42 @@ extern "C" int tb_gemm_tc(const void* X, const void* W, void* out, int M, int N,
 // Names the buffer of the timeline probe (timeline.cuh); 1 if the library was built with it, 0 if not.
 TB_TIMELINE_SETTER(tb_gemm_tc_timeline)
 
+constexpr int MAX_RUNS = 1024;
+constexpr size_t runs_smem(int bn, int stages, int runs) { return 1024 + (size_t)stages * (BM + bn) * BK * 2 + 256 + 2 * (size_t)(runs + 1) * sizeof(int); }
+
+template <int EPI>
+static int launch_runs(const void* X, int ldx, const void* W, void* out, int ldo, const int* first, int runs, int rows, int N, int K, int act, float limit, cudaStream_t stream) {
+    constexpr int BN = 256;
+    // the limit of shared memory once a device, for the most runs there may be: a limit each launch set for itself would be lowered under another thread's
+    static std::atomic<bool> configured[64];
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64 || !configured[dev].load()) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_runs_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)runs_smem(BN, stages_for<BN>(), MAX_RUNS));
+        TB_REQUIRE(e == cudaSuccess, "gemm_tc_expert_runs: cannot reserve %zu bytes of shared memory: %s", runs_smem(BN, stages_for<BN>(), MAX_RUNS), cudaGetErrorString(e));
+        if (dev < 64) configured[dev].store(true);
+    }
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    CUtensorMap ma, mb;
+    if (tb_make_map_bf16(&ma, X, rows, K, ldx, BM) || tb_make_map_bf16(&mb, W, (long long)runs * N, K, K, BN)) return 1;
+    TcArgs a = {};
+    a.out = out; a.K = K; a.ldo = ldo; a.rows_a = rows; a.rows_b = N; a.act = act; a.limit = limit;
+    const long long most = ((long long)rows / BM + runs) * ((N + BN - 1) / BN);       // tiles, if every run ends inside one
+    tb_launch(gemm_tc_runs_kernel<EPI>, dim3((unsigned)(most < sms ? most : sms)), THREADS, runs_smem(BN, stages_for<BN>(), runs), stream, ma, mb, a, first, runs);
+    return 0;
+}
+
 // The two products of every expert over rows that lie side by side, expert by expert: act = gate(X_e . Wgu_e^T) (rows of Wgu_e
 // interleaved gate, up) and y = act_e . Wd_e^T (float32), one launch each.  ``first`` [runs + 1] is on the device: the experts'
 // first rows, ascending, the last of them at most ``rows``, the rows of X, act and y.
 extern "C" int tb_gemm_tc_expert_runs(const void* X, int ldx, const void* Wgu, void* act, int ld_act, const void* Wd, void* y, int ldy,
                                       const int* first, int runs, int rows, int H, int F, int gate, float limit, cudaStream_t stream) {
-    TB_REQUIRE(first && runs > 0 && runs <= 1024 && rows > 0 && H > 0 && F > 0, "gemm_tc_expert_runs: sizes (runs=%d rows=%d H=%d F=%d)", runs, rows, H, F);
+    TB_REQUIRE(first && runs > 0 && runs <= MAX_RUNS && rows > 0 && H > 0 && F > 0, "gemm_tc_expert_runs: sizes (runs=%d rows=%d H=%d F=%d)", runs, rows, H, F);
     TB_REQUIRE((long long)runs * (2 * F > H ? 2 * F : H) < 2147483647LL, "gemm_tc_expert_runs: too many rows of weights");
     TB_REQUIRE(gate >= 0 && gate < TB_ACT_KINDS, "gemm_tc_expert_runs: unknown gate %d", gate);
     if (tb_gemm_tc_check(rows, 2 * F, H, ldx, ld_act, TB_EPI_SWIGLU, X, Wgu, act) || tb_gemm_tc_check(rows, H, F, ld_act, ldy, TB_EPI_F32, act, Wd, y)) return 1;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    constexpr int BN = 256;
-    const size_t smem = 1024 + (size_t)stages_for<BN>() * (BM + BN) * BK * 2 + 256 + 2 * (size_t)(runs + 1) * sizeof(int);
-    auto go = [&](auto kernel, const void* A, int lda, const void* W, void* out, int ldo, int N, int K) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        TB_REQUIRE(e == cudaSuccess, "gemm_tc_expert_runs: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        CUtensorMap ma, mb;
-        if (tb_make_map_bf16(&ma, A, rows, K, lda, BM) || tb_make_map_bf16(&mb, W, (long long)runs * N, K, K, BN)) return 1;
-        TcArgs a = {};
-        a.out = out; a.K = K; a.ldo = ldo; a.rows_a = rows; a.rows_b = N; a.act = gate; a.limit = limit;
-        const long long most = ((long long)rows / BM + runs) * ((N + BN - 1) / BN);       // tiles, if every run ends inside one
-        tb_launch(kernel, dim3((unsigned)(most < sms ? most : sms)), THREADS, smem, stream, ma, mb, a, first, runs);
-        return 0;
-    };
-    if (go(gemm_tc_runs_kernel<TB_EPI_SWIGLU>, X, ldx, Wgu, act, ld_act, 2 * F, H)) return 1;
-    if (go(gemm_tc_runs_kernel<TB_EPI_F32>, act, ld_act, Wd, y, ldy, H, F)) return 1;
+    if (launch_runs<TB_EPI_SWIGLU>(X, ldx, Wgu, act, ld_act, first, runs, rows, 2 * F, H, gate, limit, stream)) return 1;
+    if (launch_runs<TB_EPI_F32>(act, ld_act, Wd, y, ldy, first, runs, rows, H, F, 0, 0.f, stream)) return 1;
     TB_CHECK_LAUNCH("gemm_tc_expert_runs");
     return 0;
 }
