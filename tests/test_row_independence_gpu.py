@@ -47,6 +47,34 @@ def test_a_rows_product_is_the_same_bits_beside_any_other_rows(K, dtype, N, Kd):
         assert torch.equal(out, first[:m] + 1.0), m
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,Kd,rows", [(33000, 72, (1, 8, 9, 16, 17, 65)), (32770, 1032, (1, 3, 9, 17)), (256, 8192, (1, 3, 4, 64)), (258, 2048, (3, 4, 5)), (2, 6000, (1, 64)),
+                                       (40004, 32, (1, 2, 8)), (1030, 36, (4, 5, 64)), (600, 100, (4, 5, 8)), (4, 8, (1, 70000))])
+def test_small_few_and_tiled_products_on_both_sides_of_their_borders(K, dtype, N, Kd, rows):
+    """Every epilogue of every kernel; a row is the same bits whichever kernel takes it (a row of many is taken by the tiles)."""
+    g = torch.Generator().manual_seed(N + Kd)
+    M = max(max(rows), 130)
+    x = torch.randn(M, Kd, generator=g).to(dtype).cuda()
+    w = (torch.randn(N, Kd, generator=g) * 0.1).to(dtype).cuda()
+    f = torch.empty(M, N, device="cuda")
+    K.gemm_simt(x, w, f, K.EPI_F32, stream())
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert bool(((f.double() - want).abs() <= (16 + 1 + math.ceil(Kd / 32) + 2) * EPS32 * size + 1e-30).all())
+    for m in rows:
+        out = torch.full((m, N), 7.0, device="cuda")
+        K.gemm_simt(x[:m], w, out, K.EPI_F32, stream())
+        assert torch.equal(out, f[:m]), m
+        K.gemm_simt(x[:m], w, out.fill_(1.0), K.EPI_ADD, stream())
+        assert torch.equal(out, f[:m] + 1.0), m
+        stored = torch.full((m, N), 7.0, dtype=dtype, device="cuda")
+        K.gemm_simt(x[:m], w, stored, K.EPI_STORE, stream())
+        assert torch.equal(stored, f[:m].to(dtype)), m
+        gated, wide = torch.full((m, N // 2 + 8), 7.0, dtype=dtype, device="cuda"), torch.empty(M, N // 2, dtype=dtype, device="cuda")
+        K.gemm_simt(x[:m], w, gated[:, :N // 2], K.EPI_SWIGLU, stream())
+        K.gemm_simt(x, w, wide, K.EPI_SWIGLU, stream())
+        assert torch.equal(gated[:, :N // 2], wide[:m]) and bool((gated[:, N // 2:] == 7.0).all()), m
+
+
 def test_two_threads_launch_products_of_different_sizes(K):
     """Two engines of different widths step in two threads: no launch is refused because another has changed its kernel's limits."""
     import threading
@@ -351,7 +379,8 @@ def test_norms_of_long_prompts_are_the_bits_of_short_ones(K, dtype, rows, H):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("M,N,Kd,batch", [(1, 576, 128, 16), (8, 40, 256, 3), (9, 33, 264, 2), (64, 100, 8, 5)])
+@pytest.mark.parametrize("M,N,Kd,batch", [(1, 576, 128, 16), (8, 40, 256, 3), (9, 33, 264, 2), (64, 100, 8, 5), (2, 576, 100, 16), (3, 576, 128, 16), (12, 130, 520, 33),
+                                          (13, 130, 520, 33), (16, 70, 1032, 4), (16, 1100, 512, 4), (1, 9000, 520, 4), (1, 513, 128, 65), (9, 577, 128, 64)])
 def test_products_of_heads_side_by_side(K, dtype, M, N, Kd, batch):
     g = torch.Generator().manual_seed(N)
     x = torch.randn(M, batch * Kd, generator=g).to(dtype).cuda()

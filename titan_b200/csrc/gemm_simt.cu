@@ -6,7 +6,7 @@
 // (engine/engine-cuda/kernels/gemm_quant.cu:2331-2363 gemm_f32_kernel, :3365-3499 batched), which
 // fuse the residual into the epilogue (:3489-3493) and SwiGLU into gate/up (:2589).
 //
-// One order of sums for every kernel here, whatever M: in each run of SUM_RUN neighbouring k the products at even and those at
+// One order of sums for every kernel here but one (gemm_heads_kernel), whatever M: in each run of SUM_RUN neighbouring k the products at even and those at
 // odd k are added one after the other (fused multiply-adds from zero), then the two sums, and the runs' sums one after the
 // other.  A row's result is then the same bits alone and beside any other rows, in a decode step as in a prompt.  Even
 // and odd, because the two are neighbours in memory and one two-element instruction (fma.rn.f32x2) works on both.
@@ -50,9 +50,8 @@ template <> struct Vec<__nv_bfloat16, 8> {
         for (int i = 0; i < 4; ++i) { o[2 * i] = __uint_as_float(w[i] << 16); o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
     }
 };
-// Activations are read through L2 by instructions that stay where they are: kernels of a step are in flight together, so a line of
-// this SM's L1 may be older than what the kernel before has written, and a load that the compiler takes for a load of
-// constants may move above the wait for that kernel (a __restrict__ pointer to const; weights, which no kernel writes, may have it).
+// Loads of activations that the compiler cannot take for loads of constants (as it may through a __restrict__ pointer to const): such a load could
+// move above the wait for the kernel that writes them.  load_l2: rows that an SM reads once; load_row: rows that several of its warps read.
 template <typename V> __device__ __forceinline__ V load_l2(const void* p);
 template <> __device__ __forceinline__ float load_l2<float>(const void* p) {
     float v;
@@ -72,6 +71,27 @@ template <> __device__ __forceinline__ float4 load_l2<float4>(const void* p) {
 template <> __device__ __forceinline__ uint2 load_l2<uint2>(const void* p) {
     uint2 v;
     asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+template <typename V> __device__ __forceinline__ V load_row(const void* p);
+template <> __device__ __forceinline__ float load_row<float>(const void* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+template <> __device__ __forceinline__ __nv_bfloat16 load_row<__nv_bfloat16>(const void* p) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return __ushort_as_bfloat16(v);
+}
+template <> __device__ __forceinline__ float4 load_row<float4>(const void* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+template <> __device__ __forceinline__ uint4 load_row<uint4>(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 
@@ -370,7 +390,134 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     }
 }
 
-constexpr int SMS = 148;
+// ---------------------------------------------------------------- small products: operands straight into registers
+// The kernel above pays for its rows in shared memory in every block and for two or three barriers before the first sum: a router of
+// 128 columns of K = 4,096 in bfloat16 took 9.7 us for eight rows.  Here a thread has one column and one run of SUM_RUN at a time, ``lanes`` of
+// a block's threads along K, and a block one row: it loads both operands of the run itself (neighbouring threads have
+// neighbouring columns of the same run, a row's loads are shared by the warp) and leaves the run's sum in shared memory, where a
+// thread a column adds them in order: one barrier, 5.1 us for the router.  The weights of the first run come before the wait.  Bound by latency;
+// weights are read once a row through L2 (two and four rows a block were slower wherever this kernel is the fastest).
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256)
+gemm_small_kernel(const T* X, const T* W, void* out_, int N, int K, int ldx, int ldo, long long sx, long long sw, long long so,
+                  int lanes, int pass, int epi, int act, float limit) {
+    constexpr int PER = 16 / (int)sizeof(T), UNITS = SUM_RUN / PER;
+    pdl_launch_dependents();
+    extern __shared__ float small_sm[];                    // [pass][columns]
+    const int tid = threadIdx.x, cols = (int)blockDim.x / lanes, col = tid % cols, lane = tid / cols, n = blockIdx.x * cols + col, runs = (K + SUM_RUN - 1) / SUM_RUN;
+    const T* w = W + (size_t)blockIdx.z * sw + (size_t)n * K;
+    const T* x = X + (size_t)blockIdx.z * sx + (size_t)blockIdx.y * ldx;
+    float wf[SUM_RUN];
+    auto load_w = [&](int k) {                             // (VEC: K is a multiple of a unit; places beyond it take the row's first)
+        if constexpr (VEC) {
+            Vec<T, PER> v[UNITS];
+#pragma unroll
+            for (int i = 0; i < UNITS; ++i) v[i].load(w + (k + i * PER < K ? k + i * PER : 0));
+#pragma unroll
+            for (int i = 0; i < UNITS; ++i) v[i].get(wf + i * PER);
+        } else {
+#pragma unroll
+            for (int e = 0; e < SUM_RUN; ++e) wf[e] = k + e < K ? ldf(w + k + e) : 0.f;
+        }
+    };
+    if (lane < runs && n < N) load_w(lane * SUM_RUN);
+    pdl_wait();
+    float total = 0.f;
+    for (int p0 = 0; p0 < runs; p0 += pass) {
+        const int here = min(pass, runs - p0);
+        for (int r = p0 + lane; r < p0 + here && n < N; r += lanes) {
+            const int k = r * SUM_RUN;
+            if (r >= lanes) load_w(k);
+            unsigned long long acc = 0ull;
+            if constexpr (VEC) {
+                Vec<T, PER> v[UNITS];
+#pragma unroll
+                for (int i = 0; i < UNITS; ++i) v[i].r = load_row<decltype(v[i].r)>(x + (k + i * PER < K ? k + i * PER : 0));
+#pragma unroll
+                for (int i = 0; i < UNITS; ++i) {
+                    float xf[PER];
+                    v[i].get(xf);
+                    if (k + i * PER < K)
+#pragma unroll
+                        for (int e = 0; e < PER; e += 2) fma2(acc, pair_of(xf[e], xf[e + 1]), pair_of(wf[i * PER + e], wf[i * PER + e + 1]));
+                }
+            } else {
+                float xf[SUM_RUN];
+#pragma unroll
+                for (int e = 0; e < SUM_RUN; ++e) {
+                    xf[e] = 0.f;
+                    if (k + e < K) { const T v = load_row<T>(x + k + e); xf[e] = ldf(&v); }
+                }
+#pragma unroll
+                for (int e = 0; e < SUM_RUN; e += 2) fma2(acc, pair_of(xf[e], xf[e + 1]), pair_of(wf[e], wf[e + 1]));
+            }
+            small_sm[(r - p0) * cols + col] = both(acc);
+        }
+        __syncthreads();
+        if (tid < cols && n < N) {
+            const float* mine = small_sm + col;
+            int r = 0;
+            for (; r + 16 <= here; r += 16) {              // all loads first
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = mine[(r + i) * cols];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) total += v[i];
+            }
+            for (; r < here; ++r) total += mine[r * cols];
+        }
+        if (p0 + pass < runs) __syncthreads();
+    }
+    // the gate of a pair: its second column is the neighbouring thread's (an even number of columns a block)
+    const float right = __shfl_down_sync(0xffffffffu, total, 1);
+    if (tid >= cols || n >= N) return;
+    const size_t row = (size_t)blockIdx.z * so + (size_t)blockIdx.y * ldo;
+    if (epi == TB_EPI_SWIGLU) { if (n % 2 == 0) stf((T*)out_ + row + n / 2, tb_gated(act, limit, total, right)); }
+    else if (epi == TB_EPI_STORE) stf((T*)out_ + row + n, tb_unary(act, total));
+    else if (epi == TB_EPI_F32) ((float*)out_)[row + n] = total;
+    else ((float*)out_)[row + n] = load_l2<float>((float*)out_ + row + n) + total;
+}
+
+// ---------------------------------------------------------------- heads' products of a decode step in bfloat16: a warp an output
+// Products of a batch (STORE epilogue) whose rows are few: lanes along K with 16-byte loads of whole rows, so that weights stream at the
+// best rate of all kernels here, once for each row.  The one kernel with an order of sums of its own: what it makes is rounded to
+// bfloat16, and the products around it do not keep one order either; float32 takes the kernels above.
+__global__ void __launch_bounds__(256)
+gemm_heads_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W, __nv_bfloat16* __restrict__ out_, int N, int K, int ldx, int ldo,
+                  long long sx, long long sw, long long so, int act) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockIdx.x * 8 + warp;
+    if (n >= N) return;
+    const __nv_bfloat16* x = X + (size_t)blockIdx.z * sx + (size_t)blockIdx.y * ldx;
+    const __nv_bfloat16* w = W + (size_t)blockIdx.z * sw + (size_t)n * K;
+    float acc = 0.f;
+    if (K % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0) {
+        for (int k = lane * 8; k < K; k += 256) {
+            const uint4 a = *reinterpret_cast<const uint4*>(x + k), b = *reinterpret_cast<const uint4*>(w + k);
+            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc = fmaf(__uint_as_float(aw[i] << 16), __uint_as_float(bw[i] << 16), acc);
+                acc = fmaf(__uint_as_float(aw[i] & 0xffff0000u), __uint_as_float(bw[i] & 0xffff0000u), acc);
+            }
+        }
+    } else {
+        for (int k = lane; k < K; k += 32) acc = fmaf(ldf(x + k), ldf(w + k), acc);
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) stf(out_ + (size_t)blockIdx.z * so + (size_t)blockIdx.y * ldo + n, tb_unary(act, acc));
+}
+
+int sm_count() {
+    static std::atomic<int> count[64];                     // a device each
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && (n = count[dev].load()) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    if (dev < 64) count[dev].store(n);
+    return n;
+}
 
 // Shared memory beyond 48 KB is asked for once a device and kernel, for the largest launch there is: a limit that each launch set for itself
 // would be lowered under the launch of another thread.
@@ -406,6 +553,7 @@ constexpr size_t FEW_SMEM = 220 * 1024;
 
 template <typename T, int EPI, int MR, int COLS, bool VEC>
 int few_launch(const Product& p) {
+    const int SMS = sm_count();
     const int runs = (p.K + SUM_RUN - 1) / SUM_RUN, groups = (p.N + COLS - 1) / COLS, others = (p.M + MR - 1) / MR * p.batch;
     // One unit a block while the blocks fit the chip once: all of K at once.  Else passes of 32 runs (one a thread) and equal shares of the
     // column groups, for two blocks an SM with two stages each where their memory fits (one computes while the other waits), or
@@ -436,6 +584,20 @@ int few_rows(const Product& p) {
     return few_launch<T, EPI, MR, 8, true>(p);
 }
 
+template <typename T, bool VEC>
+int small_launch(const Product& p, int epi) {
+    const int runs = (p.K + SUM_RUN - 1) / SUM_RUN;
+    int lanes = 1, threads = 256;
+    while (lanes < runs && lanes < 128) lanes *= 2;
+    // smaller blocks while there are fewer than two an SM: a warp's columns are as many lines of the L1, which one SM would take one by one
+    while (threads > 64 && threads / 2 >= 2 * lanes && (long long)p.N * lanes / threads * p.M * p.batch < 2 * sm_count()) threads /= 2;
+    const int pass = runs < 16 * lanes ? runs : 16 * lanes, cols = threads / lanes;
+    const dim3 grid((p.N + cols - 1) / cols, p.M, p.batch);
+    tb_launch(gemm_small_kernel<T, VEC>, grid, threads, (size_t)pass * cols * sizeof(float), p.stream, (const T*)p.X, (const T*)p.W, p.out, p.N, p.K,
+              p.ldx, p.ldo, p.sx, p.sw, p.so, lanes, pass, epi, p.act, p.limit);
+    return 0;
+}
+
 template <typename T, int EPI, int RI, bool VEC>
 int tiles(const Product& p) {
     const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.batch);
@@ -445,32 +607,73 @@ int tiles(const Product& p) {
     return 0;
 }
 
+// Which kernel.  All but the warp an output add in the one order, so that these lines, measured in us, decide about time alone.
+enum Kind { SMALL, HEADS, FEW, TILES };
+template <typename T>
+Kind kind_of(const Product& p, int epi) {
+    const int M = p.M, K = p.K, groups = (M + 7) / 8;
+    const long long columns = (long long)p.N * p.batch, products = columns * M * K;
+    const bool wide = aligned<T>(p, 16 / (int)sizeof(T));
+    // Heads in bfloat16, warp an output / small / few / tiles: 128 heads of 128 columns, K = 512: 1 row 4.6 / 8.9 / 15 / 42, 8 rows 22 / 58 / 21 / 42;
+    // four of 2,048, K = 2,048: 8 rows 24 / 85 / 30 / 157, 16 rows 45 / 165 / 51 / 157; 64 of 576, K = 128: 1 row 6.6 / 5.6 / 10 / 21, 4 rows 21 / 17 /
+    // 13 / 21; 16 of 576, K = 128: 2 rows 3.5 / 2.6 / 2.6 / 10, 8 rows 11 / 8 / 4.1 / 10; four of 64, K = 64: 8 rows 1.5 / 1.6 / 3.0 / 3.5.
+    if (sizeof(T) == 2 && p.batch > 1 && epi == TB_EPI_STORE && M <= 16) {
+        if (M <= 2 && K <= 128 && wide) return SMALL;
+        if (M <= 2 || K >= 1024 || (K >= 512 && M <= 12 && !(M == 8 && columns >= 16384)) || columns * M <= 12288) return HEADS;
+    }
+    // Small / few: up to half a million products the few-rows kernel's fixed cost decides (512 columns of K = 1,024, float32: 1 row 2.3 / 2.3, 2 rows
+    // 2.8 / 2.5; 1,024 of K = 36, bfloat16: 8 rows 3.1 / 5.5); with few columns or short ones later (128 of K = 2,048: 8 rows 3.8 / 5.0, 16 rows
+    // 5.9 / 5.0; eight heads of 100, K = 96: 8 rows 2.4 / 3.3), with long ones, whose rows it would take through shared memory in every block, later still (64 of K = 8,192: 8 rows 11 / 23,
+    // 32 rows 26 / 23), and in bfloat16, whose loads are half as many, at four times the size (1,024 of K = 1,024: 2 rows 2.6 / 3.1, 4 rows 5.1 / 3.8).
+    const int most = (columns <= 256 || K <= 64 || (K <= 128 && columns <= 1024) || (sizeof(T) == 2 && columns <= 4096)) ? (K > 2048 && columns <= 256 ? 6 << 20 : 2 << 20) : 1 << 19;
+    // Rows that 16-byte loads cannot take: only short ones (1,024 of K = 1,023, bfloat16, 1 row: 5.9 / 3.2).
+    if (products <= most && M <= 64 && (wide || K <= 128)) return SMALL;
+    if (M == 1 && p.batch >= 32 && columns >= 16384) return SMALL;      // (one row of many heads, float32: 128 of 512 columns, K = 128: 11 / 16)
+    if (M > 64) return TILES;
+    // Few / tiles: every group of eight rows is a pass over the weights, which tiles read once for 64.  One group is always few (float32, K = 1,024: 8 rows
+    // of 32,768 columns 56 / 140, of 151,936 247 / 538), two up to 32,768 columns (108 / 140; of 151,936, K = 2,560: 1,786 / 1,345), more while all groups'
+    // columns stay below a bound (5,632 columns: 48 rows 58 / 67, 64 rows 77 / 69; 8,192: 32 rows 55 / 69, 48 rows 83 / 69), which is lower where K is
+    // short, as the tiles then are (8,192 of K = 128: 16 rows 7.2 / 9.7, 32 rows 13 / 10; 40,000 of K = 32: 8 rows 13 / 7.1).
+    if (K <= 64 && columns > 32768) return TILES;
+    // Rows that 16-byte loads cannot take: 5,000 columns of K = 100, bfloat16: 4 rows 8.6 / 9.0, 8 rows 12.7 / 9.1; 3,000 of K = 1,001: 48 rows 80 / 85,
+    // 64 rows 102 / 87 (float32).
+    if (!wide && K <= 128 && M > 4) return TILES;
+    if (!wide && groups > 1) return groups * columns <= 20480 ? FEW : TILES;
+    if (groups == 1 || (groups == 2 && K > 128 && columns <= 32768)) return FEW;
+    return groups * columns <= (K > 128 ? 36864 : 28672) ? FEW : TILES;
+}
+
 template <typename T, int EPI>
-int product(const Product& p, bool few) {
-    // Few rows: up to 64 while the column groups of all groups of eight rows stay near a unit's time (measured, K = 1,024, few / tiles:
-    // 64 rows of 1,024 columns 20 / 47 us, of 2,048 31 / 42; 5,632 columns 32 rows 41 / 69, 64 rows 81 / 70; 32,768 columns
-    // 8 rows 56 / 140, 24 rows 168 / 141).
-    if (few || (p.M <= 64 && (long long)((p.M + 7) / 8) * p.N * p.batch <= 32768)) {
-        if (p.M == 1) return few_rows<T, EPI, 1>(p);
-        if (p.M == 2) return few_rows<T, EPI, 2>(p);
-        if (p.M <= 4) return few_rows<T, EPI, 4>(p);
-        return few_rows<T, EPI, 8>(p);
+int product(const Product& p) {
+    switch (kind_of<T>(p, EPI)) {
+        case SMALL: return aligned<T>(p, 16 / (int)sizeof(T)) ? small_launch<T, true>(p, EPI) : small_launch<T, false>(p, EPI);
+        case HEADS:
+            if constexpr (sizeof(T) == 2)
+                tb_launch(gemm_heads_kernel, dim3((p.N + 7) / 8, p.M, p.batch), 256, 0, p.stream, (const T*)p.X, (const T*)p.W, (T*)p.out, p.N, p.K, p.ldx, p.ldo,
+                          p.sx, p.sw, p.so, p.act);
+            return 0;
+        case FEW:
+            if (p.M == 1) return few_rows<T, EPI, 1>(p);
+            if (p.M == 2) return few_rows<T, EPI, 2>(p);
+            if (p.M <= 4) return few_rows<T, EPI, 4>(p);
+            return few_rows<T, EPI, 8>(p);
+        case TILES: break;
     }
     // 8 x 4 sums a thread from four tiles an SM on (5,632 columns of K = 1,024: 1,125 rows 389 -> 357 us, 3,000 rows 980 -> 888 us);
     // below, twice the warps are worth more (1,125 rows, 1,024 columns of K = 2,816: 294 -> 203 us)
     const long long count = (long long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.batch;
     if (!aligned<T>(p, 4)) return tiles<T, EPI, 4, false>(p);
-    if (count >= 4 * SMS) return tiles<T, EPI, 8, true>(p);
+    if (count >= 4 * sm_count()) return tiles<T, EPI, 8, true>(p);
     return tiles<T, EPI, 4, true>(p);
 }
 
 template <typename T>
-int run(const Product& p, int epi, bool few = false) {
+int run(const Product& p, int epi) {
     switch (epi) {
-        case TB_EPI_STORE: return product<T, TB_EPI_STORE>(p, few);
-        case TB_EPI_F32: return product<T, TB_EPI_F32>(p, few);
-        case TB_EPI_ADD: return product<T, TB_EPI_ADD>(p, few);
-        case TB_EPI_SWIGLU: return product<T, TB_EPI_SWIGLU>(p, few);
+        case TB_EPI_STORE: return product<T, TB_EPI_STORE>(p);
+        case TB_EPI_F32: return product<T, TB_EPI_F32>(p);
+        case TB_EPI_ADD: return product<T, TB_EPI_ADD>(p);
+        case TB_EPI_SWIGLU: return product<T, TB_EPI_SWIGLU>(p);
     }
     tb_set_error("gemm: unknown epilogue %d", epi);
     return 1;
@@ -519,8 +722,8 @@ extern "C" int tb_gemm_simt(const void* X, const void* W, void* out, int dtype, 
 }
 
 // ``act``: the activation of the STORE epilogue (activation.h).
-// out (epilogue store, float32 or add) = X[M,K] . W[N,K]^T on the few-rows kernel whatever M: the products of a decode step
-// whose matrices are too small to pay for a tensor-core launch (a router, a narrow gate).
+// out (epilogue store, float32 or add) = X[M,K] . W[N,K]^T: the products of a decode step whose matrices are too small to pay for a
+// tensor-core launch (a router, a narrow gate).
 extern "C" int tb_gemm_rows(const void* X, const void* W, void* out, int dtype, int M, int N, int K, int ldx, int ldo, int epi,
                             int act, cudaStream_t stream) {
     TB_REQUIRE(epi == TB_EPI_STORE ? act >= 0 && act < TB_UNARY_KINDS : act == 0, "gemm_rows: unknown activation %d", act);
@@ -529,8 +732,8 @@ extern "C" int tb_gemm_rows(const void* X, const void* W, void* out, int dtype, 
     TB_REQUIRE(epi != TB_EPI_SWIGLU, "gemm_rows: epilogue %d is not one of store, float32, add", epi);
     const Product p{X, W, out, M, N, K, ldx, ldo, 1, 0, 0, 0, act, 0.f, stream};
     int rc;
-    if (dtype == TB_F32) rc = run<float>(p, epi, true);
-    else if (dtype == TB_BF16) rc = run<__nv_bfloat16>(p, epi, true);
+    if (dtype == TB_F32) rc = run<float>(p, epi);
+    else if (dtype == TB_BF16) rc = run<__nv_bfloat16>(p, epi);
     else { tb_set_error("gemm_rows: unknown dtype %d", dtype); return 1; }
     if (rc) return rc;
     TB_CHECK_LAUNCH("gemm_rows");

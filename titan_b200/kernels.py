@@ -431,7 +431,7 @@ def gemm_simt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: 
 
 
 def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, stream: int, unary: int = UNARY_NONE) -> None:
-    """out (epilogue store, float32 or add) = x[M,K] . w[N,K]^T on the few-rows kernel of the CUDA cores: for the few rows of a decode step and
+    """out (epilogue store, float32 or add) = x[M,K] . w[N,K]^T on the CUDA cores: for the few rows of a decode step and
     matrices too small to pay for a tensor-core launch.  ``unary``: the STORE epilogue's activation (UNARY_*)."""
     _need_cuda(x, w, out)
     M, K = x.shape

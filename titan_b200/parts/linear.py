@@ -1,7 +1,7 @@
 """Matrix products of the parts: ``out = epilogue(x . w^T)``.
 
 One function, so that which kernel runs is decided in one place.  A few rows times a small matrix (a decode step's router,
-a narrow gate) take the CUDA cores' few-rows kernel in either dtype.  Otherwise float32
+a narrow gate) take the CUDA cores in either dtype.  Otherwise float32
 always takes the CUDA-core kernel (true 32-bit).  bfloat16 takes the tcgen05
 tensor-core kernel when the shapes meet its alignment rules and the CUDA-core
 kernel otherwise; ``ctx.options["gemm"] = "plain"`` forces the latter.
@@ -15,7 +15,7 @@ from .. import kernels as K
 EPI_STORE, EPI_F32, EPI_ADD, EPI_SWIGLU = K.EPI_STORE, K.EPI_F32, K.EPI_ADD, K.EPI_SWIGLU
 
 
-# A product of at most this many rows with a matrix of at most this many elements runs on the few-rows kernel: the fixed
+# A product of at most this many rows with a matrix of at most this many elements runs on the CUDA cores: the fixed
 # cost of a tensor-core launch (or, in float32, of 64 x 64 tiles with a few live rows) is more than such a product's work.
 ROWS_MAX_M, ROWS_MAX_ELEMENTS = 8, 1 << 19
 
