@@ -332,3 +332,32 @@ def test_capture_survives_dead_engines_waiting_for_the_cycle_collector(worlds, m
     finally:
         gc.enable()
         gc.collect()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_slot_taken_on_a_busy_stream_and_used_on_another(worlds, dtype):
+    """A slot's length on the device starts from zero before the slot's first step, also when other work is still queued where the slot was taken."""
+    from titan_b200 import StepEntry
+    w = worlds["A"]
+    e = w.engine(dtype)
+    toks, busy, other = w.requests[2], torch.cuda.Stream(), torch.cuda.Stream()
+
+    def step(s):
+        with torch.cuda.stream(other):
+            return e.step([StepEntry(s, toks, list(range(len(toks))))])
+
+    for _ in range(2):                                        # (what a step allocates is there already: an allocation would wait for the device)
+        s = e.alloc_slot()
+        step(s)
+        torch.cuda.synchronize()
+        e.free_slot(s)
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(400_000_000)
+        s = e.alloc_slot()
+    logits = step(s)
+    other.synchronize()
+    assert not busy.query()
+    torch.cuda.synchronize()
+    assert int(e.cache.state.seq_len[s]) == len(toks)
+    close(logits.cpu(), w.plain(2), dtype)
+    e.free_slot(s)

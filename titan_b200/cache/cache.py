@@ -17,7 +17,7 @@ engine/engine-kvcache/src/cache.rs:166-172).
 """
 from __future__ import annotations
 
-from typing import Dict, List, Optional, Sequence, Tuple
+from typing import Dict, List, Optional, Sequence, Set, Tuple
 
 import torch
 
@@ -57,6 +57,7 @@ class SequenceCache:
         self.max_slots = max_slots
         self.device = device
         self.slots = SlotAllocator(max_slots)
+        self.fresh: Set[int] = set()           # slots handed out whose first step is still to come
         self.length: Dict[int, int] = {}
         self.state = SlotState(max_slots, device)
         self.groups: List[CacheGroup] = []
@@ -88,7 +89,7 @@ class SequenceCache:
     def alloc_slot(self) -> int:
         slot = self.slots.take()
         self.length[slot] = 0
-        self.state.seq_len[slot].zero_()    # a kernel in stream order (assigning a number would copy from the host and wait for the stream)
+        self.fresh.add(slot)
         for g in self.groups:
             g.on_alloc(slot)
         return slot
@@ -96,6 +97,7 @@ class SequenceCache:
     def free_slot(self, slot: int) -> None:
         self.slots.give_back(slot)          # raises on unknown / double free
         del self.length[slot]
+        self.fresh.discard(slot)
         for g in self.groups:
             g.release(slot, self.mark_freed)
 
@@ -104,8 +106,8 @@ class SequenceCache:
 
     # -- room ------------------------------------------------------------ #
     def reserve(self, wanted: Dict[int, int]) -> None:
-        """Make room so that each slot can hold ``wanted[slot]`` tokens in total.
-        Either every slot gets its pages or none does."""
+        """Make room so that each slot can hold ``wanted[slot]`` tokens in total, before the step that brings them is queued on the current
+        stream.  Either every slot gets its pages or none does."""
         for slot, n in wanted.items():
             if not self.is_live(slot):
                 raise CacheError(f"slot {slot} is not live")
@@ -118,6 +120,11 @@ class SequenceCache:
         for g in self.groups:
             for slot, n in wanted.items():
                 g.extend(slot, n)
+        # A new slot's length on the device starts from zero here and not where the slot was handed out: in the order of the stream its first step
+        # runs on, whatever stream took it.  (Assigning a number would copy from the host and wait for the stream.)
+        for slot in self.fresh & wanted.keys():
+            self.fresh.discard(slot)
+            self.state.seq_len[slot].zero_()
 
     def commit(self, slot: int, new_length: int) -> None:
         """Host copy of the length after a step; the device copy is advanced by the step itself."""
