@@ -1038,6 +1038,8 @@ def commit_lengths(slot_of_seq, kv_len, seq_len, stream: int) -> None:
 def wait_errors() -> dict:
     """The error words of the kernels whose waits are bounded (a wait that gave up leaves a code there and the
     step's result is invalid).  Reads and clears them; synchronises the device.  Empty if all is well."""
+    if not torch.cuda.is_initialized():
+        return {}                         # no kernel has run in this process
     found = {"gemm_few": int(lib().tb_gemm_few_error()), "lightning": int(lib().tb_lightning_error())}
     if _tlib is not None:
         found["gemm_tc"] = gemm_tc_error()
