@@ -300,6 +300,60 @@ def test_recurrence_in_chunks(K, dtype, dk, dv, plain):
     assert float((bad[:place] - out[:place]).abs().max()) < 1e-4 * float(out.abs().max()) and not bool(torch.isfinite(bad[place:, 0]).any())
 
 
+@pytest.mark.parametrize("dk,dv", [(64, 20), (128, 33)])
+def test_recurrence_room_is_bounded_and_segments_are_the_same_bits(K, monkeypatch, dk, dv):
+    """Runs beside shorter ones, cut by segments of one, two, five chunks: outputs and states are the bits of one segment, and so are those of a run alone;
+    the room for a long prompt has a bound, and is halved where memory is short."""
+    g = torch.Generator().manual_seed(dk)
+    lens, H = [63, 64, 1, 400, 65, 5, 130], 2
+    stride = 2 * H * dk + 2 * H * dv
+    proj = torch.randn(sum(lens), stride, generator=g).cuda()
+    state = torch.randn(len(lens), H, dk, dv, generator=g)
+    dec = torch.tensor([0.97, 1.0], device="cuda")
+    begin = [0] + list(itertools.accumulate(lens))
+
+    def args(which):
+        n = [lens[i] for i in which]
+        keep = (torch.cat([proj[begin[i]:begin[i + 1]] for i in which]), state.cuda().clone(), torch.tensor(list(which), dtype=torch.int32).cuda(),
+                torch.tensor([0] + list(itertools.accumulate(n)), dtype=torch.int32).cuda(), torch.empty(sum(n), H * dv, device="cuda"))
+        a = K.LightningArgs()
+        a.proj, a.stride, a.out, a.out_stride = keep[0].data_ptr(), stride, keep[4].data_ptr(), H * dv
+        a.state, a.decay, a.q_start, a.slot_of_seq = keep[1].data_ptr(), dec.data_ptr(), keep[3].data_ptr(), keep[2].data_ptr()
+        a.B, a.H, a.dk, a.dv, a.max_new, a.plain = len(n), H, dk, dv, max(n), 1
+        return a, keep, sum(n)
+
+    def run(which):
+        a, keep, tokens = args(which)
+        work = K.lightning_work(a, tokens, "cuda")
+        K.lightning_scan(a, torch.float32, stream())
+        del work
+        return keep[4].cpu(), keep[1].cpu()
+
+    out, st = run(range(7))
+    each = 4 * H * ((64 * (64 + (64 if dk <= 64 else 128) + 4)) + (64 if dk <= 64 else 128) * 68)
+    for chunks in (1, 2, 5):
+        monkeypatch.setattr(K, "LIGHTNING_ROOM", chunks * each)
+        again, st_again = run(range(7))
+        assert torch.equal(again, out) and torch.equal(st_again, st), chunks
+    alone, st_alone = run([3])
+    assert torch.equal(alone, out[begin[3]:begin[4]]) and torch.equal(st_alone[3], st[3])
+    monkeypatch.undo()
+    a, keep, _ = args(range(7))
+    a.H, a.max_new = 16, 1 << 20                                                   # (asked for only, never run)
+    assert 4 * K.lightning_work(a, 1 << 20, "cuda").numel() <= K.LIGHTNING_ROOM and a.work_chunks > 1 << 14
+    real, asked = torch.empty, []
+
+    def short(n, **kw):
+        asked.append(n)
+        if len(asked) < 3:
+            raise torch.OutOfMemoryError("short of memory")
+        return real(n, **kw)
+
+    monkeypatch.setattr(K.torch, "empty", short)
+    work = K.lightning_work(a, 1 << 20, "cuda")
+    assert work is not None and len(asked) == 3 and asked[2] < asked[0] // 3 and work.numel() == asked[2]
+
+
 @pytest.mark.parametrize("H,F,counts", [(64, 24, [1, 0, 127, 128, 129]), (264, 40, [0, 300, 0]), (2048, 136, [5, 260, 1, 0, 31, 33])])
 def test_experts_products_in_one_launch(K, H, F, counts):
     """Empty runs, runs on both sides of a row tile, columns that end inside a tile; rows behind the last run are not touched."""

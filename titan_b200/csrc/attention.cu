@@ -220,30 +220,6 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_prefill_kernel(AttnArgs a
 // tiles of 64 more cost nothing.
 constexpr int TILE_FROM = 32;
 
-// The run of the step that holds the ``left``-th of the things that count(tokens of a run) counts, -1 behind the last; ``left`` becomes the
-// place within the run.  A warp's lanes look at 32 runs at a time; every lane returns the same.
-template <typename F>
-__device__ __forceinline__ int find_run(const TbBatch& batch, int& left, F count) {
-    const int lane = threadIdx.x & 31;
-    for (int s0 = 0; s0 < batch.B; s0 += 32) {
-        const int s = s0 + lane, mine = s < batch.B ? count(batch.q_start[s + 1] - batch.q_start[s]) : 0;
-        int upto = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o *= 2) {
-            const int u = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += u;
-        }
-        const int total = __shfl_sync(0xffffffffu, upto, 31);
-        if (left < total) {
-            const int at = __ffs(__ballot_sync(0xffffffffu, upto > left)) - 1;
-            left -= __shfl_sync(0xffffffffu, upto - mine, at);
-            return s0 + at;
-        }
-        left -= total;
-    }
-    return -1;
-}
-
 // One head of one query of a short run by one warp, VW neighbouring elements of the head a lane.  A lane scores two neighbouring keys of 64;
 // weights and value rows' addresses pass through the warp's piece of shared memory, sixteen value rows are requested at once.
 // Bound by the latency of a key's row (a lane walks it alone: a sum over a row has one order).
@@ -258,7 +234,7 @@ template <int VW>
 __device__ __forceinline__ void attend_row(const AttnArgs& a, RowShared<VW>& sh, int item) {
     const int lane = threadIdx.x & 31, hd = a.hd, h = item % a.nh, kh = h / (a.nh / a.nkv);
     int place = item / a.nh;
-    const int seq = find_run(a.batch, place, [](int n) { return n < TILE_FROM ? n : 0; });
+    const int seq = tb_find_run(a.batch.q_start, a.batch.B, place, [](int n) { return n < TILE_FROM ? n : 0; });
     if (seq < 0) return;
     const int t0 = a.batch.q_start[seq], first = a.batch.start_pos[seq], slot = a.batch.slot_of_seq[seq], pos = first + place;
     const int first_new = a.kv_new ? first : 0x7fffffff;
@@ -404,7 +380,7 @@ __global__ void __launch_bounds__(256) attn_prefill_tile_kernel(AttnArgs a, int 
     }
     // which sequence, which tile of it; a sequence's last tiles, which see the most keys, start first
     int tile = blockIdx.x;
-    const int seq = find_run(a.batch, tile, [](int n) { return n >= TILE_FROM ? (n + TILE_Q - 1) / TILE_Q : 0; });
+    const int seq = tb_find_run(a.batch.q_start, a.batch.B, tile, [](int n) { return n >= TILE_FROM ? (n + TILE_Q - 1) / TILE_Q : 0; });
     if (seq < 0) return;
     const int t0 = a.batch.q_start[seq], n_new = a.batch.q_start[seq + 1] - t0;
     tile = (n_new + TILE_Q - 1) / TILE_Q - 1 - tile;

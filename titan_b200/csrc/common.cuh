@@ -114,6 +114,30 @@ __device__ __forceinline__ size_t kv_half_elems(const TbKvView& c) {
     return (size_t)c.num_pages * c.kv_heads * c.page_size * c.head_dim;
 }
 
+// The run of a step (tokens q_start[s] .. q_start[s + 1] - 1) that holds the ``left``-th of the things that count(tokens of a run) counts, -1
+// behind the last; ``left`` becomes the place within the run.  A warp's lanes look at 32 runs at a time; every lane returns the same.
+template <typename F>
+__device__ __forceinline__ int tb_find_run(const int* q_start, int B, int& left, F count) {
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < B; s0 += 32) {
+        const int s = s0 + lane, mine = s < B ? count(q_start[s + 1] - q_start[s]) : 0;
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            const int u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+        if (left < total) {
+            const int at = __ffs(__ballot_sync(0xffffffffu, upto > left)) - 1;
+            left -= __shfl_sync(0xffffffffu, upto - mine, at);
+            return s0 + at;
+        }
+        left -= total;
+    }
+    return -1;
+}
+
 // ---------------------------------------------------------------- programmatic dependent launch
 // Kernels of a step are launched so that a kernel may start while its predecessor in the stream is
 // still finishing (its blocks are scheduled once every block of the predecessor has called

@@ -4,7 +4,9 @@
 //   o_t = S_t^T q_t
 // with q = silu(.), k = silu(.), v = silu(.) of the projection's columns (the projection may be in the compute
 // dtype; the activation, the state and the sums are float32).  A sequence's tokens are taken in order, so a prompt
-// run whole, in pieces or token by token leaves the same state up to the order of float32 sums.
+// run whole, in pieces or token by token leaves the same state up to the order of float32 sums: runs of few tokens are added one
+// after the other, longer ones in chunks of 64 that begin where the step's run begins, so that a cut changes the last bits (what a
+// sequence gives does not depend on the other sequences of the step).
 //
 // tb_lightning_scan   grid (sequences, heads, ceil(dv / 32)): a block owns 32 value columns of one head's state;
 //                     four neighbouring lanes share a column (each keeps a quarter of its rows in registers) and
@@ -29,8 +31,10 @@ struct LightningArgs {
     int B; int H; int dk; int dv;
     int max_new;                            // most tokens a sequence brings in this step (1: a step of single tokens)
     int plain;                              // 1: q, k and v enter the recurrence as they stand in the rows (no silu): the retention mixer, whose rows are float32
-    float* work; int work_chunks;           // room for the chunked form (tb_lightning_work floats), work_chunks >= sum over sequences of ceil(tokens / 64); null: token by token
+    float* work; int work_chunks;           // room for the chunked form; work_chunks >= the chunks of all its runs (tb_lightning_work); null: token by token
+    int work_room;                          // chunks that ``work`` holds at a time: more go one segment after the other
     int below;                              // > 0: only runs of fewer tokens (set by the launcher)
+    int segment;                            // first chunk of the segment at work (set by the launcher)
 };
 
 namespace {
@@ -268,8 +272,14 @@ __global__ void __launch_bounds__(128) lightning_scan_vec_kernel(LightningArgs a
 // 128 blocks for one sequence of 16 heads of 128.  The FMA pipes would need 2,560 cycles a chunk (43 us of the second figure).
 // 2,000 tokens, 16 heads of 128 x 128: 34 us and 146 us, of which the outputs' product takes about 50 and the
 // state's 30; the rest is barriers, the merge of the warps' parts, values and stores.
+// Chunks are numbered through all long runs of the step; a segment of them is prepared and worked off before the next, so that their rows need
+// a bounded room however long the prompt is: the state passes from segment to segment through the cache, the bits are the same.
 constexpr int CHUNK = 64, VCOLS = 16;
-constexpr int CHUNKED_FROM = 32;        // tokens of the longest run from which the chunked form is the faster one
+// Tokens of a run from which it goes in chunks: where one sequence is the faster so (token by token / in chunks, us: 16 heads of 128 x 128, 32
+// tokens 18 / 30, 40 23 / 30, 64 33 / 29, 100 53 / 31; 32 heads of 64 x 128, 40 tokens 17 / 20, 64 24 / 22, 100 38 / 29).  Many short runs together cost more
+// in chunks (64 runs of 40 tokens of 16 heads of 128: 322 / 540; of 100: 761 / 860; 32 heads of 64 x 128: 768 / 1,329), but what a run gives
+// may not depend on the runs beside it.
+constexpr int CHUNKED_FROM = 64;
 
 __device__ __forceinline__ void lf_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
@@ -285,7 +295,7 @@ template <int DK> constexpr size_t chunk_floats() { return (size_t)chunk_a<DK>()
 __device__ unsigned int g_lightning_error = 0;
 template <int DK> constexpr size_t prep_smem() { return (size_t)(2 * CHUNK * (DK + 4) + CHUNK + 1) * sizeof(float); }
 
-// grid (work_chunks, H), 256 threads
+// grid (chunks of a segment, H), 256 threads
 template <typename T, int DK>
 __global__ void __launch_bounds__(256) lightning_prep_kernel(LightningArgs a) {
     pdl_launch_dependents();
@@ -296,14 +306,10 @@ __global__ void __launch_bounds__(256) lightning_prep_kernel(LightningArgs a) {
     float* ks = qs + CHUNK * LD;
     float* power = ks + CHUNK * LD;                     // decay^0 .. decay^64
     const int tid = threadIdx.x, h = blockIdx.y, dk = a.dk;
-    int b = 0, chunk = blockIdx.x, t0 = 0, n = 0;
-    for (; b < a.B; ++b) {
-        t0 = a.q_start[b];
-        const int left = a.q_start[b + 1] - t0, chunks = (left + CHUNK - 1) / CHUNK;
-        if (chunk < chunks) { t0 += chunk * CHUNK; n = left < CHUNKED_FROM ? 0 : min(CHUNK, left - chunk * CHUNK); break; }
-        chunk -= chunks;
-    }
-    if (b == a.B || n == 0) return;
+    int chunk = a.segment + blockIdx.x;
+    const int b = tb_find_run(a.q_start, a.B, chunk, [](int m) { return m >= CHUNKED_FROM ? (m + CHUNK - 1) / CHUNK : 0; });
+    if (b < 0) return;
+    const int t0 = a.q_start[b] + chunk * CHUNK, n = min(CHUNK, a.q_start[b + 1] - t0);
     if (tid <= CHUNK) power[tid] = (float)pow((double)a.decay[h], (double)tid);
     const T* base = (const T*)a.proj + (size_t)t0 * a.stride + h * dk;
     if (dk % 8 == 0 && a.stride % 8 == 0 && (uintptr_t)a.proj % 16 == 0) {
@@ -397,7 +403,7 @@ template <int DK> constexpr size_t chunk_smem() {
     return (size_t)(2 * (CHUNK * (chunk_row<DK>() + 4) + DK * (CHUNK + 4)) + VCOLS * (chunk_row<DK>() + 4) + 8 * VCOLS * PART_COL) * sizeof(float) + 16;
 }
 
-// grid (B, H, ceil(dv / 16)), 512 threads: warps 0 .. 7 make the outputs while warps 8 .. 15 make the state after the chunk
+// grid (long runs at most, H, ceil(dv / 16)), 512 threads: warps 0 .. 7 make the outputs while warps 8 .. 15 make the state after the chunk
 template <typename T, int DK>
 __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
     pdl_launch_dependents();
@@ -409,12 +415,22 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
     float* vals = krows + 2 * DK * LT;                  // [VCOLS][LD]: by column, the chunk's values, then the state
     float* part = vals + VCOLS * LD;                    // [8][VCOLS][PART_COL]
     uint64_t* landed = reinterpret_cast<uint64_t*>(part + 8 * VCOLS * PART_COL);      // [2]
-    const int b = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * VCOLS;
+    const int h = blockIdx.y, j0 = blockIdx.z * VCOLS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int dk = a.dk, dv = a.dv, t0 = a.q_start[b], t1 = a.q_start[b + 1];
-    if (t1 - t0 < CHUNKED_FROM) return;
-    int chunk0 = 0;                                     // the sequence's first chunk
-    for (int i = 0; i < b; ++i) chunk0 += (a.q_start[i + 1] - a.q_start[i] + CHUNK - 1) / CHUNK;
+    const int dk = a.dk, dv = a.dv;
+    int which = blockIdx.x;
+    const int b = tb_find_run(a.q_start, a.B, which, [](int m) { return m >= CHUNKED_FROM ? 1 : 0; });
+    if (b < 0) return;
+    const int t0 = a.q_start[b], t1 = a.q_start[b + 1];
+    int chunk0 = 0;                                     // the run's first chunk
+    for (int i = lane; i < b; i += 32) {
+        const int m = a.q_start[i + 1] - a.q_start[i];
+        if (m >= CHUNKED_FROM) chunk0 += (m + CHUNK - 1) / CHUNK;
+    }
+    chunk0 = __reduce_add_sync(0xffffffffu, chunk0);
+    // the run's chunks in this segment
+    const int begin = max(0, a.segment - chunk0), end = min((t1 - t0 + CHUNK - 1) / CHUNK, a.segment + a.work_room - chunk0);
+    if (begin >= end) return;
     const float decay = a.decay[h], whole = (float)pow((double)decay, (double)CHUNK);
     // the state: a thread of the second half keeps rows sk + 32 i of columns sc and sc + 8
     const bool keeps = tid >= 256;
@@ -436,7 +452,7 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
     __syncthreads();
     auto load_rows = [&](int c, int half) {             // two bulk copies, by one thread
         if (tid != 0) return;
-        const float* from = a.work + ((size_t)(chunk0 + c) * a.H + h) * chunk_floats<DK>();
+        const float* from = a.work + ((size_t)(chunk0 + c - a.segment) * a.H + h) * chunk_floats<DK>();
         tbtma::mbar_expect_tx(landed + half, (uint32_t)(chunk_floats<DK>() * sizeof(float)));
         bulk_copy(rows + half * CHUNK * LD, from, chunk_a<DK>() * 4, landed + half);
         bulk_copy(krows + half * DK * LT, from + chunk_a<DK>(), chunk_k<DK>() * 4, landed + half);
@@ -461,11 +477,10 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
         }
     };
     const bool out4 = dv % 4 == 0 && a.out_stride % 4 == 0 && (uintptr_t)a.out % 16 == 0;
-    const int chunks = (t1 - t0 + CHUNK - 1) / CHUNK;
-    load_rows(0, 0);
-    load_values(0);
-    for (int c = 0; c < chunks; ++c) {
-        const int half = c & 1, n = min(CHUNK, t1 - t0 - c * CHUNK);
+    load_rows(begin, 0);
+    load_values(begin);
+    for (int c = begin; c < end; ++c) {
+        const int half = (c - begin) & 1, n = min(CHUNK, t1 - t0 - c * CHUNK);
         int odd = 0;                                    // a value that is not finite: its product with a zero weight is no zero
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -474,8 +489,8 @@ __global__ void __launch_bounds__(512) lightning_chunk_kernel(LightningArgs a) {
             vals[(lc + i) * LD + vr] = next[i];
         }
         odd = __syncthreads_or(odd);
-        tbtma::mbar_wait(landed + half, (c >> 1) & 1, &g_lightning_error, 1);
-        if (c + 1 < chunks) { load_rows(c + 1, half ^ 1); load_values(c + 1); }
+        tbtma::mbar_wait(landed + half, ((c - begin) >> 1) & 1, &g_lightning_error, 1);
+        if (c + 1 < end) { load_rows(c + 1, half ^ 1); load_values(c + 1); }
         const float* A = rows + half * CHUNK * LD;
         if (!keeps) {   // this warp's KW of the columns of A: rows rg + 8 r, value columns cg + 4 j; sums over even and over odd places
             const int cg = lane & 3, rg = lane >> 2;
@@ -565,8 +580,12 @@ int launch_chunks(const LightningArgs& a, cudaStream_t stream) {
         TB_REQUIRE(e == cudaSuccess, "lightning_scan: cannot reserve %zu bytes of shared memory: %s", chunk_smem<DK>(), cudaGetErrorString(e));
         if (dev < 64) configured[dev].store(true);
     }
-    tb_launch(lightning_prep_kernel<T, DK>, dim3(a.work_chunks, a.H), 256, prep_smem<DK>(), stream, a);
-    tb_launch(lightning_chunk_kernel<T, DK>, dim3(a.B, a.H, (a.dv + VCOLS - 1) / VCOLS), 512, chunk_smem<DK>(), stream, a);
+    LightningArgs part = a;
+    const int runs = min(a.B, a.work_chunks);           // (a long run has a chunk at least)
+    for (part.segment = 0; part.segment < a.work_chunks; part.segment += a.work_room) {
+        tb_launch(lightning_prep_kernel<T, DK>, dim3(min(a.work_room, a.work_chunks - part.segment), a.H), 256, prep_smem<DK>(), stream, part);
+        tb_launch(lightning_chunk_kernel<T, DK>, dim3(runs, a.H, (a.dv + VCOLS - 1) / VCOLS), 512, chunk_smem<DK>(), stream, part);
+    }
     if (a.B > 1) {                                      // shorter runs beside them go token by token, as they would alone
         LightningArgs rest = a;
         rest.work = nullptr; rest.below = CHUNKED_FROM;
@@ -681,17 +700,18 @@ int launch_scan(const LightningArgs& a, bool single, cudaStream_t stream) {
 
 }  // namespace
 
-// Floats of ``work`` (and its chunks) with which a step of T tokens in B runs, the longest of max_new, takes the chunked form;
-// 0: none is wanted (short runs, where the two launches cost more than the chain; heads of more than 128 key dimensions).
+// Floats a chunk takes in ``work``, and in ``chunks`` how many chunks a step of T tokens in B runs, the longest of max_new, has at most; 0: no run is
+// long enough for the chunked form (or a head has more than 128 key dimensions).  The caller gives room for as many as it likes, one at least.
 extern "C" long long tb_lightning_work(int T, int B, int H, int dk, int dv, int max_new, int* chunks) {
-    if (max_new < CHUNKED_FROM || dk > 128 || (dv + VCOLS - 1) / VCOLS > 65535) { *chunks = 0; return 0; }
-    *chunks = T / CHUNK + B;                            // at least the sum of every run's chunks
-    return (long long)*chunks * H * (long long)(dk <= 64 ? chunk_floats<64>() : chunk_floats<128>());
+    *chunks = 0;
+    if (max_new < CHUNKED_FROM || dk > 128 || (dv + VCOLS - 1) / VCOLS > 65535) return 0;
+    *chunks = T / CHUNK + min(B, T / CHUNKED_FROM);
+    return (long long)H * (long long)(dk <= 64 ? chunk_floats<64>() : chunk_floats<128>());
 }
 
 extern "C" int tb_lightning_scan(const LightningArgs* args, int dtype, cudaStream_t stream) {
     LightningArgs a = *args;
-    a.below = 0;
+    a.below = a.segment = 0;
     TB_REQUIRE(a.B > 0 && a.H > 0 && a.dk > 0 && a.dv > 0, "lightning_scan: sizes must be positive");
     TB_REQUIRE(a.dk <= 256, "lightning_scan: %d key dimensions a head (at most 256)", a.dk);
     TB_REQUIRE(a.H <= 65535 && (a.dv + 31) / 32 <= 65535, "lightning_scan: too many heads or value columns");
@@ -699,7 +719,7 @@ extern "C" int tb_lightning_scan(const LightningArgs* args, int dtype, cudaStrea
     TB_REQUIRE(a.stride >= 2 * a.H * a.dk + a.H * a.dv, "lightning_scan: the projection row is too short");
     TB_REQUIRE(dtype == TB_F32 || dtype == TB_BF16, "lightning_scan: unknown dtype %d", dtype);
     const bool single = a.max_new <= 1;
-    TB_REQUIRE(!a.work || (a.dk <= 128 && a.work_chunks > 0 && (a.dv + VCOLS - 1) / VCOLS <= 65535 && (uintptr_t)a.work % 16 == 0),
+    TB_REQUIRE(!a.work || (a.dk <= 128 && a.work_chunks > 0 && a.work_room > 0 && (a.dv + VCOLS - 1) / VCOLS <= 65535 && (uintptr_t)a.work % 16 == 0),
                "lightning_scan: the chunked form takes heads of up to 128 key dimensions (%d)", a.dk);
     if (dtype == TB_F32 ? launch_scan<float>(a, single, stream) : launch_scan<__nv_bfloat16>(a, single, stream)) return 1;
     TB_CHECK_LAUNCH("lightning_scan");

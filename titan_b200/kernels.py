@@ -121,7 +121,7 @@ class LightningArgs(Structure):
     _fields_ = [("proj", c_void_p), ("stride", c_int), ("out", c_void_p), ("out_stride", c_int), ("state", c_void_p),
                 ("decay", c_void_p), ("q_start", c_void_p), ("slot_of_seq", c_void_p),
                 ("B", c_int), ("H", c_int), ("dk", c_int), ("dv", c_int), ("max_new", c_int), ("plain", c_int),
-                ("work", c_void_p), ("work_chunks", c_int), ("below", c_int)]
+                ("work", c_void_p), ("work_chunks", c_int), ("work_room", c_int), ("below", c_int), ("segment", c_int)]
 
 
 class WholeNormArgs(Structure):
@@ -710,12 +710,28 @@ def latent_append(rows: torch.Tensor, cache: KvView, batch: Batch, stream: int) 
     _check(lib().tb_latent_append(rows.data_ptr(), rows.stride(0), dtype_code(rows.dtype), byref(cache), byref(batch), stream))
 
 
+LIGHTNING_ROOM = 256 << 20        # bytes of room for the chunks of a recurrence at most (one chunk's where that is more)
+
+
 def lightning_work(args: "LightningArgs", tokens: int, device) -> Optional[torch.Tensor]:
-    """Room for the chunked form of the recurrence, named in ``args`` (to be held until it has run); None where the step runs token by token."""
+    """Room for the chunked form of the recurrence, named in ``args`` (to be held until it has run); None where the step runs token by token.
+    A chunk of 64 tokens takes 85 KB a head of more than 64 key dimensions (52 KB below): long prompts go through it segment by segment, and one that
+    finds less memory free in smaller segments; the result is the same bits."""
     chunks = c_int(0)
-    n = int(lib().tb_lightning_work(tokens, args.B, args.H, args.dk, args.dv, args.max_new, byref(chunks)))
-    work = torch.empty(n, dtype=torch.float32, device=device) if n else None
-    args.work, args.work_chunks = _ptr(work), chunks.value
+    each = int(lib().tb_lightning_work(tokens, args.B, args.H, args.dk, args.dv, args.max_new, byref(chunks)))
+    args.work, args.work_chunks, args.work_room = None, 0, 0
+    if not each:
+        return None
+    room = max(1, min(chunks.value, LIGHTNING_ROOM // (4 * each)))
+    while True:
+        try:
+            work = torch.empty(room * each, dtype=torch.float32, device=device)
+            break
+        except torch.OutOfMemoryError:
+            if room == 1:
+                raise
+            room = (room + 1) // 2
+    args.work, args.work_chunks, args.work_room = work.data_ptr(), chunks.value, room
     return work
 
 

@@ -7,8 +7,9 @@
 
 The state is what the mixer asks of the cache: a ``state`` group of shape [heads, dim, value_dim] in float32 per
 sequence, zeroed when a slot is handed out, read and written through the step's slot indices on the device (nothing
-of the layout is read on the host, so decode steps with this mixer are captured as graphs like any other).  The
-recurrence takes a sequence's tokens in order whatever the step brings: a whole prompt, a piece of it, or one token.
+of the layout is read on the host, so decode steps with this mixer are captured as graphs like any other).  A step may
+bring a whole prompt, a piece of it, or one token: runs of fewer than 64 tokens are added one after the other, longer
+ones in chunks of 64 from where the run begins, so that a cut changes the order of the float32 sums.
 """
 from __future__ import annotations
 

@@ -8,8 +8,8 @@
 What enters the recurrence is float32 in either dtype: the projection leaves float32 sums, the rotation (angles in float32)
 and the key's factor are applied to them in place, and the recurrence kernel of the ``lightning`` mixer reads them as they
 stand (``LightningArgs.plain``).  The state is a ``state`` cache group of shape [heads, dim, value_dim] per sequence,
-zeroed when a slot is handed out and indexed by slot on the device, so decode steps are captured as graphs; a sequence's
-tokens are taken in order whatever the step brings.  Options of the spec: ``value_dim``, ``decay`` (one number a head),
+zeroed when a slot is handed out and indexed by slot on the device, so decode steps are captured as graphs; runs of fewer
+than 64 tokens are added one after the other, longer ones in chunks of 64.  Options of the spec: ``value_dim``, ``decay`` (one number a head),
 ``norm_eps``, ``key_scale``; the rotation is ``MixerSpec.position`` (either pairing, the first ``rotary_dim`` of a head).
 """
 from __future__ import annotations
