@@ -418,9 +418,10 @@ def test_a_row_of_router_logits_that_are_not_numbers_chooses_experts_there_are(K
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,H", [(512, 1024), (513, 2048), (8192, 2052), (8193, 2564), (8192, 4092), (512, 4096), (700, 4100), (8192, 8192)])
+@pytest.mark.parametrize("rows,H", [(512, 1024), (513, 2048), (8192, 2052), (8193, 2564), (8192, 4092), (512, 4096), (700, 4100), (8192, 8192),
+                                    (799, 4096), (800, 4096), (1599, 2048), (1600, 1024), (1600, 2048)])
 def test_norms_of_long_prompts_are_the_bits_of_short_ones(K, dtype, rows, H):
-    """The kernel of 512 rows and more against the one of fewer, at both ends of every number of threads and units."""
+    """The kernel of long prompts against the one of short ones, at both ends of every number of threads and units."""
     g = torch.Generator().manual_seed(H)
     x, w = (torch.randn(rows, H, generator=g) * 3).cuda(), (1 + 0.1 * torch.randn(H, generator=g)).cuda()
     y, few = torch.empty(rows, H, dtype=dtype, device="cuda"), torch.empty(rows, H, dtype=dtype, device="cuda")

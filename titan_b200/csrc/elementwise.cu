@@ -119,8 +119,8 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restr
 
 // Long prompts: a quarter of the kernel above's threads a row and four times the 16-byte units a thread, so that an SM holds many rows' loads
 // at once (four rows of 512 threads with two units each left it waiting), and one barrier instead of three.  A thread keeps the four sums of the
-// threads whose units it has and adds them as those do: the same bits.  Bound by the bytes: 17,416 rows of
-// 4,096 in 63 us (6.8 TB/s; 111 us before), 2,048 in 11.5 (15.5), 17,416 of 2,560 in 43 (48).
+// threads whose units it has and adds them as those do: the same bits.  Bound by the bytes, part of which L2 holds: 17,416 rows of
+// 4,096 in 63 us (111 us above), 2,048 in 10.2 (13.3), 17,416 of 2,560 in 43 (48).
 template <typename T, int NV>
 __global__ void __launch_bounds__(128) rmsnorm_rows_kernel(const float* x, const float* __restrict__ w, T* y, int H, float eps) {
     pdl_launch_dependents();
@@ -159,8 +159,10 @@ template <typename T>
 static void launch_rmsnorm(const float* x, const float* w, T* y, const int* rows, int n_rows, int H, float eps, cudaStream_t stream) {
     const int threads = H >= 4096 ? 512 : (H >= 1024 ? 256 : (H >= 256 ? 64 : 32));
     const bool vec = (H % 4 == 0) && H <= 16 * threads && ((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 16 == 0);
-    // rows that need sixteen units a thread only where there are very many (2,048 of 2,560: 7.9 us above, 10.5 here)
-    if (vec && !rows && n_rows >= (H <= 8 * threads ? 512 : 8192) && threads >= 256) {
+    // From the second round of the kernel above's blocks on (four of 512 threads an SM, eight of 256): above / here, bfloat16, us: 4,096 columns, 512 rows
+    // 3.3 / 4.4, 700 4.4 / 4.6, 1,000 5.8 / 4.7; 1,024, 1,000 rows 3.0 / 3.2, 2,048 4.6 / 4.0; 2,048, 1,000 rows 3.2 / 4.3, 2,048 5.0 / 5.1, 4,000 10.8 / 9.9.
+    // Rows that need sixteen units a thread only where there are very many (2,048 of 2,560: 7.9 us above, 10.5 here).
+    if (vec && !rows && (H <= 8 * threads ? (long long)n_rows * threads >= 800 * 512 : n_rows >= 8192) && threads >= 256) {
         if (H <= 8 * threads) tb_launch(rmsnorm_rows_kernel<T, 8>, n_rows, threads / 4, 0, stream, x, w, y, H, eps);
         else tb_launch(rmsnorm_rows_kernel<T, 16>, n_rows, threads / 4, 0, stream, x, w, y, H, eps);
         return;
