@@ -417,6 +417,27 @@ def test_a_row_of_router_logits_that_are_not_numbers_chooses_experts_there_are(K
     assert bool(((ids >= 0) & (ids < 8)).all()) and ids[1].tolist() == [7, 6]
 
 
+@pytest.mark.parametrize("T,H,top", [(1, 7, 1), (3, 130, 8), (255, 1028, 2), (256, 1030, 3), (300, 4, 5)])
+def test_combining_by_single_columns_and_by_fours(K, T, H, top):
+    """Rows of whole 16-byte units and rows that are not: the sum in 64 bits, and the same bits where a row is one column longer."""
+    g = torch.Generator().manual_seed(H)
+    wide = H + 4 - H % 4 if H % 4 else H + 1                                       # the other form's width
+    ids = torch.randint(0, 6, (T, top), generator=g).to(torch.int32).cuda()
+    where = torch.randperm(T * top, generator=g).to(torch.int32).cuda()
+    y, w, shared, gate, out = (torch.randn(*s, generator=g).cuda() for s in ((T * top, wide), (T, top), (T, wide), (T,), (T, wide)))
+    x = torch.randn(T, wide, generator=g).to(torch.bfloat16).cuda()
+    found = []
+    for n in (H, wide):
+        o = out[:, :n].clone()
+        K.moe_combine(y[:, :n].contiguous(), w, shared[:, :n].contiguous(), gate, o, top, stream(), where=where, ids=ids, n_real=4, x=x[:, :n].contiguous())
+        found.append(o)
+    m = min(H, wide)
+    assert torch.equal(found[0][:, :m], found[1][:, :m])
+    rows = torch.where((ids < 4)[..., None], y.double()[where.long()].view(T, top, wide), x.double()[:, None, :])
+    want = out.double() + (w.double()[..., None] * rows).sum(1) + gate.double()[:, None] * shared.double()
+    assert float((found[1].double() - want).norm() / want.norm()) < 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,H", [(512, 1024), (513, 2048), (8192, 2052), (8193, 2564), (8192, 4092), (512, 4096), (700, 4100), (8192, 8192),
                                     (799, 4096), (800, 4096), (1599, 2048), (1600, 1024), (1600, 2048)])

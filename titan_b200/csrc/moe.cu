@@ -13,6 +13,7 @@
 //   tb_moe_rows      the same two products for a handful of pairs (decode steps): a warp per output column (or
 //                    gate/up pair) of one pair, lanes along K, weights read once per pair through L2; no plan.
 //   tb_moe_combine   out[t] += sum_k weight[t][k] * y[t * top + k] (+ gate[t] * shared[t]), float32, in pair order.
+#include <type_traits>
 #include <float.h>
 
 #include "common.cuh"
@@ -377,6 +378,28 @@ moe_rows_kernel(const T* __restrict__ X, int ldx, const T* __restrict__ W, void*
 // ------------------------------------------------------------------ combine
 // ``ids`` with ``n_real`` and ``x``: a pair whose expert is n_real or beyond has no matrices and no row in y; its output
 // is the token's own input row x[t].
+// Rows that are no whole 16-byte units, up to four choices a token: single columns, all loads as loads of constants (4,099 columns, 2,000 tokens, one / two / four
+// choices: 45 / 64 / 69 us, the kernel below 58 / 82 / 87; eight: 117 / 96).
+template <typename T>
+__global__ void moe_combine_columns_kernel(const float* __restrict__ y, const float* __restrict__ wts, const float* __restrict__ shared_y,
+                                           const float* __restrict__ gate, float* __restrict__ out, int H, int top, const int* __restrict__ where,
+                                           const int* __restrict__ ids, int n_real, const T* __restrict__ x, int ldx) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    const int per = (H + gridDim.y - 1) / gridDim.y, i0 = blockIdx.y * per, i1 = min(H, i0 + per);      // gridDim.y blocks share a row (steps of few rows)
+    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        float s = 0.f;
+        for (int k = 0; k < top; ++k) {
+            if (ids && ids[t * top + k] >= n_real) { s = fmaf(wts[t * top + k], ldf(x + t * ldx + i), s); continue; }
+            const size_t row = where ? (size_t)where[t * top + k] : t * top + k;       // pair order, or where the plan put the pair
+            s = fmaf(wts[t * top + k], y[row * H + i], s);
+        }
+        if (shared_y) s = fmaf(gate ? gate[t] : 1.f, shared_y[t * H + i], s);
+        out[t * H + i] += s;
+    }
+}
+
 template <typename T>
 __global__ void moe_combine_kernel(const float* y, const float* wts, const float* shared_y,
                                    const float* gate, float* out, int H, int top, const int* where,
@@ -522,10 +545,13 @@ extern "C" int tb_moe_combine(const float* y, const float* wts, const float* sha
     const int vec = H % 4 == 0 && (((uintptr_t)y | (uintptr_t)out | (uintptr_t)shared_y) & 15) == 0;
     const int threads = H >= 1024 ? 256 : 128, cols = vec ? 4 * threads : threads;
     const dim3 grid(T_, T_ >= 256 && !vec ? 1 : (H + cols - 1) / cols);
-    if (ids && x_dtype == TB_BF16)
-        tb_launch(moe_combine_kernel<__nv_bfloat16>, grid, threads, 0, stream, y, wts, shared_y, gate, out, H, top, where, ids, n_real, (const __nv_bfloat16*)x, ldx, vec);
-    else
-        tb_launch(moe_combine_kernel<float>, grid, threads, 0, stream, y, wts, shared_y, gate, out, H, top, where, ids, n_real, (const float*)x, ldx, vec);
+    const auto go = [&](auto* rows) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(rows)>>;
+        if (!vec && top <= 4) tb_launch(moe_combine_columns_kernel<T>, grid, threads, 0, stream, y, wts, shared_y, gate, out, H, top, where, ids, n_real, rows, ldx);
+        else tb_launch(moe_combine_kernel<T>, grid, threads, 0, stream, y, wts, shared_y, gate, out, H, top, where, ids, n_real, rows, ldx, vec);
+    };
+    if (ids && x_dtype == TB_BF16) go((const __nv_bfloat16*)x);
+    else go((const float*)x);
     TB_CHECK_LAUNCH("moe_combine");
     return 0;
 }
