@@ -354,7 +354,7 @@ def test_recurrence_room_is_bounded_and_segments_are_the_same_bits(K, monkeypatc
     assert work is not None and len(asked) == 3 and asked[2] < asked[0] // 3 and work.numel() == asked[2]
 
 
-@pytest.mark.parametrize("H,F,counts", [(64, 24, [1, 0, 127, 128, 129]), (264, 40, [0, 300, 0]), (2048, 136, [5, 260, 1, 0, 31, 33])])
+@pytest.mark.parametrize("H,F,counts", [(64, 24, [1, 0, 127, 128, 129]), (264, 40, [0, 300, 0]), (2048, 136, [5, 260, 1, 0, 31, 33]), (328, 1032, [200, 3, 129, 700])])
 def test_experts_products_in_one_launch(K, H, F, counts):
     """Empty runs, runs on both sides of a row tile, columns that end inside a tile; rows behind the last run are not touched."""
     g = torch.Generator().manual_seed(H)

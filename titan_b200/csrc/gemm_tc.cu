@@ -576,10 +576,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const float* part = reinterpret_cast<const float*>(smem_a);
             for (int idx = first + (int)threadIdx.x; idx < last; idx += THREADS) {
                 float v[16];
-    #pragma unroll
+#pragma unroll
                 for (int r = 0; r < 16; ++r) v[r] = r < n ? tbtma::ld_cluster_f32(tbtma::cluster_addr(part + idx, r)) : 0.f;     // all loads first
                 float sum = 0.f;
-    #pragma unroll
+#pragma unroll
                 for (int r = 0; r < 16; ++r) sum += v[r];                  // in the order of the slices
                 const int m = idx / BM, row = tile_a * BM + idx % BM;
                 if (row < a.rows_a) atomicAdd((float*)a.out + (size_t)m * a.ldo + row, sum);      // the element's only writer in this launch
@@ -781,7 +781,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // column tile's into the next matrix: those rows and columns are computed and not stored.
 // Bound by the tensor cores, of whose work a run's last row tile wastes half on average.  8,000 rows of 32
 // runs, 2,048 columns: K = 2,048 with the gate 93 us, K = 1,024 57 us (64 launches on four side streams took 310 us for both, and the
-// host waited for the runs' sizes before them).
+// host waited for the runs' sizes before them).  BN: columns a tile, 256, or 128 where that takes fewer rounds of the SMs (launch_runs).
 struct RunTiles {
     const int* first;       // [runs + 1]
     const int* before;      // [runs + 1] row tiles of the runs before
@@ -799,10 +799,10 @@ struct RunTiles {
     }
 };
 
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __launch_bounds__(THREADS)
 gemm_tc_runs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcArgs a, const int* first_g, int runs) {
-    constexpr int BN = 256, STAGES = stages_for<BN>();
+    constexpr int STAGES = stages_for<BN>();
     constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, TMEM_COLS = 2 * BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -1491,26 +1491,38 @@ TB_TIMELINE_SETTER(tb_gemm_tc_timeline)
 constexpr int MAX_RUNS = 1024;
 constexpr size_t runs_smem(int bn, int stages, int runs) { return 1024 + (size_t)stages * (BM + bn) * BK * 2 + 256 + 2 * (size_t)(runs + 1) * sizeof(int); }
 
-template <int EPI>
-static int launch_runs(const void* X, int ldx, const void* W, void* out, int ldo, const int* first, int runs, int rows, int N, int K, int act, float limit, cudaStream_t stream) {
-    constexpr int BN = 256;
+template <int EPI, int BN>
+static int launch_runs_of(const void* X, int ldx, const void* W, void* out, int ldo, const int* first, int runs, int rows, int N, int K, int act, float limit, int sms, cudaStream_t stream) {
     // the limit of shared memory once a device, for the most runs there may be: a limit each launch set for itself would be lowered under another thread's
     static std::atomic<bool> configured[64];
-    int dev = 0, sms = 0;
+    int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 64 || !configured[dev].load()) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_runs_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)runs_smem(BN, stages_for<BN>(), MAX_RUNS));
+        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_runs_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)runs_smem(BN, stages_for<BN>(), MAX_RUNS));
         TB_REQUIRE(e == cudaSuccess, "gemm_tc_expert_runs: cannot reserve %zu bytes of shared memory: %s", runs_smem(BN, stages_for<BN>(), MAX_RUNS), cudaGetErrorString(e));
         if (dev < 64) configured[dev].store(true);
     }
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     CUtensorMap ma, mb;
     if (tb_make_map_bf16(&ma, X, rows, K, ldx, BM) || tb_make_map_bf16(&mb, W, (long long)runs * N, K, K, BN)) return 1;
     TcArgs a = {};
     a.out = out; a.K = K; a.ldo = ldo; a.rows_a = rows; a.rows_b = N; a.act = act; a.limit = limit;
     const long long most = ((long long)rows / BM + runs) * ((N + BN - 1) / BN);       // tiles, if every run ends inside one
-    tb_launch(gemm_tc_runs_kernel<EPI>, dim3((unsigned)(most < sms ? most : sms)), THREADS, runs_smem(BN, stages_for<BN>(), runs), stream, ma, mb, a, first, runs);
+    tb_launch(gemm_tc_runs_kernel<EPI, BN>, dim3((unsigned)(most < sms ? most : sms)), THREADS, runs_smem(BN, stages_for<BN>(), runs), stream, ma, mb, a, first, runs);
     return 0;
+}
+
+// Tiles of 128 columns where the rounds of tiles they take on the SMs, at six tenths of a wide tile's time, are fewer: a few experts with a few hundred rows
+// leave SMs idle in wide ones (four of 256 rows, H = 2,048, F = 768: 38 to 49 -> 29 to 38 us for both products; H = 4,096, F = 1,536: 84 -> 81).  How many row tiles there are is known on the device
+// only: for the narrow tiles every run is taken to end inside one, for the wide ones every other.
+template <int EPI>
+static int launch_runs(const void* X, int ldx, const void* W, void* out, int ldo, const int* first, int runs, int rows, int N, int K, int act, float limit, cudaStream_t stream) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    const long long most = (long long)rows / BM + runs, fewer = rows / BM + (runs + 1) / 2;
+    const long long wide = (fewer * ((N + 255) / 256) + sms - 1) / sms, narrow = (most * ((N + 127) / 128) + sms - 1) / sms;
+    if (narrow * 3 < wide * 5) return launch_runs_of<EPI, 128>(X, ldx, W, out, ldo, first, runs, rows, N, K, act, limit, sms, stream);
+    return launch_runs_of<EPI, 256>(X, ldx, W, out, ldo, first, runs, rows, N, K, act, limit, sms, stream);
 }
 
 // The two products of every expert over rows that lie side by side, expert by expert: act = gate(X_e . Wgu_e^T) (rows of Wgu_e
