@@ -1105,14 +1105,14 @@ int launch_tc_sliced(int epi, const CUtensorMap& ma, const CUtensorMap& mb, cons
 }
 // How many clusters of ``size`` CTAs of this kernel the device holds at once (0: it places none).  Clusters are placed
 // as wholes inside one part of the chip, so this is less than the CTAs it holds divided by the size.
-template <int BN, bool NORMED>
+template <int BN, bool NORMED, int EPI = TB_EPI_ADD>
 int ordered_clusters(int size) {
     static int cached[17];
     static bool known[17] = {false};
     if (size < 1 || size > 16) return 0;
     if (!known[size]) {
-        constexpr size_t smem = smem_for<BN, true, stages_of<BN, TB_EPI_ADD, true>()>();
-        auto kernel = gemm_tc_kernel<BN, TB_EPI_ADD, true, NORMED, true>;
+        constexpr size_t smem = smem_for<BN, true, stages_of<BN, EPI, true>()>();
+        auto kernel = gemm_tc_kernel<BN, EPI, true, NORMED, true>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -1145,15 +1145,30 @@ int ordered_fit(int bn, bool normed, int tiles, int wanted) {
     return 1;
 }
 
+// The same for an epilogue that needs whole sums (0: not one of the kernels there are).
+template <int EPI>
+int whole_clusters(int bn, bool normed, int size) {
+    if constexpr (EPI == TB_EPI_SWIGLU)
+        if (normed) return bn == 16 ? ordered_clusters<16, true, EPI>(size) : (bn == 32 ? ordered_clusters<32, true, EPI>(size) : 0);
+    if (normed) return 0;
+    return bn == 16 ? ordered_clusters<16, false, EPI>(size) : (bn == 32 ? ordered_clusters<32, false, EPI>(size) : (bn == 64 ? ordered_clusters<64, false, EPI>(size) : 0));
+}
+
 // K slices of an epilogue that needs whole sums (all but ADD), the tiles of at most 64 rows: 1 or a cluster's size.  As many as give every
 // SM a CTA, at least four k-blocks each, at most four (measured at most 1 / 2 / 3 / 4 / 6 / 8: a decode step of twelve layers of
-// width 1,024 314 / 290 / 288 / 289 / 292 / 291 us, of four layers with experts of width 2,048 696 / 670 / 661 / 653 / 652 / 652).
-// The clusters take at most half of the places (two CTAs an SM), so all of them are held at once wherever they can be put.
-int whole_slices(int bn, int tiles, int kb, int sm_count) {
+// width 1,024 314 / 290 / 288 / 289 / 292 / 291 us, of four layers with experts of width 2,048 696 / 670 / 661 / 653 / 652 / 652), and no more than the
+// device places as a cluster.  The clusters take at most half of the places (two CTAs an SM), so all of them are held at once wherever they can be put.
+int whole_slices(int bn, bool normed, int epi, int tiles, int kb, int sm_count) {
     int s = sm_count / tiles;
     if (s > kb / 4) s = kb / 4;
     if (s > 4) s = 4;
-    return s < 2 || bn > 64 ? 1 : s;
+    if (bn > 64) return 1;
+    for (; s > 1; --s) {
+        const int placed = epi == TB_EPI_STORE ? whole_clusters<TB_EPI_STORE>(bn, normed, s)
+                                               : (epi == TB_EPI_F32 ? whole_clusters<TB_EPI_F32>(bn, normed, s) : whole_clusters<TB_EPI_SWIGLU>(bn, normed, s));
+        if (placed > 0) return s;
+    }
+    return 1;
 }
 
 template <int BN, int EPI>
@@ -1309,7 +1324,7 @@ static int normed_slices(int N, int K, int epi, int M = 1, bool ordered = false)
         s = s > 16 ? 16 : s;
         if (ordered) s = ordered_fit(M <= 16 ? 16 : 32, true, tiles, s);
     } else {
-        s = whole_slices(M <= 16 ? 16 : 32, tiles, kb, sm_count);
+        s = whole_slices(M <= 16 ? 16 : 32, true, epi, tiles, kb, sm_count);
     }
     const int per = (kb + s - 1) / s;
     return (kb + per - 1) / per;
@@ -1446,7 +1461,7 @@ extern "C" int tb_gemm_tc_gated(const void* X, const void* W, void* out, int M, 
             s = s < 1 ? 1 : (s > max_s ? max_s : s);
             if (ordered) s = ordered_fit(bn, false, tiles, s);
         } else {
-            s = whole_slices(bn, tiles, kb, sm_count);
+            s = whole_slices(bn, false, epi, tiles, kb, sm_count);
         }
         a.k_blocks_per_split = (kb + s - 1) / s;
         s = (kb + a.k_blocks_per_split - 1) / a.k_blocks_per_split;  // no empty slice
