@@ -827,7 +827,7 @@ gemm_tc_runs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
     pdl_wait();
-    for (int e = threadIdx.x; e <= runs; e += THREADS) first[e] = __ldcg(first_g + e);        // (through L2: see load_l2 of gemm_simt.cu)
+    for (int e = threadIdx.x; e <= runs; e += THREADS) first[e] = __ldcg(first_g + e);        // (not as a load of constants, which could move above the wait)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
