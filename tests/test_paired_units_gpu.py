@@ -1,0 +1,123 @@
+"""The prompt attention on units of 128 query rows (tcgen05), at the sizes where it can go wrong: edges of pages, tiles and blocks, odd
+groups of heads, windows that begin inside a tile, keys in two parts."""
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import Paged, layout_for, stream
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from titan_b200 import kernels
+    kernels.lib()
+    return kernels
+
+
+def attention(q, k, v, start, window, keep, scale, sink):
+    """One sequence in float64: q [n, nh, d] at positions start .., k and v [start + n, nkv, d]; also sum_j p_j |v_j|."""
+    n, nh, _ = q.shape
+    group = nh // k.shape[1]
+    kk, vv = k.double().repeat_interleave(group, 1), v.double().repeat_interleave(group, 1)
+    s = torch.einsum("ihd,jhd->hij", q.double(), kk) * scale
+    i, j = torch.arange(start, start + n, device=q.device)[:, None], torch.arange(k.shape[0], device=q.device)[None, :]
+    seen = (j <= i) & ((j > i - window) | (j < keep)) if window else j <= i
+    s = s.masked_fill(~seen, -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink.double()[:, None, None].expand(nh, n, 1)], 2)
+    p = torch.softmax(s, -1)[..., :k.shape[0]]
+    return torch.einsum("hij,jhd->ihd", p, vv), torch.einsum("hij,jhd->ihd", p, vv.abs())
+
+
+CASES = [  # nh, nkv, start positions, new tokens, window, kept first, sink, exact weights
+    (4, 2, [0, 0, 0, 0], [1, 63, 64, 65], 0, 0, False, 0),
+    (4, 2, [0, 0, 0], [127, 128, 129], 0, 0, True, 0),
+    (8, 2, [0, 0, 0], [191, 193, 1000], 0, 0, False, 1),
+    (3, 1, [0, 0, 0, 0], [1, 128, 129, 257], 0, 0, False, 0),
+    (3, 3, [0, 0], [256, 640], 0, 0, True, 1),
+    (4, 2, [0, 0], [700, 130], 100, 0, False, 0),
+    (3, 1, [0, 0], [700, 130], 130, 70, False, 0),
+    (4, 1, [64, 0, 700, 129], [1, 300, 64, 257], 0, 0, False, 0),
+    (3, 1, [64, 0, 700, 129], [1, 300, 64, 257], 0, 0, False, 0),
+    (2, 1, [640, 333], [200, 129], 65, 3, True, 0),
+]
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("nh,nkv,starts,news,window,keep,sinks,exact", CASES)
+def test_prompt_attention_at_the_edges_of_its_tiles(K, nh, nkv, starts, news, window, keep, sinks, exact, many):
+    if many:            # enough heads for two units of query rows a block
+        times = torch.cuda.get_device_properties(0).multi_processor_count // (nh * -(-sum(news) // 128)) + 1
+        nh, nkv = nh * times, nkv * times
+    hd, g = 128, torch.Generator().manual_seed(nh * 100 + sum(news))
+    slots = [3, 0, 5, 1][:len(news)]
+    lay, T, Q, KV = layout_for(slots, starts, news), sum(news), nh * hd, nkv * hd
+    scale = 1 / math.sqrt(hd)
+    rows = torch.randn(T, Q + 2 * KV, generator=g).to(torch.bfloat16).cuda()
+    sink = torch.randn(nh, generator=g).cuda() if sinks else None
+    fresh = not any(starts)
+    cache = None if fresh else Paged(K, slots, [s + n for s, n in zip(starts, news)], nkv, hd, torch.bfloat16)
+    want, weight, at = [], [], 0
+    for slot, start, n in zip(slots, starts, news):
+        mine = rows[at:at + n]
+        k, v = mine[:, Q:Q + KV].reshape(n, nkv, hd), mine[:, Q + KV:].reshape(n, nkv, hd)
+        if not fresh:
+            past = torch.randn(2, start, nkv, hd, generator=g).to(torch.bfloat16).cuda()
+            k, v = torch.cat([past[0], k]), torch.cat([past[1], v])
+            for p in range(start + n):
+                cache.put(slot, p, k[p], v[p])
+        w, a = attention(mine[:, :Q].reshape(n, nh, hd), k, v, start, window, keep, scale, sink)
+        want.append(w.reshape(n, Q)); weight.append(a.reshape(n, Q))
+        at += n
+    want, weight = torch.cat(want), torch.cat(weight)
+    out = torch.full((T, Q), float("nan"), dtype=torch.float32 if exact else torch.bfloat16, device="cuda")
+    a = K.AttnArgs()
+    a.q, a.q_stride, a.out, a.out_stride, a.out_f32, a.exact_weights = rows.data_ptr(), Q + 2 * KV, out.data_ptr(), Q, exact, exact
+    a.kv_new, a.kv_stride = rows.data_ptr() + Q * 2, Q + 2 * KV
+    if cache is not None:
+        a.cache = cache.view
+    a.batch = lay.c_struct()
+    a.nh, a.nkv, a.hd, a.window, a.keep_first, a.scale = nh, nkv, hd, window, keep, scale
+    a.sink = None if sink is None else sink.data_ptr()
+    source = K.KV_FROM_STEP if fresh else K.KV_FROM_CACHE
+    assert K.attn_prefill_tc_accepts(a, torch.bfloat16, source)
+    K.attn_prefill_tc(a, source, stream())
+    assert K.wait_errors() == {}
+    # A weight enters the product rounded to eight bits (by 2^-8 of itself at most; with exact weights 2^-16), the result is rounded once
+    # more where it leaves in bfloat16, and the scores' float32 sums (|s| below 8 here) move a weight by less than 2^-18.
+    unit = 2.0 ** -8
+    bound = weight * ((2.0 ** -16 if exact else unit) + 2.0 ** -18) + want.abs() * (2.0 ** -20 if exact else unit * 1.01) + 1e-30
+    assert bool(((out.double() - want).abs() <= bound).all()), float(((out.double() - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("nh", [2, 40])
+@pytest.mark.parametrize("news,window,sinks,exact,wide", [([1, 64, 127], 0, False, 0, True), ([130, 700], 100, True, 0, False), ([333, 65], 0, False, 1, True), ([640], 257, True, 1, False)])
+def test_prompt_attention_with_keys_in_two_parts(K, nh, news, window, sinks, exact, wide):
+    dn, dt, g = 128, 64, torch.Generator().manual_seed(nh + sum(news))
+    T, lay = sum(news), layout_for(list(range(len(news))), [0] * len(news), news)
+    scale = 1 / math.sqrt(dn + dt)
+    q = torch.randn(T, nh * (dn + dt), generator=g).to(torch.bfloat16).cuda()
+    kv = torch.randn(T, 2 * nh * dn + 8, generator=g).to(torch.bfloat16).cuda()
+    tail = torch.randn(T, 512 + dt, generator=g).to(torch.bfloat16).cuda()
+    sink = torch.randn(nh, generator=g).cuda() if sinks else None
+    room = torch.full((T, nh * dn + (8 if wide else 2)), float("nan"), dtype=torch.bfloat16, device="cuda")
+    out = room[:, :nh * dn] if wide else room[:, 2:]
+    a = K.SplitAttnArgs()
+    a.q, a.q_stride, a.kv, a.kv_stride, a.k_col0, a.v_col0 = q.data_ptr(), q.stride(0), kv.data_ptr(), kv.stride(0), 0, nh * dn + 8
+    a.tail, a.tail_stride, a.tail_col0, a.out, a.out_stride = tail.data_ptr(), tail.stride(0), 512, out.data_ptr(), room.stride(0)
+    a.batch, a.nh, a.dn, a.dt, a.dv, a.window, a.scale = lay.c_struct(), nh, dn, dt, dn, window, scale
+    a.sink, a.exact_weights = None if sink is None else sink.data_ptr(), exact
+    assert K.attn_prefill_split_accepts(a)
+    K.attn_prefill_split(a, stream())
+    assert K.wait_errors() == {}
+    at = 0
+    for n in news:
+        mine = slice(at, at + n)
+        k = torch.cat([kv[mine, :nh * dn].reshape(n, nh, dn), tail[mine, None, 512:].expand(n, nh, dt)], -1)
+        want, weight = attention(q[mine].reshape(n, nh, dn + dt), k, kv[mine, nh * dn + 8:].reshape(n, nh, dn), 0, window, 0, scale, sink)
+        bound = weight * ((2.0 ** -16 if exact else 2.0 ** -8) + 2.0 ** -18) + want.abs() * 2.0 ** -8 * 1.01 + 1e-30      # (as above)
+        assert bool(((out[mine].double().reshape(n, nh, dn) - want).abs() <= bound).all())
+        at += n

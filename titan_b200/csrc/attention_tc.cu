@@ -1,37 +1,40 @@
-// Causal attention of prompts and of continuation chunks on the tcgen05 tensor cores (head size 128).
+// Causal attention of prompts and of continuation chunks on the tcgen05 tensor cores (head size 128; keys of 128 + 64 for prompts of
+// latent attention).
 //
-// One CTA per (sequence, query head, block of 128 queries).  Per tile of 64 keys:
+// One CTA per (sequence, block of 128 queries, PAIR of query heads that share a key-value head); where a key-value head has an
+// odd number of query heads, per (sequence, 256 queries, head): two units of 128 query rows either way, over the same keys.  Steps too
+// small to fill the SMs so take one unit a CTA.
+// Per tile of 128 keys and unit:
 //     S = Q . K^T        tcgen05.mma, A = Q and B = K both K-major in shared memory, S in tensor memory
 //     P = 2^(S*c - m)    a softmax thread reads its query row of S with tcgen05.ld and writes P (pairs of
 //                        bfloat16) back over the first half of the same columns with tcgen05.st
 //     O += P . V         tcgen05.mma with A = P from tensor memory, B = V as MN-major operand from shared
 //                        memory (V's rows are keys, its contiguous dimension is the output dimension),
 //                        O accumulated in tensor memory
-// The eight softmax warps form two groups of four (a thread = a query row); group g takes the key tiles
-// j with j % 2 == g as an online softmax of its own: its own running maximum and sum, and its own O in
-// tensor memory.  A row's maximum is raised only when a tile exceeds it by more than
-// 2^RESCALE_LOG2 (P stays below that bound, which bfloat16 and the float32 sum hold easily); only then is
-// the group's O rescaled in tensor memory, which after the first tiles is rare.  At the end the groups'
-// (m, l, O) are merged like the parts of a split-key decode.  So a thread reads each score once,
-// nothing passes through registers per tile but the scores, and a group has a whole tile's time of
-// slack before its next scores are needed.
-// Warp 0 loads Q once and K and V tiles through TMA (rings of four each: K_j is free as soon as S_j is
-// done and is wanted four tiles ahead, V_j only after P.V).  Warp 1 allocates tensor memory and issues
-// the S MMAs of the even tiles, warp 11 those of the odd tiles, into four S buffers, up to four tiles
-// ahead (a buffer is free again when the P.V of the tile it held is complete); warp 10 issues the P.V
-// MMAs.  The issue is split three ways because the issuing thread is the narrow place: a tcgen05.mma
-// costs it tens of cycles however small the product.  One tcgen05.commit per event: "S_j done" serves the
-// softmax group and the K ring, "P.V_j done" the V ring, the S issuer and (for a rescale, and at the
-// end) the group.  Warps 2..9 are the softmax groups.  The step's own [T][Q | K | V] rows are the
-// only source (every sequence starts at position 0); the cache is not read.  The grid runs over heads
-// fastest, so the heaviest query blocks of all heads start first and the lightest make the tail.
-// Tensor memory: S (then P) 4 x 64 columns, O 2 x 128 columns (all 512).
+// Sixteen softmax warps, eight a unit: a query row is two threads, a page of the tile each.  While one unit's warps turn S into P, the tensor
+// cores run the other unit's P.V and next S: one thread issues P.V_0(j), S_0(j+1), P.V_1(j), S_1(j+1), ..., and MMAs run in the order they are
+// issued, so S(j+1) may take the columns of P(j), and "S(j+1) is done" also says that O holds P.V(j).  A row's maximum is raised only
+// when a tile exceeds it by more than 2^RESCALE_LOG2 (P stays below that bound, which bfloat16 and the float32 sum hold easily);
+// only then do the row's two threads exchange their maxima and rescale O in tensor memory, which after the first tiles is rare: in every
+// other tile one barrier of the two warps that says so is all they need of one another.
+//
+// What bounds it: the special-function units (16 exponentials a clock and SM: 1,024 clocks for a unit's tile) and the tensor cores
+// (1,024 clocks for S and P.V of it) are needed equally, and a unit's warps wait for their own S; two units keep both busy in turn, and
+// four warps a scheduler hide one another's fixed latencies (with two, eight warps of a whole row a thread, both pipes stood at 51 %).
+// Tiles of 128 keys: an S product of 64 keys reads 192 bytes of shared memory a clock (limit 128), one of 128 keys 128.
+//
+// Warp 0 loads Q once and K and V tiles through TMA (a ring each), warp 1 issues the MMAs and allocates tensor memory, warps 2..17 are
+// the softmax.  Keys and values come from the step's own [T][Q | K | V] rows (every sequence starts at position 0) or from the
+// cache's pages.  The grid runs over heads fastest, so the heaviest query blocks of all heads start first and the lightest make the tail.
+// Tensor memory: S (then P) 2 x 128 columns, O 2 x 128 columns (all 512).
 //
 // All waits are bounded (tma.cuh); tb_attn_tc_error() reads the error word.
 //
 // berniehans/titan: flash_attention_2_kernel, one warp per (head, query), one key per iteration,
 // scalar FMA (engine/engine-cuda/kernels/flash_attention_2.cu:22-106).
 #include <float.h>
+
+#include <atomic>
 
 #include "attention_args.h"
 #include "common.cuh"
@@ -45,13 +48,21 @@ using namespace tbtc;
 
 __device__ unsigned int g_attn_tc_error = 0;
 
-constexpr int HD = 128, BQ = 128, BKEY = 64;
-constexpr int THREADS = 384;                           // producer, S issuer (even tiles), eight softmax warps, P.V issuer, S issuer (odd tiles)
-constexpr uint32_t Q_BYTES = BQ * HD * 2;              // two boxes of 128 rows x 64 columns
-constexpr uint32_t Q_BOX = BQ * 128;
-constexpr uint32_t KV_TILE = BKEY * HD * 2;            // one K or V tile: two boxes of 64 rows x 64 columns
-constexpr uint32_t KV_BOX = BKEY * 128;
-constexpr int KV_STAGES = 4;                           // K and V tiles in flight: the loads run well ahead of P.V
+constexpr int HD = 128, BQ = 128, PAGE = 64, BKEY = 128;  // a key tile is two pages (boxes) of 64 rows
+constexpr int THREADS = 576;                           // producer, MMA issuer, sixteen softmax warps
+constexpr uint32_t Q_BOX = BQ * 128;                   // 128 rows x 64 columns
+constexpr uint32_t KV_BOX = PAGE * 128;                // 64 rows x 64 columns
+constexpr uint32_t KV_HALF = 2 * KV_BOX;               // 128 rows x 64 columns
+constexpr uint32_t V_TILE = 2 * KV_HALF;
+// DK: dimensions of a query and of a key, 128, or 192 of which the last 64 are one row for all heads (the tail); values have 128.
+// Shared memory holds two units' queries and as many K and V tiles beside them as fit.
+template <int DK> constexpr uint32_t q_unit() { return DK / 64 * Q_BOX; }
+template <int DK> constexpr uint32_t k_tile() { return DK / 64 * KV_HALF; }
+template <int DK> constexpr int k_stages() { return DK == 128 ? 3 : 2; }
+template <int DK> constexpr int v_stages() { return DK == 128 ? 2 : 1; }
+template <int DK> constexpr size_t tc_smem() {
+    return 1024 + 2 * q_unit<DK>() + k_stages<DK>() * k_tile<DK>() + v_stages<DK>() * V_TILE + 128 + 2 * BQ * sizeof(float);
+}
 
 struct TcAttnArgs {
     void* out; int out_stride; int out_f32;      // bfloat16 rows, or float32 ones
@@ -61,8 +72,12 @@ struct TcAttnArgs {
     int k_col0; int v_col0;
     // keys and values from the cache (continuation steps): the first position of each sequence's rows, its slot,
     // the block table, and the row of the first V page in the cache's tensor map; paged = 0: from the step's rows
+    int units;               // of 128 query rows a CTA: 1 or 2
+    int pair_heads;          // 1: a CTA's two units are query heads 2x and 2x + 1, 0: blocks of 128 queries of one head
     int paged; const int* start_pos; const int* slot_of_seq; const int* table; int table_width; int v_row0;
     const float* sink;       // [nh] or null: one more term exp(sink) of every head's softmax denominator, without key or value
+    int tail_col0;           // DK = 192: first column of the shared key part in the tail's rows
+    int out_wide;            // output rows take 16-byte stores
 };
 
 __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity, unsigned code) {
@@ -75,13 +90,14 @@ __device__ __forceinline__ uint64_t desc_k_major(uint32_t addr) {
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 // MN-major operand tile: 64 contiguous elements of the MN dimension per 128-byte row, rows are K;
-// leading byte offset = distance between 64-element MN blocks (one box), stride byte offset = 8 rows.
+// leading byte offset = distance between 64-element MN blocks, stride byte offset = 8 rows.
 __device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(KV_BOX >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(KV_HALF >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// kind::f16, D float32, A and B bfloat16, M = 128; S: N = 64 keys; P.V: N = 128 dims, bit 16: B is MN-major.
+// kind::f16, D float32, A and B bfloat16, M = 128; S: N = 128 keys, 64 in a last tile of one page; P.V: N = 128 dims, bit 16: B is MN-major.
 constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKEY >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+constexpr uint32_t IDESC_S_PAGE = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PAGE >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 constexpr uint32_t IDESC_PV = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
@@ -99,78 +115,85 @@ __device__ __forceinline__ float ex2(float x) {          // 2^x, one instruction
     return y;
 }
 
+// Whether ``mine`` is true in any thread of the two warps that meet at the barrier.
+__device__ __forceinline__ bool any_of_two_warps(int barrier, bool mine) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, %2, 64, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any) : "r"((uint32_t)mine), "r"(barrier) : "memory");
+    return any != 0;
+}
+
 constexpr float RESCALE_LOG2 = 8.0f;
 
-// Barriers and why no waiter can fall behind.  A parity wait only tells "the phase with this parity is
-// over" from the barrier's CURRENT phase, so a waiter must see phase k before phase k + 1 ends; every
-// barrier below keeps that by construction (tile j uses slot j % 4; a slot's phases are tiles j, j + 4, ..).
-//   k_full[s], v_full[s]   TMA bytes of K_j, V_j.  Waited by the S issuer of tile j / the P.V issuer.  The
-//                          next load into the slot needs s_done / pv_done of tile j, i.e. the MMAs that
-//                          the waiter issued after its wait.
-//   s_done[s]              tcgen05.commit after S_j.  Waited by the softmax group of tile j (every phase)
-//                          and polled by the producer for K_{j+4}; S_{j+4} needs that K tile and pv_done(j),
-//                          which needs the group's P_j.
-//   p_full[g]              four arrivals (the group's warps) per tile of group g.  Waited by the P.V issuer,
-//                          every phase.  The group arrives for tile j only after pv_done(j - 2): without
-//                          that, a group that never rescales could arrive for j and j + 2 before the
-//                          issuer had looked once (an intermittent deadlock on long prompts).
-//   pv_done[s]             tcgen05.commit after P.V_j.  Polled by the producer for V_{j+4}, waited by the S
-//                          issuer of tile j + 4 (both every phase) and by the group of tile j + 2 before it
-//                          arrives (and before a rescale, and once after its last tile); P.V_{j+4} needs
-//                          all three to have moved on.
+// Barriers and why no waiter can fall behind.  A parity wait only tells "the phase with this parity is over" from the barrier's
+// CURRENT phase, so a waiter must see phase k before phase k + 1 ends.
+//   k_full, k_empty,    the rings' stages: TMA bytes of a tile, and the commit behind the last MMA that reads it.  Loads go out in the order
+//   v_full, v_empty     K_0 V_0 K_1 V_1 ...; a load waits for a commit that needs no tile behind it in that order.
+//   s_done[u]           commit behind S_u(j) (phase j), and once more behind the last P.V_u.  The unit's warps wait for every phase; the
+//                       issuer commits phase j + 1 only after p_full of tile j, which the warps arrive at after seeing phase j.
+//   p_full[u]           eight arrivals (the unit's warps) a tile.  The issuer waits for every phase; the warps arrive for tile
+//                       j + 1 only after s_done(j + 1), which the issuer commits after it has seen p_full of tile j.
 
 // EXACT: the softmax weights enter P . V as two bfloat16 halves (AttnArgs.exact_weights): the rounded weights over the first
 // half of the tile's S columns, what rounding left over over the second half, and each value tile is multiplied by both.
-template <bool EXACT>
+template <bool EXACT, int DK>
 __global__ void __launch_bounds__(THREADS, 1)
-attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, TcAttnArgs a) {
+attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap tail_map, TcAttnArgs a) {
+    constexpr int KB = DK / 64, KS = k_stages<DK>(), VS = v_stages<DK>();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* q_smem = base;                                       // 32 KB
-    uint8_t* kv_smem = base + Q_BYTES;                            // KV_STAGES x (K 16 KB + V 16 KB)
-    uint64_t* bars = (uint64_t*)(kv_smem + KV_STAGES * 2 * KV_TILE);
+    uint8_t* q_smem = base;                                       // [unit][64 dims] boxes of 16 KB
+    uint8_t* k_smem = base + 2 * q_unit<DK>();
+    uint8_t* v_smem = k_smem + KS * k_tile<DK>();
+    uint64_t* bars = (uint64_t*)(v_smem + VS * V_TILE);
     uint64_t* q_full = bars;
-    uint64_t* k_full = bars + 1;             // [4] K and V have rings of their own: K_j is free as soon as S_j is
-    uint64_t* v_full = bars + 5;             // [4] done, long before V_j, and is wanted four tiles ahead
-    uint64_t* s_done = bars + 9;             // [4] S of tile j is in tensor-memory buffer j % 4 (and K stage j % 4 is free)
-    uint64_t* pv_done = bars + 13;           // [4] P.V of tile j is complete: V stage j % 4 and S buffer j % 4 are free, O holds it
-    uint64_t* p_full = bars + 17;            // [2] the group's four warps have written P
-    uint32_t* tmem_slot = (uint32_t*)(bars + 19);
-    float* ml_sh = (float*)(bars + 20);      // [2 groups][m, l][128 rows]
+    uint64_t* k_full = bars + 1;             // [KS]
+    uint64_t* k_empty = k_full + KS;         // [KS]
+    uint64_t* v_full = k_empty + KS;         // [VS]
+    uint64_t* v_empty = v_full + VS;         // [VS]
+    uint64_t* s_done = bars + 11;            // [2]
+    uint64_t* p_full = bars + 13;            // [2]
+    uint32_t* tmem_slot = (uint32_t*)(bars + 15);
+    float* row_sh = (float*)(bars + 16);     // [2 units][128 rows]: what the two threads of a row tell one another
 
     pdl_launch_dependents();
     pdl_wait();
-    // blockIdx.y: which sequence and which block of 128 queries (a sequence's blocks from the heaviest,
-    // the last, down); blockIdx.x, which runs fastest in the dispatch order: the head
+    // blockIdx.y: which sequence and which block of queries (a sequence's blocks from the heaviest,
+    // the last, down); blockIdx.x, which runs fastest in the dispatch order: the head or pair of heads
+    const int units = a.units, rows_cta = a.pair_heads ? BQ : units * BQ;
     int rem = blockIdx.y, seq = -1, blk = 0, tok0 = 0, n = 0;
     for (int s = 0; s < a.B; ++s) {
-        const int t0 = a.q_start[s], ns = a.q_start[s + 1] - t0, nb = (ns + BQ - 1) / BQ;
+        const int t0 = a.q_start[s], ns = a.q_start[s + 1] - t0, nb = (ns + rows_cta - 1) / rows_cta;
         if (rem < nb) { seq = s; blk = nb - 1 - rem; tok0 = t0; n = ns; break; }
         rem -= nb;
     }
     if (seq < 0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.x, kh = h / (a.nh / a.nkv);
-    const int r0 = blk * BQ;                                      // first row of the block among the sequence's rows of this step
+    const int h0 = a.pair_heads ? 2 * blockIdx.x : blockIdx.x, kh = h0 / (a.nh / a.nkv);
+    const int r0 = blk * rows_cta;                                // first row of the CTA among the sequence's rows of this step
     const int p0 = a.paged ? a.start_pos[seq] : 0;                // position of the sequence's first row
-    const int last_key = p0 + min(n - 1, r0 + BQ - 1);
+    const int last_key = p0 + min(n - 1, r0 + rows_cta - 1);
     const int first_key = a.window > 0 ? max(0, p0 + r0 - a.window + 1) : 0;
-    // Key tiles of this block: the window's, from tile kt0 to the last query's; and, where the window has left a
-    // sequence's kept first keys behind by at least a tile, the n_keep tiles that hold those, ahead of the window's.
-    int kt0 = first_key / BKEY, n_keep = 0;
+    // Pages of 64 keys of this CTA: the window's, from page kt0 to the last query's; and, where the window has left a
+    // sequence's kept first keys behind by at least a page, the n_keep pages that hold those, ahead of the window's.
+    int kt0 = first_key / PAGE, n_keep = 0;
     if (a.keep_first > 0 && a.window > 0) {
-        const int kept_tiles = (a.keep_first + BKEY - 1) / BKEY;
-        if (kt0 > kept_tiles) n_keep = kept_tiles; else kt0 = 0;
+        const int kept_pages = (a.keep_first + PAGE - 1) / PAGE;
+        if (kt0 > kept_pages) n_keep = kept_pages; else kt0 = 0;
     }
-    const int n_tiles = n_keep + last_key / BKEY - kt0 + 1;
-    const int kskip = kt0 - n_keep;                               // tile j holds keys of tile j (j < n_keep) or j + kskip
+    const int n_pages = n_keep + last_key / PAGE - kt0 + 1;
+    const int n_tiles = (n_pages + 1) >> 1;                       // tile j: pages 2 j and, if there is one, 2 j + 1 of that list
+    const int kskip = kt0 - n_keep;                               // place i of the list is page i (i < n_keep) or i + kskip
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        for (int s = 0; s < KV_STAGES; ++s) {
-            mbar_init(k_full + s, 1); mbar_init(v_full + s, 1); mbar_init(s_done + s, 1); mbar_init(pv_done + s, 1);
-        }
-        for (int s = 0; s < 2; ++s) mbar_init(p_full + s, 4);
+        for (int s = 0; s < KS; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, 1); }
+        for (int s = 0; s < VS; ++s) { mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(s_done + s, 1); mbar_init(p_full + s, 8); }
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -178,101 +201,102 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_s = tmem;             // S of tile j: columns 64 (j % 4) ..; a group owns two of the four buffers
-    const uint32_t tmem_o = tmem + 256;       // O of group g: columns 256 + 128 g ..
+    const uint32_t tmem_s = tmem;             // S of unit u: columns 128 u ..
+    const uint32_t tmem_o = tmem + 256;       // O of unit u: columns 256 + 128 u ..
 
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_expect_tx(q_full, Q_BYTES);
-            tma_load_2d(q_smem, &q_map, q_full, h * HD, tok0 + r0);
-            tma_load_2d(q_smem + Q_BOX, &q_map, q_full, h * HD + 64, tok0 + r0);
-            // K and V tiles as their rings allow, whichever is free first (bounded polling)
+    if (warp < 2) {
+        if (warp == 0 && lane == 0) {
+            mbar_expect_tx(q_full, units * q_unit<DK>());
+            for (int u = 0; u < units; ++u)
+                for (int c = 0; c < KB; ++c)
+                    tma_load_2d(q_smem + (KB * u + c) * Q_BOX, &q_map, q_full, (h0 + (a.pair_heads ? u : 0)) * DK + c * 64,
+                                tok0 + r0 + (a.pair_heads ? 0 : u * BQ));
             const int* tab = a.paged ? a.table + (size_t)a.slot_of_seq[seq] * a.table_width : nullptr;
-            const int kx = a.paged ? 0 : a.k_col0 + kh * HD, vx = a.paged ? 0 : a.v_col0 + kh * HD;
-            int ki = 0, vi = 0;
-            for (uint32_t spin = 0; (ki < n_tiles || vi < n_tiles) && spin < (tbtma::WAIT_LIMIT << 4); ++spin) {
-                if (ki < n_tiles && (ki < KV_STAGES || tbtma::mbar_test(s_done + ki % KV_STAGES, (ki / KV_STAGES - 1) & 1))) {
-                    const int s = ki % KV_STAGES, kt = ki < n_keep ? ki : ki + kskip;
-                    const int row = a.paged ? (tab[kt] * a.nkv + kh) * BKEY : tok0 + kt * BKEY;
-                    uint8_t* kd = kv_smem + s * 2 * KV_TILE;
-                    mbar_expect_tx(k_full + s, KV_TILE);
-                    tma_load_2d(kd, &kv_map, k_full + s, kx, row);
-                    tma_load_2d(kd + KV_BOX, &kv_map, k_full + s, kx + 64, row);
-                    ++ki; spin = 0;
-                }
-                if (vi < n_tiles && (vi < KV_STAGES || tbtma::mbar_test(pv_done + vi % KV_STAGES, (vi / KV_STAGES - 1) & 1))) {
-                    const int s = vi % KV_STAGES, kt = vi < n_keep ? vi : vi + kskip;
-                    const int row = a.paged ? a.v_row0 + (tab[kt] * a.nkv + kh) * BKEY : tok0 + kt * BKEY;
-                    uint8_t* vd = kv_smem + s * 2 * KV_TILE + KV_TILE;
-                    mbar_expect_tx(v_full + s, KV_TILE);
-                    tma_load_2d(vd, &kv_map, v_full + s, vx, row);
-                    tma_load_2d(vd + KV_BOX, &kv_map, v_full + s, vx + 64, row);
-                    ++vi; spin = 0;
+            for (int i = 0; i < 2 * n_tiles; ++i) {               // K_0 V_0 K_1 V_1 ...
+                const int j = i >> 1, is_v = i & 1, stages = is_v ? VS : KS, s = j % stages, pages = min(2, n_pages - 2 * j);
+                uint64_t* full = (is_v ? v_full : k_full) + s;
+                if (j >= stages) wait((is_v ? v_empty : k_empty) + s, (j / stages - 1) & 1, 1);
+                uint8_t* dst = is_v ? v_smem + s * V_TILE : k_smem + s * k_tile<DK>();
+                mbar_expect_tx(full, pages * (is_v ? 2 : KB) * KV_BOX);
+                const int x = a.paged ? 0 : (is_v ? a.v_col0 : a.k_col0) + kh * HD;
+                for (int p = 0; p < pages; ++p) {
+                    const int at = 2 * j + p, page = at < n_keep ? at : at + kskip;
+                    const int row = a.paged ? (is_v ? a.v_row0 : 0) + (tab[page] * a.nkv + kh) * PAGE : tok0 + page * PAGE;
+                    tma_load_2d(dst + p * KV_BOX, &kv_map, full, x, row);
+                    tma_load_2d(dst + KV_HALF + p * KV_BOX, &kv_map, full, x + 64, row);
+                    if (DK > HD && !is_v) tma_load_2d(dst + 2 * KV_HALF + p * KV_BOX, &tail_map, full, a.tail_col0, row);
                 }
             }
-            if (ki < n_tiles || vi < n_tiles) atomicCAS(&g_attn_tc_error, 0u, 1u);
-        }
-    } else if (warp == 1 || warp == 11) {
-        // ---- S issuers (warp 1: even tiles, warp 11: odd tiles): S_i = Q . K_i^T into S buffer i % 4, up to
-        // four tiles ahead of the softmax; a tile's descriptors differ from a base by constants.
-        if (lane == 0) {
+        } else if (warp == 1 && lane == 0) {
+            // ---- every MMA; a tile's descriptors differ from a base by constants
             const uint64_t q_desc = desc_k_major(smem_u32(q_smem));
-            wait(q_full, 0, 3);
-            for (int i = warp == 1 ? 0 : 1; i < n_tiles; i += 2) {
-                const int s = i % KV_STAGES;
-                if (i >= 4) wait(pv_done + (i & 3), ((i >> 2) - 1) & 1, 9);       // the buffer held S, then P, of tile i - 4
-                wait(k_full + s, (i / KV_STAGES) & 1, 2);
-                tc_fence_after();
-                const uint64_t k_desc = desc_k_major(smem_u32(kv_smem + s * 2 * KV_TILE));
-                const uint32_t d = tmem_s + (i & 3) * BKEY;
+            auto issue_s = [&](int u, int j) {                    // S_u = Q_u . K_j^T
+                const uint64_t k_desc = desc_k_major(smem_u32(k_smem + j % KS * k_tile<DK>()));
+                const uint32_t d = tmem_s + u * BKEY, idesc = 2 * j + 1 < n_pages ? IDESC_S : IDESC_S_PAGE;
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)        // 16 dims per step: box ks / 4, 32 bytes per step inside it
-                    tc_mma(d, q_desc + (uint64_t)(((ks >> 2) * Q_BOX + (ks & 3) * 32) >> 4),
-                           k_desc + (uint64_t)(((ks >> 2) * KV_BOX + (ks & 3) * 32) >> 4), IDESC_S, ks > 0 ? 1u : 0u);
-                tc_commit(s_done + (i & 3));                // one arrival for the softmax group and for the K ring
-            }
-        }
-    } else if (warp == 10) {
-        // ---- P.V issuer: O_g += P_j . V_j for the group g = j % 2
-        if (lane == 0) {
-            for (int j = 0; j < n_tiles; ++j) {
-                const int g = j & 1, s = j % KV_STAGES;
-                wait(v_full + s, (j / KV_STAGES) & 1, 5);
-                wait(p_full + g, (j >> 1) & 1, 4);          // the group has rescaled O if it had to and written P_j
-                tc_fence_after();
-                const uint64_t v_desc = desc_mn_major(smem_u32(kv_smem + s * 2 * KV_TILE + KV_TILE));
-                const uint32_t p_tmem = tmem_s + (j & 3) * BKEY;      // P_j lies over the first half of S_j
-                const uint32_t d = tmem_o + g * HD;
+                for (int ks = 0; ks < DK / 16; ++ks)              // 16 dims per step: box ks / 4, 32 bytes per step inside it
+                    tc_mma(d, q_desc + (uint64_t)((u * q_unit<DK>() + (ks >> 2) * Q_BOX + (ks & 3) * 32) >> 4),
+                           k_desc + (uint64_t)(((ks >> 2) * KV_HALF + (ks & 3) * 32) >> 4), idesc, ks > 0 ? 1u : 0u);
+                tc_commit(s_done + u);
+            };
+            auto issue_pv = [&](int u, int j, int half) {         // O_u += P_u . V_j, the keys of one page
+                const uint64_t v_desc = desc_mn_major(smem_u32(v_smem + j % VS * V_TILE));
+                const uint32_t p = tmem_s + u * BKEY, d = tmem_o + u * HD;
 #pragma unroll
-                for (int ks = 0; ks < BKEY / 16; ++ks)      // 16 keys per step: 8 columns of P, 16 rows of V
-                    tc_mma_a_tmem(d, p_tmem + ks * 8, v_desc + (uint64_t)((ks * 2048) >> 4), IDESC_PV, (j >= 2 || ks > 0) ? 1u : 0u);
+                for (int ks = 4 * half; ks < 4 * half + 4; ++ks)  // 16 keys per step: 8 columns of P, 16 rows of V
+                    tc_mma_a_tmem(d, p + ks * 8, v_desc + (uint64_t)((ks * 2048) >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
                 if (EXACT) {
 #pragma unroll
-                    for (int ks = 0; ks < BKEY / 16; ++ks)
-                        tc_mma_a_tmem(d, p_tmem + BKEY / 2 + ks * 8, v_desc + (uint64_t)((ks * 2048) >> 4), IDESC_PV, 1u);
+                    for (int ks = 4 * half; ks < 4 * half + 4; ++ks)
+                        tc_mma_a_tmem(d, p + BKEY / 2 + ks * 8, v_desc + (uint64_t)((ks * 2048) >> 4), IDESC_PV, 1u);
                 }
-                tc_commit(pv_done + (j & 3));               // one arrival for the V ring, the S issuer and the group
+            };
+            wait(q_full, 0, 3);
+            wait(k_full, 0, 2);
+            tc_fence_after();
+            for (int u = 0; u < units; ++u) issue_s(u, 0);
+            tc_commit(k_empty);
+            for (int j = 0; j < n_tiles; ++j) {
+                const bool both = 2 * j + 1 < n_pages;
+                for (int u = 0; u < units; ++u) {
+                    if (u == 0) wait(v_full + j % VS, (j / VS) & 1, 5);
+                    wait(p_full + u, j & 1, 4);                   // the unit has rescaled O if it had to and written P
+                    tc_fence_after();
+                    issue_pv(u, j, 0);
+                    if (both) issue_pv(u, j, 1);
+                    if (u == units - 1) tc_commit(v_empty + j % VS);
+                    if (j + 1 < n_tiles) {
+                        if (u == 0) { wait(k_full + (j + 1) % KS, ((j + 1) / KS) & 1, 2); tc_fence_after(); }
+                        issue_s(u, j + 1);
+                        if (u == units - 1) tc_commit(k_empty + (j + 1) % KS);
+                    } else {
+                        tc_commit(s_done + u);                    // O is complete
+                    }
+                }
             }
         }
-    } else {
-        const int g = (warp - 2) >> 2, quarter = warp & 3;       // a warp may touch the tensor-memory lanes 32 * (warp % 4) ..
-        const int row = quarter * 32 + lane;
+    } else if ((warp - 2) >> 3 < units) {
+        const int u = (warp - 2) >> 3, p = ((warp - 2) >> 2) & 1, quarter = warp & 3;      // a warp may touch the tensor-memory lanes 32 * (warp % 4) ..
+        const int lane_row = quarter * 32 + lane, row = lane_row + (a.pair_heads ? 0 : u * BQ);       // among the unit's and the CTA's rows
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+        const uint32_t s_cols = tmem_s + u * BKEY + lane_addr, o_cols = tmem_o + u * HD + p * 64 + lane_addr;
+        float* told = row_sh + u * BQ + lane_row;
+        const int pair_barrier = 1 + u * 4 + quarter;            // the two warps that share rows
         const int qpos = p0 + r0 + row;                          // the row's position in its sequence
         const int lo = a.window > 0 ? qpos - a.window + 1 : 0;
-        float m_run = -1e30f, l_run = 0.f;                       // the maximum P is taken against (may lag), the sum
-        int mine = 0;                                            // tiles of this group so far
-        for (int j = g; j < n_tiles; j += 2, ++mine) {
-            const int key0 = (j < n_keep ? j : j + kskip) * BKEY;
-            const bool tile_visible = key0 + BKEY - 1 <= qpos && (key0 >= lo || key0 + BKEY <= a.keep_first);       // no mask needed in this tile
-            wait(s_done + (j & 3), (j >> 2) & 1, 6);
+        float m_run = -1e30f, l_run = 0.f;                       // the maximum P is taken against (may lag), this thread's part of the sum
+        for (int j = 0; j < n_tiles; ++j) {
+            const int at = 2 * j + p;                            // this thread's page of the tile, if there is one
+            const int key0 = at < n_pages ? (at < n_keep ? at : at + kskip) * PAGE : 0x40000000;      // (else behind every query)
+            const bool visible = key0 + PAGE - 1 <= qpos && (key0 >= lo || key0 + PAGE <= a.keep_first);      // no mask needed
+            wait(s_done + u, j & 1, 6);
             tc_fence_after();
             float v[64];
-            tmem_ld32_nowait(tmem_s + (j & 3) * BKEY + lane_addr, v);
-            tmem_ld32_nowait(tmem_s + (j & 3) * BKEY + lane_addr + 32, v + 32);
-            tmem_wait_ld<64>(v);
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            if (!tile_visible) {
+            tmem_ld32_nowait(s_cols + p * PAGE, v);
+            tmem_ld32_nowait(s_cols + p * PAGE + 32, v + 32);
+            tmem_wait_ld<64>(v);
+            if (!visible) {
 #pragma unroll
                 for (int i = 0; i < 64; ++i) v[i] = (key0 + i <= qpos && (key0 + i >= lo || key0 + i < a.keep_first)) ? v[i] : -INFINITY;
             }
@@ -281,93 +305,86 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 mx4[0] = max3(mx4[0], v[i], v[i + 1]); mx4[1] = max3(mx4[1], v[i + 2], v[i + 3]);
                 mx4[2] = max3(mx4[2], v[i + 4], v[i + 5]); mx4[3] = max3(mx4[3], v[i + 6], v[i + 7]);
             }
-            const float cand = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;
-            // Raise the row's maximum only when the tile exceeds it by more than the bound.
-            const bool raise = cand > m_run + RESCALE_LOG2;
-            const float m_new = raise ? cand : m_run;
-            const float f = raise ? ex2(m_run - m_new) : 1.f;
-            // Only a rescale touches O, and only then must the group's earlier P.V be complete (P itself goes
-            // into this tile's own S buffer).  f = 1 for the rows of the warp that keep their maximum.
-            if (mine >= 1 && __any_sync(0xffffffffu, raise)) {
-                wait(pv_done + ((j - 2) & 3), ((j - 2) >> 2) & 1, 7);
-                tc_fence_after();
+            float cand = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;
+            // Raise the row's maximum only when the tile exceeds it by more than the bound.  The two warps that share rows ask one another; the
+            // barrier also says that both have read their scores, over which P goes.
+            float f = 1.f;
+            if (any_of_two_warps(pair_barrier, cand > m_run + RESCALE_LOG2)) {
+                if (p == 0) *told = cand;
+                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                if (p == 1) *told = cand = fmaxf(cand, *told);
+                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                if (p == 0) cand = *told;
+                const float m_old = m_run;
+                if (cand > m_run + RESCALE_LOG2) m_run = cand;
+                f = ex2(m_old - m_run);                          // 1 for the rows that keep their maximum
+                // Only a rescale touches O, a warp half of its columns (P.V of the tile before is complete: S of this one was issued behind it).
+                if (j > 0) {
 #pragma unroll 1
-                for (int c = 0; c < HD; c += 32) {
-                    float o[32];
-                    tmem_ld32(tmem_o + g * HD + lane_addr + c, o);
+                    for (int c = 0; c < 64; c += 16) {
+                        float o[16];
+                        uint32_t bits[16];
+                        tmem_ld16(o_cols + c, o);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] *= f;
-                    tmem_st32(tmem_o + g * HD + lane_addr + c, o);
+                        for (int i = 0; i < 16; ++i) bits[i] = __float_as_uint(o[i] * f);
+                        tmem_st16_nowait(o_cols + c, bits);
+                    }
+                    tmem_wait_st();
                 }
             }
-            // two scores per instruction where the hardware has one (packed float32 FMA and add on sm_100):
-            // the softmax warps are short of issue slots, not only of special-function units
-            const float2 scale2 = make_float2(a.scale_log2, a.scale_log2), shift2 = make_float2(-m_new, -m_new);
+            // two scores per instruction where the hardware has one (packed float32 FMA and add on sm_100)
+            const float2 scale2 = make_float2(a.scale_log2, a.scale_log2), shift2 = make_float2(-m_run, -m_run);
             float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            // P as bfloat16 pairs over the first columns of the unit's S: the A operand of P.V, which never touches shared memory
 #pragma unroll
-            for (int i = 0; i < 64; i += 2) {
-                const float2 x = __ffma2_rn(make_float2(v[i], v[i + 1]), scale2, shift2);
-                v[i] = ex2(x.x); v[i + 1] = ex2(x.y);
-                sum2[(i >> 1) & 1] = __fadd2_rn(sum2[(i >> 1) & 1], make_float2(v[i], v[i + 1]));
+            for (int c = 0; c < 64; c += 32) {
+                uint32_t pk[16];
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    float* w = v + c + i;
+                    const float2 x = __ffma2_rn(make_float2(w[0], w[1]), scale2, shift2);
+                    w[0] = ex2(x.x); w[1] = ex2(x.y);
+                    sum2[(i >> 1) & 1] = __fadd2_rn(sum2[(i >> 1) & 1], make_float2(w[0], w[1]));
+                    pk[i >> 1] = pack_bf16x2(w[0], w[1]);
+                }
+                tmem_st16_nowait(s_cols + 32 * p + c / 2, pk);
+                if (EXACT) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        pk[i] = pack_bf16x2(v[c + 2 * i] - __uint_as_float(pk[i] << 16), v[c + 2 * i + 1] - __uint_as_float(pk[i] & 0xffff0000u));
+                    tmem_st16_nowait(s_cols + BKEY / 2 + 32 * p + c / 2, pk);
+                }
             }
-            l_run = l_run * f + ((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
-            m_run = m_new;
-            // P as bfloat16 pairs over the first 32 columns of this tile's S buffer (this thread's lane: its
-            // scores are all in registers by now): the A operand of P.V, which never touches shared memory
-            uint32_t pk[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-            tmem_st32_bits(tmem_s + (j & 3) * BKEY + lane_addr, pk);
-            if (EXACT) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    pk[i] = pack_bf16x2(v[2 * i] - __uint_as_float(pk[i] << 16), v[2 * i + 1] - __uint_as_float(pk[i] & 0xffff0000u));
-                tmem_st32_bits(tmem_s + (j & 3) * BKEY + lane_addr + BKEY / 2, pk);
-            }
-            // The P.V issuer must have seen this group's previous arrival before the next one, or the
-            // barrier would run two phases ahead of it and its parity wait would never end.  P.V of that
-            // tile complete implies it; by now (a whole tile later) this wait is almost always over.
-            if (mine >= 1) wait(pv_done + ((j - 2) & 3), ((j - 2) >> 2) & 1, 10);
+            tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(p_full + g);
+            if (lane == 0) mbar_arrive(p_full + u);
+            l_run = l_run * f + ((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
         }
-        if (mine >= 1) {                                         // the group's last P.V
-            const int last = g + 2 * (mine - 1);
-            wait(pv_done + (last & 3), (last >> 2) & 1, 8);
-            tc_fence_after();
-        }
-        // merge the two groups: weights 2^(m_g - M) / L
-        ml_sh[(g * 2 + 0) * 128 + row] = mine ? m_run : -1e30f;
-        ml_sh[(g * 2 + 1) * 128 + row] = mine ? l_run : 0.f;
-        tc_fence_before();
-        asm volatile("bar.sync 1, 256;" ::: "memory");           // all eight softmax warps
+        wait(s_done + u, n_tiles & 1, 8);                        // the unit's last P.V
         tc_fence_after();
-        const float m0 = ml_sh[0 * 128 + row], l0 = ml_sh[1 * 128 + row], m1 = ml_sh[2 * 128 + row], l1 = ml_sh[3 * 128 + row];
+        if (p == 0) *told = l_run;
+        asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+        if (p == 1) *told = l_run = *told + l_run;
+        asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+        const float l0 = p == 0 ? *told : l_run;
+        const int h = h0 + (a.pair_heads ? u : 0);
         const float sk = a.sink ? a.sink[h] * 1.4426950408889634f : -1e30f;      // the sink, in units of log2 like the maxima
-        const float M = fmaxf(fmaxf(m0, m1), sk);
-        const float w0 = ex2(m0 - M), w1 = n_tiles > 1 ? ex2(m1 - M) : 0.f;
-        const float inv = 1.0f / (l0 * w0 + l1 * w1 + (a.sink ? ex2(sk - M) : 0.f));
-        // this thread: output dims 64 g .. 64 g + 63 of its row, from both groups' O
-        float o0[64], o1[64];
-        tmem_ld32_nowait(tmem_o + lane_addr + g * 64, o0);
-        tmem_ld32_nowait(tmem_o + lane_addr + g * 64 + 32, o0 + 32);
-        if (n_tiles > 1) {                                       // uniform over the CTA
-            tmem_ld32_nowait(tmem_o + HD + lane_addr + g * 64, o1);
-            tmem_ld32_nowait(tmem_o + HD + lane_addr + g * 64 + 32, o1 + 32);
-        }
-        tmem_wait_ld<64>(o0);
-        if (n_tiles > 1) tmem_wait_ld<64>(o1);
+        const float M = fmaxf(m_run, sk), w0 = ex2(m_run - M);
+        const float c0 = w0 / (l0 * w0 + (a.sink ? ex2(sk - M) : 0.f));
+        const size_t at = (size_t)(tok0 + r0 + row) * a.out_stride + h * HD + p * 64;      // this thread: half of its row's output
+        float o[64];
+        tmem_ld32_nowait(o_cols, o);
+        tmem_ld32_nowait(o_cols + 32, o + 32);
+        tmem_wait_ld<64>(o);
         if (r0 + row < n) {
-            const float c0 = w0 * inv, c1 = w1 * inv;
-            const size_t at = (size_t)(tok0 + r0 + row) * a.out_stride + h * HD + g * 64;
             __nv_bfloat16* dst = (__nv_bfloat16*)a.out + at;
             float* dst32 = (float*)a.out + at;
 #pragma unroll
             for (int i = 0; i < 64; i += 8) {
                 float r[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) r[e] = n_tiles > 1 ? o0[i + e] * c0 + o1[i + e] * c1 : o0[i + e] * c0;
+                for (int e = 0; e < 8; ++e) r[e] = o[i + e] * c0;
                 if (a.out_f32) {
                     *reinterpret_cast<float4*>(dst32 + i) = make_float4(r[0], r[1], r[2], r[3]);
                     *reinterpret_cast<float4*>(dst32 + i + 4) = make_float4(r[4], r[5], r[6], r[7]);
@@ -376,7 +393,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 uint4 pk;
                 pk.x = pack_bf16x2(r[0], r[1]); pk.y = pack_bf16x2(r[2], r[3]);
                 pk.z = pack_bf16x2(r[4], r[5]); pk.w = pack_bf16x2(r[6], r[7]);
-                *reinterpret_cast<uint4*>(dst + i) = pk;
+                uint32_t* narrow = reinterpret_cast<uint32_t*>(dst + i);
+                if (DK == HD || a.out_wide) *reinterpret_cast<uint4*>(dst + i) = pk;
+                else { narrow[0] = pk.x; narrow[1] = pk.y; narrow[2] = pk.z; narrow[3] = pk.w; }
             }
         }
     }
@@ -409,10 +428,34 @@ extern "C" int tb_attn_prefill_tc_check(const AttnArgs* a, int dtype, int source
         const long long off = ((const char*)a->kv_new - (const char*)a->q) / 2;
         TB_REQUIRE(off == (long long)a->nh * a->hd, "attn_prefill_tc: K must follow Q in the buffer");
     } else {
-        TB_REQUIRE(a->cache.storage && a->cache.page_size == BKEY && a->cache.ring_rows == 0, "attn_prefill_tc: needs a cache of %d-row pages that keeps every key", BKEY);
+        TB_REQUIRE(a->cache.storage && a->cache.page_size == PAGE && a->cache.ring_rows == 0, "attn_prefill_tc: needs a cache of %d-row pages that keeps every key", PAGE);
         TB_REQUIRE(a->cache.head_dim == a->hd && a->cache.kv_heads == a->nkv, "attn_prefill_tc: the cache view does not match the heads");
     }
     TB_REQUIRE(a->out_stride % 8 == 0 && ((uintptr_t)a->out & 15) == 0, "attn_prefill_tc: the output must be 16-byte aligned");
+    return 0;
+}
+
+template <bool EXACT, int DK>
+static int launch_tc(const CUtensorMap& q_map, const CUtensorMap& kv_map, const CUtensorMap& tail_map, TcAttnArgs& p, int T, cudaStream_t stream) {
+    // once a device: the limit of shared memory, and the SMs
+    static std::atomic<int> configured[64];
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64) sms = configured[dev].load();
+    if (sms <= 0) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<EXACT, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem<DK>());
+        TB_REQUIRE(e == cudaSuccess, "attn_prefill_tc: cannot reserve %zu bytes of shared memory: %s", tc_smem<DK>(), cudaGetErrorString(e));
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+        if (dev < 64) configured[dev].store(sms);
+    }
+    // Two units a CTA where that leaves no SM idle that one unit a CTA would use: a unit alone waits for its own chain of S, P and P.V.
+    p.units = (long long)p.nh * ((T + BQ - 1) / BQ) <= sms ? 1 : 2;
+    p.pair_heads = p.units == 2 && (p.nh / p.nkv) % 2 == 0;
+    const int rows_cta = p.pair_heads ? BQ : p.units * BQ;
+    const int blocks = (T + rows_cta - 1) / rows_cta + p.B;      // upper bound on sum over sequences of ceil(n / rows_cta)
+    TB_REQUIRE(blocks <= 65535, "attn_prefill_tc: too many query blocks (%d)", blocks);
+    tb_launch(attn_prefill_tc_kernel<EXACT, DK>, dim3(p.pair_heads ? p.nh / 2 : p.nh, blocks), THREADS, tc_smem<DK>(), stream, q_map, kv_map, tail_map, p);      // heads fastest: the heaviest blocks of all heads start first
+    TB_CHECK_LAUNCH("attn_prefill_tc");
     return 0;
 }
 
@@ -425,29 +468,60 @@ extern "C" int tb_attn_prefill_tc(const AttnArgs* args, int source, cudaStream_t
     TcAttnArgs p;
     p.paged = source == TB_KV_FROM_CACHE;
     if (p.paged) {
-        const long long rows = 2LL * a.cache.num_pages * a.nkv * BKEY;
-        if (tb_make_map_bf16(&kv_map, a.cache.storage, rows, a.hd, a.hd, BKEY)) return 1;
-    } else if (tb_make_map_bf16(&kv_map, a.q, a.batch.T, a.q_stride, a.q_stride, BKEY)) return 1;
+        const long long rows = 2LL * a.cache.num_pages * a.nkv * PAGE;
+        if (tb_make_map_bf16(&kv_map, a.cache.storage, rows, a.hd, a.hd, PAGE)) return 1;
+    } else if (tb_make_map_bf16(&kv_map, a.q, a.batch.T, a.q_stride, a.q_stride, PAGE)) return 1;
     p.start_pos = a.batch.start_pos; p.slot_of_seq = a.batch.slot_of_seq; p.table = a.cache.table; p.table_width = a.cache.table_width;
-    p.v_row0 = a.cache.num_pages * a.nkv * BKEY;
+    p.v_row0 = a.cache.num_pages * a.nkv * PAGE;
     p.out = a.out; p.out_stride = a.out_stride; p.out_f32 = a.out_f32; p.q_start = a.batch.q_start; p.B = a.batch.B;
     p.nh = a.nh; p.nkv = a.nkv; p.window = a.window; p.scale_log2 = a.scale * 1.4426950408889634f; p.sink = a.sink;
     p.keep_first = a.window > 0 ? a.keep_first : 0;
     p.k_col0 = a.nh * a.hd; p.v_col0 = (a.nh + a.nkv) * a.hd;
-    constexpr size_t smem = 1024 + Q_BYTES + KV_STAGES * 2 * KV_TILE + 256 + 4 * 128 * sizeof(float);
-    static_assert(KV_STAGES == 4, "the second kernel's barrier layout and S buffers assume four stages");
-    auto kernel = a.exact_weights ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>;
-    static bool configured[2] = {false, false};
-    if (!configured[a.exact_weights != 0]) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        TB_REQUIRE(e == cudaSuccess, "attn_prefill_tc: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        configured[a.exact_weights != 0] = true;
-    }
-    const int blocks = (a.batch.T + BQ - 1) / BQ + a.batch.B;      // upper bound on sum over sequences of ceil(n / 128)
-    TB_REQUIRE(blocks <= 65535, "attn_prefill_tc: too many query blocks (%d)", blocks);
-    tb_launch(kernel, dim3(a.nh, blocks), THREADS, smem, stream, q_map, kv_map, p);      // heads fastest: the heaviest blocks of all heads start first
-    TB_CHECK_LAUNCH("attn_prefill_tc");
+    p.tail_col0 = 0; p.out_wide = 1;
+    return a.exact_weights ? launch_tc<true, HD>(q_map, kv_map, kv_map, p, a.batch.T, stream) : launch_tc<false, HD>(q_map, kv_map, kv_map, p, a.batch.T, stream);
+}
+
+// Prompts whose sequences all start at position 0, with keys in two parts:
+//   query of head h   q[t][h * (dn + dt) ..]                      [own part dn | shared part dt]
+//   key of head h     kv[t][k_col0 + h * dn ..] | tail[t][tail_col0 ..]   (the second part is one for all heads)
+//   value of head h   kv[t][v_col0 + h * dv ..],  output out[t][h * dv ..]
+// (latent attention with keys and values expanded per head).  2,000 tokens, 16 heads of 128 + 64 and 128, a window of 1,024: 95 us on mma.sync.
+struct SplitAttnArgs {
+    const void* q; int q_stride;
+    const void* kv; int kv_stride; int k_col0; int v_col0;
+    const void* tail; int tail_stride; int tail_col0;
+    void* out; int out_stride;
+    TbBatch batch;
+    int nh; int dn; int dt; int dv; int window; float scale;
+    const float* sink;       // [nh] or null: one more term exp(sink) of every head's softmax denominator
+    int exact_weights;       // softmax weights enter P . V as two bfloat16 halves (AttnArgs.exact_weights)
+};
+
+extern "C" int tb_attn_prefill_split_check(const SplitAttnArgs* a) {
+    TB_REQUIRE(a->dn == 128 && a->dt == 64 && a->dv == 128, "attn_prefill_split: built for keys of 128 + 64 and values of 128, not %d + %d and %d", a->dn, a->dt, a->dv);
+    TB_REQUIRE(a->q && a->kv && a->tail && a->out && a->nh > 0, "attn_prefill_split: missing buffers");
+    TB_REQUIRE(a->q_stride % 8 == 0 && a->kv_stride % 8 == 0 && a->tail_stride % 8 == 0 && a->k_col0 % 8 == 0 && a->v_col0 % 8 == 0 && a->tail_col0 % 8 == 0,
+               "attn_prefill_split: rows and first columns must be multiples of 8 elements (16-byte TMA coordinates)");
+    TB_REQUIRE((((uintptr_t)a->q | (uintptr_t)a->kv | (uintptr_t)a->tail) & 15) == 0, "attn_prefill_split: buffers must be 16-byte aligned");
+    TB_REQUIRE(a->out_stride % 2 == 0 && ((uintptr_t)a->out & 3) == 0, "attn_prefill_split: the output must be 4-byte aligned");
+    TB_REQUIRE(a->window >= 0, "attn_prefill_split: negative window");
     return 0;
+}
+
+extern "C" int tb_attn_prefill_split(const SplitAttnArgs* args, cudaStream_t stream) {
+    const SplitAttnArgs& a = *args;
+    if (tb_attn_prefill_split_check(args)) return 1;
+    TB_REQUIRE(a.batch.T > 0 && a.batch.B > 0, "attn_prefill_split: no tokens");
+    CUtensorMap q_map, kv_map, tail_map;
+    if (tb_make_map_bf16(&q_map, a.q, a.batch.T, a.q_stride, a.q_stride, BQ)) return 1;
+    if (tb_make_map_bf16(&kv_map, a.kv, a.batch.T, a.kv_stride, a.kv_stride, PAGE)) return 1;
+    if (tb_make_map_bf16(&tail_map, a.tail, a.batch.T, a.tail_stride, a.tail_stride, PAGE)) return 1;
+    TcAttnArgs p = {};
+    p.out = a.out; p.out_stride = a.out_stride; p.q_start = a.batch.q_start; p.B = a.batch.B;
+    p.nh = a.nh; p.nkv = a.nh; p.window = a.window; p.scale_log2 = a.scale * 1.4426950408889634f;
+    p.k_col0 = a.k_col0; p.v_col0 = a.v_col0; p.tail_col0 = a.tail_col0; p.sink = a.sink;
+    p.out_wide = a.out_stride % 8 == 0 && ((uintptr_t)a.out & 15) == 0;
+    return a.exact_weights ? launch_tc<true, 192>(q_map, kv_map, tail_map, p, a.batch.T, stream) : launch_tc<false, 192>(q_map, kv_map, tail_map, p, a.batch.T, stream);
 }
 
 

@@ -109,7 +109,7 @@ class LatentArgs(Structure):
 
 
 class SplitAttnArgs(Structure):
-    """Arguments of the tensor-core prompt attention with keys in two parts (csrc/attention_mma.cu: tb_attn_prefill_split)."""
+    """Arguments of the tensor-core prompt attention with keys in two parts (csrc/attention_tc.cu: tb_attn_prefill_split)."""
     _fields_ = [("q", c_void_p), ("q_stride", c_int), ("kv", c_void_p), ("kv_stride", c_int), ("k_col0", c_int), ("v_col0", c_int),
                 ("tail", c_void_p), ("tail_stride", c_int), ("tail_col0", c_int), ("out", c_void_p), ("out_stride", c_int),
                 ("batch", Batch), ("nh", c_int), ("dn", c_int), ("dt", c_int), ("dv", c_int), ("window", c_int), ("scale", c_float),
