@@ -1,0 +1,67 @@
+"""The experts' products of a few pairs: pairs of one expert in every number around a fragment's eight."""
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import stream
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("K_,N_out,same", [(128, 16, 1), (128, 32, 8), (384, 48, 9), (2048, 16, 17), (1024, 64, 24), (96, 32, 3), (128, 12, 5)])
+def test_experts_of_a_few_pairs(mode, K_, N_out, same):
+    """``same`` pairs choose one expert, the others each their own, one an expert without matrices.  The last two sizes are not whole
+    fragments (K = 96; 12 or 24 rows) and take the kernel of a warp an output."""
+    from titan_b200 import kernels as K
+    E, top = 6, 3
+    g = torch.Generator().manual_seed(K_ + same)
+    ids = [4] * same + [0, 5, E, 2, 5]
+    while len(ids) % top:
+        ids.append(1)
+    ids = torch.tensor(ids, dtype=torch.int32)[torch.randperm(len(ids), generator=g)]
+    P = len(ids)
+    rows = P // top if mode == 0 else P
+    x = torch.randn(rows, K_ + 8, generator=g).to(torch.bfloat16).cuda()[:, :K_]
+    w = (torch.randn(E, 2 * N_out if mode == 0 else N_out, K_, generator=g) / math.sqrt(K_)).to(torch.bfloat16).cuda()
+    out = torch.full((P, N_out), 768.0, dtype=torch.bfloat16 if mode == 0 else torch.float32, device="cuda")
+    K.moe_rows(x, w, out, mode, ids.cuda(), top, stream())
+    for p in range(P):
+        e = int(ids[p])
+        if e == E:
+            assert bool((out[p] == 768.0).all())
+            continue
+        s = w[e].double() @ x[p // top if mode == 0 else p].double()
+        size = w[e].double().abs() @ x[p // top if mode == 0 else p].double().abs()
+        err = size * K_ * 2.0 ** -23                      # float32 sums of exact products, each addition off by at most one unit of the sum's size
+        if mode == 0:
+            gate, up = s[0::2], s[1::2]
+            want = torch.nn.functional.silu(gate) * up
+            err = 1.1 * err[0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * err[1::2] + want.abs() * 2.0 ** -8
+        else:
+            want = s
+        assert bool(((out[p].double() - want).abs() <= err + 1e-30).all()), (p, e)
+    # a pair alone is the same bits as beside the others
+    first = int((ids == 4).nonzero()[0])
+    one = torch.empty_like(out[:1])
+    K.moe_rows(x[first // top:first // top + 1] if mode == 0 else x[first:first + 1], w, one, mode, ids[first:first + 1].cuda(), 1, stream())
+    assert torch.equal(one[0], out[first])
+
+
+@pytest.mark.parametrize("P,E", [(1, 1), (37, 5), (8192, 33), (8193, 64), (20000, 3)])
+def test_plan_groups_every_pair_once(P, E):
+    """Around the number of pairs that the block keeps in registers, and of experts around a warp's lanes."""
+    from titan_b200 import kernels as K
+    g = torch.Generator().manual_seed(P)
+    ids = torch.randint(0, E, (P, 1), generator=g, dtype=torch.int32)
+    plan = K.moe_plan(ids.cuda(), E, torch.empty(K.MoePlan.size(P, E), dtype=torch.int32, device="cuda"), stream())
+    offsets, perm, inverse = plan.offsets[:E + 1].cpu(), plan.perm[:P].cpu().long(), plan.inverse[:P].cpu().long()
+    counts = torch.bincount(ids[:, 0].long(), minlength=E)
+    assert offsets.tolist() == [0] + counts.cumsum(0).tolist()
+    assert torch.equal(perm.sort().values, torch.arange(P)) and torch.equal(perm[inverse], torch.arange(P))
+    assert torch.equal(ids[perm, 0].long(), torch.repeat_interleave(torch.arange(E), counts))
+    n = int(plan.n_tiles[0])
+    tiles = list(zip(plan.tile_e[:n].tolist(), plan.tile_row0[:n].tolist(), plan.tile_rows[:n].tolist()))
+    want = [(e, int(offsets[e]) + r, min(64, int(counts[e]) - r)) for e in range(E) for r in range(0, int(counts[e]), 64)]
+    assert tiles == want
