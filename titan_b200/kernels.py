@@ -1035,6 +1035,10 @@ def set_attn_decode_late_trigger(on: bool) -> None:
     alib().tb_attn_decode_set_late_trigger(int(bool(on)))
 
 
+def set_attn_decode_ahead(mb: int) -> None:
+    """Decode attention: at most this many MB of the weights after it (``AttnArgs.next_w``) are requested into L2 (0: none; -1: the default)."""
+    alib().tb_attn_decode_set_ahead(int(mb))
+
 # Where the tensor-core prompt kernels take keys and values from: nowhere they can (0), the step's own rows (every
 # sequence starts at position 0), or the cache's pages (the step's keys are appended already; no ring).
 KV_NOWHERE, KV_FROM_STEP, KV_FROM_CACHE = 0, 1, 2
