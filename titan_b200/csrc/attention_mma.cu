@@ -18,6 +18,8 @@
 // scalar FMA (engine/engine-cuda/kernels/paged_attention.cu:200-309).
 #include <float.h>
 
+#include <atomic>
+
 #include "attention_args.h"
 #include "common.cuh"
 #include "mma.cuh"
@@ -62,6 +64,7 @@ struct DecArgs {
     const float* sink;                             // [nh] or null: one more term exp(sink) of every head's softmax denominator
     int keep_first;                                // with a window: the sequence's first keep_first keys stay visible
     const char* next_w[2]; long long next_bytes[2];     // weights of the kernels behind this one, to be requested into L2
+    int by_length;                                 // the blocks take the sequences from the longest down
 };
 
 // This CTA's share of the next kernels' weights, by one thread, as bulk requests of up to 16 KB that bring nothing into the SM.
@@ -135,7 +138,8 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kv_map, DecArgs a) {
     float* recv = reinterpret_cast<float*>(q_sh + 16 * HD);          // CL: [split][per + 32]: every split's values for this CTA's share of the output, its maxima and sums
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x, kh = blockIdx.y, split = blockIdx.z;
+    int b = blockIdx.x, kh = blockIdx.y;
+    const int split = blockIdx.z;
     TimelineProbe probe;              // stamps: 1 wait for the kernels before passed, 2 queries ready, 3 pages done, 5 all parts here, 4 end
     probe.begin(100000 + gridDim.z, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
     // The kernel after this one may start (and request its first weight tiles) while this one runs.  Those requests
@@ -147,7 +151,24 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kv_map, DecArgs a) {
     // only older positions are requested before the wait, while those kernels still run.
     const bool early = a.early_mode != 0;
     if (!early) pdl_wait();
-    const int len = a.early_mode == 2 ? a.early_len[a.slot_of_seq[b]] + 1 : (early ? a.early_len[b] : a.kv_len[b]);
+    auto length_of = [&](int s) { return a.early_mode == 2 ? a.early_len[a.slot_of_seq[s]] + 1 : (early ? a.early_len[s] : a.kv_len[s]); };
+    if (a.by_length) {
+        // More blocks than the device holds at once: they start in the order of their numbers, so block i takes kv head i % nkv of the
+        // sequence with i / nkv longer ones before it, and the shortest fill the last places (64 sequences of 64 to 512 keys in
+        // batch order, a block a kv head: 22 us, of which the last longest ones alone a third).  A sequence's own arithmetic is the same.
+        __shared__ int lens[DEC_THREADS], chosen;
+        const int i = blockIdx.x + gridDim.x * blockIdx.y, t = threadIdx.x, mine = t < (int)gridDim.x ? length_of(t) : 0;
+        lens[t] = mine;
+        __syncthreads();
+        if (t < (int)gridDim.x) {
+            int before = 0;
+            for (int s = 0; s < (int)gridDim.x; ++s) before += lens[s] > mine || (lens[s] == mine && s < t);
+            if (before == i / a.nkv) chosen = t;
+        }
+        __syncthreads();
+        b = chosen; kh = i % a.nkv;
+    }
+    const int len = length_of(b);
     const int keys = tb_split_keys(len, a.chunk, a.n_splits);
     if (!CL && (long long)split * keys >= len) return;  // uniform over the CTA; the merge skips these splits (in a cluster the CTA stays, with no pages, for the barrier)
     const int group = a.nh / a.nkv;
@@ -778,6 +799,16 @@ int g_late_trigger = 1;
 // When the kernel after decode attention may start: once this one's pages have been read (1, default) or at once (0).
 // Measured after 2,048-token prompts: batch 1 2.85 -> 2.81 ms per step, batch 4 3.11 -> 3.06, batch 8 3.27 -> 3.24; no
 // difference at 7,000 tokens or at batch 64.
+static int sm_count() {
+    static std::atomic<int> count[64];                     // a device each
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && (n = count[dev].load()) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    if (dev < 64) count[dev].store(n);
+    return n;
+}
+
 constexpr int AHEAD_MB = 48;
 static int g_ahead_mb = -1;
 // MB of the next kernels' weights that are requested into L2 (0: none, -1: the default).
@@ -852,6 +883,7 @@ extern "C" int tb_attn_decode_mma(const AttnArgs* args, cudaStream_t stream) {
         room -= d.next_bytes[r];
     }
     dim3 grid(a.batch.B, a.nkv, a.n_splits);
+    d.by_length = a.n_splits == 1 && a.batch.B <= DEC_THREADS && (long long)a.batch.B * a.nkv > 2 * sm_count();      // two blocks an SM
     d.late_trigger = g_late_trigger;
     const bool wide = a.nh / a.nkv > 8;
     int rc;
