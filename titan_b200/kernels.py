@@ -95,7 +95,8 @@ class AttnArgs(Structure):
                 ("softcap", c_float), ("rel_bias", c_void_p), ("rel_far", c_int), ("head_mix", c_void_p),
                 ("head_gate", c_void_p), ("head_gate_stride", c_int),
                 ("pair_lambda", c_void_p), ("pair_eps", c_float), ("pair_scale", c_float), ("pair_width", c_int),
-                ("out_f32", c_int), ("exact_weights", c_int)]
+                ("out_f32", c_int), ("exact_weights", c_int),
+                ("next_w", c_void_p * 2), ("next_bytes", c_longlong * 2)]
 
 
 class LatentArgs(Structure):
