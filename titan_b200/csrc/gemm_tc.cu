@@ -953,7 +953,7 @@ __device__ __forceinline__ void lanes_out(const float* v, const TcArgs& a, int r
     for (int i = 0; i < 32; i += 2) {
         const float other = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
         const float x = odd ? other : v[i], y = odd ? v[i + 1] : other;           // columns n & ~1 and its neighbour
-        if (i + odd >= rows || n >= a.rows_b) continue;
+        if (i + odd >= rows || (n & ~1) >= a.rows_b) continue;
         if (EPI == TB_EPI_SWIGLU) o[(size_t)i * a.ldo] = __float2bfloat16_rn(silu_mul(x, y));
         else if ((n | 1) < a.rows_b) *reinterpret_cast<uint32_t*>(o + (size_t)i * a.ldo) = pack_bf16(tb_unary(a.act, x), tb_unary(a.act, y));
         else o[(size_t)i * a.ldo] = __float2bfloat16_rn(tb_unary(a.act, x));      // the last of an odd number of columns
