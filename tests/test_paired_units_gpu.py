@@ -46,12 +46,9 @@ CASES = [  # nh, nkv, start positions, new tokens, window, kept first, sink, exa
 ]
 
 
-@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("units", [1, 2])
 @pytest.mark.parametrize("nh,nkv,starts,news,window,keep,sinks,exact", CASES)
-def test_prompt_attention_at_the_edges_of_its_tiles(K, nh, nkv, starts, news, window, keep, sinks, exact, many):
-    if many:            # enough heads for two units of query rows a block
-        times = torch.cuda.get_device_properties(0).multi_processor_count // (nh * -(-sum(news) // 128)) + 1
-        nh, nkv = nh * times, nkv * times
+def test_prompt_attention_at_the_edges_of_its_tiles(K, nh, nkv, starts, news, window, keep, sinks, exact, units):
     hd, g = 128, torch.Generator().manual_seed(nh * 100 + sum(news))
     slots = [3, 0, 5, 1][:len(news)]
     lay, T, Q, KV = layout_for(slots, starts, news), sum(news), nh * hd, nkv * hd
@@ -84,7 +81,11 @@ def test_prompt_attention_at_the_edges_of_its_tiles(K, nh, nkv, starts, news, wi
     a.sink = None if sink is None else sink.data_ptr()
     source = K.KV_FROM_STEP if fresh else K.KV_FROM_CACHE
     assert K.attn_prefill_tc_accepts(a, torch.bfloat16, source)
-    K.attn_prefill_tc(a, source, stream())
+    K.set_attn_tc_units(units)
+    try:
+        K.attn_prefill_tc(a, source, stream())
+    finally:
+        K.set_attn_tc_units(0)
     assert K.wait_errors() == {}
     # A weight enters the product rounded to eight bits (by 2^-8 of itself at most; with exact weights 2^-16), the result is rounded once
     # more where it leaves in bfloat16, and the scores' float32 sums (|s| below 8 here) move a weight by less than 2^-18.
@@ -93,9 +94,9 @@ def test_prompt_attention_at_the_edges_of_its_tiles(K, nh, nkv, starts, news, wi
     assert bool(((out.double() - want).abs() <= bound).all()), float(((out.double() - want).abs() / bound).max())
 
 
-@pytest.mark.parametrize("nh", [2, 40])
+@pytest.mark.parametrize("nh,units", [(2, 1), (2, 2), (40, 0)])
 @pytest.mark.parametrize("news,window,sinks,exact,wide", [([1, 64, 127], 0, False, 0, True), ([130, 700], 100, True, 0, False), ([333, 65], 0, False, 1, True), ([640], 257, True, 1, False)])
-def test_prompt_attention_with_keys_in_two_parts(K, nh, news, window, sinks, exact, wide):
+def test_prompt_attention_with_keys_in_two_parts(K, nh, units, news, window, sinks, exact, wide):
     dn, dt, g = 128, 64, torch.Generator().manual_seed(nh + sum(news))
     T, lay = sum(news), layout_for(list(range(len(news))), [0] * len(news), news)
     scale = 1 / math.sqrt(dn + dt)
@@ -111,7 +112,11 @@ def test_prompt_attention_with_keys_in_two_parts(K, nh, news, window, sinks, exa
     a.batch, a.nh, a.dn, a.dt, a.dv, a.window, a.scale = lay.c_struct(), nh, dn, dt, dn, window, scale
     a.sink, a.exact_weights = None if sink is None else sink.data_ptr(), exact
     assert K.attn_prefill_split_accepts(a)
-    K.attn_prefill_split(a, stream())
+    K.set_attn_tc_units(units)
+    try:
+        K.attn_prefill_split(a, stream())
+    finally:
+        K.set_attn_tc_units(0)
     assert K.wait_errors() == {}
     at = 0
     for n in news:

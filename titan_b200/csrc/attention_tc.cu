@@ -3,7 +3,7 @@
 //
 // One CTA per (sequence, block of 128 queries, PAIR of query heads that share a key-value head); where a key-value head has an
 // odd number of query heads, per (sequence, 256 queries, head): two units of 128 query rows either way, over the same keys.  Steps too
-// small to fill the SMs so take one unit a CTA.
+// small to fill the SMs so take one unit a CTA (the second form below).
 // Per tile of 128 keys and unit:
 //     S = Q . K^T        tcgen05.mma, A = Q and B = K both K-major in shared memory, S in tensor memory
 //     P = 2^(S*c - m)    a softmax thread reads its query row of S with tcgen05.ld and writes P (pairs of
@@ -11,19 +11,22 @@
 //     O += P . V         tcgen05.mma with A = P from tensor memory, B = V as MN-major operand from shared
 //                        memory (V's rows are keys, its contiguous dimension is the output dimension),
 //                        O accumulated in tensor memory
-// Sixteen softmax warps, eight a unit: a query row is two threads, a page of the tile each.  While one unit's warps turn S into P, the tensor
-// cores run the other unit's P.V and next S: one thread issues P.V_0(j), S_0(j+1), P.V_1(j), S_1(j+1), ..., and MMAs run in the order they are
-// issued, so S(j+1) may take the columns of P(j), and "S(j+1) is done" also says that O holds P.V(j).  A row's maximum is raised only
-// when a tile exceeds it by more than 2^RESCALE_LOG2 (P stays below that bound, which bfloat16 and the float32 sum hold easily);
-// only then do the row's two threads exchange their maxima and rescale O in tensor memory, which after the first tiles is rare: in every
-// other tile one barrier of the two warps that says so is all they need of one another.
+// Two units: eight softmax warps, four a unit, a thread a query row.  While one unit's warps turn S into P, the tensor cores run the
+// other unit's P.V and next S: one thread issues P.V_0(j), S_0(j+1), P.V_1(j), S_1(j+1), ..., and MMAs run in the order they are issued, so
+// S(j+1) may take the columns of P(j), and "S(j+1) is done" also says that O holds P.V(j).
+// One unit: two threads a query row, a page of the tile each, and S in two buffers (the second unit's columns), so that S(j+1) runs while
+// the warps are at tile j.  The two threads exchange their maxima only when one of them has to raise the row's; in every other tile one barrier of
+// the two warps that says so is all they need of one another.
+// P is handed over in two halves of 64 keys.  A row's maximum is raised only when a tile exceeds it by more than 2^RESCALE_LOG2 (P
+// stays below that bound, which bfloat16 and the float32 sum hold easily); only then are rows of O rescaled in tensor memory, which
+// after the first tiles is rare.
 //
 // What bounds it: the special-function units (16 exponentials a clock and SM: 1,024 clocks for a unit's tile) and the tensor cores
-// (1,024 clocks for S and P.V of it) are needed equally, and a unit's warps wait for their own S; two units keep both busy in turn, and
-// four warps a scheduler hide one another's fixed latencies (with two, eight warps of a whole row a thread, both pipes stood at 51 %).
+// (1,024 clocks for S and P.V of it) are needed equally, and a unit's warps wait for their own S; two units keep both busy in turn (51 % each).
+// Sixteen softmax warps of half rows, which have 96 registers a thread, were slower (8,192 tokens of 32 heads on 8: 527 us; as it is 470).
 // Tiles of 128 keys: an S product of 64 keys reads 192 bytes of shared memory a clock (limit 128), one of 128 keys 128.
 //
-// Warp 0 loads Q once and K and V tiles through TMA (a ring each), warp 1 issues the MMAs and allocates tensor memory, warps 2..17 are
+// Warp 0 loads Q once and K and V tiles through TMA (a ring each), warp 1 issues the MMAs and allocates tensor memory, warps 4..11 are
 // the softmax.  Keys and values come from the step's own [T][Q | K | V] rows (every sequence starts at position 0) or from the
 // cache's pages.  The grid runs over heads fastest, so the heaviest query blocks of all heads start first and the lightest make the tail.
 // Tensor memory: S (then P) 2 x 128 columns, O 2 x 128 columns (all 512).
@@ -49,7 +52,10 @@ using namespace tbtc;
 __device__ unsigned int g_attn_tc_error = 0;
 
 constexpr int HD = 128, BQ = 128, PAGE = 64, BKEY = 128;  // a key tile is two pages (boxes) of 64 rows
-constexpr int THREADS = 576;                           // producer, MMA issuer, sixteen softmax warps
+constexpr int THREADS = 384;                           // producer, MMA issuer, two idle warps, eight softmax warps
+// Registers: the launch gives every thread 168 (65,536 / 384, in steps of eight); with two units the first four warps keep 96 and the softmax
+// warps, which hold whole rows of 128 scores, take 200: 128 * 96 + 256 * 200 = 63,488 of 64,512.
+constexpr int REGS_OTHER = 96, REGS_SOFTMAX = 200;
 constexpr uint32_t Q_BOX = BQ * 128;                   // 128 rows x 64 columns
 constexpr uint32_t KV_BOX = PAGE * 128;                // 64 rows x 64 columns
 constexpr uint32_t KV_HALF = 2 * KV_BOX;               // 128 rows x 64 columns
@@ -61,7 +67,7 @@ template <int DK> constexpr uint32_t k_tile() { return DK / 64 * KV_HALF; }
 template <int DK> constexpr int k_stages() { return DK == 128 ? 3 : 2; }
 template <int DK> constexpr int v_stages() { return DK == 128 ? 2 : 1; }
 template <int DK> constexpr size_t tc_smem() {
-    return 1024 + 2 * q_unit<DK>() + k_stages<DK>() * k_tile<DK>() + v_stages<DK>() * V_TILE + 128 + 2 * BQ * sizeof(float);
+    return 1024 + 2 * q_unit<DK>() + k_stages<DK>() * k_tile<DK>() + v_stages<DK>() * V_TILE + 160 + BQ * sizeof(float);
 }
 
 struct TcAttnArgs {
@@ -72,7 +78,6 @@ struct TcAttnArgs {
     int k_col0; int v_col0;
     // keys and values from the cache (continuation steps): the first position of each sequence's rows, its slot,
     // the block table, and the row of the first V page in the cache's tensor map; paged = 0: from the step's rows
-    int units;               // of 128 query rows a CTA: 1 or 2
     int pair_heads;          // 1: a CTA's two units are query heads 2x and 2x + 1, 0: blocks of 128 queries of one head
     int paged; const int* start_pos; const int* slot_of_seq; const int* table; int table_width; int v_row0;
     const float* sink;       // [nh] or null: one more term exp(sink) of every head's softmax denominator, without key or value
@@ -133,14 +138,17 @@ constexpr float RESCALE_LOG2 = 8.0f;
 // CURRENT phase, so a waiter must see phase k before phase k + 1 ends.
 //   k_full, k_empty,    the rings' stages: TMA bytes of a tile, and the commit behind the last MMA that reads it.  Loads go out in the order
 //   v_full, v_empty     K_0 V_0 K_1 V_1 ...; a load waits for a commit that needs no tile behind it in that order.
-//   s_done[u]           commit behind S_u(j) (phase j), and once more behind the last P.V_u.  The unit's warps wait for every phase; the
+//   s_done[u]           Two units: commit behind S_u(j) (phase j), and once more behind the last P.V_u.  The unit's warps wait for every phase; the
 //                       issuer commits phase j + 1 only after p_full of tile j, which the warps arrive at after seeing phase j.
-//   p_full[u]           eight arrivals (the unit's warps) a tile.  The issuer waits for every phase; the warps arrive for tile
-//                       j + 1 only after s_done(j + 1), which the issuer commits after it has seen p_full of tile j.
+//   p_full[u][half]     four arrivals (warps) a tile.  The issuer waits for every phase; the warps arrive for tile j + 1 only after
+//                       s_done(j + 1), which the issuer commits after it has seen both halves of tile j.
+//   One unit: the same with u the buffer j & 1 and its tiles j, j + 2, ... as phases: S(j + 2) is issued after both halves of P(j).
+//   o_done              one unit: commit behind P.V(j) (phase j).  Who rescales O in tile j waits for phase j - 1, and phase j needs that
+//                       thread's own P(j); the others need not look.
 
 // EXACT: the softmax weights enter P . V as two bfloat16 halves (AttnArgs.exact_weights): the rounded weights over the first
 // half of the tile's S columns, what rounding left over over the second half, and each value tile is multiplied by both.
-template <bool EXACT, int DK>
+template <bool EXACT, int DK, int UNITS>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap tail_map, TcAttnArgs a) {
     constexpr int KB = DK / 64, KS = k_stages<DK>(), VS = v_stages<DK>();
@@ -156,15 +164,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     uint64_t* v_full = k_empty + KS;         // [VS]
     uint64_t* v_empty = v_full + VS;         // [VS]
     uint64_t* s_done = bars + 11;            // [2]
-    uint64_t* p_full = bars + 13;            // [2]
-    uint32_t* tmem_slot = (uint32_t*)(bars + 15);
-    float* row_sh = (float*)(bars + 16);     // [2 units][128 rows]: what the two threads of a row tell one another
+    uint64_t* p_full = bars + 13;            // [2][2 halves]
+    uint64_t* o_done = bars + 17;
+    uint32_t* tmem_slot = (uint32_t*)(bars + 18);
+    float* row_sh = (float*)(bars + 20);     // [128 rows]: what the two threads of a row tell one another (one unit)
 
     pdl_launch_dependents();
     pdl_wait();
     // blockIdx.y: which sequence and which block of queries (a sequence's blocks from the heaviest,
     // the last, down); blockIdx.x, which runs fastest in the dispatch order: the head or pair of heads
-    const int units = a.units, rows_cta = a.pair_heads ? BQ : units * BQ;
+    const int rows_cta = a.pair_heads ? BQ : UNITS * BQ;
     int rem = blockIdx.y, seq = -1, blk = 0, tok0 = 0, n = 0;
     for (int s = 0; s < a.B; ++s) {
         const int t0 = a.q_start[s], ns = a.q_start[s + 1] - t0, nb = (ns + rows_cta - 1) / rows_cta;
@@ -193,7 +202,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         mbar_init(q_full, 1);
         for (int s = 0; s < KS; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, 1); }
         for (int s = 0; s < VS; ++s) { mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(s_done + s, 1); mbar_init(p_full + s, 8); }
+        for (int s = 0; s < 2; ++s) mbar_init(s_done + s, 1);
+        for (int s = 0; s < 4; ++s) mbar_init(p_full + s, 4);
+        mbar_init(o_done, 1);
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -201,13 +212,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_s = tmem;             // S of unit u: columns 128 u ..
+    const uint32_t tmem_s = tmem;             // S of unit (or buffer) u: columns 128 u ..
     const uint32_t tmem_o = tmem + 256;       // O of unit u: columns 256 + 128 u ..
 
-    if (warp < 2) {
+    if (warp < 4) {
+        if (UNITS == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
         if (warp == 0 && lane == 0) {
-            mbar_expect_tx(q_full, units * q_unit<DK>());
-            for (int u = 0; u < units; ++u)
+            mbar_expect_tx(q_full, UNITS * q_unit<DK>());
+            for (int u = 0; u < UNITS; ++u)
                 for (int c = 0; c < KB; ++c)
                     tma_load_2d(q_smem + (KB * u + c) * Q_BOX, &q_map, q_full, (h0 + (a.pair_heads ? u : 0)) * DK + c * 64,
                                 tok0 + r0 + (a.pair_heads ? 0 : u * BQ));
@@ -230,18 +242,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         } else if (warp == 1 && lane == 0) {
             // ---- every MMA; a tile's descriptors differ from a base by constants
             const uint64_t q_desc = desc_k_major(smem_u32(q_smem));
-            auto issue_s = [&](int u, int j) {                    // S_u = Q_u . K_j^T
+            auto issue_s = [&](int u, int buf, int j) {           // S_u = Q_u . K_j^T
                 const uint64_t k_desc = desc_k_major(smem_u32(k_smem + j % KS * k_tile<DK>()));
-                const uint32_t d = tmem_s + u * BKEY, idesc = 2 * j + 1 < n_pages ? IDESC_S : IDESC_S_PAGE;
+                const uint32_t d = tmem_s + buf * BKEY, idesc = 2 * j + 1 < n_pages ? IDESC_S : IDESC_S_PAGE;
 #pragma unroll
                 for (int ks = 0; ks < DK / 16; ++ks)              // 16 dims per step: box ks / 4, 32 bytes per step inside it
                     tc_mma(d, q_desc + (uint64_t)((u * q_unit<DK>() + (ks >> 2) * Q_BOX + (ks & 3) * 32) >> 4),
                            k_desc + (uint64_t)(((ks >> 2) * KV_HALF + (ks & 3) * 32) >> 4), idesc, ks > 0 ? 1u : 0u);
-                tc_commit(s_done + u);
+                tc_commit(s_done + buf);
             };
-            auto issue_pv = [&](int u, int j, int half) {         // O_u += P_u . V_j, the keys of one page
+            auto issue_pv = [&](int u, int buf, int j, int half) {      // O_u += P_u . V_j, the keys of one page
                 const uint64_t v_desc = desc_mn_major(smem_u32(v_smem + j % VS * V_TILE));
-                const uint32_t p = tmem_s + u * BKEY, d = tmem_o + u * HD;
+                const uint32_t p = tmem_s + buf * BKEY, d = tmem_o + u * HD;
 #pragma unroll
                 for (int ks = 4 * half; ks < 4 * half + 4; ++ks)  // 16 keys per step: 8 columns of P, 16 rows of V
                     tc_mma_a_tmem(d, p + ks * 8, v_desc + (uint64_t)((ks * 2048) >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
@@ -254,74 +266,108 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             wait(q_full, 0, 3);
             wait(k_full, 0, 2);
             tc_fence_after();
-            for (int u = 0; u < units; ++u) issue_s(u, 0);
+            for (int u = 0; u < UNITS; ++u) issue_s(u, u, 0);
             tc_commit(k_empty);
             for (int j = 0; j < n_tiles; ++j) {
                 const bool both = 2 * j + 1 < n_pages;
-                for (int u = 0; u < units; ++u) {
+                auto next_k = [&] { wait(k_full + (j + 1) % KS, ((j + 1) / KS) & 1, 2); tc_fence_after(); };
+                if (UNITS == 1 && j + 1 < n_tiles) {
+                    next_k();
+                    issue_s(0, (j + 1) & 1, j + 1);
+                    tc_commit(k_empty + (j + 1) % KS);
+                }
+                for (int u = 0; u < UNITS; ++u) {
+                    const int buf = UNITS == 2 ? u : j & 1, parity = UNITS == 2 ? j & 1 : (j >> 1) & 1;
                     if (u == 0) wait(v_full + j % VS, (j / VS) & 1, 5);
-                    wait(p_full + u, j & 1, 4);                   // the unit has rescaled O if it had to and written P
+                    wait(p_full + 2 * buf, parity, 4);            // O is rescaled if it had to be, and the first half of P is written
                     tc_fence_after();
-                    issue_pv(u, j, 0);
-                    if (both) issue_pv(u, j, 1);
-                    if (u == units - 1) tc_commit(v_empty + j % VS);
-                    if (j + 1 < n_tiles) {
-                        if (u == 0) { wait(k_full + (j + 1) % KS, ((j + 1) / KS) & 1, 2); tc_fence_after(); }
-                        issue_s(u, j + 1);
-                        if (u == units - 1) tc_commit(k_empty + (j + 1) % KS);
+                    issue_pv(u, buf, j, 0);
+                    wait(p_full + 2 * buf + 1, parity, 7);
+                    tc_fence_after();
+                    if (both) issue_pv(u, buf, j, 1);
+                    if (u == UNITS - 1) tc_commit(v_empty + j % VS);
+                    if (UNITS == 1) {
+                        tc_commit(o_done);
+                    } else if (j + 1 < n_tiles) {
+                        if (u == 0) next_k();
+                        issue_s(u, u, j + 1);
+                        if (u == UNITS - 1) tc_commit(k_empty + (j + 1) % KS);
                     } else {
                         tc_commit(s_done + u);                    // O is complete
                     }
                 }
             }
         }
-    } else if ((warp - 2) >> 3 < units) {
-        const int u = (warp - 2) >> 3, p = ((warp - 2) >> 2) & 1, quarter = warp & 3;      // a warp may touch the tensor-memory lanes 32 * (warp % 4) ..
+    } else {
+        if (UNITS == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_SOFTMAX));
+        constexpr int OWN = UNITS;                               // pages of a tile that this thread has scores of
+        const int team = (warp - 4) >> 2, u = UNITS == 2 ? team : 0, p0s = UNITS == 2 ? 0 : team, quarter = warp & 3;      // a warp may touch the tensor-memory lanes 32 * (warp % 4) ..
         const int lane_row = quarter * 32 + lane, row = lane_row + (a.pair_heads ? 0 : u * BQ);       // among the unit's and the CTA's rows
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-        const uint32_t s_cols = tmem_s + u * BKEY + lane_addr, o_cols = tmem_o + u * HD + p * 64 + lane_addr;
-        float* told = row_sh + u * BQ + lane_row;
-        const int pair_barrier = 1 + u * 4 + quarter;            // the two warps that share rows
+        const uint32_t o_cols = tmem_o + u * HD + p0s * 64 + lane_addr;          // of this thread's part of the row of O
+        constexpr int O_COLS = UNITS == 2 ? HD : HD / 2;
+        float* told = row_sh + lane_row;
+        const int pair_barrier = 1 + quarter;                    // the two warps that share rows (one unit)
         const int qpos = p0 + r0 + row;                          // the row's position in its sequence
         const int lo = a.window > 0 ? qpos - a.window + 1 : 0;
         float m_run = -1e30f, l_run = 0.f;                       // the maximum P is taken against (may lag), this thread's part of the sum
         for (int j = 0; j < n_tiles; ++j) {
-            const int at = 2 * j + p;                            // this thread's page of the tile, if there is one
-            const int key0 = at < n_pages ? (at < n_keep ? at : at + kskip) * PAGE : 0x40000000;      // (else behind every query)
-            const bool visible = key0 + PAGE - 1 <= qpos && (key0 >= lo || key0 + PAGE <= a.keep_first);      // no mask needed
-            wait(s_done + u, j & 1, 6);
-            tc_fence_after();
-            float v[64];
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            tmem_ld32_nowait(s_cols + p * PAGE, v);
-            tmem_ld32_nowait(s_cols + p * PAGE + 32, v + 32);
-            tmem_wait_ld<64>(v);
-            if (!visible) {
+            const int buf = UNITS == 2 ? u : j & 1, parity = UNITS == 2 ? j & 1 : (j >> 1) & 1;
+            const uint32_t s_cols = tmem_s + buf * BKEY + lane_addr;
+            int key0[OWN];
+            bool visible = true;                                 // no mask needed
 #pragma unroll
-                for (int i = 0; i < 64; ++i) v[i] = (key0 + i <= qpos && (key0 + i >= lo || key0 + i < a.keep_first)) ? v[i] : -INFINITY;
+            for (int p = 0; p < OWN; ++p) {
+                const int at = 2 * j + p0s + p;
+                key0[p] = at < n_pages ? (at < n_keep ? at : at + kskip) * PAGE : 0x40000000;        // no such page: behind every query
+                visible = visible && key0[p] + PAGE - 1 <= qpos && (key0[p] >= lo || key0[p] + PAGE <= a.keep_first);
+            }
+            wait(s_done + buf, parity, 6);
+            tc_fence_after();
+            float v[64 * OWN];
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            tmem_ld32_nowait(s_cols + p0s * PAGE, v);
+            tmem_ld32_nowait(s_cols + p0s * PAGE + 32, v + 32);
+            tmem_wait_ld<64>(v);
+            if (OWN == 2) {
+                tmem_ld32_nowait(s_cols + 64, v + 64 * (OWN - 1));
+                tmem_ld32_nowait(s_cols + 96, v + 64 * (OWN - 1) + 32);
             }
 #pragma unroll
-            for (int i = 0; i < 64; i += 8) {               // four chains of three-input maxima
-                mx4[0] = max3(mx4[0], v[i], v[i + 1]); mx4[1] = max3(mx4[1], v[i + 2], v[i + 3]);
-                mx4[2] = max3(mx4[2], v[i + 4], v[i + 5]); mx4[3] = max3(mx4[3], v[i + 6], v[i + 7]);
+            for (int p = 0; p < OWN; ++p) {
+                if (p == 1) tmem_wait_ld<64>(v + 64 * p);
+                float* w = v + 64 * p;
+                if (!visible) {
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) w[i] = (key0[p] + i <= qpos && (key0[p] + i >= lo || key0[p] + i < a.keep_first)) ? w[i] : -INFINITY;
+                }
+#pragma unroll
+                for (int i = 0; i < 64; i += 8) {           // four chains of three-input maxima
+                    mx4[0] = max3(mx4[0], w[i], w[i + 1]); mx4[1] = max3(mx4[1], w[i + 2], w[i + 3]);
+                    mx4[2] = max3(mx4[2], w[i + 4], w[i + 5]); mx4[3] = max3(mx4[3], w[i + 6], w[i + 7]);
+                }
             }
             float cand = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;
-            // Raise the row's maximum only when the tile exceeds it by more than the bound.  The two warps that share rows ask one another; the
-            // barrier also says that both have read their scores, over which P goes.
+            // Raise the row's maximum only when the tile exceeds it by more than the bound.  One unit: the two warps that share rows ask one another;
+            // the barrier also says that both have read their scores, over which P goes.
             float f = 1.f;
-            if (any_of_two_warps(pair_barrier, cand > m_run + RESCALE_LOG2)) {
-                if (p == 0) *told = cand;
-                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-                if (p == 1) *told = cand = fmaxf(cand, *told);
-                asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-                if (p == 0) cand = *told;
+            const bool above = cand > m_run + RESCALE_LOG2;
+            if (UNITS == 2 ? __any_sync(0xffffffffu, above) : any_of_two_warps(pair_barrier, above)) {
+                if (UNITS == 1) {
+                    if (team == 0) *told = cand;
+                    asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                    if (team == 1) *told = cand = fmaxf(cand, *told);
+                    asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+                    if (team == 0) cand = *told;
+                }
                 const float m_old = m_run;
                 if (cand > m_run + RESCALE_LOG2) m_run = cand;
                 f = ex2(m_old - m_run);                          // 1 for the rows that keep their maximum
-                // Only a rescale touches O, a warp half of its columns (P.V of the tile before is complete: S of this one was issued behind it).
                 if (j > 0) {
+                    // Only a rescale touches O.  Two units: P.V of the tile before is complete, S of this one was issued behind it.
+                    if (UNITS == 1) { wait(o_done, (j - 1) & 1, 9); tc_fence_after(); }
 #pragma unroll 1
-                    for (int c = 0; c < 64; c += 16) {
+                    for (int c = 0; c < O_COLS; c += 16) {
                         float o[16];
                         uint32_t bits[16];
                         tmem_ld16(o_cols + c, o);
@@ -337,49 +383,58 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
             // P as bfloat16 pairs over the first columns of the unit's S: the A operand of P.V, which never touches shared memory
 #pragma unroll
-            for (int c = 0; c < 64; c += 32) {
-                uint32_t pk[16];
+            for (int p = 0; p < OWN; ++p) {
+                const int half = p0s + p;
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float* w = v + c + i;
-                    const float2 x = __ffma2_rn(make_float2(w[0], w[1]), scale2, shift2);
-                    w[0] = ex2(x.x); w[1] = ex2(x.y);
-                    sum2[(i >> 1) & 1] = __fadd2_rn(sum2[(i >> 1) & 1], make_float2(w[0], w[1]));
-                    pk[i >> 1] = pack_bf16x2(w[0], w[1]);
-                }
-                tmem_st16_nowait(s_cols + 32 * p + c / 2, pk);
-                if (EXACT) {
+                for (int c = 0; c < 64; c += 32) {
+                    uint32_t pk[16];
+                    float* w = v + 64 * p + c;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        pk[i] = pack_bf16x2(v[c + 2 * i] - __uint_as_float(pk[i] << 16), v[c + 2 * i + 1] - __uint_as_float(pk[i] & 0xffff0000u));
-                    tmem_st16_nowait(s_cols + BKEY / 2 + 32 * p + c / 2, pk);
+                    for (int i = 0; i < 32; i += 2) {
+                        const float2 x = __ffma2_rn(make_float2(w[i], w[i + 1]), scale2, shift2);
+                        w[i] = ex2(x.x); w[i + 1] = ex2(x.y);
+                        sum2[(i >> 1) & 1] = __fadd2_rn(sum2[(i >> 1) & 1], make_float2(w[i], w[i + 1]));
+                        pk[i >> 1] = pack_bf16x2(w[i], w[i + 1]);
+                    }
+                    tmem_st16_nowait(s_cols + 32 * half + c / 2, pk);
+                    if (EXACT) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            pk[i] = pack_bf16x2(w[2 * i] - __uint_as_float(pk[i] << 16), w[2 * i + 1] - __uint_as_float(pk[i] & 0xffff0000u));
+                        tmem_st16_nowait(s_cols + BKEY / 2 + 32 * half + c / 2, pk);
+                    }
                 }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_full + 2 * buf + half);
             }
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_full + u);
             l_run = l_run * f + ((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
         }
-        wait(s_done + u, n_tiles & 1, 8);                        // the unit's last P.V
+        if (UNITS == 2) wait(s_done + u, n_tiles & 1, 8);        // the last P.V
+        else wait(o_done, (n_tiles - 1) & 1, 8);
         tc_fence_after();
-        if (p == 0) *told = l_run;
-        asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-        if (p == 1) *told = l_run = *told + l_run;
-        asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
-        const float l0 = p == 0 ? *told : l_run;
+        if (UNITS == 1) {
+            if (team == 0) *told = l_run;
+            asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+            if (team == 1) *told = l_run = *told + l_run;
+            asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier) : "memory");
+            if (team == 0) l_run = *told;
+        }
         const int h = h0 + (a.pair_heads ? u : 0);
         const float sk = a.sink ? a.sink[h] * 1.4426950408889634f : -1e30f;      // the sink, in units of log2 like the maxima
         const float M = fmaxf(m_run, sk), w0 = ex2(m_run - M);
-        const float c0 = w0 / (l0 * w0 + (a.sink ? ex2(sk - M) : 0.f));
-        const size_t at = (size_t)(tok0 + r0 + row) * a.out_stride + h * HD + p * 64;      // this thread: half of its row's output
-        float o[64];
-        tmem_ld32_nowait(o_cols, o);
-        tmem_ld32_nowait(o_cols + 32, o + 32);
-        tmem_wait_ld<64>(o);
-        if (r0 + row < n) {
-            __nv_bfloat16* dst = (__nv_bfloat16*)a.out + at;
-            float* dst32 = (float*)a.out + at;
+        const float c0 = w0 / (l_run * w0 + (a.sink ? ex2(sk - M) : 0.f));
+        const size_t at = (size_t)(tok0 + r0 + row) * a.out_stride + h * HD + p0s * 64;      // this thread's part of its row's output
+#pragma unroll 1
+        for (int c = 0; c < O_COLS; c += 64) {
+            float o[64];
+            tmem_ld32_nowait(o_cols + c, o);
+            tmem_ld32_nowait(o_cols + c + 32, o + 32);
+            tmem_wait_ld<64>(o);
+            if (r0 + row >= n) continue;
+            __nv_bfloat16* dst = (__nv_bfloat16*)a.out + at + c;
+            float* dst32 = (float*)a.out + at + c;
 #pragma unroll
             for (int i = 0; i < 64; i += 8) {
                 float r[8];
@@ -435,28 +490,41 @@ extern "C" int tb_attn_prefill_tc_check(const AttnArgs* a, int dtype, int source
     return 0;
 }
 
-template <bool EXACT, int DK>
-static int launch_tc(const CUtensorMap& q_map, const CUtensorMap& kv_map, const CUtensorMap& tail_map, TcAttnArgs& p, int T, cudaStream_t stream) {
-    // once a device: the limit of shared memory, and the SMs
-    static std::atomic<int> configured[64];
-    int dev = 0, sms = 0;
+static int g_units = 0;
+// 1 or 2: units of 128 query rows a CTA whatever the size (0: by the rule below).
+extern "C" void tb_attn_tc_set_units(int units) { g_units = units; }
+
+template <bool EXACT, int DK, int UNITS>
+static int launch_units(const CUtensorMap& q_map, const CUtensorMap& kv_map, const CUtensorMap& tail_map, TcAttnArgs& p, int T, cudaStream_t stream) {
+    static std::atomic<bool> configured[64];              // a device each
+    int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 64) sms = configured[dev].load();
-    if (sms <= 0) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<EXACT, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem<DK>());
+    if (dev >= 64 || !configured[dev].load()) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<EXACT, DK, UNITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem<DK>());
         TB_REQUIRE(e == cudaSuccess, "attn_prefill_tc: cannot reserve %zu bytes of shared memory: %s", tc_smem<DK>(), cudaGetErrorString(e));
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-        if (dev < 64) configured[dev].store(sms);
+        if (dev < 64) configured[dev].store(true);
     }
-    // Two units a CTA where that leaves no SM idle that one unit a CTA would use: a unit alone waits for its own chain of S, P and P.V.
-    p.units = (long long)p.nh * ((T + BQ - 1) / BQ) <= sms ? 1 : 2;
-    p.pair_heads = p.units == 2 && (p.nh / p.nkv) % 2 == 0;
-    const int rows_cta = p.pair_heads ? BQ : p.units * BQ;
+    p.pair_heads = UNITS == 2 && (p.nh / p.nkv) % 2 == 0;
+    const int rows_cta = p.pair_heads ? BQ : UNITS * BQ;
     const int blocks = (T + rows_cta - 1) / rows_cta + p.B;      // upper bound on sum over sequences of ceil(n / rows_cta)
     TB_REQUIRE(blocks <= 65535, "attn_prefill_tc: too many query blocks (%d)", blocks);
-    tb_launch(attn_prefill_tc_kernel<EXACT, DK>, dim3(p.pair_heads ? p.nh / 2 : p.nh, blocks), THREADS, tc_smem<DK>(), stream, q_map, kv_map, tail_map, p);      // heads fastest: the heaviest blocks of all heads start first
+    tb_launch(attn_prefill_tc_kernel<EXACT, DK, UNITS>, dim3(p.pair_heads ? p.nh / 2 : p.nh, blocks), THREADS, tc_smem<DK>(), stream, q_map, kv_map, tail_map, p);      // heads fastest: the heaviest blocks of all heads start first
     TB_CHECK_LAUNCH("attn_prefill_tc");
     return 0;
+}
+template <bool EXACT, int DK>
+static int launch_tc(const CUtensorMap& q_map, const CUtensorMap& kv_map, const CUtensorMap& tail_map, TcAttnArgs& p, int T, cudaStream_t stream) {
+    static std::atomic<int> count[64];                     // SMs, a device each
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64) sms = count[dev].load();
+    if (sms <= 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+        if (dev < 64) count[dev].store(sms);
+    }
+    // Two units a CTA where that leaves no SM idle that one unit a CTA would use: a unit alone waits for its own chain of S, P and P.V.
+    const bool one = g_units ? g_units == 1 : (long long)p.nh * ((T + BQ - 1) / BQ) <= sms;
+    return one ? launch_units<EXACT, DK, 1>(q_map, kv_map, tail_map, p, T, stream) : launch_units<EXACT, DK, 2>(q_map, kv_map, tail_map, p, T, stream);
 }
 
 extern "C" int tb_attn_prefill_tc(const AttnArgs* args, int source, cudaStream_t stream) {

@@ -1073,6 +1073,11 @@ def attn_prefill_tc(args: AttnArgs, source: int, stream: int) -> None:
     _check(alib().tb_attn_prefill_tc(byref(args), int(source), stream))
 
 
+def set_attn_tc_units(units: int) -> None:
+    """Prompt attention: 1 or 2 units of 128 query rows a block whatever the size (0: by its rule)."""
+    alib().tb_attn_tc_set_units(int(units))
+
+
 def attn_tc_error() -> int:
     return int(alib().tb_attn_tc_error())
 
