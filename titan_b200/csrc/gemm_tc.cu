@@ -1078,123 +1078,6 @@ gemm_tc_runs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
 }
 
-// ---------------------------------------------------------------- prompts: equal tiles of rows
-// gemm_tc_pair_kernel with the operands' sides exchanged, as above, for one matrix: 256 rows of W against tiles of ``cols`` rows of X, a multiple of
-// 16 that the launcher chooses so that the tiles take the pairs of CTAs the least time (equal_tiles).  Tiles of 256 rows cost 905 rows of X
-// as much as 1,024, and a last round of tiles as much as a full one; the ADD epilogue cuts that one along K, the others cannot.
-template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
-gemm_tc_equal_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, TcArgs a, int cols) {
-    constexpr int STAGES = PAIR_STAGES;
-    constexpr uint32_t A_BYTES = PAIR_A_BYTES, B_BYTES = PAIR_B_BYTES;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* smem_a = base;
-    uint8_t* smem_b = base + STAGES * A_BYTES;
-    uint64_t* full = (uint64_t*)(base + STAGES * (A_BYTES + B_BYTES));
-    uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;          // [2]
-    uint64_t* acc_empty = acc_full + 2;           // [2]
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = tbtma::cluster_rank();
-    const int n_kb = (a.K + BK - 1) / BK, half = cols / 2, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, total = a.tiles_m * a.tiles_n;
-
-    pdl_launch_dependents();
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 8); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
-    tc_fence_before();
-    tbtma::cluster_sync();                         // both CTAs' barriers exist before either signals the other's
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    // tile t: rows t % tiles_m of X, so that the pairs at work share panels of weights
-
-    if (warp == 0) {
-        if (lane == 0) {
-            const uint32_t bytes = 2 * (A_BYTES + (uint32_t)half * BK * 2);
-            auto load_w = [&](int s, int t, int k) {
-                tbtma::tma_load_2d_pair(smem_a + s * A_BYTES, &map_w, tbtma::cluster_addr(full + s, 0), k * BK, t / a.tiles_m * 2 * BM + (int)rank * BM);
-            };
-            auto load_x = [&](int s, int t, int k) {
-                tbtma::tma_load_2d_pair(smem_b + s * B_BYTES, &map_x, tbtma::cluster_addr(full + s, 0), k * BK, t % a.tiles_m * cols + (int)rank * half);
-            };
-            // the first tile's first stages: weights before the wait, which no kernel writes
-            const int pre = pair < total ? min(STAGES, n_kb) : 0;
-            for (int k = 0; k < pre; ++k) {
-                if (rank == 0) mbar_expect_tx(full + k, bytes);
-                load_w(k, pair, k);
-            }
-            pdl_wait();
-            for (int k = 0; k < pre; ++k) load_x(k, pair, k);
-            int it = pre;
-            for (int t = pair; t < total; t += pairs)
-                for (int k = t == pair ? pre : 0; k < n_kb; ++k, ++it) {
-                    const int s = it % STAGES, round = it / STAGES;
-                    if (round > 0) mbar_wait(empty + s, (round - 1) & 1, 1);
-                    if (rank == 0) mbar_expect_tx(full + s, bytes);
-                    load_w(s, t, k);
-                    load_x(s, t, k);
-                }
-        }
-    } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            pdl_wait();
-            const uint32_t idesc = instr_desc(2 * BM, cols);
-            int it = 0, j = 0;
-            for (int t = pair; t < total; t += pairs, ++j) {
-                const int buf = j & 1;
-                if (j >= 2) mbar_wait(acc_empty + buf, ((j >> 1) - 1) & 1, 4);     // both CTAs' epilogues have drained this buffer
-                tc_fence_after();
-                const uint32_t acc = tmem + buf * PAIR_N;
-                for (int i = 0; i < n_kb; ++i, ++it) {
-                    const int s = it % STAGES, round = it / STAGES;
-                    mbar_wait(full + s, round & 1, 2);
-                    tc_fence_after();
-                    const uint64_t da = smem_desc(smem_u32(smem_a + s * A_BYTES));
-                    const uint64_t db = smem_desc(smem_u32(smem_b + s * B_BYTES));
-#pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        tc_mma_pair(acc, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                    tc_commit_pair(empty + s, 3);
-                }
-                tc_commit_pair(acc_full + buf, 3);
-            }
-        }
-    } else {
-        pdl_wait();
-        const int quarter = warp & 3;
-        int j = 0;
-        for (int t = pair; t < total; t += pairs, ++j) {
-            const int buf = j & 1, row0 = t % a.tiles_m * cols, rows = min(cols, a.rows_a - row0);
-            mbar_wait(acc_full + buf, (j >> 1) & 1, 3);
-            tc_fence_after();
-            const int n = t / a.tiles_m * 2 * BM + (int)rank * BM + quarter * 32 + lane;          // this lane's row of W: an output column, or half of one
-            const uint32_t taddr = tmem + buf * PAIR_N + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll 1
-            for (int c = 0; c < rows; c += 32) {
-                float v[32];
-                tmem_ld32(taddr + c, v);
-                lanes_out<EPI>(v, a, row0 + c, rows - c, n, lane);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tbtma::mbar_arrive_cluster(tbtma::cluster_addr(acc_empty + buf, 0));
-        }
-    }
-    pdl_wait();
-    tc_fence_before();
-    tbtma::cluster_sync();                         // nobody leaves while the other still reads its shared memory or signals it
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc_pair(tmem, 512);
-    }
-}
-
 // ---------------------------------------------------------------- host side
 template <int BN, int EPI, bool SWAP>
 int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, dim3 grid, cudaStream_t stream) {
@@ -1390,34 +1273,6 @@ int launch_pair(int epi, const CUtensorMap& ma, const CUtensorMap& mb, const TcA
     return 1;
 }
 
-// Rows a tile of the kernel of equal tiles for M rows and N columns on ``pairs`` pairs of CTAs: what makes rounds times rows of a tile (and 16 rows' time a
-// round for what a tile costs beside its products) least, at most 256; ``cost`` of that.
-int equal_tiles(int M, int N, int pairs, double* cost) {
-    const long long panels = (N + 2 * BM - 1) / (2 * BM);
-    const int fewest = (M + PAIR_N - 1) / PAIR_N;
-    int best = 0;
-    *cost = 1e30;
-    for (int t = fewest; t <= (M + 63) / 64 && t <= 4 * fewest + 4; ++t) {
-        const int each = ((M + t - 1) / t + 15) & ~15;
-        const double c = (double)((panels * ((M + each - 1) / each) + pairs - 1) / pairs) * ((each < 128 ? 128 : each) + 16);       // (an instruction of fewer than 128 columns waits for its operands)
-        if (c < *cost) { *cost = c; best = each; }
-    }
-    return best;
-}
-template <int EPI>
-int launch_equal_epi(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& a, int cols, int pairs, cudaStream_t stream) {
-    static std::atomic<bool> configured[64];              // a device each
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 64 || !configured[dev].load()) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_equal_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM);
-        TB_REQUIRE(e == cudaSuccess, "gemm_tc: cannot reserve %zu bytes of shared memory: %s", PAIR_SMEM, cudaGetErrorString(e));
-        if (dev < 64) configured[dev].store(true);
-    }
-    tb_launch(gemm_tc_equal_kernel<EPI>, dim3(2 * pairs, 1, 1), THREADS, PAIR_SMEM, stream, mw, mx, a, cols);
-    return 0;
-}
-
 template <int BN, bool SWAP>
 int launch_epi(int epi, const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, dim3 grid, cudaStream_t stream) {
     switch (epi) {
@@ -1437,7 +1292,7 @@ int launch_epi(int epi, const CUtensorMap& ma, const CUtensorMap& mb, const TcAr
 int g_plain_tile = 0;
 int g_swap_below = 128;
 extern "C" void tb_gemm_tc_set_swap_below(int m) { g_swap_below = m; }
-// Prompt products: 0 chooses the tile shape, 1 forces CTA pairs (256 x 256), 2 single CTAs with 128 x 256, 3 with 128 x 128, 4 equal tiles of rows.
+// Prompt products: 0 chooses the tile shape, 1 forces CTA pairs (256 x 256), 2 single CTAs with 128 x 256, 3 with 128 x 128.
 extern "C" void tb_gemm_tc_set_plain_tile(int which) { g_plain_tile = which; }
 
 int g_pair = 1;
@@ -1601,29 +1456,10 @@ extern "C" int tb_gemm_tc_gated(const void* X, const void* W, void* out, int M, 
         if (t_128 < t_pair && t_128 < t_256) { pairs_max = 0; single_bn = 128; }
         else if (t_256 < t_pair) pairs_max = 0;
     }
-    // Equal tiles of rows, sides exchanged, where they take the pairs less time than the shapes above do by their own rule.
-    const int pairs_all = (!swap && g_pair && M > 128 && N >= 256 && (epi == TB_EPI_SWIGLU || epi == TB_EPI_STORE)) ? pair_clusters_for(epi) : 0;
-    int equal = 0;
-    if (pairs_all > 0 && (g_plain_tile == 0 || g_plain_tile == 4)) {
-        double cost, now;
-        const int each = equal_tiles(M, N, pairs_all, &cost);
-        const long long m256 = (M + 255) / 256, m128 = (M + 127) / 128, n256 = (N + 255) / 256, n128 = (N + 127) / 128;
-        if (pairs_max > 0) now = (double)((m256 * n256 + pairs_max - 1) / pairs_max) * (256 + 16);
-        else if (single_bn == 256) now = (double)((m128 * n256 + sm_count - 1) / sm_count) * (256 + 16) * 1.1;
-        else now = (double)((m128 * n128 + sm_count - 1) / sm_count) * (256 + 16) * 0.85;
-        if (cost < 0.97 * now || g_plain_tile == 4) equal = each;
-    }
     if (!swap && g_plain_tile == 1 && M > 128 && N >= 256) pairs_max = pair_clusters_for(epi);
     if (!swap && g_plain_tile == 2) { pairs_max = 0; single_bn = N >= 256 ? 256 : 128; }
     if (!swap && g_plain_tile == 3) { pairs_max = 0; single_bn = 128; }
-    if (equal > 0) {
-        a.rows_a = M; a.rows_b = N;
-        a.tiles_m = (M + equal - 1) / equal; a.tiles_n = (N + 2 * BM - 1) / (2 * BM);
-        if (tb_make_map_bf16(&ma, W, N, K, K, BM) || tb_make_map_bf16(&mb, X, M, K, ldx, equal / 2)) return 1;
-        TB_REQUIRE((long long)a.tiles_m * a.tiles_n < (1LL << 30), "gemm_tc: too many tiles");
-        const int total = a.tiles_m * a.tiles_n, pairs = total < pairs_all ? total : pairs_all;
-        rc = epi == TB_EPI_SWIGLU ? launch_equal_epi<TB_EPI_SWIGLU>(ma, mb, a, equal, pairs, stream) : launch_equal_epi<TB_EPI_STORE>(ma, mb, a, equal, pairs, stream);
-    } else if (pairs_max > 0) {
+    if (pairs_max > 0) {
         a.rows_a = M; a.rows_b = N;
         a.tiles_m = (M + 2 * BM - 1) / (2 * BM); a.tiles_n = (N + PAIR_N - 1) / PAIR_N;
         if (tb_make_map_bf16(&ma, X, M, K, ldx, BM) || tb_make_map_bf16(&mb, W, N, K, K, 128)) return 1;

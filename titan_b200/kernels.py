@@ -1146,8 +1146,7 @@ def set_gemm_swap_below(m: int) -> None:
 
 def set_gemm_plain_tile(which: int) -> None:
     """Prompt products: 0 lets the launcher choose the tile shape (default), 1 forces CTA pairs with 256 x 256 tiles
-    (from 256 x 256 outputs on), 2 single CTAs with 128 x 256 tiles, 3 single CTAs with 128 x 128 tiles, 4 CTA pairs with equal
-    tiles of rows (the store and gate epilogues)."""
+    (from 256 x 256 outputs on), 2 single CTAs with 128 x 256 tiles, 3 single CTAs with 128 x 128 tiles."""
     tlib().tb_gemm_tc_set_plain_tile(int(which))
 
 
