@@ -65,9 +65,6 @@ struct AttnArgs {
     // The tensor-core kernels: softmax weights enter the product with the values as two bfloat16 halves (the rounded weight
     // and what rounding left over), so that they keep sixteen bits instead of eight.
     int exact_weights;
-    // Decode on tensor cores: weights that the kernels after this one read, in their order (null: none).  They are requested into L2
-    // while this kernel's own chain of dependent steps leaves the memory idle.
-    const void* next_w[2]; long long next_bytes[2];
 };
 
 // How decode attention cuts the keys of ONE sequence into splits: ``chunk`` keys each while ``n_splits`` of

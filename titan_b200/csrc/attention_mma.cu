@@ -63,20 +63,8 @@ struct DecArgs {
     int late_trigger;                              // the next kernel may start once this one's pages are read (else: at once)
     const float* sink;                             // [nh] or null: one more term exp(sink) of every head's softmax denominator
     int keep_first;                                // with a window: the sequence's first keep_first keys stay visible
-    const char* next_w[2]; long long next_bytes[2];     // weights of the kernels behind this one, to be requested into L2
     int by_length;                                 // the blocks take the sequences from the longest down
 };
-
-// This CTA's share of the next kernels' weights, by one thread, as bulk requests of up to 16 KB that bring nothing into the SM.
-__device__ __forceinline__ void request_next_weights(const DecArgs& a) {
-    const long long ctas = (long long)gridDim.x * gridDim.y * gridDim.z, cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const long long units = a.next_bytes[r] >> 12, first = units * cta / ctas, last = units * (cta + 1) / ctas;      // units of 4 KB
-        for (long long u = first; u < last; u += 4)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.next_w[r] + (u << 12)), "r"((uint32_t)min(4ll, last - u) << 12) : "memory");
-    }
-}
 
 // HD: head size (64 or 128).  WIDE: the group has more than 8 query heads (rows 8..15 of the tile are live).
 // CL: the splits of a (sequence, kv head) are the CTAs of one thread-block cluster (up to 16).  Every CTA merges a
@@ -231,7 +219,6 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kv_map, DecArgs a) {
                 pdl_wait();
                 if (a.kv_len[b] != len) atomicCAS(&g_attn_error, 0u, 7u);
             }
-            request_next_weights(a);                        // behind the pages, which this kernel waits for
         }
         if (a.late_trigger) pdl_launch_dependents();
         if (!CL) return;
@@ -809,11 +796,6 @@ static int sm_count() {
     return n;
 }
 
-constexpr int AHEAD_MB = 48;
-static int g_ahead_mb = -1;
-// MB of the next kernels' weights that are requested into L2 (0: none, -1: the default).
-extern "C" void tb_attn_decode_set_ahead(int mb) { g_ahead_mb = mb; }
-
 extern "C" void tb_attn_decode_set_late_trigger(int on) { g_late_trigger = on ? 1 : 0; }
 // The splits of decode attention merge inside a thread-block cluster (1, default, up to 16 splits where the device places such clusters) or through scratch memory and the merge kernel (0).
 extern "C" void tb_attn_decode_set_cluster(int on) { g_decode_cluster = on ? 1 : 0; }
@@ -875,12 +857,6 @@ extern "C" int tb_attn_decode_mma(const AttnArgs* args, cudaStream_t stream) {
         d.acc = (float*)const_cast<void*>(q.in); d.acc_stride = q.in_stride; d.q_w = q.q_w; d.k_w = q.k_w; d.qk_eps = q.eps; d.rope = q.rope;
         d.row_sumsq = q.row_sumsq; d.row_parts = q.row_parts; d.row_width = q.row_width; d.row_eps = q.row_eps;
         d.storage = (__nv_bfloat16*)a.cache.storage; d.v_half = (long long)a.cache.num_pages * a.nkv * PAGE * a.hd;
-    }
-    long long room = (long long)(g_ahead_mb >= 0 ? g_ahead_mb : AHEAD_MB) << 20;
-    for (int r = 0; r < 2; ++r) {
-        const bool ok = a.next_w[r] && a.next_bytes[r] > 0 && ((uintptr_t)a.next_w[r] & 15) == 0;
-        d.next_w[r] = (const char*)a.next_w[r]; d.next_bytes[r] = ok ? (a.next_bytes[r] < room ? a.next_bytes[r] : room) : 0;
-        room -= d.next_bytes[r];
     }
     dim3 grid(a.batch.B, a.nkv, a.n_splits);
     d.by_length = a.n_splits == 1 && a.batch.B <= DEC_THREADS && (long long)a.batch.B * a.nkv > 2 * sm_count();      // two blocks an SM

@@ -522,8 +522,11 @@ static int launch_tc(const CUtensorMap& q_map, const CUtensorMap& kv_map, const 
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
         if (dev < 64) count[dev].store(sms);
     }
-    // Two units a CTA where that leaves no SM idle that one unit a CTA would use: a unit alone waits for its own chain of S, P and P.V.
-    const bool one = g_units ? g_units == 1 : (long long)p.nh * ((T + BQ - 1) / BQ) <= sms;
+    // Two units a CTA keep both pipes busy, but a CTA's chain of tiles, which a small step waits for, is shorter with one.  One: up to a CTA an SM
+    // (us with one / two units: 8 heads of 2,048 tokens 27 / 40, 32 heads of 300 9.4 / 12.8), and up to two where one sequence's long chains
+    // are all there is (16 heads of 2,000 31 / 41, 32 heads of 1,000 22.5 / 23.9; 1,300 36 / 28; four sequences of 60 to 250 14.8 / 12.6).
+    const long long ctas = (long long)p.nh * ((T + BQ - 1) / BQ);
+    const bool one = g_units ? g_units == 1 : ctas <= (p.B == 1 ? 2 : 1) * sms;
     return one ? launch_units<EXACT, DK, 1>(q_map, kv_map, tail_map, p, T, stream) : launch_units<EXACT, DK, 2>(q_map, kv_map, tail_map, p, T, stream);
 }
 

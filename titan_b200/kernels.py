@@ -95,8 +95,7 @@ class AttnArgs(Structure):
                 ("softcap", c_float), ("rel_bias", c_void_p), ("rel_far", c_int), ("head_mix", c_void_p),
                 ("head_gate", c_void_p), ("head_gate_stride", c_int),
                 ("pair_lambda", c_void_p), ("pair_eps", c_float), ("pair_scale", c_float), ("pair_width", c_int),
-                ("out_f32", c_int), ("exact_weights", c_int),
-                ("next_w", c_void_p * 2), ("next_bytes", c_longlong * 2)]
+                ("out_f32", c_int), ("exact_weights", c_int)]
 
 
 class LatentArgs(Structure):
@@ -1035,10 +1034,6 @@ def set_attn_decode_late_trigger(on: bool) -> None:
     default), or at once: the next kernel's first weight requests then queue in front of the pages."""
     alib().tb_attn_decode_set_late_trigger(int(bool(on)))
 
-
-def set_attn_decode_ahead(mb: int) -> None:
-    """Decode attention: at most this many MB of the weights after it (``AttnArgs.next_w``) are requested into L2 (0: none; -1: the default)."""
-    alib().tb_attn_decode_set_ahead(int(mb))
 
 # Where the tensor-core prompt kernels take keys and values from: nowhere they can (0), the step's own rows (every
 # sequence starts at position 0), or the cache's pages (the step's keys are appended already; no ring).

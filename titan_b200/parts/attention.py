@@ -553,10 +553,6 @@ class AttentionMixer(Mixer):
                     aa.early_len, aa.early_mode = lay.kv_len.data_ptr(), 1
                 elif lay.committed_len is not None:
                     aa.early_len, aa.early_mode = lay.committed_len.data_ptr(), 2
-            # what the kernels behind the attention read, in their order
-            for r, w in enumerate((self.w_o, ctx.upcoming)):
-                if w is not None:
-                    aa.next_w[r], aa.next_bytes[r] = w.data_ptr(), w.numel() * w.element_size()
             if folds_head_norm:
                 aa.fused_qk = ctypes.pointer(qa)
                 if not (fast and K.attn_decode_mma_accepts(aa, q_buf.dtype)):      # the kernel cannot take it in: as a kernel of its own, then

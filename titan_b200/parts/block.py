@@ -55,9 +55,7 @@ class PreNormBlock(Part):
         return norm.deferred(x, ctx) if getattr(consumer, "starts_norm", False) and not ctx.layout.all_single else norm.forward(x, ctx)
 
     def forward(self, x: torch.Tensor, ctx, cache) -> None:
-        ctx.upcoming = getattr(self.feed_forward, "first_weights", None)
         self.mixer.forward(self._normed(self.mixer_norm, self.mixer, x, ctx), ctx, cache, x)
-        ctx.upcoming = None
         self.feed_forward.forward(self._normed(self.feed_forward_norm, self.feed_forward, x, ctx), ctx, x)
 
 

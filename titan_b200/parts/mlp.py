@@ -63,11 +63,6 @@ class GatedMLP(FeedForward):
         del gate, up
         self.w_down = get(p + n["down"])
 
-    @property
-    def first_weights(self) -> torch.Tensor:
-        """What the first product reads, whole, in every step."""
-        return self.w_gate_up
-
     def forward(self, h, ctx, out: torch.Tensor) -> None:
         act = ctx.room("act", (h.shape[0], self.spec.intermediate_size))
         if (isinstance(h, DeferredNorm) and self.gate == K.ACT_SILU and ctx.options.get("gemm", "fast") != "plain" and self.w_gate_up.dtype == torch.bfloat16
