@@ -600,60 +600,35 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attn_decode_kernel(AttnArgs a)
 // a head together and meet in shared memory.  They are as many as leave a stream a whole round of eight keys of the launch's ``chunk``
 // (more only add parts to merge: 32 keys a split, 64 sequences of 2,000, 8 heads of 8: 2,700 us with sixteen warps a head).
 // Bound by the latency of the loads at a few hundred keys a split: three
-// sequences of 500 tokens, 16 heads of 64 on 8, float32: 210 -> 12.3 us a layer.  Given a length that was final before the step began, the first
-// round of older keys is requested before the wait for the kernels before.
+// sequences of 500 tokens, 16 heads of 64 on 8, float32: 210 -> 12.3 us a layer.
 constexpr int VEC_WARPS = 16, VEC_KEYS = 8;
 
 template <typename T, int LPK>
 __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArgs a, int share) {
     constexpr int PER = 16 / (int)sizeof(T), STREAMS = 32 / LPK;
     pdl_launch_dependents();
-    const bool early = a.early_mode != 0;               // the lengths, the block tables and all rows but the newest are there before the wait
-    if (!early) pdl_wait();
+    pdl_wait();
     extern __shared__ float parts[];                   // [warps][hdv + 2]: what a warp made of its keys (share > 1)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, unit = lane % LPK;
     const int blocks_y = a.head_blocks > 0 ? a.head_blocks : a.nkv;
     const int b = blockIdx.x, kh = (int)blockIdx.y * a.nkv / blocks_y, split = blockIdx.z;
     const int hd = a.hd, hdv = value_width(a), group = a.nh / blocks_y;
-    const int slot = a.batch.slot_of_seq[b];
-    const int len = a.early_mode == 2 ? a.early_len[slot] + 1 : (early ? a.early_len[b] : a.batch.kv_len[b]);
+    const int len = a.batch.kv_len[b];
     const int keys = tb_split_keys(len, a.chunk, a.n_splits);
-    if ((long long)split * keys >= len) {           // the merge reads ceil(len / keys) splits only
-        pdl_wait();
-        return;
-    }
+    if ((long long)split * keys >= len) return;     // the merge reads ceil(len / keys) splits only
     const int pos = len - 1;
+    const int slot = a.batch.slot_of_seq[b];
     const int wlo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
     const int lo = max(wlo, split * keys), hi = min(len, (split + 1) * keys);
     // the kept first tokens that lie in this split and before the window
     const int klo = split * keys, khi = a.window > 0 ? min(min(a.keep_first, wlo), hi) : 0;
-    if (lo >= hi && a.keep_first <= 0) {               // a split before the window: the merge begins behind it
-        pdl_wait();
-        return;
-    }
+    if (lo >= hi && a.keep_first <= 0) return;         // a split before the window: the merge begins behind it
     const T* cache = (const T*)a.cache.storage;
     const size_t vhalf = a.v_alias ? 0 : kv_half_elems(a.cache);
     const int shift = page_shift(a.cache);
     const int streams = share * STREAMS, st = (warp % share) * STREAMS + lane / LPK;
     const int at = unit * PER, at_once = (int)(blockDim.x >> 5) / share;
     const bool key_part = at < hd, value_part = at < hdv;
-    // A round's keys and values: all of them, all but the newest key's (before the wait), or that one alone.
-    uint4 kr[VEC_KEYS], vr[VEC_KEYS];
-    enum Which { ALL, OLDER, NEWEST };
-    auto fetch = [&](int base, int last, Which which) {
-#pragma unroll
-        for (int u = 0; u < VEC_KEYS; ++u) {
-            const int key = min(base + u * streams + st, last - 1);
-            if (which != ALL && (key == pos) != (which == NEWEST)) continue;
-            const T* row = cache + row_offset(a.cache, slot, key, kh, shift) + at;
-            kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
-            if (key_part) kr[u] = *reinterpret_cast<const uint4*>(row);
-            if (value_part) vr[u] = *reinterpret_cast<const uint4*>(row + vhalf);
-        }
-    };
-    bool fetched = early && klo >= khi && lo < hi;     // the first round of the first heads: on its way while the kernels before still run
-    if (fetched) fetch(lo, hi, OLDER);
-    if (early) pdl_wait();
     for (int g0 = 0; g0 < group; g0 += at_once) {
         const int g = g0 + warp / share;
         const int h = (int)blockIdx.y * group + min(g, group - 1);
@@ -665,8 +640,14 @@ __global__ void __launch_bounds__(VEC_WARPS * 32) attn_decode_vec_kernel(AttnArg
         }
         auto attend = [&](int first, int last) {
             for (int base = first; base < last; base += VEC_KEYS * streams) {      // (the bounds are the warp's: its lanes stay together)
-                fetch(base, last, fetched ? NEWEST : ALL);
-                fetched = false;
+                uint4 kr[VEC_KEYS], vr[VEC_KEYS];
+#pragma unroll
+                for (int u = 0; u < VEC_KEYS; ++u) {
+                    const T* row = cache + row_offset(a.cache, slot, min(base + u * streams + st, last - 1), kh, shift) + at;
+                    kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
+                    if (key_part) kr[u] = *reinterpret_cast<const uint4*>(row);
+                    if (value_part) vr[u] = *reinterpret_cast<const uint4*>(row + vhalf);
+                }
                 float s[VEC_KEYS], top = m;
 #pragma unroll
                 for (int u = 0; u < VEC_KEYS; ++u) {

@@ -317,11 +317,6 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int u = 1; u < stages - 1; ++u) asm volatile("cp.async.commit_group;" ::: "memory");
     for (int u = 0; u < units; ++u) {
-        // what a thread's sum is added to, requested before the operands are waited for: nothing of this launch changes it
-        const int m = m0 + om, n = (blockIdx.x + u / passes * gridDim.x) * COLS + on;
-        const bool stores = tid < MR * COLS && u % passes == passes - 1 && m < M && n < N;
-        float old = 0.f;
-        if (EPI == TB_EPI_ADD && stores) old = load_l2<float>((float*)out_ + (size_t)z * so + (size_t)m * ldo + n);
         if (stages > 1 && u + stages - 1 < units) {
             stage_w(u + stages - 1);
             if (passes > 1) stage_x(u + stages - 1);
@@ -381,14 +376,15 @@ gemm_few_kernel(const T* X, const T* W, void* out_, int M, int N, int K, int ldx
             for (; r < here; ++r) total += mine[r * MR * COLS];
         }
         if (u % passes != passes - 1) continue;
+        const int m = m0 + om, n = (blockIdx.x + u / passes * gridDim.x) * COLS + on;
         // the gate of a pair: its second column is the neighbouring thread's
         const float right = __shfl_down_sync(MR * COLS >= 32 ? 0xffffffffu : (1u << (MR * COLS % 32)) - 1u, total, 1);
-        if (stores) {
+        if (m < M && n < N) {
             const size_t at = (size_t)z * so + (size_t)m * ldo + n;
             if (EPI == TB_EPI_SWIGLU) { if (n % 2 == 0) stf((T*)out_ + (size_t)z * so + (size_t)m * ldo + n / 2, tb_gated(act, limit, total, right)); }
             if (EPI == TB_EPI_STORE) stf((T*)out_ + at, tb_unary(act, total));
             if (EPI == TB_EPI_F32) ((float*)out_)[at] = total;
-            if (EPI == TB_EPI_ADD) ((float*)out_)[at] = old + total;
+            if (EPI == TB_EPI_ADD) ((float*)out_)[at] = load_l2<float>((float*)out_ + at) + total;
         }
         total = 0.f;
     }
