@@ -18,8 +18,6 @@
 // scalar FMA (engine/engine-cuda/kernels/paged_attention.cu:200-309).
 #include <float.h>
 
-#include <atomic>
-
 #include "attention_args.h"
 #include "common.cuh"
 #include "mma.cuh"
@@ -63,7 +61,6 @@ struct DecArgs {
     int late_trigger;                              // the next kernel may start once this one's pages are read (else: at once)
     const float* sink;                             // [nh] or null: one more term exp(sink) of every head's softmax denominator
     int keep_first;                                // with a window: the sequence's first keep_first keys stay visible
-    int by_length;                                 // the blocks take the sequences from the longest down
 };
 
 // HD: head size (64 or 128).  WIDE: the group has more than 8 query heads (rows 8..15 of the tile are live).
@@ -126,8 +123,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kv_map, DecArgs a) {
     float* recv = reinterpret_cast<float*>(q_sh + 16 * HD);          // CL: [split][per + 32]: every split's values for this CTA's share of the output, its maxima and sums
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int b = blockIdx.x, kh = blockIdx.y;
-    const int split = blockIdx.z;
+    const int b = blockIdx.x, kh = blockIdx.y, split = blockIdx.z;
     TimelineProbe probe;              // stamps: 1 wait for the kernels before passed, 2 queries ready, 3 pages done, 5 all parts here, 4 end
     probe.begin(100000 + gridDim.z, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
     // The kernel after this one may start (and request its first weight tiles) while this one runs.  Those requests
@@ -139,24 +135,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kv_map, DecArgs a) {
     // only older positions are requested before the wait, while those kernels still run.
     const bool early = a.early_mode != 0;
     if (!early) pdl_wait();
-    auto length_of = [&](int s) { return a.early_mode == 2 ? a.early_len[a.slot_of_seq[s]] + 1 : (early ? a.early_len[s] : a.kv_len[s]); };
-    if (a.by_length) {
-        // More blocks than the device holds at once: they start in the order of their numbers, so block i takes kv head i % nkv of the
-        // sequence with i / nkv longer ones before it, and the shortest fill the last places (64 sequences of 64 to 512 keys in
-        // batch order, a block a kv head: 22 us, of which the last longest ones alone a third).  A sequence's own arithmetic is the same.
-        __shared__ int lens[DEC_THREADS], chosen;
-        const int i = blockIdx.x + gridDim.x * blockIdx.y, t = threadIdx.x, mine = t < (int)gridDim.x ? length_of(t) : 0;
-        lens[t] = mine;
-        __syncthreads();
-        if (t < (int)gridDim.x) {
-            int before = 0;
-            for (int s = 0; s < (int)gridDim.x; ++s) before += lens[s] > mine || (lens[s] == mine && s < t);
-            if (before == i / a.nkv) chosen = t;
-        }
-        __syncthreads();
-        b = chosen; kh = i % a.nkv;
-    }
-    const int len = length_of(b);
+    const int len = a.early_mode == 2 ? a.early_len[a.slot_of_seq[b]] + 1 : (early ? a.early_len[b] : a.kv_len[b]);
     const int keys = tb_split_keys(len, a.chunk, a.n_splits);
     if (!CL && (long long)split * keys >= len) return;  // uniform over the CTA; the merge skips these splits (in a cluster the CTA stays, with no pages, for the barrier)
     const int group = a.nh / a.nkv;
@@ -786,15 +765,6 @@ int g_late_trigger = 1;
 // When the kernel after decode attention may start: once this one's pages have been read (1, default) or at once (0).
 // Measured after 2,048-token prompts: batch 1 2.85 -> 2.81 ms per step, batch 4 3.11 -> 3.06, batch 8 3.27 -> 3.24; no
 // difference at 7,000 tokens or at batch 64.
-static int sm_count() {
-    static std::atomic<int> count[64];                     // a device each
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && (n = count[dev].load()) > 0) return n;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
-    if (dev < 64) count[dev].store(n);
-    return n;
-}
 
 extern "C" void tb_attn_decode_set_late_trigger(int on) { g_late_trigger = on ? 1 : 0; }
 // The splits of decode attention merge inside a thread-block cluster (1, default, up to 16 splits where the device places such clusters) or through scratch memory and the merge kernel (0).
@@ -859,7 +829,6 @@ extern "C" int tb_attn_decode_mma(const AttnArgs* args, cudaStream_t stream) {
         d.storage = (__nv_bfloat16*)a.cache.storage; d.v_half = (long long)a.cache.num_pages * a.nkv * PAGE * a.hd;
     }
     dim3 grid(a.batch.B, a.nkv, a.n_splits);
-    d.by_length = a.n_splits == 1 && a.batch.B <= DEC_THREADS && (long long)a.batch.B * a.nkv > 2 * sm_count();      // two blocks an SM
     d.late_trigger = g_late_trigger;
     const bool wide = a.nh / a.nkv > 8;
     int rc;
