@@ -40,13 +40,9 @@
 
 #include "common.cuh"
 #include "gemm.h"
-#include "qk_args.h"
 #include "tcgen05.cuh"
 #include "timeline.cuh"
 #include "tma.cuh"
-
-extern "C" int tb_rmsnorm(const float* x, const float* w, void* y, int dtype, const int* rows, int n_rows, int H, float eps, cudaStream_t stream);
-extern "C" int tb_qk_norm_rope(const QkArgs* args, int in_dtype, int out_dtype, cudaStream_t stream);
 
 namespace {
 
@@ -1581,28 +1577,4 @@ extern "C" int tb_gemm_tc_expert_runs(const void* X, int ldx, const void* Wgu, v
     if (launch_runs<TB_EPI_F32>(act, ld_act, Wd, y, ldy, first, runs, rows, H, F, 0, 0.f, stream)) return 1;
     TB_CHECK_LAUNCH("gemm_tc_expert_runs");
     return 0;
-}
-
-// ---------------------------------------------------------------- whole sublayers of a prompt in one call
-// A prompt of a few hundred tokens keeps the device for 2 to 20 us a kernel, and a kernel's launch from Python costs the host 9 to 11 us (arguments,
-// a buffer, the call itself): the host was what such a step waited for.  These two start a sublayer's kernels, the same ones in the same order,
-// with one call.  3: a product that tb_gemm_tc does not take; nothing has been launched.
-
-// x[M][H] (float32, row stride H) += W_down . gate(W_gu . rmsnorm(x)); h [M][H] and act [M][F] are room for the rows between.
-extern "C" int tb_norm_gated_mlp(float* x, const float* norm_w, float eps, const void* W_gu, const void* W_down, void* h, void* act, int M, int H, int F,
-                                 int gate, float limit, int splits, cudaStream_t stream) {
-    if (tb_gemm_tc_check(M, 2 * F, H, H, F, TB_EPI_SWIGLU, h, W_gu, act) || tb_gemm_tc_check(M, H, F, F, H, TB_EPI_ADD, act, W_down, x)) return 3;
-    if (int rc = tb_rmsnorm(x, norm_w, h, TB_BF16, nullptr, M, H, eps, stream)) return rc;
-    if (int rc = tb_gemm_tc_gated(h, W_gu, act, M, 2 * F, H, H, F, TB_EPI_SWIGLU, splits, gate, limit, stream)) return rc == 3 ? 1 : rc;
-    const int rc = tb_gemm_tc_gated(act, W_down, x, M, H, F, F, H, TB_EPI_ADD, splits, 0, 0.f, stream);
-    return rc == 3 ? 1 : rc;
-}
-
-// qkv[M][N] = W . rmsnorm(x), then head norm, rotation and append as *qk says (its rows are qkv's).
-extern "C" int tb_norm_qkv(const float* x, const float* norm_w, float eps, const void* W, void* h, void* qkv, int M, int H, int N, const QkArgs* qk,
-                           int splits, cudaStream_t stream) {
-    if (tb_gemm_tc_check(M, N, H, H, N, TB_EPI_STORE, h, W, qkv)) return 3;
-    if (int rc = tb_rmsnorm(x, norm_w, h, TB_BF16, nullptr, M, H, eps, stream)) return rc;
-    if (int rc = tb_gemm_tc_gated(h, W, qkv, M, N, H, H, N, TB_EPI_STORE, splits, 0, 0.f, stream)) return rc == 3 ? 1 : rc;
-    return tb_qk_norm_rope(qk, TB_BF16, TB_BF16, stream);
 }

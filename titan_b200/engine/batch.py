@@ -132,13 +132,5 @@ class StepContext:
         self.sites_taken += 1
         return places[self.sites_taken - 1]
 
-    def room(self, name: str, shape) -> torch.Tensor:
-        """Rows in the compute dtype that live until the next part of THIS step asks for the same name and shape: for what a part makes and uses up
-        before it returns.  Every kernel that reads or writes them runs on the step's stream, one behind the other."""
-        kept = self.carried.get((name, tuple(shape)))
-        if kept is None:
-            kept = self.carried[(name, tuple(shape))] = self.empty(tuple(shape))
-        return kept
-
     def empty(self, shape, dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         return torch.empty(shape, dtype=dtype or self.dtype, device=self.device)

@@ -307,8 +307,6 @@ def tlib():
         l.tb_gemm_tc_normed_check.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
         l.tb_gemm_tc_expert_runs.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                              c_int, c_int, c_float, c_void_p]
-        l.tb_norm_gated_mlp.argtypes = [c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]
-        l.tb_norm_qkv.argtypes = [c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, POINTER(QkArgs), c_int, c_void_p]
         l.tb_gemm_tc_check.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]
         _tlib = l
     return _tlib
@@ -350,14 +348,6 @@ def _check(rc: int) -> None:
     if rc:
         raise KernelError(lib().tb_last_error().decode())
 
-
-def _count(*names: str) -> None:
-    """Counts launchers that a call started beside the one that ``_check`` counts."""
-    global launch_count
-    launch_count += len(names)
-    if _launch_log is not None:
-        for name in names:
-            _launch_log[name] = _launch_log.get(name, 0) + 1
 
 def dtype_code(dt: torch.dtype) -> int:
     if dt == torch.float32:
@@ -894,46 +884,6 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, strea
     _check(rc)
     return True
 
-
-def norm_gated_mlp(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w_gate_up: torch.Tensor, w_down: torch.Tensor, h: torch.Tensor, act: torch.Tensor,
-                   stream: int, gate: int = ACT_SILU, limit: float = 0.0, ordered: bool = False) -> bool:
-    """x (float32 [M, H], contiguous) += w_down . gate(w_gate_up . rmsnorm(x; norm_w, eps)): a prompt's norm and its two products, started by one
-    call; ``h`` [M, H] and ``act`` [M, F] (bfloat16, contiguous) are room for what lies between.  False, and nothing launched, where the tensor-core
-    kernel takes neither product."""
-    _need_cuda(x, norm_w, w_gate_up, w_down, h, act)
-    M, H = x.shape
-    F = act.shape[1]
-    bf16 = torch.bfloat16
-    if (x.dtype != torch.float32 or norm_w.dtype != torch.float32 or norm_w.numel() != H or h.dtype != bf16 or act.dtype != bf16 or w_gate_up.dtype != bf16
-            or w_down.dtype != bf16 or w_gate_up.shape != (2 * F, H) or w_down.shape != (H, F) or h.shape != (M, H) or act.shape[0] != M
-            or not all(t.is_contiguous() for t in (x, norm_w, w_gate_up, w_down, h, act))):
-        return False
-    rc = tlib().tb_norm_gated_mlp(x.data_ptr(), norm_w.data_ptr(), eps, w_gate_up.data_ptr(), w_down.data_ptr(), h.data_ptr(), act.data_ptr(), M, H, F,
-                                  gate, limit, -1 if ordered else 0, stream)
-    if rc == 3:
-        return False
-    _count("rmsnorm", "gemm_tc")
-    _check(rc)
-    return True
-
-def norm_qkv(x: torch.Tensor, norm_w: torch.Tensor, eps: float, w: torch.Tensor, h: torch.Tensor, qkv: torch.Tensor, qk: QkArgs, stream: int,
-             ordered: bool = False) -> bool:
-    """qkv [M, N] = w . rmsnorm(x; norm_w, eps), then what ``qk`` says of its heads (norm, rotation, append): a prompt's three kernels in front of its
-    attention, started by one call.  False, and nothing launched, where the tensor-core kernel does not take the product."""
-    _need_cuda(x, norm_w, w, h, qkv)
-    M, H = x.shape
-    N = w.shape[0]
-    bf16 = torch.bfloat16
-    if (x.dtype != torch.float32 or norm_w.dtype != torch.float32 or norm_w.numel() != H or h.dtype != bf16 or qkv.dtype != bf16 or w.dtype != bf16
-            or w.shape[1] != H or h.shape != (M, H) or qkv.shape != (M, N) or not all(t.is_contiguous() for t in (x, norm_w, w, h, qkv))):
-        return False
-    rc = tlib().tb_norm_qkv(x.data_ptr(), norm_w.data_ptr(), eps, w.data_ptr(), h.data_ptr(), qkv.data_ptr(), M, H, N, byref(qk),
-                            -1 if ordered else 0, stream)
-    if rc == 3:
-        return False
-    _count("rmsnorm", "gemm_tc")
-    _check(rc)
-    return True
 
 def gemm_tc_expert_runs(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, w_down: torch.Tensor, y: torch.Tensor, first: torch.Tensor,
                         stream: int, gate: int = ACT_SILU, limit: float = 0.0) -> None:

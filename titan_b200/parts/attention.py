@@ -121,7 +121,6 @@ def distance_rows(rows: int, far: float) -> List[int]:
 
 class AttentionMixer(Mixer):
     folds_norm = True           # a decode step's Q|K|V product takes the norm before it in
-    starts_norm = True          # a prompt's norm, Q|K|V product and head norms are started by one call
 
     def __init__(self, spec):
         s = spec
@@ -197,8 +196,6 @@ class AttentionMixer(Mixer):
                 raise ValueError(f"a convolution of {self.taps} taps (1 to 64)")
             if self.shaped or self.shared or self.unit_norm or self.value_mix is not None or self.value_norm is not None or s.qk_norm is not None:
                 raise ValueError("a convolution on q, k and v comes without head norms, normed or blended values, shaped scores or another layer's cache")
-        # one norm's rows, one product and one kernel in front of the attention: what starts_norm stands for
-        self.starts_norm = not (self.shaped or self.shared or self.taps is not None or self.value_mix is not None or self.value_norm is not None or self.gate_name)
         self.bias = self.b_o = self.whole_q_w = self.whole_k_w = self.rel_table = self.head_mix = None
 
     # -- declaration ------------------------------------------------------ #
@@ -457,7 +454,7 @@ class AttentionMixer(Mixer):
         # A decode step in bfloat16 sums Q | K | V in float32 (K slices of the product add into a zeroed
         # buffer), and the norm/rotary kernel rounds once, into the query buffer and the cache.
         wide_sum = decode and not self.shared and h.dtype == torch.bfloat16 and ctx.options.get("gemm", "fast") != "plain"
-        row_sums, started = None, False           # started: the norm, the product and the head norms by one call, below
+        row_sums = None
         if wide_sum:
             key = f"acc_qkv_{T}x{width}"            # zeroed once; the norm/rotary kernel leaves it zeroed again (Engine.reset_accumulators after a failed step)
             qkv = ctx.scratch.get(key)
@@ -476,9 +473,6 @@ class AttentionMixer(Mixer):
             if row_sums is None:
                 linear.matmul(rows_of(h), self.w_qkv, qkv, linear.EPI_ADD, ctx)
             q_buf, q_stride = ctx.empty((T, Q)), Q
-        elif isinstance(h, DeferredNorm) and self.starts_norm and not decode and linear.on_tensor_cores(ctx):
-            qkv, started = ctx.room("qkv", (T, width)), True
-            q_buf, q_stride = qkv, width
         else:
             qkv = ctx.empty((T, width))
             linear.matmul(rows_of(h), self.w_qkv, qkv, linear.EPI_STORE, ctx)
@@ -522,14 +516,10 @@ class AttentionMixer(Mixer):
             # the normed values are what a prompt's attention reads: written back over the step's own V columns
             qa.v_keep, qa.v_keep_stride = qkv.data_ptr() + (Q + KV) * qkv.element_size(), width
         folds_head_norm = wide_sum and ctx.options.get("fold_head_norm", True) and not self.extended
-        if started and not K.norm_qkv(h.x, h.weight, h.eps, self.w_qkv, ctx.room("normed", h.shape), qkv, qa, ctx.stream,
-                                      ordered=bool(ctx.options.get("reproducible", False))):
-            started = False
-            linear.matmul(rows_of(h), self.w_qkv, qkv, linear.EPI_STORE, ctx)
-        if not (started or folds_head_norm) and self.taps is None:
+        if not folds_head_norm and self.taps is None:
             K.qk_norm_rope(qa, qkv.dtype, q_buf.dtype, ctx.stream)
 
-        attn = ctx.empty((T, Q)) if decode else ctx.room("attn", (T, Q))
+        attn = ctx.empty((T, Q))
         aa = K.AttnArgs()
         aa.q, aa.q_stride = q_buf.data_ptr(), q_stride
         aa.out, aa.out_stride = attn.data_ptr(), Q
@@ -579,7 +569,7 @@ class AttentionMixer(Mixer):
                 source = K.KV_NOWHERE
             if hd not in (64, 128):                       # what the tensor-core kernels are built for: nothing else asks for (and compiles) them
                 source = K.KV_NOWHERE
-            if mode == "fast" and source and hd == 128 and K.attn_prefill_tc_accepts(aa, q_buf.dtype, source):
+            if mode == "fast" and source and K.attn_prefill_tc_accepts(aa, q_buf.dtype, source):
                 K.attn_prefill_tc(aa, source, ctx.stream)
             elif mode in ("fast", "mma") and source and K.attn_prefill_mma_accepts(aa, q_buf.dtype, source):
                 K.attn_prefill_mma(aa, source, ctx.stream)

@@ -47,12 +47,10 @@ class PreNormBlock(Part):
         deferred and the part can fold it into its first product."""
         # up to 16 rows: measured after 2,048-token prompts, folding gains 3 % of the step at 12 and 16 sequences and
         # loses 1 to 3 % at 20 to 32 (the kernels take up to 32 rows: twice the float32 rows per weight tile through L2)
-        if not (hasattr(norm, "deferred") and getattr(norm, "groups", 1) == 1):
-            return norm.forward(x, ctx)
-        if getattr(consumer, "folds_norm", False) and ctx.options.get("fold_norms", True) and x.shape[0] <= int(ctx.options.get("fold_norms_rows", 16)):
+        if (getattr(consumer, "folds_norm", False) and hasattr(norm, "deferred") and getattr(norm, "groups", 1) == 1 and ctx.options.get("fold_norms", True)
+                and x.shape[0] <= int(ctx.options.get("fold_norms_rows", 16))):
             return norm.deferred(x, ctx)
-        # a prompt's part that starts the norm's kernel and its own with one call
-        return norm.deferred(x, ctx) if getattr(consumer, "starts_norm", False) and not ctx.layout.all_single else norm.forward(x, ctx)
+        return norm.forward(x, ctx)
 
     def forward(self, x: torch.Tensor, ctx, cache) -> None:
         self.mixer.forward(self._normed(self.mixer_norm, self.mixer, x, ctx), ctx, cache, x)

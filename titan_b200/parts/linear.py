@@ -20,10 +20,6 @@ EPI_STORE, EPI_F32, EPI_ADD, EPI_SWIGLU = K.EPI_STORE, K.EPI_F32, K.EPI_ADD, K.E
 ROWS_MAX_M, ROWS_MAX_ELEMENTS = 8, 1 << 19
 
 
-def on_tensor_cores(ctx) -> bool:
-    """Whether a prompt's bfloat16 products go to the tensor-core kernel first (rows beyond those of the small products' rule)."""
-    return ctx.dtype == torch.bfloat16 and ctx.layout.T > ROWS_MAX_M and ctx.options.get("gemm", "fast") != "plain"
-
 def matmul(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epi: int, ctx, gate: int = K.ACT_SILU, limit: float = 0.0,
            unary: int = K.UNARY_NONE) -> None:
     """``gate``, ``limit``: what the SWIGLU epilogue makes of a (gate, up) pair (``kernels.ACT_*``); ``unary``: what the STORE

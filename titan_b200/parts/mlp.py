@@ -26,7 +26,6 @@ from .norm import DeferredNorm, rows_of
 
 class GatedMLP(FeedForward):
     folds_norm = True           # a decode step's gate-and-up product takes the norm before it in
-    starts_norm = True          # a prompt's norm and products are started by one call
 
     def __init__(self, spec):
         if spec.activation not in ("silu", "gelu_tanh"):
@@ -64,14 +63,10 @@ class GatedMLP(FeedForward):
         self.w_down = get(p + n["down"])
 
     def forward(self, h, ctx, out: torch.Tensor) -> None:
-        act = ctx.room("act", (h.shape[0], self.spec.intermediate_size))
+        act = ctx.empty((h.shape[0], self.spec.intermediate_size))
         if (isinstance(h, DeferredNorm) and self.gate == K.ACT_SILU and ctx.options.get("gemm", "fast") != "plain" and self.w_gate_up.dtype == torch.bfloat16
                 and K.gemm_tc_normed_accepts(h.x, h.weight, self.w_gate_up, act, linear.EPI_SWIGLU, None)):
             K.gemm_tc_normed(h.x, h.weight, h.eps, self.w_gate_up, act, linear.EPI_SWIGLU, ctx.stream)
-        elif (isinstance(h, DeferredNorm) and not ctx.layout.all_single and out.data_ptr() == h.x.data_ptr() and linear.on_tensor_cores(ctx)
-                and K.norm_gated_mlp(h.x, h.weight, h.eps, self.w_gate_up, self.w_down, ctx.room("normed", h.shape), act, ctx.stream, self.gate,
-                                     ordered=bool(ctx.options.get("reproducible", False)))):
-            return
         else:
             linear.matmul(rows_of(h), self.w_gate_up, act, linear.EPI_SWIGLU, ctx, gate=self.gate)
         linear.matmul(act, self.w_down, out, linear.EPI_ADD, ctx)
