@@ -12,8 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("K_,N_out,same", [(128, 16, 1), (128, 32, 8), (384, 48, 9), (2048, 16, 17), (1024, 64, 24), (96, 32, 3), (128, 12, 5)])
 def test_experts_of_a_few_pairs(mode, K_, N_out, same):
-    """``same`` pairs choose one expert, the others each their own, one an expert without matrices.  The last two sizes are not whole
-    fragments (K = 96; 12 or 24 rows) and take the kernel of a warp an output."""
+    """``same`` pairs choose one expert, the others each their own, one an expert without matrices."""
     from titan_b200 import kernels as K
     E, top = 6, 3
     g = torch.Generator().manual_seed(K_ + same)

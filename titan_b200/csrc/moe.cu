@@ -10,16 +10,14 @@
 //   tb_moe_grouped   out = epilogue(X . W_e^T) on the CUDA cores for every tile of the plan, any size, either dtype:
 //                    rows gathered from the tokens (gate-and-up, SwiGLU epilogue) or scattered back to pair order
 //                    (down, float32).  The plain path and the true 32-bit path.
-//   tb_moe_rows      the same two products for a handful of pairs (decode steps), without a plan: in bfloat16 an expert's pairs together on
-//                    mma.sync, its weights read once; else (float32, odd sizes) a warp per output column (or gate/up pair) of one
-//                    pair, lanes along K, weights read once per pair through L2.
+//   tb_moe_rows      the same two products for a handful of pairs (decode steps): a warp per output column (or
+//                    gate/up pair) of one pair, lanes along K, weights read once per pair through L2; no plan.
 //   tb_moe_combine   out[t] += sum_k weight[t][k] * y[t * top + k] (+ gate[t] * shared[t]), float32, in pair order.
 #include <type_traits>
 #include <float.h>
 
 #include "common.cuh"
 #include "gemm.h"
-#include "mma.cuh"
 
 #define MOE_BM 64
 #define MOE_BN 64
@@ -410,75 +408,6 @@ moe_rows_kernel(const T* __restrict__ X, int ldx, const T* __restrict__ W, void*
     }
 }
 
-// ------------------------------------------------------------------ a few pairs in bfloat16: an expert's pairs together
-// Bound by the chosen experts' matrices, read from DRAM once an expert; a warp an output read them once a PAIR through L2 (268 MB where 176 are
-// distinct) and kept two rows a warp in flight.  Here the block of an expert's FIRST pair (found in ids; the blocks of its other pairs leave)
-// multiplies 32 rows with up to eight of the expert's pairs at once: mma.sync m16n8k16, rows of W on the 16-side and pairs on
-// the 8-side.  A lane's 16 bytes of a row are k = 8 t .. 8 t + 7 of 32 (t = lane % 4): both operands take K in that order, so
-// fragments come straight from global memory, 64 contiguous bytes a row.  Warps: two tiles of 16 rows times four quarters of K, added
-// up in that order, which depends on nothing but K: a pair is the same bits alone and beside others.
-constexpr int MMA_MAX_PAIRS = 1024;
-template <int MODE>
-__global__ void __launch_bounds__(256, 3)
-moe_rows_mma_kernel(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* __restrict__ W, void* out, int ldo,        // (X and ids: no loads of constants, which could move above the wait)
-                    const int* ids, int P, int N_rows, int K, int top, int n_real, int act, float limit) {
-    __shared__ int list[MMA_MAX_PAIRS];
-    __shared__ int n_list;
-    __shared__ float part[2][4][8][17];               // [row tile][quarter][pair][row]
-    pdl_launch_dependents();
-    pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = warp >> 2, quarter = warp & 3, g = lane >> 2, t = lane & 3;
-    const int p = blockIdx.x, e = ids[p];
-    if (e >= n_real) return;                          // an expert without matrices: the combine kernel adds the input itself
-    bool earlier = false;
-    for (int q = threadIdx.x; q < p; q += 256) earlier = earlier || ids[q] == e;
-    if (__syncthreads_or(earlier)) return;
-    if (warp == 0) {
-        int n = 0;
-        for (int q0 = p; q0 < P; q0 += 32) {
-            const bool same = q0 + lane < P && ids[q0 + lane] == e;
-            const unsigned m = __ballot_sync(0xffffffffu, same);
-            if (same) list[n + __popc(m & ((1u << lane) - 1u))] = q0 + lane;
-            n += __popc(m);
-        }
-        if (lane == 0) n_list = n;
-    }
-    __syncthreads();
-    const int span = K / 4, r0 = blockIdx.y * 32;
-    const __nv_bfloat16* w_lo = W + ((size_t)e * N_rows + r0 + tile * 16 + g) * K + quarter * span + t * 8;
-    const __nv_bfloat16* w_hi = w_lo + (size_t)8 * K;
-    for (int g0 = 0; g0 < n_list; g0 += 8) {
-        const bool live = g0 + g < n_list;
-        const int q = live ? list[g0 + g] : 0;
-        const __nv_bfloat16* x = X + (size_t)(MODE == 0 ? q / top : q) * ldx + quarter * span + t * 8;
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int k = 0; k < span; k += 32) {
-            const uint4 a = __ldcs(reinterpret_cast<const uint4*>(w_lo + k)), b = __ldcs(reinterpret_cast<const uint4*>(w_hi + k));
-            const uint4 v = live ? *reinterpret_cast<const uint4*>(x + k) : make_uint4(0, 0, 0, 0);
-            tbmma::mma_bf16(c, a.x, b.x, a.y, b.y, v.x, v.y);
-            tbmma::mma_bf16(c, a.z, b.z, a.w, b.w, v.z, v.w);
-        }
-        part[tile][quarter][2 * t][g] = c[0]; part[tile][quarter][2 * t + 1][g] = c[1];
-        part[tile][quarter][2 * t][g + 8] = c[2]; part[tile][quarter][2 * t + 1][g + 8] = c[3];
-        __syncthreads();
-        const int pair = threadIdx.x >> 5, row = threadIdx.x & 31;          // a warp a pair, a lane a row
-        if (g0 + pair < n_list) {
-            float s = 0.f;
-#pragma unroll
-            for (int z = 0; z < 4; ++z) s += part[row >> 4][z][pair][row & 15];
-            const size_t to = (size_t)list[g0 + pair] * ldo;
-            if (MODE == 0) {
-                const float u = __shfl_down_sync(0xffffffffu, s, 1);
-                if ((row & 1) == 0) ((__nv_bfloat16*)out)[to + (r0 + row) / 2] = __float2bfloat16_rn(tb_gated(act, limit, s, u));
-            } else {
-                ((float*)out)[to + r0 + row] = s;
-            }
-        }
-        __syncthreads();
-    }
-}
-
 // ------------------------------------------------------------------ combine
 // ``ids`` with ``n_real`` and ``x``: a pair whose expert is n_real or beyond has no matrices and no row in y; its output
 // is the token's own input row x[t].
@@ -619,14 +548,6 @@ extern "C" int tb_moe_rows(const void* X, int ldx, const void* W, void* out, int
                            int P, int N_out, int K, int top, int n_real, int act, float limit, cudaStream_t stream) {
     TB_REQUIRE(P > 0 && N_out > 0 && K > 0 && top > 0 && (N_out + 7) / 8 <= 65535, "moe_rows: sizes (P=%d N=%d K=%d)", P, N_out, K);
     TB_REQUIRE(act >= 0 && act < TB_ACT_KINDS && n_real > 0, "moe_rows: unknown gate %d or no expert", act);
-    const int n_rows = mode == 0 ? 2 * N_out : N_out;
-    if (dtype == TB_BF16 && P <= MMA_MAX_PAIRS && K % 128 == 0 && n_rows % 32 == 0 && ldx % 8 == 0 && (((uintptr_t)X | (uintptr_t)W) & 15) == 0) {
-        // whole fragments of 16 bytes: every size that the loads below would take as 16-byte units and that cuts evenly
-        tb_launch(mode == 0 ? moe_rows_mma_kernel<0> : moe_rows_mma_kernel<1>, dim3(P, n_rows / 32), 256, 0, stream, (const __nv_bfloat16*)X, ldx,
-                  (const __nv_bfloat16*)W, out, ldo, ids, P, n_rows, K, top, n_real, act, limit);
-        TB_CHECK_LAUNCH("moe_rows");
-        return 0;
-    }
     dim3 grid(P, (N_out + 7) / 8);
 #define MOE_R(TT, MM) tb_launch(moe_rows_kernel<TT, MM>, grid, 256, 0, stream, (const TT*)X, ldx, (const TT*)W, out, ldo, ids, N_out, K, top, n_real, act, limit)
     if (dtype == TB_F32) { if (mode == 0) MOE_R(float, 0); else MOE_R(float, 1); }
